@@ -31,6 +31,20 @@ struct BvhTri { float4 p1, e1, e2; };
 // empty leaf).
 struct BvhNode4 { float4 lox, hix, loy, hiy, loz, hiz; int4 ref; int4 pad; };
 
+// The 4-wide node with quantised boxes (64 bytes): the four children's planes as one byte each
+// on the node's own grid, rounded outward. Byte q of an axis is the plane p + s (1 + q 2^-15): p
+// lies one s below the grid's origin and s is 2^15 cells, so that the byte placed in a float's
+// mantissa (1 + q 2^-15) decodes with a single FMA. Same children and refs as the full-precision
+// node, at the same index; unused slots have an inverted box (255, 0) and ref ~0.
+// Its boxes contain the full-precision ones, so the traversals find the same hits; only the
+// visiting order differs, which decides a hit's identity where two triangles lie at exactly the
+// same distance. Such ties are detected and traced again over the full-precision nodes.
+struct __align__(64) BvhNode4Q {
+    float p[3], s[3];
+    uint32_t lox, hix, loy, hiy, loz, hiz;
+    int ref[4];
+};
+
 struct DeviceBvh {
     BvhNode* nodes = nullptr;     // num_nodes records, root at 0
     BvhTri* tris = nullptr;       // num_tris records in leaf order
@@ -39,9 +53,20 @@ struct DeviceBvh {
     int depth = 0;                // longest root-to-leaf path (interior levels + 1)
     float lo[3] = {0, 0, 0}, hi[3] = {0, 0, 0};   // scene bounds
     BvhNode4* nodes4 = nullptr;   // the 4-wide form, root at 0 (same triangles)
+    BvhNode4Q* nodes4q = nullptr; // the same with quantised boxes
     int num_nodes4 = 0;
     int depth4 = 0;               // 4-wide levels on the longest path
 };
+
+// From this many 4-wide nodes on, closest-hit and any-hit rays traverse the quantised nodes; below
+// it the full-precision ones, which then sit in the L1, where their requests are cheap and the
+// byte decoding is not. Measured on the 512 x 512, 64 sample sphere frame with 644 / 5,444 /
+// 20,804 / 82,244 triangles (about a third as many nodes), closest hit full vs quantised: 2.34
+// vs 2.60, 3.35 vs 3.57, 3.89 vs 4.05, 4.55 vs 4.56 ms; on the 3.4 M triangle terrain 106.8 vs
+// 95.9. Any hit: 1.67 vs 1.62, 2.23 vs 2.10, 2.57 vs 2.38, 3.04 vs 2.75 ms; terrain 54.8 vs 44.2;
+// 344 triangles 1.38 vs 1.37; a batch of 36-triangle boxes 5.65 vs 5.81 ms.
+constexpr int kQuantMinNodes4 = 1 << 15;
+constexpr int kQuantMinNodes4Any = 1 << 7;
 
 struct BvhBuildOptions {
     int max_leaf = 4;             // triangles per leaf at most (<= 31)

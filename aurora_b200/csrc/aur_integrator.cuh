@@ -22,6 +22,7 @@ struct DevScene {
     const BvhNode* nodes;
     const BvhTri* tris;
     const BvhNode4* nodes4;   // the 4-wide form of the same tree, or null
+    const BvhNode4Q* nodes4q; // its quantised form (with nodes4)
     ShadeScene sh;
     Camera cam;
 };
@@ -52,18 +53,24 @@ __device__ __forceinline__ int pick_visible_light(const ShadeScene& sh, float3 P
     return -1;
 }
 
-// Traversal of the scene's binary (kWidth 2) or 4-wide (kWidth 4) tree.
+// Traversal of the scene's binary (kWidth 2), 4-wide (kWidth 4) or quantised 4-wide (kWidth 8) tree.
 template <int kWidth>
 __device__ __forceinline__ bool trace_closest(const DevScene& sc, float3 o, float3 d, float mint, float maxt, Hit* h,
                                               TraceWork& w) {
-    if constexpr (kWidth == 4) return bvh_trace4<false>(sc.nodes4, sc.tris, o, d, mint, maxt, h, w);
+    if constexpr (kWidth == 8) {
+        bool tie = false;
+        const bool hit = bvh_trace4<false>(sc.nodes4q, sc.tris, o, d, mint, maxt, h, w, &tie);
+        return tie ? bvh_trace4<false>(sc.nodes4, sc.tris, o, d, mint, maxt, h, w) : hit;
+    }
+    else if constexpr (kWidth == 4) return bvh_trace4<false>(sc.nodes4, sc.tris, o, d, mint, maxt, h, w);
     else return bvh_trace<false>(sc.nodes, sc.tris, o, d, mint, maxt, h, w);
 }
 template <int kWidth>
 __device__ __forceinline__ bool trace_occluded(const DevScene& sc, float3 o, float3 d, float mint, float maxt,
                                                TraceWork& w) {
     Hit h;
-    if constexpr (kWidth == 4) return bvh_trace4<true>(sc.nodes4, sc.tris, o, d, mint, maxt, &h, w);
+    if constexpr (kWidth == 8) return bvh_trace4<true>(sc.nodes4q, sc.tris, o, d, mint, maxt, &h, w);
+    else if constexpr (kWidth == 4) return bvh_trace4<true>(sc.nodes4, sc.tris, o, d, mint, maxt, &h, w);
     else return bvh_trace<true>(sc.nodes, sc.tris, o, d, mint, maxt, &h, w);
 }
 

@@ -16,10 +16,11 @@ cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_
 cudaError_t launch_kelemen_table(int refl_index, float* out, cudaStream_t s);
 
 // render_plain.cu — one thread per pixel, spp paths per thread.
-// counters[0..3] = camera rays, closest rays, shadow rays, paths; with count_work
+// counters[0..3] = camera rays, closest rays, shadow rays, paths; with count_width (the width of the
+// tree walked while counting: 2 binary, 4 four-wide, 8 quantised four-wide; 0 not counting)
 // also [4..5] interior-node visits / triangle tests of closest-hit rays and
 // [6..7] those of shadow rays (accumulated).
 cudaError_t launch_render_plain(const DevScene& sc, const PathParams& p, float4* film, double* film64,
-                                unsigned long long* counters, bool count_work, cudaStream_t s);
+                                unsigned long long* counters, int count_width, cudaStream_t s);
 
 }  // namespace aur

@@ -150,12 +150,98 @@ __device__ __forceinline__ bool bvh_trace(const BvhNode* __restrict__ nodes, con
     return best >= 0;
 }
 
-// The same traversal over the 4-wide tree (one 128-byte record per node visit; hit
-// children nearest first).
-constexpr int kTraversalStack4Local = 96;
+// Entry distances of the four children of a full-precision 4-wide node (+inf where missed) and
+// their references.
 template <bool kAnyHit>
-__device__ __forceinline__ bool bvh_trace4(const BvhNode4* __restrict__ nodes, const BvhTri* __restrict__ tris,
-                                           float3 o, float3 d, float mint, float maxt, Hit* hit, TraceWork& work) {
+__device__ __forceinline__ void boxes4(const BvhNode4* __restrict__ q, float3 id, float3 ood, float tmin, float tmax,
+                                       float (&t)[4], int (&r)[4]) {
+    const Planes4 pl = load_planes4<kAnyHit>(q, id);
+    const float4 rf = ld_node(reinterpret_cast<const float4*>(&q->ref));
+    const float kMiss = __int_as_float(0x7f800000);
+    float tc;
+    t[0] = slab_nf(pl.nx.x, pl.fx.x, pl.ny.x, pl.fy.x, pl.nz.x, pl.fz.x, id, ood, tmin, tmax, &tc) ? tc : kMiss;
+    t[1] = slab_nf(pl.nx.y, pl.fx.y, pl.ny.y, pl.fy.y, pl.nz.y, pl.fz.y, id, ood, tmin, tmax, &tc) ? tc : kMiss;
+    t[2] = slab_nf(pl.nx.z, pl.fx.z, pl.ny.z, pl.fy.z, pl.nz.z, pl.fz.z, id, ood, tmin, tmax, &tc) ? tc : kMiss;
+    t[3] = slab_nf(pl.nx.w, pl.fx.w, pl.ny.w, pl.fy.w, pl.nz.w, pl.fz.w, id, ood, tmin, tmax, &tc) ? tc : kMiss;
+    r[0] = __float_as_int(rf.x); r[1] = __float_as_int(rf.y); r[2] = __float_as_int(rf.z); r[3] = __float_as_int(rf.w);
+}
+
+__device__ __forceinline__ void ld_words8(const uint32_t* a, uint32_t (&v)[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+        : "l"(a));
+}
+// byte k of w as 1 + byte * 2^-15: one byte permutation, no integer conversion
+__device__ __forceinline__ float plane_f(uint32_t w, int k) {
+    return __uint_as_float(__byte_perm(w, 0x3f800000u, 0x7604u | ((uint32_t)k << 4)));
+}
+// a * m + c for two planes in one packed FMA (each half rounded as fmaf)
+__device__ __forceinline__ float2 fma_pair(float2 a, float m, float c) {
+    float2 r;
+    asm("{.reg .b64 x, y, z, w;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %4};\n mov.b64 z, {%5, %5};\n"
+        " fma.rn.f32x2 w, x, y, z;\n mov.b64 {%0, %1}, w;}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(m), "f"(c));
+    return r;
+}
+
+// The same for a quantised node. The traversals are bound by the L1's request rate and by the
+// latency of dependent fetches, not by instruction issue alone (an extra prefetch per leaf made
+// the any-hit kernel 15% slower; 68% of issue slots are busy): two 256-bit loads a visit replace
+// seven requests (four in the any-hit form). A plane at byte q lies at p + s (1 + q 2^-15), so
+// its distance is one FMA of the byte permuted into a float's mantissa; packed FMAs take two
+// children at a time. 1080p terrain frame, closest hit / any hit: full precision 106.8 / 54.8 ms,
+// quantised 102.0 / 49.1, with packed FMAs 98.0 / 45.5, with the rounds below free of a lane's
+// live flags and 12 idle lanes to a refill 95.9 / 44.2.
+template <bool kAnyHit>
+__device__ __forceinline__ void boxes4(const BvhNode4Q* __restrict__ node, float3 id, float3 ood, float tmin, float tmax,
+                                       float (&t)[4], int (&r)[4]) {
+    uint32_t a[8], b[8];
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(node);
+    ld_words8(q, a);
+    ld_words8(q + 8, b);
+    const float kMiss = __int_as_float(0x7f800000);
+    const float3 S = mk(__uint_as_float(a[3]) * id.x, __uint_as_float(a[4]) * id.y, __uint_as_float(a[5]) * id.z);
+    const float3 B = mk(fmaf(__uint_as_float(a[0]), id.x, -ood.x), fmaf(__uint_as_float(a[1]), id.y, -ood.y),
+                        fmaf(__uint_as_float(a[2]), id.z, -ood.z));
+    const bool sx = id.x < 0.f, sy = id.y < 0.f, sz = id.z < 0.f;
+    const uint32_t nx = sx ? a[7] : a[6], fx = sx ? a[6] : a[7];
+    const uint32_t ny = sy ? b[1] : b[0], fy = sy ? b[0] : b[1];
+    const uint32_t nz = sz ? b[3] : b[2], fz = sz ? b[2] : b[3];
+#pragma unroll
+    for (int k = 0; k < 4; k += 2) {
+        auto two = [&](uint32_t w, float m, float c) {
+            return fma_pair(make_float2(plane_f(w, k), plane_f(w, k + 1)), m, c);
+        };
+        const float2 ax = two(nx, S.x, B.x), ay = two(ny, S.y, B.y), az = two(nz, S.z, B.z);
+        const float2 bx = two(fx, S.x, B.x), by = two(fy, S.y, B.y), bz = two(fz, S.z, B.z);
+        const float n0 = fmaxf(fmaxf(ax.x, ay.x), fmaxf(az.x, tmin)), f0 = fminf(fminf(bx.x, by.x), fminf(bz.x, tmax));
+        const float n1 = fmaxf(fmaxf(ax.y, ay.y), fmaxf(az.y, tmin)), f1 = fminf(fminf(bx.y, by.y), fminf(bz.y, tmax));
+        t[k] = n0 <= f0 ? n0 : kMiss;
+        t[k + 1] = n1 <= f1 ? n1 : kMiss;
+    }
+    for (int k = 0; k < 4; ++k) r[k] = (int)b[4 + k];
+}
+
+// Puts the entered children in ascending order of entry distance, misses last: a five-exchange
+// network; unless kSorted only the first place is right (any hit, where the order of the rest
+// matters less than its cost: 45.1 vs 45.5 ms per 1080p terrain frame).
+template <bool kSorted>
+__device__ __forceinline__ void order4(float (&t)[4], int (&r)[4]) {
+    auto cx = [&](int i, int j) {
+        if (t[j] < t[i]) { const float tt = t[i]; t[i] = t[j]; t[j] = tt; const int rr = r[i]; r[i] = r[j]; r[j] = rr; }
+    };
+    cx(0, 1); cx(2, 3); cx(0, 2);
+    if (kSorted) { cx(1, 3); cx(1, 2); }
+}
+
+// The same traversal over a 4-wide tree, children nearest first. *tie (may be null): a second
+// triangle was accepted at exactly the best distance, so that the hit's identity depends on the
+// visiting order.
+constexpr int kTraversalStack4Local = 96;
+template <bool kAnyHit, class Node4>
+__device__ __forceinline__ bool bvh_trace4(const Node4* __restrict__ nodes, const BvhTri* __restrict__ tris,
+                                           float3 o, float3 d, float mint, float maxt, Hit* hit, TraceWork& work,
+                                           bool* tie = nullptr) {
     const float3 id = mk(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
     const float3 ood = mk(o.x * id.x, o.y * id.y, o.z * id.z);
     const float box_tmin = mint > 0.f ? mint * 0.99999905f : mint * 1.00000095f;
@@ -170,20 +256,10 @@ __device__ __forceinline__ bool bvh_trace4(const BvhNode4* __restrict__ nodes, c
     while (true) {
         if (node >= 0) {
             ++work.nodes;
-            const BvhNode4* q = nodes + node;
-            const Planes4 pl = load_planes4<kAnyHit>(q, id);
-            const int4 rf = __ldg(&q->ref);
             float t[4];
-            int r[4] = {rf.x, rf.y, rf.z, rf.w};
-            float tc;
-            t[0] = slab_nf(pl.nx.x, pl.fx.x, pl.ny.x, pl.fy.x, pl.nz.x, pl.fz.x, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-            t[1] = slab_nf(pl.nx.y, pl.fx.y, pl.ny.y, pl.fy.y, pl.nz.y, pl.fz.y, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-            t[2] = slab_nf(pl.nx.z, pl.fx.z, pl.ny.z, pl.fy.z, pl.nz.z, pl.fz.z, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-            t[3] = slab_nf(pl.nx.w, pl.fx.w, pl.ny.w, pl.fy.w, pl.nz.w, pl.fz.w, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-            auto cx = [&](int i, int j) {   // nearest first, as the resumable traversal
-                if (t[j] < t[i]) { const float tt = t[i]; t[i] = t[j]; t[j] = tt; const int rr = r[i]; r[i] = r[j]; r[j] = rr; }
-            };
-            cx(0, 1); cx(2, 3); cx(0, 2); cx(1, 3); cx(1, 2);
+            int r[4];
+            boxes4<kAnyHit>(nodes + node, id, ood, box_tmin, box_tmax, t, r);
+            order4<true>(t, r);
             if (t[0] != kMiss) {
                 if (t[3] != kMiss && sp < kTraversalStack4Local) stack[sp++] = r[3];
                 if (t[2] != kMiss && sp < kTraversalStack4Local) stack[sp++] = r[2];
@@ -203,6 +279,7 @@ __device__ __forceinline__ bool bvh_trace4(const BvhNode4* __restrict__ nodes, c
                 if (tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
                                   &t, &u, &v)) {
                     if (kAnyHit) return true;
+                    if (tie) *tie = *tie || (t == tbest && best >= 0);
                     tbest = t; bu = u; bv = v;
                     best = __float_as_int(p.w);
                     box_tmax = tbest * 1.00000095f;
@@ -265,16 +342,30 @@ struct LaneStackT {
 using LaneStack = LaneStackT<kTraversalStack>;
 using LaneStack4 = LaneStackT<kTraversalStack4>;
 
-// Resumable traversal of one ray, for persistent kernels whose lanes take a new
-// ray as soon as theirs finishes (lane refill). Same visiting order, slack and
-// exact triangle test as bvh_trace; round() advances every lane of a warp by one
-// while-while round and returns true when this lane's ray is finished.
-template <bool kAnyHit>
-struct TraceState {
+// Resumable traversal of one ray, for persistent kernels whose lanes take a new ray as soon
+// as theirs finishes (lane refill). Same slack and exact triangle test as bvh_trace.
+//
+// round() advances every lane of a warp by one round of "while-while" traversal with
+// speculative leaf postponing (Aila & Laine, "Understanding the Efficiency of Ray Traversal
+// on GPUs", HPG 2009): in the interior phase a lane walks down until it holds a leaf, and one
+// that holds one walks on speculatively; then all lanes test their leaf's triangles together.
+// The interior phase ends when at most kMaxSearching lanes are still without a leaf (they go on
+// in the next round) instead of when none is: waiting for the last few left most of the warp
+// idle. Measured per 1080p terrain frame on the full-precision 4-wide nodes, at a limit of 0 /
+// 4 / 6 / 8 / 10 lanes: closest hit 120.9 / 107.7 / 106.8 / 107.0 / 107.2 ms, any hit 60.3 /
+// 55.0 / 54.8 / 55.2 / 55.6 ms. The order in which a ray tests its leaves does not depend on it.
+// All 32 lanes of the warp must call round(); lanes without a ray hold node = leaf = kNoNode.
+constexpr int kMaxSearching = 6;
+constexpr int kNoNode = INT_MIN;
+
+// What every form of the resumable traversal keeps per ray.
+struct TraceLane {
     float3 o, d, id, ood;
     float mint, tbest, box_tmin, box_tmax, bu, bv;
-    int node, sp, best;
-    bool hit_any;
+    int node = kNoNode, leaf = kNoNode;   // next node (>= 0) or leaf reference; the postponed leaf
+    int sp = 0, best;                 // stack entries: none once finished
+    bool hit_any;                     // any hit: something was hit
+    bool tie;                         // closest hit: a second triangle lies at exactly the best distance
 
     __device__ __forceinline__ void begin(float3 o_, float3 d_, float mint_, float maxt_) {
         o = o_; d = d_;
@@ -286,165 +377,97 @@ struct TraceState {
         box_tmax = tbest * 1.00000095f;
         bu = bv = 0.f;
         node = 0; sp = 0; best = -1;
-        leaf = kNone;
-        hit_any = false;
+        leaf = kNoNode;
+        hit_any = tie = false;
     }
+    __device__ __forceinline__ bool finished() const { return node == kNoNode && leaf == kNoNode; }
 
-    // One round of "while-while" traversal with speculative leaf postponing (Aila &
-    // Laine, "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009): the
-    // interior loop runs until every lane of the warp holds a leaf (or has finished),
-    // lanes that already hold one keep descending speculatively, then all lanes test
-    // their leaf's triangles together. `live` marks lanes that have a ray; all 32
-    // lanes of the warp must call round(). Returns true when this lane's ray is done.
-    int leaf;        // postponed leaf reference, kNone if none
-    static constexpr int kNone = INT_MIN;
+    template <class Stack>
+    __device__ __forceinline__ int pop(Stack& stack) { return sp > 0 ? stack.get(--sp) : kNoNode; }
 
-    __device__ __forceinline__ bool round(const BvhNode* __restrict__ nodes, const BvhTri* __restrict__ tris,
-                                          LaneStack& stack, bool live) {
-        bool finished = !live;
-        if (live && leaf == kNone && node == kNone) finished = true;
-        // interior phase
-        while (true) {
-            bool searching = false;
-            if (!finished && node != kNone && node >= 0) {
-                const float4 a = __ldg(&nodes[node].a);
-                const float4 b = __ldg(&nodes[node].b);
-                const float4 c = __ldg(&nodes[node].c);
-                const float4 e = __ldg(&nodes[node].d);
-                float t0, t1;
-                const bool h0 = slab(a.x, a.y, a.z, a.w, c.x, c.y, id, ood, box_tmin, box_tmax, &t0);
-                const bool h1 = slab(b.x, b.y, b.z, b.w, c.z, c.w, id, ood, box_tmin, box_tmax, &t1);
-                const int r0 = __float_as_int(e.x), r1 = __float_as_int(e.y);
-                if (h0 && h1) {
-                    const bool first0 = t0 <= t1;
-                    if (sp < kTraversalStack) stack.set(sp++, first0 ? r1 : r0);   // depth <= 63 is checked at build
-                    node = first0 ? r0 : r1;
-                } else if (h0) node = r0;
-                else if (h1) node = r1;
-                else node = sp > 0 ? stack.get(--sp) : kNone;
-            }
-            if (!finished && node != kNone && node < 0 && leaf == kNone) {   // postpone this leaf
-                leaf = node;
-                node = sp > 0 ? stack.get(--sp) : kNone;
-            }
-            if (!finished) searching = leaf == kNone && node != kNone;   // still looking for a leaf
-            if (!__any_sync(0xffffffffu, searching)) break;
-        }
-        // leaf phase
-        if (!finished && leaf != kNone) {
-            const int packed = ~leaf;
-            const int start = packed >> 5, end = start + (packed & 31);
-            leaf = kNone;
-            for (int k = start; k < end; ++k) {
-                const float4 p = __ldg(&tris[k].p1);
-                const float4 e1 = __ldg(&tris[k].e1);
-                const float4 e2 = __ldg(&tris[k].e2);
-                float t, u, v;
-                if (tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
-                                  &t, &u, &v)) {
-                    if (kAnyHit) { hit_any = true; return true; }
-                    tbest = t; bu = u; bv = v;
-                    best = __float_as_int(p.w);
-                    box_tmax = tbest * 1.00000095f;
-                }
+    // The postponed leaf's triangles.
+    template <bool kAnyHit>
+    __device__ __forceinline__ void test_leaf(const BvhTri* __restrict__ tris) {
+        const int packed = ~leaf;
+        const int start = packed >> 5, end = start + (packed & 31);
+        leaf = kNoNode;
+        for (int k = start; k < end; ++k) {
+            const float4 p = __ldg(&tris[k].p1);
+            const float4 e1 = __ldg(&tris[k].e1);
+            const float4 e2 = __ldg(&tris[k].e2);
+            float t, u, v;
+            if (tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
+                              &t, &u, &v)) {
+                if (kAnyHit) { hit_any = true; node = kNoNode; sp = 0; return; }
+                tie = tie || (t == tbest && best >= 0);
+                tbest = t; bu = u; bv = v;
+                best = __float_as_int(p.w);
+                box_tmax = tbest * 1.00000095f;
             }
         }
-        if (finished) return live;
-        return leaf == kNone && node == kNone;
     }
 };
 
-// The same resumable while-while traversal over the 4-wide tree: a node visit loads
-// one 128-byte record, tests four boxes, and continues with the nearest hit child
-// while the other hit children go on the stack, farthest first. Boxes and the triangle
-// test are the binary tree's, so the closest hit equals it whenever the minimum is unique.
-template <bool kAnyHit>
-struct TraceState4 {
-    float3 o, d, id, ood;
-    float mint, tbest, box_tmin, box_tmax, bu, bv;
-    int node, sp, best;
-    bool hit_any;
-    int leaf;
-    static constexpr int kNone = INT_MIN;
-
-    __device__ __forceinline__ void begin(float3 o_, float3 d_, float mint_, float maxt_) {
-        o = o_; d = d_;
-        id = mk(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
-        ood = mk(o.x * id.x, o.y * id.y, o.z * id.z);
-        mint = mint_;
-        box_tmin = mint > 0.f ? mint * 0.99999905f : mint * 1.00000095f;
-        tbest = maxt_;
-        box_tmax = tbest * 1.00000095f;
-        bu = bv = 0.f;
-        node = 0; sp = 0; best = -1;
-        leaf = kNone;
-        hit_any = false;
+// One round over any of the trees: `visit` steps a lane whose node is an interior one.
+template <bool kAnyHit, class Stack, class Visit>
+__device__ __forceinline__ void trace_round(TraceLane& s, const BvhTri* __restrict__ tris, Stack& stack, Visit visit) {
+    while (true) {
+        if (s.node >= 0) visit();
+        if (s.node < 0 && s.leaf == kNoNode) {   // postpone this leaf (kNoNode stays kNoNode: the stack is empty then)
+            s.leaf = s.node;
+            s.node = s.pop(stack);
+        }
+        const bool searching = s.leaf == kNoNode && s.node != kNoNode;
+        if (__popc(__ballot_sync(0xffffffffu, searching)) <= kMaxSearching) break;
     }
+    if (s.leaf != kNoNode) s.test_leaf<kAnyHit>(tris);
+}
 
-    __device__ __forceinline__ void visit(const BvhNode4* __restrict__ nodes, LaneStack4& stack) {
-        const BvhNode4* q = nodes + node;
-        const Planes4 pl = load_planes4<kAnyHit>(q, id);
-        const float4 rff = ld_node(reinterpret_cast<const float4*>(&q->ref));
-        const int4 rf = make_int4(__float_as_int(rff.x), __float_as_int(rff.y), __float_as_int(rff.z),
-                                  __float_as_int(rff.w));
+// Over the binary tree, in the visiting order of bvh_trace.
+template <bool kAnyHit>
+struct TraceState : TraceLane {
+    __device__ __forceinline__ void visit(const BvhNode* __restrict__ nodes, LaneStack& stack) {
+        const float4 a = __ldg(&nodes[node].a);
+        const float4 b = __ldg(&nodes[node].b);
+        const float4 c = __ldg(&nodes[node].c);
+        const float4 e = __ldg(&nodes[node].d);
+        float t0, t1;
+        const bool h0 = slab(a.x, a.y, a.z, a.w, c.x, c.y, id, ood, box_tmin, box_tmax, &t0);
+        const bool h1 = slab(b.x, b.y, b.z, b.w, c.z, c.w, id, ood, box_tmin, box_tmax, &t1);
+        const int r0 = __float_as_int(e.x), r1 = __float_as_int(e.y);
+        if (h0 && h1) {
+            const bool first0 = t0 <= t1;
+            if (sp < kTraversalStack) stack.set(sp++, first0 ? r1 : r0);   // depth <= 63 is checked at build
+            node = first0 ? r0 : r1;
+        } else if (h0) node = r0;
+        else if (h1) node = r1;
+        else node = pop(stack);
+    }
+    __device__ __forceinline__ void round(const BvhNode* __restrict__ nodes, const BvhTri* __restrict__ tris,
+                                          LaneStack& stack) {
+        trace_round<kAnyHit>(*this, tris, stack, [&]() { visit(nodes, stack); });
+    }
+};
+
+// Over a 4-wide tree: the nearest child entered comes next, the others go on the stack, farthest
+// first (three entries a level at most: checked against the stack at build).
+template <bool kAnyHit, class Node4>
+struct TraceState4 : TraceLane {
+    __device__ __forceinline__ void visit(const Node4* __restrict__ nodes, LaneStack4& stack) {
         const float kMiss = __int_as_float(0x7f800000);
         float t[4];
-        int r[4] = {rf.x, rf.y, rf.z, rf.w};
-        float tc;
-        t[0] = slab_nf(pl.nx.x, pl.fx.x, pl.ny.x, pl.fy.x, pl.nz.x, pl.fz.x, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-        t[1] = slab_nf(pl.nx.y, pl.fx.y, pl.ny.y, pl.fy.y, pl.nz.y, pl.fz.y, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-        t[2] = slab_nf(pl.nx.z, pl.fx.z, pl.ny.z, pl.fy.z, pl.nz.z, pl.fz.z, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-        t[3] = slab_nf(pl.nx.w, pl.fx.w, pl.ny.w, pl.fy.w, pl.nz.w, pl.fz.w, id, ood, box_tmin, box_tmax, &tc) ? tc : kMiss;
-        // ascending by entry distance (misses last): a five-exchange network. Any-hit rays
-        // take the same order (nearest first measured 1.6% faster than slot order for the
-        // next-event rays, whose occluders tend to lie near the shading point).
-        auto cx = [&](int i, int j) {
-            if (t[j] < t[i]) { const float tt = t[i]; t[i] = t[j]; t[j] = tt; const int rr = r[i]; r[i] = r[j]; r[j] = rr; }
-        };
-        cx(0, 1); cx(2, 3); cx(0, 2); cx(1, 3); cx(1, 2);
-        if (t[0] == kMiss) { node = sp > 0 ? stack.get(--sp) : kNone; return; }
-        if (t[3] != kMiss && sp < kTraversalStack4) stack.set(sp++, r[3]);
-        if (t[2] != kMiss && sp < kTraversalStack4) stack.set(sp++, r[2]);
-        if (t[1] != kMiss && sp < kTraversalStack4) stack.set(sp++, r[1]);
+        int r[4];
+        boxes4<kAnyHit>(nodes + node, id, ood, box_tmin, box_tmax, t, r);
+        order4<!kAnyHit>(t, r);
+        if (t[0] == kMiss) { node = pop(stack); return; }
+        if (t[3] != kMiss) stack.set(sp++, r[3]);
+        if (t[2] != kMiss) stack.set(sp++, r[2]);
+        if (t[1] != kMiss) stack.set(sp++, r[1]);
         node = r[0];
     }
-
-    // As TraceState::round: interior phase until every live lane holds a leaf, then the
-    // leaf phase. All 32 lanes of the warp must call it.
-    __device__ __forceinline__ bool round(const BvhNode4* __restrict__ nodes, const BvhTri* __restrict__ tris,
-                                          LaneStack4& stack, bool live) {
-        bool finished = !live;
-        if (live && leaf == kNone && node == kNone) finished = true;
-        while (true) {
-            bool searching = false;
-            if (!finished && node != kNone && node >= 0) visit(nodes, stack);
-            if (!finished && node != kNone && node < 0 && leaf == kNone) {   // postpone this leaf
-                leaf = node;
-                node = sp > 0 ? stack.get(--sp) : kNone;
-            }
-            if (!finished) searching = leaf == kNone && node != kNone;
-            if (!__any_sync(0xffffffffu, searching)) break;
-        }
-        if (!finished && leaf != kNone) {
-            const int packed = ~leaf;
-            const int start = packed >> 5, end = start + (packed & 31);
-            leaf = kNone;
-            for (int k = start; k < end; ++k) {
-                const float4 p = __ldg(&tris[k].p1);
-                const float4 e1 = __ldg(&tris[k].e1);
-                const float4 e2 = __ldg(&tris[k].e2);
-                float t, u, v;
-                if (tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
-                                  &t, &u, &v)) {
-                    if (kAnyHit) { hit_any = true; return true; }
-                    tbest = t; bu = u; bv = v;
-                    best = __float_as_int(p.w);
-                    box_tmax = tbest * 1.00000095f;
-                }
-            }
-        }
-        if (finished) return live;
-        return leaf == kNone && node == kNone;
+    __device__ __forceinline__ void round(const Node4* __restrict__ nodes, const BvhTri* __restrict__ tris,
+                                          LaneStack4& stack) {
+        trace_round<kAnyHit>(*this, tris, stack, [&]() { visit(nodes, stack); });
     }
 };
 

@@ -560,6 +560,7 @@ void bvh_free_device(DeviceBvh* bvh, cudaStream_t s) {
     if (bvh->nodes) cudaFreeAsync(bvh->nodes, s);
     if (bvh->tris) cudaFreeAsync(bvh->tris, s);
     if (bvh->nodes4) cudaFreeAsync(bvh->nodes4, s);
+    if (bvh->nodes4q) cudaFreeAsync(bvh->nodes4q, s);
     *bvh = DeviceBvh();
 }
 
@@ -749,6 +750,56 @@ __global__ void k_collapse4_dp(const BvhNode* __restrict__ n2, const uchar4* __r
     write_node4(lo, hi, ref, n, f.y, out, counters, next, cap);
 }
 
+// One axis of a node's quantised boxes. The decoded plane of byte q is p + s (1 + q 2^-15) in
+// exact arithmetic; planes are rounded outward with a margin of 1/64 cell for the traversal's
+// rounding (2^-8 cell at most). The cell grows until every plane fits.
+__device__ void quantise_axis(const float (&lo)[4], const float (&hi)[4], const bool (&used)[4], float* p_out,
+                              float* s_out, uint32_t* qlo, uint32_t* qhi) {
+    double mn = 1e300, mx = -1e300;
+    for (int k = 0; k < 4; ++k)
+        if (used[k]) { mn = fmin(mn, (double)lo[k]); mx = fmax(mx, (double)hi[k]); }
+    double cell = fmax((mx - mn) / 250.0, 1e-30);
+    float p = 0.f, s = 0.f;
+    int l[4], h[4];
+    for (int it = 0; it < 64; ++it) {
+        s = (float)(cell * 32768.0);
+        p = (float)(mn - (double)s - 2.0 * cell);
+        bool ok = true;
+        for (int k = 0; k < 4; ++k) {
+            if (!used[k]) { l[k] = 255; h[k] = 0; continue; }
+            const double a = floor((((double)lo[k] - p) / s - 1.0) * 32768.0 - 1.0 / 64.0);
+            const double b = ceil((((double)hi[k] - p) / s - 1.0) * 32768.0 + 1.0 / 64.0);
+            ok = ok && a >= 0.0 && b <= 255.0;
+            l[k] = (int)fmin(fmax(a, 0.0), 255.0);
+            h[k] = (int)fmin(fmax(b, 0.0), 255.0);
+        }
+        if (ok) break;
+        cell *= 1.25;
+    }
+    *p_out = p;
+    *s_out = s;
+    *qlo = *qhi = 0u;
+    for (int k = 0; k < 4; ++k) { *qlo |= (uint32_t)l[k] << (8 * k); *qhi |= (uint32_t)h[k] << (8 * k); }
+}
+
+__global__ void k_quantise4(const BvhNode4* __restrict__ in, int n, BvhNode4Q* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const BvhNode4 nd = in[i];
+    const int r[4] = {nd.ref.x, nd.ref.y, nd.ref.z, nd.ref.w};
+    const float lx[4] = {nd.lox.x, nd.lox.y, nd.lox.z, nd.lox.w}, hx[4] = {nd.hix.x, nd.hix.y, nd.hix.z, nd.hix.w};
+    const float ly[4] = {nd.loy.x, nd.loy.y, nd.loy.z, nd.loy.w}, hy[4] = {nd.hiy.x, nd.hiy.y, nd.hiy.z, nd.hiy.w};
+    const float lz[4] = {nd.loz.x, nd.loz.y, nd.loz.z, nd.loz.w}, hz[4] = {nd.hiz.x, nd.hiz.y, nd.hiz.z, nd.hiz.w};
+    bool used[4];
+    for (int k = 0; k < 4; ++k) used[k] = r[k] != ~0 && lx[k] <= hx[k] && ly[k] <= hy[k] && lz[k] <= hz[k];
+    BvhNode4Q q;
+    quantise_axis(lx, hx, used, &q.p[0], &q.s[0], &q.lox, &q.hix);
+    quantise_axis(ly, hy, used, &q.p[1], &q.s[1], &q.loy, &q.hiy);
+    quantise_axis(lz, hz, used, &q.p[2], &q.s[2], &q.loz, &q.hiz);
+    for (int k = 0; k < 4; ++k) q.ref[k] = r[k];
+    out[i] = q;
+}
+
 }  // namespace
 
 cudaError_t bvh_collapse4(DeviceBvh* b, cudaStream_t s) {
@@ -800,6 +851,8 @@ cudaError_t bvh_collapse4(DeviceBvh* b, cudaStream_t s) {
         bound = hc[2];
     }
     b->num_nodes4 = hc[0];
+    CK(dalloc(&b->nodes4q, b->num_nodes4, s));
+    k_quantise4<<<div_up(b->num_nodes4, 128), 128, 0, s>>>(b->nodes4, b->num_nodes4, b->nodes4q);
     b->depth4 = hc[3];
     dfree(fa, s);
     dfree(fb, s);

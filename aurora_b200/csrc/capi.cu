@@ -273,7 +273,9 @@ aur_status aur_bvh_build(aur_ctx* ctx, const float* verts, uint32_t nvert, const
     if (e == cudaSuccess && 3 * b->bvh.depth4 + 1 > kTraversalStack4) {
         // a 4-wide node pushes up to three entries: too deep for its stack, keep the binary tree only
         cudaFreeAsync(b->bvh.nodes4, s);
+        cudaFreeAsync(b->bvh.nodes4q, s);
         b->bvh.nodes4 = nullptr;
+        b->bvh.nodes4q = nullptr;
         b->bvh.num_nodes4 = 0;
     }
     if (e == cudaSuccess && tri_attr) {

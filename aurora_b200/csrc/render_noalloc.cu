@@ -89,7 +89,7 @@ extern "C" aur_status aur_render_fp64acc_noalloc(aur_scene* sc, const aur_render
     if ((st = device_addresses(&a)) != AUR_OK) return st;
     cudaStream_t s = sc->ctx->stream;
     cudaError_t e = cudaMemsetAsync(a.counters, 0, sizeof(unsigned long long) * 8, s);
-    if (e == cudaSuccess) e = launch_render_plain(sc->dev(), p, (float4*)film, a.accum, a.counters, false, s);
+    if (e == cudaSuccess) e = launch_render_plain(sc->dev(), p, (float4*)film, a.accum, a.counters, 0, s);
     unsigned long long cnt[4] = {0, 0, 0, 0};
     if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, a.counters, sizeof(cnt), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -26,7 +26,7 @@ __device__ __forceinline__ void add_counters(unsigned long long* counters, const
         for (int k = 0; k < kN; ++k) atomicAdd(&counters[k], v[k]);
 }
 
-// kWidth: the tree traversed (2 binary, 4 four-wide). The timed kernels use the binary
+// kWidth: the tree traversed (2 binary, 4 four-wide, 8 quantised four-wide). The timed kernels use the binary
 // tree, on which this one-thread-per-path kernel is fastest (its code holds five
 // traversals; the 4-wide ones made it 30% slower); the counting pass can use either, to
 // count the work of the wavefront renderer's traversal.
@@ -89,16 +89,18 @@ __global__ void __launch_bounds__(kPlainBlock) k_render_plain(DevScene sc, PathP
 }  // namespace
 
 cudaError_t launch_render_plain(const DevScene& sc, const PathParams& p, float4* film, double* film64,
-                                unsigned long long* counters, bool count_work, cudaStream_t s) {
+                                unsigned long long* counters, int count_width, cudaStream_t s) {
     const int npix = sc.cam.w * sc.cam.h;
     const int grid = (npix + kPlainBlock - 1) / kPlainBlock;
     const bool multi = p.light_samples > 1;
     if (film64 && multi) k_render_plain<true, false, 2, true><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
     else if (film64) k_render_plain<true, false, 2, false><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
-    else if (count_work && multi) return cudaErrorNotSupported;   // the counting pass counts one path per sample
-    else if (count_work && sc.nodes4)
+    else if (count_width && multi) return cudaErrorNotSupported;   // the counting pass counts one path per sample
+    else if (count_width == 8)
+        k_render_plain<false, true, 8, false><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
+    else if (count_width == 4)
         k_render_plain<false, true, 4, false><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
-    else if (count_work) k_render_plain<false, true, 2, false><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
+    else if (count_width) k_render_plain<false, true, 2, false><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
     else if (multi) k_render_plain<false, false, 2, true><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
     else k_render_plain<false, false, 2, false><<<grid, kPlainBlock, 0, s>>>(sc, p, film, film64, counters);
     return cudaGetLastError();

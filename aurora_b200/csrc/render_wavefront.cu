@@ -34,9 +34,9 @@ namespace {
 enum : uint32_t { PS_EMPTY = 0, PS_ACTIVE = 1, PS_DONE = 2, PS_MASK = 3, PS_PENDING = 4 };
 // lane refill: a warp takes new rays once this many lanes are idle, and runs kRounds
 // traversal rounds (interior phase + leaf phase) between refill checks
-// (swept on the 4-wide tree: rounds 2 / 3 / 4 / 6 / 8 at 16 idle lanes 479.6 / 481.8 /
-// 488.1 / 472.7 / 463.8 M samples/s; refill 8-20 idle lanes within 0.5% at 4 rounds)
-constexpr int kRefill = 16;
+// (swept on the quantised 4-wide tree, 1080p terrain frame, closest + any hit: rounds 3 / 4 / 5 at
+// 16 idle lanes 142.6 / 141.0 / 141.0 ms; 12 / 16 / 20 idle lanes at 4 rounds 140.1 / 141.0 / 143.8)
+constexpr int kRefill = 12;
 constexpr int kRounds = 4;
 // resident 256-thread blocks per SM the traversal kernels are compiled for (register cap)
 #ifndef AUR_TRAV_MINB
@@ -266,14 +266,34 @@ __device__ __forceinline__ int bucket_of(const ShadeScene& sh, int prim) {
          : mt == MAT_METAL ? B_METAL : B_CONST;
 }
 
+// The tree a traversal kernel walks.
+enum : int { TREE_BINARY = 0, TREE_WIDE = 1, TREE_QUANT = 2 };
+template <int kTree, bool kAnyHit> struct TreeTypes;
+template <bool kAnyHit> struct TreeTypes<TREE_BINARY, kAnyHit> {
+    using Node = BvhNode;
+    using Stack = LaneStack;
+    using Trace = TraceState<kAnyHit>;
+    __device__ static const Node* nodes(const DevScene& sc) { return sc.nodes; }
+};
+template <bool kAnyHit> struct TreeTypes<TREE_WIDE, kAnyHit> {
+    using Node = BvhNode4;
+    using Stack = LaneStack4;
+    using Trace = TraceState4<kAnyHit, BvhNode4>;
+    __device__ static const Node* nodes(const DevScene& sc) { return sc.nodes4; }
+};
+template <bool kAnyHit> struct TreeTypes<TREE_QUANT, kAnyHit> {
+    using Node = BvhNode4Q;
+    using Stack = LaneStack4;
+    using Trace = TraceState4<kAnyHit, BvhNode4Q>;
+    __device__ static const Node* nodes(const DevScene& sc) { return sc.nodes4q; }
+};
+
 // Closest hit for the extension queue. Each lane keeps a resumable traversal;
 // finished lanes are refilled from the queue (one atomic per warp) while the
 // others continue, so a warp is not held up by its slowest ray.
-template <bool kSort, bool kWide>
+template <bool kSort, int kTree>
 __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_q) {
-    using Stack = std::conditional_t<kWide, LaneStack4, LaneStack>;
-    using Trace = std::conditional_t<kWide, TraceState4<false>, TraceState<false>>;
-    using Node = std::conditional_t<kWide, BvhNode4, BvhNode>;
+    using Tree = TreeTypes<kTree, false>;
     const uint32_t* qin = in_q ? w.q_ext1 : w.q_ext0;
     const uint32_t n = w.ctr[in_q ? C_EXT1 : C_EXT0];
     // Outputs of the later stages start empty. Only counters that no block of
@@ -290,13 +310,15 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
     }
     extern __shared__ int s_stack[];
     __shared__ uint32_t s_bucket[kBuckets];   // per-block material counts, added to the global ones at exit
+    __shared__ uint32_t s_tie[256];           // per thread: first slot of its list of exact-distance ties
     if (kSort && threadIdx.x < kBuckets) s_bucket[threadIdx.x] = 0;
+    s_tie[threadIdx.x] = 0xffffffffu;
     __syncthreads();
-    Stack stack;
+    typename Tree::Stack stack;
     stack.col = s_stack + threadIdx.x;
     stack.stride = blockDim.x;
-    Trace ts;
-    const Node* nodes = nullptr;
+    typename Tree::Trace ts;
+    const typename Tree::Node* nodes = nullptr;
     const BvhTri* tris = nullptr;
     const WfScene* S = nullptr;
     uint32_t slot = 0;
@@ -315,8 +337,7 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
                 if (k < n) {
                     slot = qin[k];
                     S = &w.scenes[w.id(slot).x];
-                    if constexpr (kWide) nodes = S->sc.nodes4;
-                    else nodes = S->sc.nodes;
+                    nodes = Tree::nodes(S->sc);
                     tris = S->sc.tris;
                     const float4 o = w.ray_o(slot), d = w.ray_d(slot);
                     ts.begin(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, d.w);
@@ -327,17 +348,19 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
             }
         }
         if (__ballot_sync(0xffffffffu, has || !exhausted) == 0) break;
-        bool done = false;
-        for (int k = 0; k < kRounds; ++k) {          // all lanes take part in every round
-            if (ts.round(nodes, tris, stack, has && !done)) done = true;
-        }
-        done = done && has;
+        for (int k = 0; k < kRounds; ++k) ts.round(nodes, tris, stack);   // all lanes take part in every round
+        const bool done = has && ts.finished();
         int bucket = -1;
         if (done) {
-            w.hit(slot) = make_float4(ts.tbest, ts.bu, ts.bv, __int_as_float(ts.best));
-            if (kSort) {
-                bucket = bucket_of(S->sc.sh, ts.best);
-                w.bucket[slot] = (uint8_t)bucket;   // the scatter reads it instead of the hit's material
+            if (kTree == TREE_QUANT && ts.tie) {   // traced again below; the thread's ties are a list through q_sort
+                w.q_sort[slot] = s_tie[threadIdx.x];
+                s_tie[threadIdx.x] = slot;
+            } else {
+                w.hit(slot) = make_float4(ts.tbest, ts.bu, ts.bv, __int_as_float(ts.best));
+                if (kSort) {
+                    bucket = bucket_of(S->sc.sh, ts.best);
+                    w.bucket[slot] = (uint8_t)bucket;   // the scatter reads it instead of the hit's material
+                }
             }
             has = false;
         }
@@ -346,6 +369,24 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
             if (bucket >= 0) {
                 const uint32_t peers = __match_any_sync(fin, bucket);
                 if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(&s_bucket[bucket], (uint32_t)__popc(peers));
+            }
+        }
+    }
+    if constexpr (kTree == TREE_QUANT) {
+        // rays that met two triangles at exactly the same distance take the hit that the
+        // full-precision tree's visiting order gives (out of the main loop, so that the second
+        // traversal adds no registers to it)
+        for (uint32_t i = s_tie[threadIdx.x]; i != 0xffffffffu; i = w.q_sort[i]) {
+            const WfScene& T = w.scenes[w.id(i).x];
+            const float4 o = w.ray_o(i), d = w.ray_d(i);
+            Hit h;
+            TraceWork work;
+            bvh_trace4<false>(T.sc.nodes4, T.sc.tris, mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, d.w, &h, work);
+            w.hit(i) = make_float4(h.t, h.u, h.v, __int_as_float(h.prim));
+            if (kSort) {
+                const int b = bucket_of(T.sc.sh, h.prim);
+                w.bucket[i] = (uint8_t)b;
+                atomicAdd(&s_bucket[b], 1u);
             }
         }
     }
@@ -582,11 +623,9 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
 // ------------------------------------------------------------------ shadow
 // Occlusion of the next-event rays (entries slot << 1 | ray); lanes are refilled as in
 // k_extend. An unoccluded ray sets its bit in sh_vis; the next regen adds the light.
-template <bool kWide>
+template <int kTree>
 __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
-    using Stack = std::conditional_t<kWide, LaneStack4, LaneStack>;
-    using Trace = std::conditional_t<kWide, TraceState4<true>, TraceState<true>>;
-    using Node = std::conditional_t<kWide, BvhNode4, BvhNode>;
+    using Tree = TreeTypes<kTree, true>;
     const uint32_t n = w.ctr[C_SHADOW];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.rays[1] += n;
@@ -595,11 +634,11 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
         for (int k = 0; k < kBuckets; ++k) { w.ctr[C_BUCKET + k] = 0; w.ctr[C_FILL + k] = 0; }
     }
     extern __shared__ int s_stack[];
-    Stack stack;
+    typename Tree::Stack stack;
     stack.col = s_stack + threadIdx.x;
     stack.stride = blockDim.x;
-    Trace ts;
-    const Node* nodes = nullptr;
+    typename Tree::Trace ts;
+    const typename Tree::Node* nodes = nullptr;
     const BvhTri* tris = nullptr;
     uint32_t entry = 0;
     bool has = false, exhausted = false;
@@ -618,8 +657,7 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
                     entry = w.q_shadow[k];
                     const uint32_t slot = entry >> 1;
                     const WfScene& S = w.scenes[w.id(slot).x];
-                    if constexpr (kWide) nodes = S.sc.nodes4;
-                    else nodes = S.sc.nodes;
+                    nodes = Tree::nodes(S.sc);
                     tris = S.sc.tris;
                     const float4 p = w.sh_p(slot);
                     const float4 d = (entry & 1u) ? w.sh_d1(slot) : w.sh_d0(slot);
@@ -631,11 +669,8 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
             }
         }
         if (__ballot_sync(0xffffffffu, has || !exhausted) == 0) break;
-        bool done = false;
-        for (int k = 0; k < kRounds; ++k) {
-            if (ts.round(nodes, tris, stack, has && !done)) done = true;
-        }
-        if (done && has) {
+        for (int k = 0; k < kRounds; ++k) ts.round(nodes, tris, stack);
+        if (has && ts.finished()) {
             if (!ts.hit_any) atomicOr(&w.sh_vis[entry >> 1], 1u << (entry & 1u));
             has = false;
         }
@@ -704,7 +739,9 @@ struct WfConfig {
     int block = 128;
     int sort = 1;
     int record = 0;   // record mode: hit records + unclamped radiance per item instead of samples
-    int wide = 0;     // traverse the 4-wide trees (every scene of the batch has one)
+    // the trees traversed by closest-hit and any-hit rays (TREE_*; the 4-wide ones only when every
+    // scene has them), chosen by tree_for
+    int tree = TREE_BINARY, tree_any = TREE_BINARY;
 };
 
 // The 4-wide traversal is used when every scene of a batch has a 4-wide tree.
@@ -712,7 +749,17 @@ struct WfConfig {
 #define AUR_WIDE_TRAVERSAL 1
 #endif
 struct BatchItem;
-static int wide_for(const std::vector<BatchItem>& items);
+static void tree_for(const std::vector<BatchItem>& items, WfConfig* cfg);
+
+static auto extend_kernel(const WfConfig& c) -> void (*)(WfPool, int) {
+    if (c.tree == TREE_QUANT) return c.sort ? k_extend<true, TREE_QUANT> : k_extend<false, TREE_QUANT>;
+    if (c.tree == TREE_WIDE) return c.sort ? k_extend<true, TREE_WIDE> : k_extend<false, TREE_WIDE>;
+    return c.sort ? k_extend<true, TREE_BINARY> : k_extend<false, TREE_BINARY>;
+}
+static auto shadow_kernel(const WfConfig& c) -> void (*)(WfPool) {
+    return c.tree_any == TREE_QUANT ? k_shadow<TREE_QUANT>
+         : c.tree_any == TREE_WIDE ? k_shadow<TREE_WIDE> : k_shadow<TREE_BINARY>;
+}
 
 // ------------------------------------------------------------------ host driver
 struct WfRun {
@@ -778,13 +825,11 @@ struct WfRun {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, c.block, smem);
             return std::max(1, nb) * sms;
         };
-        const void* ext = c.wide ? (c.sort ? (const void*)k_extend<true, true> : (const void*)k_extend<false, true>)
-                                 : (c.sort ? (const void*)k_extend<true, false> : (const void*)k_extend<false, false>);
-        grid_ext = persist(ext, stack_smem);
+        grid_ext = persist((const void*)extend_kernel(c), stack_smem);
         grid_shade = persist(c.record ? (const void*)k_shade<true, SHADE_ALL> : (const void*)k_shade<false, SHADE_ALL>, 0);
         grid_shade_m = persist(c.record ? (const void*)k_shade<true, SHADE_MATTE> : (const void*)k_shade<false, SHADE_MATTE>, 0);
         grid_shade_r = persist(c.record ? (const void*)k_shade<true, SHADE_REST> : (const void*)k_shade<false, SHADE_REST>, 0);
-        grid_shadow = persist(c.wide ? (const void*)k_shadow<true> : (const void*)k_shadow<false>, stack_smem);
+        grid_shadow = persist((const void*)shadow_kernel(c), stack_smem);
         grid_sort = persist((const void*)k_sort_scatter, 0);
         // 64 blocks per SM (about 10 resident waves of the 40-register kernel): 14.8 ms per
         // 1080p frame against 15.3 at 16 and 16.5 at exactly the resident 6
@@ -799,13 +844,7 @@ struct WfRun {
         if (cfg.record) k_regen<true><<<grid_regen, cfg.block, 0, stream>>>(w, in_q);
         else k_regen<false><<<grid_regen, cfg.block, 0, stream>>>(w, in_q);
         cudaEventRecordWithFlags(e[0], stream, cudaEventRecordExternal);
-        if (cfg.wide) {
-            if (cfg.sort) k_extend<true, true><<<grid_ext, cfg.block, stack_smem, stream>>>(w, in_q);
-            else k_extend<false, true><<<grid_ext, cfg.block, stack_smem, stream>>>(w, in_q);
-        } else {
-            if (cfg.sort) k_extend<true, false><<<grid_ext, cfg.block, stack_smem, stream>>>(w, in_q);
-            else k_extend<false, false><<<grid_ext, cfg.block, stack_smem, stream>>>(w, in_q);
-        }
+        extend_kernel(cfg)<<<grid_ext, cfg.block, stack_smem, stream>>>(w, in_q);
         cudaEventRecordWithFlags(e[1], stream, cudaEventRecordExternal);
         if (cfg.sort) k_sort_scatter<<<grid_sort, cfg.block, 0, stream>>>(w, in_q);
         cudaEventRecordWithFlags(e[2], stream, cudaEventRecordExternal);
@@ -823,8 +862,7 @@ struct WfRun {
             k_shade<false, SHADE_ALL><<<grid_shade, cfg.block, 0, stream>>>(w, in_q, 0);
         }
         cudaEventRecordWithFlags(e[3], stream, cudaEventRecordExternal);
-        if (cfg.wide) k_shadow<true><<<grid_shadow, cfg.block, stack_smem, stream>>>(w);
-        else k_shadow<false><<<grid_shadow, cfg.block, stack_smem, stream>>>(w);
+        shadow_kernel(cfg)<<<grid_shadow, cfg.block, stack_smem, stream>>>(w);
         cudaEventRecordWithFlags(e[4], stream, cudaEventRecordExternal);
     }
 
@@ -1001,7 +1039,7 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
                 c.pool = pools[pi];
                 c.block = blocks[bi];
                 c.sort = so;
-                c.wide = wide_for(items);
+                tree_for(items, &c);
                 WfRun run;
                 e = run.init(c, (int)items.size(), s);
                 if (e == cudaSuccess)
@@ -1033,11 +1071,11 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
 // Engines (pool buffers, captured graph, events, sample buffer) are cached per
 // (context, configuration) and reused by later calls; aur_ctx_destroy releases them.
 static std::mutex g_engine_mutex;
-static std::map<std::tuple<aur_ctx*, uint32_t, int, int, int, int>, std::unique_ptr<WfRun>> g_engines;
+static std::map<std::tuple<aur_ctx*, uint32_t, int, int, int, int, int>, std::unique_ptr<WfRun>> g_engines;
 
 static WfRun* engine_for(aur_ctx* ctx, const WfConfig& cfg, int nscenes, cudaError_t* err) {
     std::lock_guard<std::mutex> lock(g_engine_mutex);
-    const auto key = std::make_tuple(ctx, cfg.pool, cfg.block, cfg.sort, cfg.record, cfg.wide);
+    const auto key = std::make_tuple(ctx, cfg.pool, cfg.block, cfg.sort, cfg.record, cfg.tree, cfg.tree_any);
     auto it = g_engines.find(key);
     if (it != g_engines.end() && it->second->cap_scenes >= nscenes) return it->second.get();
     if (it != g_engines.end()) { it->second->release(); g_engines.erase(it); }
@@ -1051,7 +1089,7 @@ static WfRun* engine_for(aur_ctx* ctx, const WfConfig& cfg, int nscenes, cudaErr
 
 static void wf_drop_engine(aur_ctx* ctx, const WfConfig& cfg) {
     std::lock_guard<std::mutex> lock(g_engine_mutex);
-    auto it = g_engines.find(std::make_tuple(ctx, cfg.pool, cfg.block, cfg.sort, cfg.record, cfg.wide));
+    auto it = g_engines.find(std::make_tuple(ctx, cfg.pool, cfg.block, cfg.sort, cfg.record, cfg.tree, cfg.tree_any));
     if (it != g_engines.end()) { it->second->release(); g_engines.erase(it); }
 }
 
@@ -1063,11 +1101,15 @@ void wf_release_context(aur_ctx* ctx) {
     }
 }
 
-static int wide_for(const std::vector<BatchItem>& items) {
-    if (!AUR_WIDE_TRAVERSAL) return 0;
-    for (const BatchItem& it : items)
-        if (!it.scene->bvh.bvh.nodes4) return 0;
-    return 1;
+static void tree_for(const std::vector<BatchItem>& items, WfConfig* cfg) {
+    int largest = 0;
+    cfg->tree = cfg->tree_any = TREE_BINARY;
+    for (const BatchItem& it : items) {
+        if (!AUR_WIDE_TRAVERSAL || !it.scene->bvh.bvh.nodes4) return;
+        largest = std::max(largest, it.scene->bvh.bvh.num_nodes4);
+    }
+    cfg->tree = largest >= kQuantMinNodes4 ? TREE_QUANT : TREE_WIDE;
+    cfg->tree_any = largest >= kQuantMinNodes4Any ? TREE_QUANT : TREE_WIDE;
 }
 
 // Renders a batch of scenes with the wavefront engine. films[i]: device float4[npix].
@@ -1075,7 +1117,7 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
                                   std::vector<float4*>& films, aur_render_stats* stats, float* kernel_ms) {
     const int n = (int)items.size();
     WfConfig cfg = cfg_in;
-    cfg.wide = wide_for(items);
+    tree_for(items, &cfg);
     // The engine runs on the context's own non-blocking stream (graph capture is not
     // allowed on the legacy default stream), ordered after the caller's stream.
     cudaStream_t s = ctx->work_stream;
@@ -1168,7 +1210,7 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
         stats->wf_pool = (int32_t)cfg.pool;
         stats->wf_block = cfg.block;
         stats->wf_sort = cfg.sort;
-        stats->node_bytes = cfg.wide ? (int32_t)sizeof(BvhNode4) : (int32_t)sizeof(BvhNode);
+        stats->node_bytes = (int32_t)(cfg.tree == TREE_QUANT ? sizeof(BvhNode4Q) : cfg.tree == TREE_WIDE ? sizeof(BvhNode4) : sizeof(BvhNode));
     }
     return AUR_OK;
 }
@@ -1185,7 +1227,7 @@ aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsampl
     cfg.record = 1;
     std::vector<BatchItem> items(1);
     items[0] = {sc, p, (uint32_t)sc->cam.w * (uint32_t)sc->cam.h, nullptr, nullptr};
-    cfg.wide = wide_for(items);
+    tree_for(items, &cfg);
     cudaStream_t s = ctx->work_stream;
     cudaEventRecord(ctx->ev_order, ctx->stream);
     cudaStreamWaitEvent(s, ctx->ev_order, 0);

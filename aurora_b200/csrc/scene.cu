@@ -123,6 +123,7 @@ DevScene aur_scene::dev() const {
     d.nodes = bvh.bvh.nodes;
     d.tris = bvh.bvh.tris;
     d.nodes4 = bvh.bvh.nodes4;
+    d.nodes4q = bvh.bvh.nodes4q;
     d.sh.mats = mats;
     d.sh.attrs = attrs;
     d.sh.lights = lights;
@@ -427,7 +428,10 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
-    cudaError_t e = launch_render_plain(sc->dev(), p, f32, d64, sc->ctx->counters, o->count_work != 0, s);
+    // the counting pass walks the tree that the wavefront renderer's closest-hit rays do
+    const DeviceBvh& tree = sc->bvh.bvh;
+    const int count_width = !o->count_work ? 0 : !tree.nodes4 ? 2 : tree.num_nodes4 >= kQuantMinNodes4 ? 8 : 4;
+    cudaError_t e = launch_render_plain(sc->dev(), p, f32, d64, sc->ctx->counters, count_width, s);
     cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = f64 ? fo64.finish() : fo.finish();
     unsigned long long cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -451,7 +455,8 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
         stats->shadow_tri_tests = cnt[7];
         stats->launches = 1;
         stats->kernel_ms = ms;
-        stats->node_bytes = o->count_work && sc->bvh.bvh.nodes4 ? (int32_t)sizeof(BvhNode4) : (int32_t)sizeof(BvhNode);
+        stats->node_bytes = (int32_t)(count_width == 4 ? sizeof(BvhNode4) : count_width == 8 ? sizeof(BvhNode4Q)
+                                                                                             : sizeof(BvhNode));
     }
     return AUR_OK;
 }
