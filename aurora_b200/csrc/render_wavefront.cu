@@ -5,13 +5,14 @@
 // a pool of P path slots lives in HBM (structure of arrays) and every
 // iteration runs one bounce of every live path as separate stages:
 //
-//   regen   finished slots write their sample and take the next work item
-//           (scene, pixel, sample) from a global counter -> camera ray
+//   regen   the slots that the shading stage listed: next-event radiance is added, finished
+//           slots write their sample and take the next work item (scene, pixel, sample)
+//           from a global counter -> camera ray
 //   extend  closest hit for the extension queue (persistent warps, traversal only)
 //   sort    optional: counting sort of the hits by material type
 //   shade   emission, lobe choice, next-event rays + their contributions, BRDF
 //           continuation, throughput and roulette -> next extension queue
-//   shadow  occlusion for the next-event rays, Lo += direct * T
+//   shadow  occlusion for the next-event rays
 //
 // Queue appends and work fetches are aggregated per block (one atomic per block). Many scenes of
 // different resolution, spp and depth share one pool (batched launch). The
@@ -21,6 +22,8 @@
 // produce the same film for the same seed.
 #include "aur_capi_internal.h"
 #include <algorithm>
+#include <climits>
+#include <cstddef>
 #include <cstring>
 #include <map>
 #include <memory>
@@ -31,7 +34,9 @@
 namespace aur {
 namespace {
 
-enum : uint32_t { PS_EMPTY = 0, PS_ACTIVE = 1, PS_DONE = 2, PS_MASK = 3, PS_PENDING = 4 };
+// What regen has to do for a slot, alone or above the slot's number (below 2^26).
+constexpr uint32_t kPending = 1u << 31;   // next-event rays in flight: their radiance is to be added
+constexpr uint32_t kDone = 1u << 30;      // the path is finished: write its sample, take new work
 // lane refill: a warp takes new rays once this many lanes are idle, and runs kRounds
 // traversal rounds (interior phase + leaf phase) between refill checks
 // (swept on the quantised 4-wide tree, 1080p terrain frame, closest + any hit: rounds 3 / 4 / 5 at
@@ -46,7 +51,18 @@ enum : int { B_MISS = 0, B_MATTE = 1, B_KELEMEN = 2, B_CT = 3, B_METAL = 4, B_CO
 // counters
 enum : int {
     C_EXT0 = 0, C_EXT1 = 1, C_SHADOW = 2, C_WORK = 3, C_TOTAL = 4, C_CUR_EXT = 5, C_CUR_SHADE = 6,
-    C_CUR_SHADOW = 7, C_CUR_SORT = 8, C_CUR_SHADE2 = 9, C_BUCKET = 16, C_FILL = 24, kCounters = 32
+    C_CUR_SHADOW = 7, C_CUR_SORT = 8, C_CUR_SHADE2 = 9, C_LIST = 10, C_FRESH = 11, C_SCENES = 12,
+    C_BUCKET = 16, C_FILL = 24, kCounters = 32
+};
+// What a pass keeps beside the queues; copied to the host in one piece.
+struct WfState {
+    uint32_t ctr[kCounters];
+    int32_t stage;                    // the stage that is running (-1: none yet)
+    int32_t pad;
+    unsigned long long stamp;         // when it began
+    // summed over the passes of a render:
+    unsigned long long rays[2];       // closest-hit rays, any-hit rays
+    unsigned long long stage_ns[5];   // device time of regen, extend, sort, shade, shadow
 };
 
 struct WfScene {
@@ -61,6 +77,9 @@ struct WfScene {
     // has one path only (renderer.cpp:231-258): its sub-samples j > 0 are skipped.
     uint32_t lsub, rng_offset;
     float4* samples;       // [spp_pass * lsub][npix]
+    // resolve: the film and, for renders of several passes, the sums between them
+    float4 *film, *acc_s, *acc_c;
+    int32_t total_spp, first_pass, last_pass;
     // record mode (path-replay adjoint): per item (sample-major, sl * npix + pixel)
     float4* rec;           // [items][rec_depth] hit records (t, u, v, prim | visibility << 30)
     float4* lo_raw;        // [items] unclamped path radiance, w = number of recorded vertices
@@ -78,15 +97,14 @@ struct WfScene {
 //   neeC   first next-event contribution, throughput + nvis            (regen)
 struct WfPool {
     float4 *ray, *hitid, *tplo, *neeA, *neeB, *neeC;   // [P][2] each
-    uint32_t* state;            // PS_* in the low bits, PS_PENDING when next-event rays are in flight
+    uint32_t* q_regen;          // what regen has to do: by slot (sweep), or a list of the slots (see k_regen)
     uint32_t* sh_vis;           // bit k: next-event ray k of the slot is unoccluded
     uint32_t* rec_cur;          // record mode: record index of the vertex whose next-event rays are in flight
     uint8_t* bucket;            // material bucket of the slot's last hit (written by the sorting extend)
     uint32_t *q_ext0, *q_ext1, *q_sort, *q_shadow;
-    uint32_t* ctr;
-    unsigned long long* rays;   // [0] closest-hit rays, [1] shadow rays
+    uint32_t* ctr;              // WfState::ctr
+    WfState* st;
     const WfScene* scenes;
-    int nscenes;                // table capacity; unused entries start at item UINT32_MAX
     uint32_t P;
     __device__ __forceinline__ float4& ray_o(uint32_t i) const { return ray[2 * (size_t)i]; }
     __device__ __forceinline__ float4& ray_d(uint32_t i) const { return ray[2 * (size_t)i + 1]; }
@@ -116,29 +134,42 @@ __device__ __forceinline__ bool f_matte(uint32_t f) { return (f >> 20) & 1; }
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << lane_id()) - 1u; }
 
-// Block-aggregated append to up to three queues: every thread of the block calls it
-// (uniform control flow) with its flags; it returns each flagged thread's slot in the
-// queue. One atomic per queue per block instead of one per warp.
-struct BlockScan { uint32_t cnt[16][3]; uint32_t base[3]; };
-__device__ __forceinline__ void block_reserve(BlockScan& sh, const bool (&p)[3], uint32_t* const (&ctr)[3],
-                                              uint32_t (&pos)[3]) {
+// Block 0's first thread charges the time since the previous stage began to that stage: two
+// timer reads and a few stores a launch, where event records between the launches cost every
+// graph as many nodes again.
+__device__ __forceinline__ void stage_begins(const WfPool& w, int stage) {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    unsigned long long now;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
+    if (w.st->stage >= 0) w.st->stage_ns[w.st->stage] += now - w.st->stamp;
+    w.st->stamp = now;
+    w.st->stage = stage;
+}
+
+// Block-aggregated append to kQ queues: every thread of the block calls it (uniform control
+// flow) with its flags; it returns each flagged thread's slot in the queue. One atomic per
+// queue per block instead of one per warp.
+struct BlockScan { uint32_t cnt[16][4]; uint32_t base[4]; };
+template <int kQ>
+__device__ __forceinline__ void block_reserve(BlockScan& sh, const bool (&p)[kQ], uint32_t* const (&ctr)[kQ],
+                                              uint32_t (&pos)[kQ]) {
     const int warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint32_t m[3];
+    uint32_t m[kQ];
 #pragma unroll
-    for (int q = 0; q < 3; ++q) m[q] = __ballot_sync(0xffffffffu, p[q]);
+    for (int q = 0; q < kQ; ++q) m[q] = __ballot_sync(0xffffffffu, p[q]);
     if (lane_id() == 0)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) sh.cnt[warp][q] = __popc(m[q]);
+        for (int q = 0; q < kQ; ++q) sh.cnt[warp][q] = __popc(m[q]);
     __syncthreads();
-    if (threadIdx.x < 3) {
+    if (threadIdx.x < kQ) {
         const int q = threadIdx.x;
         uint32_t t = 0;
         for (int j = 0; j < nw; ++j) { const uint32_t c = sh.cnt[j][q]; sh.cnt[j][q] = t; t += c; }
-        sh.base[q] = (t && ctr[q]) ? atomicAdd(ctr[q], t) : 0u;
+        sh.base[q] = t ? atomicAdd(ctr[q], t) : 0u;
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 3; ++q) pos[q] = sh.base[q] + sh.cnt[warp][q] + __popc(m[q] & lanemask_lt());
+    for (int q = 0; q < kQ; ++q) pos[q] = sh.base[q] + sh.cnt[warp][q] + __popc(m[q] & lanemask_lt());
     __syncthreads();   // sh is reused by the next call
 }
 
@@ -147,13 +178,14 @@ __device__ __forceinline__ uint32_t rng_index(const WfScene& S, uint32_t q) { re
 __device__ __forceinline__ uint32_t cam_index(const WfScene& S, uint32_t q) {
     return S.lsub > 1 ? S.rng_offset + q - q % S.lsub : S.rng_offset + q;
 }
-// sub-samples j > 0 of the render's sample 0 trace nothing (one path in the first pass)
-__device__ __forceinline__ bool skipped_sub(const WfScene& S, uint32_t q) {
-    return S.lsub > 1 && q % S.lsub != 0 && (uint32_t)S.p.sample_offset + q / S.lsub == 0;
+// The k-th sub-sample that a pass traces per pixel: all of them, but for the render's sample 0,
+// which has one path (its sub-samples j > 0 are no work items).
+__device__ __forceinline__ uint32_t sub_sample(const WfScene& S, uint32_t k) {
+    return S.p.sample_offset == 0 && k > 0 ? k + S.lsub - 1 : k;
 }
 
 __device__ __forceinline__ int scene_of(const WfPool& w, uint32_t item) {
-    int lo = 0, hi = w.nscenes - 1;
+    int lo = 0, hi = (int)w.ctr[C_SCENES] - 1;
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (w.scenes[mid].item_base <= item) lo = mid; else hi = mid - 1;
@@ -162,79 +194,82 @@ __device__ __forceinline__ int scene_of(const WfPool& w, uint32_t item) {
 }
 
 // ------------------------------------------------------------------ regen
-template <bool kRec>
+// Slots that the last shading stage left something to do for (next-event radiance to add, or a
+// finished path); in a pass's first iteration (C_FRESH) as many unused slots as there is work.
+// Two ways to find them. kSweep: every slot's flags are read in slot order, and the records of
+// those that have work. Otherwise the shading stage appends them to a list. A pass whose paths
+// all fit the pool takes the list, where nothing is refilled and ever fewer slots are left: the
+// 512 x 512 sphere frame's regen 3.0 -> 1.2 ms of 14.4. One that refills its slots takes the
+// sweep, which hands consecutive pixels to consecutive slots; the list hands them out in the
+// shading stage's order, and on the 1080p terrain frame the pool's gathers lost what locality
+// they had (regen 13.6 -> 30.5, shade 51.7 -> 62.8 ms).
+template <bool kRec, bool kSweep>
 __global__ void k_regen(WfPool w, int in_q) {
     __shared__ BlockScan s_scan;
+    stage_begins(w, 0);
     uint32_t* qin = in_q ? w.q_ext1 : w.q_ext0;
     uint32_t* cin = &w.ctr[in_q ? C_EXT1 : C_EXT0];
     const uint32_t total = w.ctr[C_TOTAL];
+    const bool fresh = w.ctr[C_FRESH] != 0;
+    const uint32_t n = fresh ? (total < w.P ? total : w.P) : kSweep ? w.P : w.ctr[C_LIST];
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t base = blockIdx.x * blockDim.x; base < w.P; base += stride) {
-        const uint32_t i = base + threadIdx.x;
-        const bool valid = i < w.P;
-        uint32_t st = PS_ACTIVE, vis = 0;
-        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), t = lo, c0 = lo;
-        uint4 id = make_uint4(0, 0, 0, 0);
-        if (valid) {
-            // the slot's records are loaded together, before its state says which of them it
-            // uses, so that their latencies overlap (c0 and t share one 32-byte pair)
-            st = w.state[i];
-            vis = w.sh_vis[i];
-            t = w.sh_t(i);
-            c0 = w.sh_c0(i);
-            lo = w.lo(i);
-            id = w.id(i);
-        }
-        if (st & PS_PENDING) {
-            // next-event estimate of the last vertex: Lo += ((vis0 c0 + vis1 c1) nvis) T, the
-            // plain kernel's order of operations (integrate_direct)
-            const float nvis = t.w;   // the number of visible lights rides in the throughput record
-            float3 res = mk(0.f, 0.f, 0.f);
-            if (vis & 1u) res += mk(c0.x, c0.y, c0.z);   // only unoccluded contributions are added
-            if (vis & 2u) { const float4 c1 = w.sh_c1(i); res += mk(c1.x, c1.y, c1.z); }
-            const float3 add = (res * nvis) * mk(t.x, t.y, t.z);
-            lo.x += add.x; lo.y += add.y; lo.z += add.z;
-            w.lo(i) = lo;
-            st &= ~PS_PENDING;
-            if (kRec) {   // the visibility of the vertex's next-event rays goes into its record
-                float4* r = w.scenes[id.x].rec + w.rec_cur[i];
-                r->w = __int_as_float(__float_as_int(r->w) | (int)(vis << 30));
+    for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += stride) {
+        const uint32_t k = base + threadIdx.x;
+        bool want = false;
+        uint32_t i = k;
+        if (fresh) {
+            want = k < n;
+        } else if (const uint32_t e = k < n ? w.q_regen[k] : 0u) {
+            if (kSweep) w.q_regen[k] = 0u;
+            else i = e & (kDone - 1);
+            // the slot's records are loaded together, so that their latencies overlap (c0 and t
+            // share one 32-byte pair)
+            float4 lo = w.lo(i);
+            const uint4 id = w.id(i);
+            if (e & kPending) {
+                // next-event estimate of the last vertex: Lo += ((vis0 c0 + vis1 c1) nvis) T, the
+                // plain kernel's order of operations (integrate_direct)
+                const uint32_t vis = w.sh_vis[i];
+                const float4 t = w.sh_t(i), c0 = w.sh_c0(i);
+                const float nvis = t.w;   // the number of visible lights rides in the throughput record
+                float3 res = mk(0.f, 0.f, 0.f);
+                if (vis & 1u) res += mk(c0.x, c0.y, c0.z);   // only unoccluded contributions are added
+                if (vis & 2u) { const float4 c1 = w.sh_c1(i); res += mk(c1.x, c1.y, c1.z); }
+                const float3 add = (res * nvis) * mk(t.x, t.y, t.z);
+                lo.x += add.x; lo.y += add.y; lo.z += add.z;
+                if (!(e & kDone)) w.lo(i) = lo;
+                if (kRec) {   // the visibility of the vertex's next-event rays goes into its record
+                    float4* r = w.scenes[id.x].rec + w.rec_cur[i];
+                    r->w = __int_as_float(__float_as_int(r->w) | (int)(vis << 30));
+                }
+            }
+            if (e & kDone) {
+                const WfScene& S = w.scenes[id.x];
+                if (kRec) {
+                    S.lo_raw[(size_t)id.z * S.npix + id.y] = make_float4(lo.x, lo.y, lo.z, __int_as_float(f_vtx(id.w)));
+                } else {
+                    const float3 L = (id.w & kNoClamp) ? mk(lo.x, lo.y, lo.z) : firefly_clamp(mk(lo.x, lo.y, lo.z));
+                    // with light samples, alpha 2 marks the environment seen by the camera ray: the
+                    // sample is that radiance, not the mean of its sub-samples (integrator.cpp:287-298)
+                    const float a = (S.lsub > 1 && (id.w & kNoClamp)) ? 2.f : lo.w;
+                    S.samples[(size_t)id.z * S.npix + id.y] = make_float4(L.x, L.y, L.z, a);
+                }
+                want = *(volatile uint32_t*)&w.ctr[C_WORK] < total;
             }
         }
-        if (st == PS_DONE) {
-            const WfScene& S = w.scenes[id.x];
-            if (kRec) {
-                S.lo_raw[(size_t)id.z * S.npix + id.y] = make_float4(lo.x, lo.y, lo.z, __int_as_float(f_vtx(id.w)));
-            } else {
-                const float3 L = (id.w & kNoClamp) ? mk(lo.x, lo.y, lo.z) : firefly_clamp(mk(lo.x, lo.y, lo.z));
-                // with light samples, alpha 2 marks the environment seen by the camera ray: the
-                // sample is that radiance, not the mean of its sub-samples (integrator.cpp:287-298)
-                const float a = (S.lsub > 1 && (id.w & kNoClamp)) ? 2.f : lo.w;
-                S.samples[(size_t)id.z * S.npix + id.y] = make_float4(L.x, L.y, L.z, a);
-            }
-            st = PS_EMPTY;
-        }
-        const bool want = st == PS_EMPTY && *(volatile uint32_t*)&w.ctr[C_WORK] < total;
-        uint32_t item = 0xffffffffu;
+        uint32_t pos[1];
         {
-            const bool pw[3] = {want, false, false};
-            uint32_t* const cw[3] = {&w.ctr[C_WORK], nullptr, nullptr};
-            uint32_t pos[3];
+            const bool pw[1] = {want};
+            uint32_t* const cw[1] = {&w.ctr[C_WORK]};
             block_reserve(s_scan, pw, cw, pos);
-            if (want) item = pos[0];
         }
-        bool start = want && item < total;
-        int s = 0;
-        uint32_t pixel = 0, q = 0;
+        const uint32_t item = pos[0];
+        const bool start = want && item < total;
         if (start) {
-            s = scene_of(w, item);
-            const uint32_t local = item - w.scenes[s].item_base;
-            pixel = local % w.scenes[s].npix;
-            q = local / w.scenes[s].npix;
-            start = !skipped_sub(w.scenes[s], q);
-        }
-        if (start) {
+            const int s = scene_of(w, item);
             const WfScene& S = w.scenes[s];
+            const uint32_t local = item - S.item_base;
+            const uint32_t pixel = local % S.npix, q = sub_sample(S, local / S.npix);
             PathRng rng;
             rng.key = S.key;
             rng.base = path_base(pixel, cam_index(S, q));
@@ -245,16 +280,13 @@ __global__ void k_regen(WfPool w, int in_q) {
             w.tp(i) = make_float4(1.f, 1.f, 1.f, 1.f);
             w.lo(i) = make_float4(0.f, 0.f, 0.f, 0.f);
             w.id(i) = make_uint4((uint32_t)s, pixel, q, pack_flags(0, 0, RAY_CAMERA, false));
-            st = PS_ACTIVE;
         }
         {
-            const bool pp[3] = {start, false, false};
-            uint32_t* const cp[3] = {cin, nullptr, nullptr};
-            uint32_t pos[3];
+            const bool pp[1] = {start};
+            uint32_t* const cp[1] = {cin};
             block_reserve(s_scan, pp, cp, pos);
             if (start) qin[pos[0]] = i;
         }
-        if (valid) w.state[i] = st;
     }
 }
 
@@ -299,14 +331,17 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
     // Outputs of the later stages start empty. Only counters that no block of
     // this kernel touches are reset here; the bucket counters this kernel
     // increments were reset by the previous next-event stage (or the pass start).
+    stage_begins(w, 1);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
+        w.ctr[C_LIST] = 0;
+        w.ctr[C_FRESH] = 0;
         w.ctr[in_q ? C_EXT0 : C_EXT1] = 0;
         w.ctr[C_SHADOW] = 0;
         w.ctr[C_CUR_SHADE] = 0;
         w.ctr[C_CUR_SHADE2] = 0;
         w.ctr[C_CUR_SHADOW] = 0;
         w.ctr[C_CUR_SORT] = 0;
-        w.rays[0] += n;
+        w.st->rays[0] += n;
     }
     extern __shared__ int s_stack[];
     __shared__ uint32_t s_bucket[kBuckets];   // per-block material counts, added to the global ones at exit
@@ -398,6 +433,7 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
 
 // counting-sort scatter of the extension queue into q_sort, grouped by bucket
 __global__ void k_sort_scatter(WfPool w, int in_q) {
+    stage_begins(w, 2);
     const uint32_t* qin = in_q ? w.q_ext1 : w.q_ext0;
     const uint32_t n = w.ctr[in_q ? C_EXT1 : C_EXT0];
     __shared__ uint32_t s_ofs[kBuckets], s_cnt[kBuckets], s_base[kBuckets];
@@ -468,7 +504,8 @@ enum : int { SHADE_ALL = 0, SHADE_MATTE = 1, SHADE_REST = 2 };
 #define AUR_SHADE_MATTE_MINB 4
 #endif
 template <bool kRec, int kPart>
-__global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MINB : 3) k_shade(WfPool w, int in_q, int sorted) {
+__global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MINB : 3) k_shade(WfPool w, int in_q, int sorted,
+                                                                                                 bool sweep) {
     const uint32_t* qin = sorted ? w.q_sort : (in_q ? w.q_ext1 : w.q_ext0);
     const uint32_t n_all = w.ctr[in_q ? C_EXT1 : C_EXT0];
     // the sorted queue holds the misses first, then the matte bucket
@@ -479,13 +516,14 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
     uint32_t* cout = &w.ctr[in_q ? C_EXT0 : C_EXT1];
     __shared__ BlockScan s_scan;
     __shared__ uint32_t s_fetch;
+    if (kPart != SHADE_REST) stage_begins(w, 3);
     while (true) {
         if (threadIdx.x == 0) s_fetch = atomicAdd(&w.ctr[kPart == SHADE_MATTE ? C_CUR_SHADE2 : C_CUR_SHADE], blockDim.x);
         __syncthreads();
         const uint32_t b = s_fetch;   // rewritten only after block_reserve's barriers below
         if (b >= n) break;
         const uint32_t k = b + threadIdx.x;
-        bool push_ext = false, push_sh0 = false, push_sh1 = false;
+        bool push_ext = false, push_sh0 = false, push_sh1 = false, done = false;
         uint32_t slot = 0;
         if (k < n) {
             slot = qin[kPart == SHADE_ALL ? k : kPart == SHADE_MATTE ? nmiss + k : (k < nmiss ? k : k + nm)];
@@ -498,10 +536,10 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                 const int kind = f_kind(id.w), vtx = f_vtx(id.w);
                 if (S.sc.sh.nenv && (vtx == 0 || kind == RAY_MIRROR))
                     lo = shade_env_miss(&w, &S, slot, id, vtx, lo);
-                w.state[slot] = PS_DONE;
+                done = true;
             } else if (f_vtx(w.id(slot).w) >= w.scenes[w.id(slot).x].p.max_depth) {
                 // the reference's unshaded last ray hit something: the path ends
-                w.state[slot] = PS_DONE;
+                done = true;
             } else {
                 const uint4 id = w.id(slot);
                 const WfScene& S = w.scenes[id.x];
@@ -603,19 +641,22 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                 lo = make_float4(Lo.x, Lo.y, Lo.z, lo.w);
                 // a finished path's flags count its recorded vertices (a missed ray's vertex is not recorded)
                 if (kRec && !alive) w.id(slot).w = pack_flags(vtx + 1, bounces, kind, matte);
-                w.state[slot] = (alive ? PS_ACTIVE : PS_DONE) | (push_sh0 || push_sh1 ? PS_PENDING : 0u);
+                done = !alive;
                 push_ext = alive;
             }
             w.lo(slot) = lo;
         }
         {
-            const bool pp[3] = {push_ext, push_sh0, push_sh1};
-            uint32_t* const cp[3] = {cout, &w.ctr[C_SHADOW], &w.ctr[C_SHADOW]};
-            uint32_t pos[3];
+            const bool nee = push_sh0 || push_sh1;
+            const uint32_t todo = (done ? kDone : 0u) | (nee ? kPending : 0u);
+            const bool pp[4] = {push_ext, push_sh0, push_sh1, todo && !sweep};
+            uint32_t* const cp[4] = {cout, &w.ctr[C_SHADOW], &w.ctr[C_SHADOW], &w.ctr[C_LIST]};
+            uint32_t pos[4];
             block_reserve(s_scan, pp, cp, pos);
             if (push_ext) qout[pos[0]] = slot;
             if (push_sh0) w.q_shadow[pos[1]] = slot << 1;
             if (push_sh1) w.q_shadow[pos[2]] = (slot << 1) | 1u;
+            if (todo) w.q_regen[sweep ? slot : pos[3]] = sweep ? todo : slot | todo;
         }
     }
 }
@@ -627,8 +668,9 @@ template <int kTree>
 __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
     using Tree = TreeTypes<kTree, true>;
     const uint32_t n = w.ctr[C_SHADOW];
+    stage_begins(w, 4);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        w.rays[1] += n;
+        w.st->rays[1] += n;
         // extend, scatter and shade are finished: reset their fetch and bucket counters
         w.ctr[C_CUR_EXT] = 0;
         for (int k = 0; k < kBuckets; ++k) { w.ctr[C_BUCKET + k] = 0; w.ctr[C_FILL + k] = 0; }
@@ -678,58 +720,65 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
 }
 
 // ------------------------------------------------------------------ resolve
-// Adds this pass's samples of every pixel, in sample order, to the per-pixel
-// compensated sums (the plain kernel's accumulation order).
-__global__ void k_resolve(const WfScene* scenes, int s, float4* acc_s, float4* acc_c) {
-    const WfScene& S = scenes[s];
-    const uint32_t pixel = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pixel >= S.npix) return;
-    const float4 a = acc_s[pixel], c = acc_c[pixel];
-    Kahan3 k;
-    k.s = mk(a.x, a.y, a.z);
-    k.c = mk(c.x, c.y, c.z);
-    float alpha = a.w;
-    if (S.lsub <= 1) {
-        for (int j = 0; j < S.p.spp; ++j) {
-            const float4 v = S.samples[(size_t)j * S.npix + pixel];
-            k.add(mk(v.x, v.y, v.z));
-            alpha += v.w;
+// Adds this pass's samples of every pixel of every scene (blockIdx.y), in sample order, to the
+// pixel's compensated sum (the plain kernel's accumulation order), and after a scene's last pass
+// writes its film. A render of one pass keeps no sums in memory.
+__global__ void k_resolve(const WfScene* scenes) {
+    const WfScene& S = scenes[blockIdx.y];
+    if (S.p.spp == 0) return;
+    for (uint32_t pixel = blockIdx.x * blockDim.x + threadIdx.x; pixel < S.npix; pixel += gridDim.x * blockDim.x) {
+        Kahan3 k;
+        k.init();
+        float alpha = 0.f;
+        if (!S.first_pass) {
+            const float4 a = S.acc_s[pixel], c = S.acc_c[pixel];
+            k.s = mk(a.x, a.y, a.z);
+            k.c = mk(c.x, c.y, c.z);
+            alpha = a.w;
         }
-    } else {
-        // a camera sample with light samples is the mean of its n sub-samples, added in their
-        // order as Lo / n (integrate_camera_sample); n = 1 for the render's sample 0
-        for (int sl = 0; sl < S.p.spp; ++sl) {
-            const float4* sub = S.samples + (size_t)sl * S.lsub * S.npix + pixel;
-            const float4 v0 = sub[0];
-            if (v0.w == 2.f) {               // the camera ray saw the environment
-                k.add(mk(v0.x, v0.y, v0.z));
-                alpha += 1.f;
-                continue;
+        if (S.lsub <= 1) {
+            const float4* v = S.samples + pixel;
+            const int n = S.p.spp;
+            const size_t step = S.npix;
+#pragma unroll 8
+            for (int j = 0; j < n; ++j) {
+                const float4 x = __ldg(v + j * step);
+                k.add(mk(x.x, x.y, x.z));
+                alpha += x.w;
             }
-            const int n = S.p.sample_offset + sl == 0 ? 1 : (int)S.lsub;
-            float3 sum = mk(v0.x, v0.y, v0.z);
-            if (n > 1) {
-                sum = cdiv(sum, (float)n);
-                for (int j = 1; j < n; ++j) {
-                    const float4 v = sub[(size_t)j * S.npix];
-                    sum += cdiv(mk(v.x, v.y, v.z), (float)n);
+        } else {
+            // a camera sample with light samples is the mean of its n sub-samples, added in their
+            // order as Lo / n (integrate_camera_sample); n = 1 for the render's sample 0
+            for (int sl = 0; sl < S.p.spp; ++sl) {
+                const float4* sub = S.samples + (size_t)sl * S.lsub * S.npix + pixel;
+                const float4 v0 = sub[0];
+                if (v0.w == 2.f) {               // the camera ray saw the environment
+                    k.add(mk(v0.x, v0.y, v0.z));
+                    alpha += 1.f;
+                    continue;
                 }
+                const int n = S.p.sample_offset + sl == 0 ? 1 : (int)S.lsub;
+                float3 sum = mk(v0.x, v0.y, v0.z);
+                if (n > 1) {
+                    sum = cdiv(sum, (float)n);
+                    for (int j = 1; j < n; ++j) {
+                        const float4 v = sub[(size_t)j * S.npix];
+                        sum += cdiv(mk(v.x, v.y, v.z), (float)n);
+                    }
+                }
+                k.add(sum);
+                alpha += v0.w;
             }
-            k.add(sum);
-            alpha += v0.w;
+        }
+        if (S.last_pass) {
+            const float inv = 1.f / (float)S.total_spp;
+            const float3 t = k.total();
+            S.film[pixel] = make_float4(t.x * inv, t.y * inv, t.z * inv, alpha * inv);
+        } else {
+            S.acc_s[pixel] = make_float4(k.s.x, k.s.y, k.s.z, alpha);
+            S.acc_c[pixel] = make_float4(k.c.x, k.c.y, k.c.z, 0.f);
         }
     }
-    acc_s[pixel] = make_float4(k.s.x, k.s.y, k.s.z, alpha);
-    acc_c[pixel] = make_float4(k.c.x, k.c.y, k.c.z, 0.f);
-}
-
-__global__ void k_finish(const float4* acc_s, const float4* acc_c, uint32_t npix, int spp, float4* film) {
-    const uint32_t pixel = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pixel >= npix) return;
-    const float inv = 1.f / (float)spp;
-    const float4 a = acc_s[pixel], c = acc_c[pixel];
-    const float3 t = mk(a.x, a.y, a.z) + mk(c.x, c.y, c.z);
-    film[pixel] = make_float4(t.x * inv, t.y * inv, t.z * inv, a.w * inv);
 }
 
 }  // namespace
@@ -763,7 +812,7 @@ static auto shadow_kernel(const WfConfig& c) -> void (*)(WfPool) {
 
 // ------------------------------------------------------------------ host driver
 struct WfRun {
-    // one wavefront engine: pool buffers + a captured graph of kItersPerGraph iterations
+    // one wavefront engine: pool buffers + captured graphs of 1 to kItersPerGraph iterations
     WfConfig cfg;
     WfPool w{};
     void* mem = nullptr;
@@ -773,30 +822,34 @@ struct WfRun {
     size_t samples_bytes = 0;
     float4* acc = nullptr;                     // per-pixel compensated sums, grown on demand
     size_t acc_bytes = 0;
-    cudaGraphExec_t exec = nullptr;
     cudaStream_t stream = nullptr;
     int grid_regen = 0, grid_ext = 0, grid_shade = 0, grid_shade_m = 0, grid_shade_r = 0, grid_shadow = 0, grid_sort = 0;
     size_t stack_smem = 0;                     // shared traversal stack of one block
-    uint32_t* h_ctr = nullptr;   // pinned
+    WfState* h_state = nullptr;                // pinned: [0] as read back, [1] as uploaded
+    WfScene* h_scenes = nullptr;               // pinned scene table
     static constexpr int kItersPerGraph = 8;
     static constexpr int kStages = 5;          // regen, extend, sort, shade, shadow
-    cudaEvent_t ev[kItersPerGraph * kStages + 1] = {};
-    int launches_per_graph = 0;
-    double stage_ms[kStages] = {0, 0, 0, 0, 0};
+    cudaEvent_t e0 = nullptr, e1 = nullptr;    // around a whole render
+    // by iterations and kind of pass: one that refills its slots, one that fits the pool, and one of
+    // at most kSmallPass paths, whose launches need few blocks
+    enum Kind : int { REFILL = 0, FITS = 1, SMALL = 2 };
+    cudaGraphExec_t exec[kItersPerGraph + 1][3] = {};
+    static constexpr uint32_t kSmallPass = 1u << 18;
+
+    int launches_per_iteration() const { return cfg.sort ? 6 : 4; }
 
     cudaError_t init(const WfConfig& c, int nscenes, cudaStream_t s) {
         cfg = c;
         stream = s;
         const size_t P = c.pool;
-        const size_t bytes = P * (12 * sizeof(float4) + 8 * sizeof(uint32_t) + 1) + 21 * 256 +
-                             kCounters * sizeof(uint32_t) + 2 * sizeof(unsigned long long);
+        const size_t bytes = P * (12 * sizeof(float4) + 8 * sizeof(uint32_t) + 1) + 21 * 256 + sizeof(WfState);
         cudaError_t e = cudaMalloc(&mem, bytes);
         if (e != cudaSuccess) return e;
         char* p = (char*)mem;
         auto take = [&](size_t n) { char* r = p; p += (n + 255) & ~(size_t)255; return (void*)r; };
         float4** pairs[] = {&w.ray, &w.hitid, &w.tplo, &w.neeA, &w.neeB, &w.neeC};
         for (float4** q : pairs) *q = (float4*)take(2 * P * sizeof(float4));
-        w.state = (uint32_t*)take(P * 4);
+        w.q_regen = (uint32_t*)take(P * 4);
         w.q_ext0 = (uint32_t*)take(P * 4);
         w.q_ext1 = (uint32_t*)take(P * 4);
         w.q_sort = (uint32_t*)take(P * 4);
@@ -804,18 +857,19 @@ struct WfRun {
         w.sh_vis = (uint32_t*)take(P * 4);
         w.rec_cur = (uint32_t*)take(P * 4);
         w.bucket = (uint8_t*)take(P);
-        w.ctr = (uint32_t*)take(kCounters * 4);
-        w.rays = (unsigned long long*)take(2 * sizeof(unsigned long long));
+        w.st = (WfState*)take(sizeof(WfState));
+        w.ctr = w.st->ctr;
         if ((size_t)(p - (char*)mem) > bytes) return cudaErrorMemoryAllocation;
         cap_scenes = std::max(nscenes, 64);
         e = cudaMalloc(&d_scenes, sizeof(WfScene) * cap_scenes);
         if (e != cudaSuccess) return e;
         w.scenes = d_scenes;
-        w.nscenes = cap_scenes;
         w.P = (uint32_t)P;
-        e = cudaMallocHost(&h_ctr, kCounters * 4);
+        e = cudaMallocHost(&h_state, 2 * sizeof(WfState));
+        if (e == cudaSuccess) e = cudaMallocHost(&h_scenes, sizeof(WfScene) * cap_scenes);
+        if (e == cudaSuccess) e = cudaEventCreate(&e0);
+        if (e == cudaSuccess) e = cudaEventCreate(&e1);
         if (e != cudaSuccess) return e;
-        for (auto& x : ev) if ((e = cudaEventCreate(&x)) != cudaSuccess) return e;
         int dev = 0, sms = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -831,86 +885,113 @@ struct WfRun {
         grid_shade_r = persist(c.record ? (const void*)k_shade<true, SHADE_REST> : (const void*)k_shade<false, SHADE_REST>, 0);
         grid_shadow = persist((const void*)shadow_kernel(c), stack_smem);
         grid_sort = persist((const void*)k_sort_scatter, 0);
-        // 64 blocks per SM (about 10 resident waves of the 40-register kernel): 14.8 ms per
-        // 1080p frame against 15.3 at 16 and 16.5 at exactly the resident 6
         grid_regen = (int)std::min<size_t>((P + c.block - 1) / c.block, (size_t)sms * 64);
         return cudaSuccess;
     }
 
-    // One iteration; an event after every stage so the graph reports per-stage device time.
-    void enqueue_iteration(int in_q, int it) {
-        // inside stream capture only an "external" record becomes an event-record node
-        cudaEvent_t* e = &ev[it * kStages + 1];
-        if (cfg.record) k_regen<true><<<grid_regen, cfg.block, 0, stream>>>(w, in_q);
-        else k_regen<false><<<grid_regen, cfg.block, 0, stream>>>(w, in_q);
-        cudaEventRecordWithFlags(e[0], stream, cudaEventRecordExternal);
-        extend_kernel(cfg)<<<grid_ext, cfg.block, stack_smem, stream>>>(w, in_q);
-        cudaEventRecordWithFlags(e[1], stream, cudaEventRecordExternal);
-        if (cfg.sort) k_sort_scatter<<<grid_sort, cfg.block, 0, stream>>>(w, in_q);
-        cudaEventRecordWithFlags(e[2], stream, cudaEventRecordExternal);
-        if (cfg.sort) {   // the matte bucket, then the others
-            if (cfg.record) {
-                k_shade<true, SHADE_MATTE><<<grid_shade_m, cfg.block, 0, stream>>>(w, in_q, 1);
-                k_shade<true, SHADE_REST><<<grid_shade_r, cfg.block, 0, stream>>>(w, in_q, 1);
-            } else {
-                k_shade<false, SHADE_MATTE><<<grid_shade_m, cfg.block, 0, stream>>>(w, in_q, 1);
-                k_shade<false, SHADE_REST><<<grid_shade_r, cfg.block, 0, stream>>>(w, in_q, 1);
-            }
-        } else if (cfg.record) {
-            k_shade<true, SHADE_ALL><<<grid_shade, cfg.block, 0, stream>>>(w, in_q, 0);
-        } else {
-            k_shade<false, SHADE_ALL><<<grid_shade, cfg.block, 0, stream>>>(w, in_q, 0);
-        }
-        cudaEventRecordWithFlags(e[3], stream, cudaEventRecordExternal);
-        shadow_kernel(cfg)<<<grid_shadow, cfg.block, stack_smem, stream>>>(w);
-        cudaEventRecordWithFlags(e[4], stream, cudaEventRecordExternal);
+    Kind kind_of(uint32_t total) const { return total > w.P ? REFILL : total > kSmallPass ? FITS : SMALL; }
+
+    void regen(int in_q, Kind kind) {
+        const int grid = kind == SMALL ? std::min(grid_regen, (int)(kSmallPass / 4 / cfg.block)) : grid_regen;
+        auto kern = kind == REFILL ? (cfg.record ? k_regen<true, true> : k_regen<false, true>)
+                                   : (cfg.record ? k_regen<true, false> : k_regen<false, false>);
+        kern<<<grid, cfg.block, 0, stream>>>(w, in_q);
     }
 
-    cudaError_t build_graph() {
-        cudaGraph_t g;
-        cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
-        if (e != cudaSuccess) return e;
-        cudaEventRecordWithFlags(ev[0], stream, cudaEventRecordExternal);
-        for (int it = 0; it < kItersPerGraph; ++it) enqueue_iteration(it & 1, it);
-        e = cudaStreamEndCapture(stream, &g);
-        if (e != cudaSuccess) return e;
-        e = cudaGraphInstantiate(&exec, g, 0);
-        cudaGraphDestroy(g);
-        launches_per_graph = kItersPerGraph * (cfg.sort ? 6 : 4);
+    void enqueue_iteration(int in_q, Kind kind) {
+        const int cap = kind == SMALL ? (int)(kSmallPass / cfg.block) : INT_MAX;
+        const bool sweep = kind == REFILL;
+        regen(in_q, kind);
+        extend_kernel(cfg)<<<std::min(grid_ext, cap), cfg.block, stack_smem, stream>>>(w, in_q);
+        if (cfg.sort) {   // the matte bucket, then the others
+            k_sort_scatter<<<std::min(grid_sort, cap), cfg.block, 0, stream>>>(w, in_q);
+            auto matte = cfg.record ? k_shade<true, SHADE_MATTE> : k_shade<false, SHADE_MATTE>;
+            auto rest = cfg.record ? k_shade<true, SHADE_REST> : k_shade<false, SHADE_REST>;
+            matte<<<std::min(grid_shade_m, cap), cfg.block, 0, stream>>>(w, in_q, 1, sweep);
+            rest<<<std::min(grid_shade_r, cap), cfg.block, 0, stream>>>(w, in_q, 1, sweep);
+        } else {
+            auto all = cfg.record ? k_shade<true, SHADE_ALL> : k_shade<false, SHADE_ALL>;
+            all<<<std::min(grid_shade, cap), cfg.block, 0, stream>>>(w, in_q, 0, sweep);
+        }
+        shadow_kernel(cfg)<<<std::min(grid_shadow, cap), cfg.block, stack_smem, stream>>>(w);
+    }
+
+    cudaError_t launch_graph(int iters, Kind kind) {
+        cudaGraphExec_t& x = exec[iters][kind];
+        if (!x) {
+            cudaGraph_t g;
+            cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+            if (e != cudaSuccess) return e;
+            for (int it = 0; it < iters; ++it) enqueue_iteration(it & 1, kind);
+            e = cudaStreamEndCapture(stream, &g);
+            if (e != cudaSuccess) return e;
+            e = cudaGraphInstantiate(&x, g, 0);
+            cudaGraphDestroy(g);
+            if (e != cudaSuccess) { x = nullptr; return e; }
+        }
+        return cudaGraphLaunch(x, stream);
+    }
+
+    // Uploads the first n entries of h_scenes and the pass's counters; `reset` also clears what a
+    // render sums over its passes.
+    cudaError_t begin_pass(uint32_t total, int n, bool reset) {
+        WfState& h = h_state[1];
+        memset(&h, 0, sizeof(h));
+        h.ctr[C_TOTAL] = total;
+        h.ctr[C_FRESH] = 1;
+        h.ctr[C_SCENES] = (uint32_t)n;
+        h.stage = -1;
+        cudaError_t e = cudaMemcpyAsync(d_scenes, h_scenes, sizeof(WfScene) * n, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(w.st, &h, reset ? sizeof(WfState) : offsetof(WfState, rays), cudaMemcpyHostToDevice, stream);
+        // the sweep reads every slot's flags: none set from a pass before
+        if (e == cudaSuccess && kind_of(total) == REFILL) e = cudaMemsetAsync(w.q_regen, 0, (size_t)w.P * 4, stream);
         return e;
     }
+    cudaError_t read_state() {
+        return cudaMemcpyAsync(&h_state[0], w.st, sizeof(WfState), cudaMemcpyDeviceToHost, stream);
+    }
 
-    // Runs one pass over `total` work items of the uploaded scene table.
-    cudaError_t run_pass(uint32_t total, uint64_t* launches) {
-        cudaError_t e = cudaMemsetAsync(w.ctr, 0, kCounters * 4, stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(w.state, 0, (size_t)w.P * 4, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&w.ctr[C_TOTAL], &total, 4, cudaMemcpyHostToDevice, stream);
-        if (e != cudaSuccess) return e;
-        if (!exec && (e = build_graph()) != cudaSuccess) return e;
-        // Bound on graph launches: each launch advances every live path by 8 bounces
-        // and refills the pool, so a pass needs about total / P * depth / 8 launches.
-        const uint64_t max_launches = (uint64_t)total * 64ull / ((uint64_t)w.P) + 4096ull;
-        for (uint64_t it = 0; it < max_launches; ++it) {
-            e = cudaGraphLaunch(exec, stream);
+    // Runs one pass over `total` work items of the uploaded scene table, whose paths have at most
+    // `depth` rays. A pass that fits the pool starts all its paths in its first iteration and is
+    // done after `depth` of them: one graph of that many, nothing to wait for. A larger one runs
+    // graphs of kItersPerGraph iterations and reads the counters between them. The stream is not
+    // synchronised at the end; drained() tells after that, and after read_state(), whether the
+    // pass finished.
+    cudaError_t run_pass(uint32_t total, int depth, uint64_t* launches) {
+        const Kind kind = kind_of(total);
+        cudaError_t e = cudaSuccess;
+        if (kind != REFILL && depth <= kItersPerGraph) {   // as graph_iters
+            e = launch_graph(depth, kind);
             if (e != cudaSuccess) return e;
-            *launches += launches_per_graph;
-            e = cudaMemcpyAsync(h_ctr, w.ctr, 8 * 4, cudaMemcpyDeviceToHost, stream);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-            if (e != cudaSuccess) return e;
-            for (int k = 0; k < kItersPerGraph * kStages; ++k) {
-                float ms = 0.f;
-                if (cudaEventElapsedTime(&ms, ev[k], ev[k + 1]) == cudaSuccess) stage_ms[k % kStages] += ms;
-                else cudaGetLastError();   // timing is informational; never leave a stale error behind
+            *launches += depth * launches_per_iteration();
+        } else {
+            // Bound on graph launches: each launch advances every live path by 8 bounces
+            // and refills the pool, so a pass needs about total / P * depth / 8 launches.
+            const uint64_t max_launches = (uint64_t)total * 64ull / ((uint64_t)w.P) + 4096ull;
+            bool done = false;
+            for (uint64_t it = 0; it < max_launches && !done; ++it) {
+                e = launch_graph(kItersPerGraph, kind);
+                if (e == cudaSuccess) e = read_state();
+                if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+                if (e != cudaSuccess) return e;
+                *launches += kItersPerGraph * launches_per_iteration();
+                done = drained(total, kItersPerGraph);
             }
-            if (h_ctr[C_WORK] >= total && h_ctr[C_EXT0] == 0) {
-                // writes the last finished samples
-                if (cfg.record) k_regen<true><<<grid_regen, cfg.block, 0, stream>>>(w, 0);
-                else k_regen<false><<<grid_regen, cfg.block, 0, stream>>>(w, 0);
-                *launches += 1;
-                return cudaGetLastError();
-            }
+            if (!done) return cudaErrorLaunchTimeout;
         }
-        return cudaErrorLaunchTimeout;
+        regen(0, kind);   // writes the last finished samples
+        *launches += 1;
+        return cudaGetLastError();
+    }
+    // By the counters as last read, after `iters` iterations of the last graph: no work left and
+    // no ray in the queue that the next iteration would take.
+    bool drained(uint32_t total, int iters) const {
+        const uint32_t* c = h_state[0].ctr;
+        return c[C_WORK] >= total && c[iters & 1 ? C_EXT1 : C_EXT0] == 0;
+    }
+    int graph_iters(uint32_t total, int depth) const {
+        return total <= w.P && depth <= kItersPerGraph ? depth : kItersPerGraph;
     }
 
     cudaError_t ensure_samples(size_t bytes) {
@@ -937,16 +1018,18 @@ struct WfRun {
         if (acc) cudaFree(acc);
         acc = nullptr;
         acc_bytes = 0;
-        if (exec) cudaGraphExecDestroy(exec);
+        for (auto& row : exec)
+            for (auto& x : row) { if (x) cudaGraphExecDestroy(x); x = nullptr; }
         if (mem) cudaFree(mem);
         if (d_scenes) cudaFree(d_scenes);
         if (samples) cudaFree(samples);
         samples = nullptr;
         samples_bytes = 0;
-        if (h_ctr) cudaFreeHost(h_ctr);
-        for (auto& x : ev) if (x) cudaEventDestroy(x);
-        exec = nullptr; mem = nullptr; d_scenes = nullptr; h_ctr = nullptr;
-        for (auto& x : ev) x = nullptr;
+        if (h_state) cudaFreeHost(h_state);
+        if (h_scenes) cudaFreeHost(h_scenes);
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+        mem = nullptr; d_scenes = nullptr; h_state = nullptr; h_scenes = nullptr; e0 = e1 = nullptr;
     }
 };
 
@@ -954,41 +1037,59 @@ struct BatchItem {
     aur_scene* scene;
     PathParams p;
     uint32_t npix;
+    float4* film;
     float4* acc_s;
     float4* acc_c;
     uint32_t lsub() const { return p.light_samples > 1 ? (uint32_t)p.light_samples : 1u; }
-    // work items (one per traced or skipped sub-sample) of one camera sample of every pixel
+    // sub-samples of one camera sample of every pixel (the sample buffer's unit)
     uint64_t items_per_sample() const { return (uint64_t)npix * lsub(); }
-    // paths traced for spp samples from sample_offset (the render's sample 0 traces one)
+    // paths traced for spp samples from sample_offset (the render's sample 0 traces one): the
+    // work items of a pass
     uint64_t paths(int spp, int offset) const {
         return (uint64_t)npix * ((uint64_t)spp * lsub() - (offset == 0 && spp > 0 ? lsub() - 1 : 0));
     }
+    // rays on the longest path: one per vertex, and with an environment light the one after the last
+    int depth() const {
+        int rays = p.max_depth;
+        for (const Light& l : scene->h_lights) if (l.type == LIGHT_ENV) return rays + 1;
+        return rays;
+    }
 };
+static int max_rays(const std::vector<BatchItem>& items) {
+    int d = 1;
+    for (const BatchItem& it : items) d = std::max(d, it.depth());
+    return d;
+}
 
-// Fills the scene table of one pass: samples [s0, s0 + chunk) of every scene.
-static uint32_t fill_table(std::vector<BatchItem>& items, int s0, int chunk, float4* samples, std::vector<WfScene>& tab,
-                           int capacity) {
+// Fills the scene table of one pass: samples [s0, s0 + chunk) of every scene. Returns the
+// number of work items.
+static uint32_t fill_table(std::vector<BatchItem>& items, int s0, int chunk, float4* samples, WfScene* tab) {
     uint32_t base = 0;
     size_t off = 0;
-    tab.assign(capacity, WfScene());
-    for (int i = (int)items.size(); i < capacity; ++i) tab[i].item_base = 0xffffffffu;   // never selected
     for (size_t i = 0; i < items.size(); ++i) {
         WfScene& t = tab[i];
+        const BatchItem& it = items[i];
         memset(&t, 0, sizeof(t));
-        t.sc = items[i].scene->dev();
-        t.p = items[i].p;
-        const int pass_spp = std::max(0, std::min(chunk, items[i].p.spp - s0));
+        t.sc = it.scene->dev();
+        t.p = it.p;
+        const int pass_spp = std::max(0, std::min(chunk, it.p.spp - s0));
         t.p.spp = pass_spp;
-        t.p.sample_offset = items[i].p.sample_offset + s0;
-        t.key = seed_key(items[i].p.seed);
-        t.npix = items[i].npix;
-        t.lsub = items[i].lsub();
+        t.p.sample_offset = it.p.sample_offset + s0;
+        t.key = seed_key(it.p.seed);
+        t.npix = it.npix;
+        t.lsub = it.lsub();
         t.rng_offset = (uint32_t)t.p.sample_offset * t.lsub;
         t.item_base = base;
-        t.items = (uint32_t)(items[i].items_per_sample() * (uint32_t)pass_spp);
+        t.items = (uint32_t)it.paths(pass_spp, t.p.sample_offset);
         t.samples = samples ? samples + off : nullptr;
+        t.film = it.film;
+        t.acc_s = it.acc_s;
+        t.acc_c = it.acc_c;
+        t.total_spp = it.p.spp;
+        t.first_pass = s0 == 0;
+        t.last_pass = s0 + pass_spp >= it.p.spp;
         base += t.items;
-        off += (size_t)items[i].items_per_sample() * chunk;
+        off += (size_t)it.items_per_sample() * chunk;
     }
     return base;
 }
@@ -1007,7 +1108,7 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
         per_sample += (size_t)it.items_per_sample() * sizeof(float4);
         total += it.items_per_sample() * it.p.spp;
     }
-    const uint32_t limit = (uint32_t)std::min<uint64_t>(total, 1ull << 25);
+    uint32_t limit = (uint32_t)std::min<uint64_t>(total, 1ull << 25);
     int chunk = 1;   // samples buffer large enough for the probe's first `limit` items
     {
         uint64_t covered = 0;
@@ -1020,8 +1121,9 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
     float4* samples = nullptr;
     cudaError_t e = cudaMallocAsync(&samples, per_sample * chunk, s);
     if (e != cudaSuccess) return cuda_fail(e, "wavefront autotune");
-    std::vector<WfScene> tab;
-    fill_table(items, 0, chunk, samples, tab, std::max((int)items.size(), 64));
+    std::vector<WfScene> tab(items.size());
+    limit = std::min(limit, fill_table(items, 0, chunk, samples, tab.data()));
+    const int depth = max_rays(items), n = (int)items.size();
     constexpr int kPools = 5;
     const uint32_t pools[kPools] = {1u << 20, 1u << 21, 1u << 22, 1u << 23, 1u << 24};
     const int blocks[2] = {128, 256};
@@ -1030,7 +1132,6 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    bool warmed = false;
     for (int pi = 0; pi < kPools && e == cudaSuccess; ++pi) {
         if (pi > 0 && (uint64_t)pools[pi] > 2ull * limit) break;   // a pool that would stay mostly empty
         for (int bi = 0; bi < 2 && e == cudaSuccess; ++bi)
@@ -1042,14 +1143,19 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
                 tree_for(items, &c);
                 WfRun run;
                 e = run.init(c, (int)items.size(), s);
-                if (e == cudaSuccess)
-                    e = cudaMemcpyAsync(run.d_scenes, tab.data(), sizeof(WfScene) * tab.size(), cudaMemcpyHostToDevice, s);
+                if (e == cudaSuccess) memcpy(run.h_scenes, tab.data(), sizeof(WfScene) * n);
+                // a short probe runs twice: the first pass also builds its graph
                 uint64_t l = 0;
-                if (e == cudaSuccess && !warmed) { e = run.run_pass(std::min<uint32_t>(limit, 1u << 20), &l); warmed = true; }
-                cudaEventRecord(e0, s);
-                if (e == cudaSuccess) e = run.run_pass(limit, &l);
-                cudaEventRecord(e1, s);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+                auto pass = [&](uint32_t items_in_pass) {
+                    cudaError_t pe = run.begin_pass(items_in_pass, n, true);
+                    if (pe == cudaSuccess) pe = cudaEventRecord(e0, s);
+                    if (pe == cudaSuccess) pe = run.run_pass(items_in_pass, depth, &l);
+                    if (pe == cudaSuccess) pe = cudaEventRecord(e1, s);
+                    const cudaError_t se = cudaStreamSynchronize(s);
+                    return pe != cudaSuccess ? pe : se;
+                };
+                if (e == cudaSuccess && limit <= (1u << 22)) e = pass(limit);
+                if (e == cudaSuccess) e = pass(limit);
                 float ms = 0.f;
                 if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
                 run.release();
@@ -1112,9 +1218,9 @@ static void tree_for(const std::vector<BatchItem>& items, WfConfig* cfg) {
     cfg->tree_any = largest >= kQuantMinNodes4Any ? TREE_QUANT : TREE_WIDE;
 }
 
-// Renders a batch of scenes with the wavefront engine. films[i]: device float4[npix].
+// Renders a batch of scenes with the wavefront engine into items[i].film (device float4[npix]).
 static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, const WfConfig& cfg_in,
-                                  std::vector<float4*>& films, aur_render_stats* stats, float* kernel_ms) {
+                                  aur_render_stats* stats) {
     const int n = (int)items.size();
     WfConfig cfg = cfg_in;
     tree_for(items, &cfg);
@@ -1131,17 +1237,18 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
     const size_t budget = (size_t)3 << 30;
     size_t per_sample = 0;
     int max_spp = 0;
+    uint32_t max_pix = 0;
     for (auto& it : items) {
         per_sample += (size_t)it.items_per_sample() * sizeof(float4);
         max_spp = std::max(max_spp, it.p.spp);
+        max_pix = std::max(max_pix, it.npix);
     }
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)max_spp, budget / std::max<size_t>(per_sample, 1)));
     e = run.ensure_samples(per_sample * chunk);
-    float4* samples = run.samples;
-    size_t per_pixel_set = 0;
-    for (auto& it : items) per_pixel_set += (size_t)it.npix * sizeof(float4);
-    if (e == cudaSuccess) e = run.ensure_acc(2 * per_pixel_set);   // two float4 per pixel
-    {
+    if (chunk < max_spp) {   // several passes: two float4 sums per pixel between them
+        size_t pixels = 0;
+        for (auto& it : items) pixels += it.npix;
+        if (e == cudaSuccess) e = run.ensure_acc(2 * pixels * sizeof(float4));
         size_t off = 0;
         for (auto& it : items) {
             it.acc_s = run.acc + off;
@@ -1149,54 +1256,38 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
             off += 2 * (size_t)it.npix;
         }
     }
-    for (auto& it : items) {
-        if (e == cudaSuccess) e = cudaMemsetAsync(it.acc_s, 0, sizeof(float4) * it.npix, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(it.acc_c, 0, sizeof(float4) * it.npix, s);
-    }
-    if (e == cudaSuccess) e = cudaMemsetAsync(run.w.rays, 0, 2 * sizeof(unsigned long long), s);
-    for (double& x : run.stage_ms) x = 0.0;
     if (e != cudaSuccess) return cuda_fail(e, "wavefront: sample buffers");
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, s);
+    const int depth = max_rays(items);
     uint64_t launches = 0;
-    std::vector<WfScene> tab;
+    cudaEventRecord(run.e0, s);
     for (int s0 = 0; s0 < max_spp && e == cudaSuccess; s0 += chunk) {
-        const uint32_t total = fill_table(items, s0, chunk, samples, tab, run.cap_scenes);
-        e = cudaMemcpyAsync(run.d_scenes, tab.data(), sizeof(WfScene) * run.cap_scenes, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = run.run_pass(total, &launches);
-        for (int i = 0; i < n && e == cudaSuccess; ++i) {
-            if (tab[i].p.spp == 0) continue;
-            k_resolve<<<(items[i].npix + 255) / 256, 256, 0, s>>>(run.d_scenes, i, items[i].acc_s, items[i].acc_c);
+        const uint32_t total = fill_table(items, s0, chunk, run.samples, run.h_scenes);
+        e = run.begin_pass(total, n, s0 == 0);
+        if (e == cudaSuccess) e = run.run_pass(total, depth, &launches);
+        if (e != cudaSuccess) break;
+        for (int i = 0; i < n; i += 65535) {
+            const dim3 grid((unsigned)std::min<uint32_t>((max_pix + 255) / 256, 1u << 20), (unsigned)std::min(n - i, 65535));
+            k_resolve<<<grid, 256, 0, s>>>(run.d_scenes + i);
             ++launches;
-            e = cudaGetLastError();
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // the scene table is rewritten next pass
-    }
-    for (int i = 0; i < n && e == cudaSuccess; ++i) {
-        k_finish<<<(items[i].npix + 255) / 256, 256, 0, s>>>(items[i].acc_s, items[i].acc_c, items[i].npix,
-                                                             items[i].p.spp, films[i]);
-        ++launches;
         e = cudaGetLastError();
+        const bool last = s0 + chunk >= max_spp;
+        if (e == cudaSuccess && last) e = cudaEventRecord(run.e1, s);
+        if (e == cudaSuccess) e = run.read_state();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // the scene table is rewritten next pass
+        if (e == cudaSuccess && !run.drained(total, run.graph_iters(total, depth))) e = cudaErrorLaunchTimeout;
     }
-    cudaEventRecord(e1, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     float ms = 0.f;
-    if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    unsigned long long rays[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(rays, run.w.rays, sizeof(rays), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) cudaEventElapsedTime(&ms, run.e0, run.e1);
+    const WfState& hs = run.h_state[0];
+    const unsigned long long rays[2] = {hs.rays[0], hs.rays[1]};
     cudaEventRecord(ctx->ev_order, s);              // the caller's stream continues after this work
     cudaStreamWaitEvent(ctx->stream, ctx->ev_order, 0);
     double stage[WfRun::kStages];
-    for (int k = 0; k < WfRun::kStages; ++k) stage[k] = run.stage_ms[k];
+    for (int k = 0; k < WfRun::kStages; ++k) stage[k] = 1e-6 * (double)hs.stage_ns[k];
     if (e != cudaSuccess) wf_drop_engine(ctx, cfg);   // never reuse an engine left in an unknown state
     if (e == cudaErrorLaunchTimeout) return fail(AUR_ERR_TIMEOUT, "wavefront: the path pool did not drain");
     if (e != cudaSuccess) return cuda_fail(e, "wavefront");
-    *kernel_ms = ms;
     if (stats) {
         uint64_t paths = 0, cams = 0;
         for (auto& it : items) { paths += it.paths(it.p.spp, it.p.sample_offset); cams += (uint64_t)it.npix * it.p.spp; }
@@ -1226,7 +1317,7 @@ aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsampl
     if (sc->wf_tuned) { cfg.pool = (uint32_t)sc->wf_pool; cfg.block = sc->wf_block; cfg.sort = sc->wf_sort; }
     cfg.record = 1;
     std::vector<BatchItem> items(1);
-    items[0] = {sc, p, (uint32_t)sc->cam.w * (uint32_t)sc->cam.h, nullptr, nullptr};
+    items[0] = {sc, p, (uint32_t)sc->cam.w * (uint32_t)sc->cam.h, nullptr, nullptr, nullptr};
     tree_for(items, &cfg);
     cudaStream_t s = ctx->work_stream;
     cudaEventRecord(ctx->ev_order, ctx->stream);
@@ -1235,18 +1326,16 @@ aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsampl
     WfRun* engine = engine_for(ctx, cfg, 1, &e);
     if (!engine) return cuda_fail(e, "adjoint record pass: pool allocation");
     WfRun& run = *engine;
-    std::vector<WfScene> tab;
-    const uint32_t total = fill_table(items, s0, nsamples, nullptr, tab, run.cap_scenes);
-    tab[0].rec = rec;
-    tab[0].lo_raw = lo_raw;
-    tab[0].rec_depth = (uint32_t)p.max_depth;
-    e = cudaMemsetAsync(run.w.rays, 0, 2 * sizeof(unsigned long long), s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(run.d_scenes, tab.data(), sizeof(WfScene) * run.cap_scenes, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = run.run_pass(total, launches);
-    unsigned long long r[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(r, run.w.rays, sizeof(r), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // the host table and counters are read back
+    const uint32_t total = fill_table(items, s0, nsamples, nullptr, run.h_scenes);
+    run.h_scenes[0].rec = rec;
+    run.h_scenes[0].lo_raw = lo_raw;
+    run.h_scenes[0].rec_depth = (uint32_t)p.max_depth;
+    e = run.begin_pass(total, 1, true);
+    if (e == cudaSuccess) e = run.run_pass(total, max_rays(items), launches);
+    if (e == cudaSuccess) e = run.read_state();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // the host table and counters are reused
+    if (e == cudaSuccess && !run.drained(total, run.graph_iters(total, max_rays(items)))) e = cudaErrorLaunchTimeout;
+    const unsigned long long r[2] = {run.h_state[0].rays[0], run.h_state[0].rays[1]};
     cudaEventRecord(ctx->ev_order, s);
     cudaStreamWaitEvent(ctx->stream, ctx->ev_order, 0);
     if (e != cudaSuccess) wf_drop_engine(ctx, cfg);
@@ -1293,7 +1382,7 @@ aur_status render_wavefront(aur_scene* sc, const aur_render_opts* o, float* film
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);   // film staging allocated on the caller's stream
     if (e != cudaSuccess) return cuda_fail(e, "aur_render(wavefront)");
     std::vector<BatchItem> items(1);
-    items[0] = {sc, p, npix, nullptr, nullptr};
+    items[0] = {sc, p, npix, (float4*)fo.ptr, nullptr, nullptr};
     if (wants_tuning(o)) {
         // Tuned once per render shape (triangles, materials, lights, resolution, spp, depths)
         // on this context: a scene rendered at another spp or depth is tuned for that too,
@@ -1313,9 +1402,7 @@ aur_status render_wavefront(aur_scene* sc, const aur_render_opts* o, float* film
         sc->wf_tuned = true;
         cfg.pool = sc->wf_pool; cfg.block = sc->wf_block; cfg.sort = sc->wf_sort;
     }
-    std::vector<float4*> films = {(float4*)fo.ptr};
-    float ms = 0.f;
-    st = wavefront_batch(sc->ctx, items, cfg, films, stats, &ms);
+    st = wavefront_batch(sc->ctx, items, cfg, stats);
     if (st == AUR_OK) {
         e = fo.finish();
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -1342,22 +1429,20 @@ extern "C" aur_status aur_render_batch(aur_scene* const* scenes, const aur_rende
     cudaStream_t s = ctx->stream;
     std::vector<BatchItem> items(n);
     std::vector<DevOut> outs(n);
-    std::vector<float4*> fl(n);
     uint64_t total = 0;
     for (uint32_t i = 0; i < n; ++i) {
         PathParams p;
         if ((st = render_options(scenes[i], &opts[i], &p)) != AUR_OK) return st;
         const uint32_t npix = (uint32_t)scenes[i]->cam.w * scenes[i]->cam.h;
         total += (uint64_t)npix * p.spp * (uint64_t)p.light_samples;
-        items[i] = {scenes[i], p, npix, nullptr, nullptr};
+        items[i] = {scenes[i], p, npix, nullptr, nullptr, nullptr};
     }
     if (total >= (1ull << 31)) return fail(AUR_ERR_INVALID_ARG, "aur_render_batch: more than 2^31 paths");
     cudaError_t e = cudaSuccess;
     for (uint32_t i = 0; i < n && e == cudaSuccess; ++i) {
         e = outs[i].init(films[i], sizeof(float4) * items[i].npix, 16, s);
-        fl[i] = (float4*)outs[i].ptr;
+        items[i].film = (float4*)outs[i].ptr;
     }
-    float ms = 0.f;
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e == cudaSuccess && wants_tuning(&opts[0])) {
         // tuned once per (scene count, path count) on this context
@@ -1370,7 +1455,7 @@ extern "C" aur_status aur_render_batch(aur_scene* const* scenes, const aur_rende
         }
         if (st == AUR_OK) { cfg.pool = (uint32_t)it->second[0]; cfg.block = it->second[1]; cfg.sort = it->second[2]; }
     }
-    if (e == cudaSuccess && st == AUR_OK) st = wavefront_batch(ctx, items, cfg, fl, stats, &ms);
+    if (e == cudaSuccess && st == AUR_OK) st = wavefront_batch(ctx, items, cfg, stats);
     else if (e != cudaSuccess) st = cuda_fail(e, "aur_render_batch");
     for (uint32_t i = 0; i < n && st == AUR_OK; ++i) {
         e = outs[i].finish();
