@@ -21,9 +21,13 @@
 // colour drives Lambert lobes (matte, Kelemen's diffuse lobe); roughness drives
 // Cook-Torrance lobes (Kelemen, Cook-Torrance, metal roughnessA); a diffuse
 // texture receives the diffuse gradient of the texel the lookup used. Gradients
-// are summed in FP32 with TwoSum-compensated atomics (shared, then global).
+// are summed in FP32 with TwoSum-compensated atomics (shared, then global) by the megakernel,
+// in FP64 by the wavefront form, which computes a vertex's derivative factors where the wavefront
+// engine shades it (record mode) instead of shading it again.
 #define AUR_MATH_OUT_OF_LINE 1
 #include "aur_capi_internal.h"
+#include "aur_adjoint.cuh"
+#include <algorithm>
 
 namespace aur {
 namespace {
@@ -31,6 +35,15 @@ namespace {
 constexpr int kAdjBlock = 128;
 constexpr int kAdjMaxDepth = 16;
 constexpr int kAdjMaxMat = 64;
+constexpr size_t kRecBudget = (size_t)4 << 30;   // bytes of vertex records in one record pass
+
+// float4s per vertex record: the three texels of a triplanar diffuse shader take two more
+int record_stride(const aur_scene* sc) {
+    for (const Material& m : sc->h_mats)
+        if ((m.type == MAT_MATTE || m.type == MAT_KELEMEN) && m.diff_tex >= 0 && sc->h_texs[m.diff_tex].tri_scale != 0.f)
+            return kVertexRec + 2;
+    return kVertexRec;
+}
 
 // hit record of one vertex: (t, u, v, prim | visibility of its next-event rays << 30)
 __device__ __forceinline__ float4 pack_rec(const Hit& h, uint32_t vis) {
@@ -58,8 +71,7 @@ __device__ __forceinline__ void two_sum_add(float& sum, float& comp, float x) {
 // Per-thread compensated accumulators of the per-material gradients (diffuse rgb,
 // roughness) of the two most recently touched materials. A pixel's paths mostly revisit
 // the same materials, so the block's shared sums see one flush per eviction instead of
-// one atomic per vertex (the megakernel: 11% faster; the replay kernel, one path per
-// thread, is faster with DirectAcc). Register-resident: slots resolved by selects.
+// one atomic per vertex (11% faster). Register-resident: slots resolved by selects.
 struct MatCache {
     int tag0 = -1, tag1 = -1;
     float s0[4] = {0.f, 0.f, 0.f, 0.f}, c0[4] = {0.f, 0.f, 0.f, 0.f};
@@ -102,43 +114,6 @@ struct MatCache {
     }
 };
 
-// Accumulator that adds every contribution to the block's shared sums at once.
-struct DirectAcc {
-    template <int Q>
-    __device__ __forceinline__ void add(int mat, float x, float* s_g, float* s_c) {
-        if (x != 0.f) comp_add(&s_g[4 * mat + Q], &s_c[4 * mat + Q], x);
-    }
-    __device__ __forceinline__ void add3(int mat, float3 v, float* s_g, float* s_c) {
-        add<0>(mat, v.x, s_g, s_c);
-        add<1>(mat, v.y, s_g, s_c);
-        add<2>(mat, v.z, s_g, s_c);
-    }
-    __device__ __forceinline__ void flush(float*, float*) {}
-};
-
-// ln D derivative w.r.t. roughness r of the Beckmann term, with tan^2(alpha) given
-// and the reference's max(0.001, r^2) floor (eval uses r^2 unfloored).
-__device__ __forceinline__ float dlnD_dr(float r, float tan2, bool floored) {
-    const float r2 = r * r;
-    if (floored && r2 <= 0.001f) return 0.f;
-    return 2.f * tan2 / (r2 * r) - 2.f / r;
-}
-__device__ __forceinline__ float tan2_of(float ndoth) {
-    const float t = xtanf(xacosf(ndoth));
-    return t * t;
-}
-
-// d ln f / d roughness of a Cook-Torrance sample (cookTorrance.cpp:47-99): the sampled
-// half vector is normalize(L + V); a clamped D (>= 1000) or the 0.001 floor on r^2
-// makes the sample's colour independent of roughness.
-__device__ __forceinline__ float sample_dlnD(const Brdf& b, const Frame& f, const BrdfSample& bs) {
-    const float3 H = normalize(bs.dir + f.V);
-    const float ndoth = dot(f.N, H);
-    const float tana = ndoth > 0.999f ? 0.f : xtanf(xacosf(ndoth));
-    if (ct_d(b.rough, ndoth, tana) >= 1000.f) return 0.f;
-    return dlnD_dr(b.rough, tana * tana, true);
-}
-
 // Next-event estimation of one vertex (integrateDirect with integrateDirectLight /
 // integrateDirectMIS). kTrace: traces the shadow rays and records their visibility
 // in *vis; otherwise replays `vis`. With kGrad it also returns dD/dtheta of the lobe's
@@ -178,10 +153,7 @@ __device__ __forceinline__ float3 direct(const DevScene& sc, const Frame& f, con
                     const float w = power_heuristic(ls.pdf, bp);
                     const float3 c0 = cdiv(((ls.color * w) * brdf_eval(brdf, ls.dir, f.V, f.N)) * cost, ls.pdf);
                     res += c0;
-                    if (kGrad) {
-                        const float3 H = normalize(ls.dir + f.V);
-                        dres += c0 * dlnD_dr(brdf.rough, tan2_of(dot(H, f.N)), false);
-                    }
+                    if (kGrad) dres += c0 * eval_dlnD(brdf.rough, f.N, f.V, ls.dir);
                 }
             }
         }
@@ -199,7 +171,7 @@ __device__ __forceinline__ float3 direct(const DevScene& sc, const Frame& f, con
                     const float w = power_heuristic(bs.pdf, lp);
                     const float3 c1 = cdiv(((bs.color * w) * light_eval(sc.sh, L, bs.dir)) * cost, bs.pdf);
                     res += c1;
-                    if (kGrad) dres += c1 * sample_dlnD(brdf, f, bs);
+                    if (kGrad) dres += c1 * sample_dlnD(brdf.rough, f.N, f.V, bs.dir);
                 }
             }
         }
@@ -208,77 +180,11 @@ __device__ __forceinline__ float3 direct(const DevScene& sc, const Frame& f, con
     return res * (float)nvis;
 }
 
-// d A / d roughness of the Kelemen directional-albedo lookup (kelemen_albedo): the
-// lookup is linear in roughness * 31 between the two columns it reads.
-__device__ __forceinline__ float kelemen_dalbedo_dr(const float* table, float costheta, float roughness) {
-    int i = aur_floor(costheta * (kAlbedoCos - 1));
-    int ra = aur_floor(roughness * (kAlbedoRough - 1));
-    int rb = ra + 1 > kAlbedoRough - 1 ? ra + 1 : kAlbedoRough - 1;
-    i = i < 0 ? 0 : (i > kAlbedoCos - 1 ? kAlbedoCos - 1 : i);
-    ra = ra < 0 ? 0 : (ra > kAlbedoRough - 1 ? kAlbedoRough - 1 : ra);
-    rb = rb > kAlbedoRough - 1 ? kAlbedoRough - 1 : rb;
-    const int i1 = i + 1 < kAlbedoCos - 1 ? i + 1 : kAlbedoCos - 1;
-    const float mixc = costheta * (kAlbedoCos - 1) - (float)i;
-    const float resA = (1.f - mixc) * table[i * kAlbedoRough + ra] + mixc * table[i1 * kAlbedoRough + ra];
-    const float resB = (1.f - mixc) * table[i * kAlbedoRough + rb] + mixc * table[i1 * kAlbedoRough + rb];
-    return (resB - resA) * (float)(kAlbedoRough - 1);
-}
-
-// Score-function factor d ln P(chosen lobe) / d roughness of Kelemen's lobe choice
-// (kelemenMaterial.cpp:236-253): P(spec) = min(1, A(cos, r_eff)), P(diffuse) = 1 - A.
-__device__ __forceinline__ float kelemen_score(const ShadeScene& sh, const Material& m, const Frame& f, const Brdf& b,
-                                               bool matte) {
-    float r = m.rough;
-    if (matte) r = caustic_blur(r);
-    float c = dot(f.N, f.V);
-    c = c < 0.f ? 0.f : (c > 1.f ? 1.f : c);
-    const float* table = sh.albedo + (size_t)m.table * (kAlbedoCos * kAlbedoRough);
-    const float A = kelemen_albedo(table, c, r);
-    const float dA = kelemen_dalbedo_dr(table, c, r) * (matte ? (float)(1.0 - 0.2) : 1.f);
-    if (b.lobe == LOBE_SPEC) return A < 1.f && A > 0.f ? dA / A : 0.f;
-    return A < 1.f ? -dA / (1.f - A) : 0.f;
-}
-
-// Which parameter a vertex's lobe depends on.
-struct ParamRef {
-    int kind;        // 0 none, 1 diffuse colour of material `index`, 2 texels `taps`, 3 roughness
-    int index;
-    float dr;        // roughness: d r_eff / d r (caustic blur on matte paths)
-    Taps taps;       // kind 2: texel blocks (3 floats each, index from the texel array start) and
-                     // the weights the shader blends them with (1 for the uv lookup; 0 = unused)
-};
-
-__device__ __forceinline__ ParamRef param_of(const ShadeScene& sh, int mat_id, const Brdf& b, const Frame& f,
-                                             bool matte, float lobe_u) {
-    ParamRef p;
-    p.kind = 0; p.index = 0; p.dr = 0.f;
-    for (int k = 0; k < 3; ++k) { p.taps.idx[k] = 0; p.taps.w[k] = 0.f; }
-    const Material m = sh.mats[mat_id];
-    if (b.lobe == LOBE_MATTE) {
-        if (m.type != MAT_MATTE && m.type != MAT_KELEMEN) return p;
-        if (m.diff_tex >= 0) {
-            const Texture t = sh.texs[m.diff_tex];
-            p.kind = 2;
-            if (t.tri_scale == 0.f) {
-                p.taps.idx[0] = uv_texel_index(t, f.su, f.sv);
-                p.taps.w[0] = 1.f;
-            } else {
-                p.taps = triplanar_taps(sh.attr_c2o + (size_t)f.attr * 16, t, f.P, f.Ng, false);
-            }
-            for (int k = 0; k < 3; ++k) p.taps.idx[k] += t.offset / 3;
-        } else {
-            p.kind = 1;
-            p.index = mat_id;
-        }
-        return p;
-    }
-    if (b.lobe == LOBE_SPEC && m.rough_tex < 0 &&
-        (m.type == MAT_KELEMEN || m.type == MAT_COOKTORRANCE || (m.type == MAT_METAL && lobe_u > m.mix))) {
-        p.kind = 3;
-        p.index = mat_id;
-        p.dr = matte ? (float)(1.0 - 0.2) : 1.f;
-    }
-    return p;
+// The firefly clamp's factor of a path of radiance c (detached).
+__device__ __forceinline__ float firefly_factor(float3 c) {
+    float f = 1.f;
+    for (int k = 0; k < 64 && (c.x > kFirefly || c.y > kFirefly || c.z > kFirefly); ++k) { c *= 0.2f; f *= 0.2f; }
+    return f;
 }
 
 // Pass 2 of one camera path: re-shades the recorded vertices rec[0, nv) (no ray
@@ -286,18 +192,12 @@ __device__ __forceinline__ ParamRef param_of(const ShadeScene& sh, int mat_id, c
 // n paths of a camera sample with light samples). Lo is the path's unclamped radiance
 // from pass 1; cam_rng draws the camera ray (the path's own rng but for light samples,
 // whose paths share their sample's camera ray).
-template <class Acc>
 __device__ __forceinline__ void replay_path(const DevScene& sc, const PathParams& p, int px, int py,
                                             const PathRng& cam_rng, const PathRng& rng, const float4* rec, int nv,
-                                            float3 Lo, float3 delta, Acc& mc, float* s_g, float* s_c, float* g_tex,
+                                            float3 Lo, float3 delta, MatCache& mc, float* s_g, float* s_c, float* g_tex,
                                             float* g_tex_c, RayCounts& rc) {
     if (nv == 0 || !isfinite(Lo.x) || !isfinite(Lo.y) || !isfinite(Lo.z)) return;
-    float clampf = 1.f;             // firefly clamp factor (detached)
-    {
-        float3 c = Lo;
-        for (int k = 0; k < 64 && (c.x > kFirefly || c.y > kFirefly || c.z > kFirefly); ++k) { c *= 0.2f; clampf *= 0.2f; }
-    }
-    const float3 dp = delta * clampf;
+    const float3 dp = delta * firefly_factor(Lo);
     RayF ray = camera_ray(sc.cam, px, py, cam_rng.u(kDimCamera), cam_rng.u(kDimCamera + 1));
     float3 T = mk(1.f, 1.f, 1.f), collected = mk(0.f, 0.f, 0.f);
     float cont = 1.f;
@@ -330,13 +230,13 @@ __device__ __forceinline__ void replay_path(const DevScene& sc, const PathParams
             // the lobe choice depends on roughness: score-function term on the subtree radiance
             const float score = kelemen_score(sc.sh, mat, f, brdf, matte);
             const float3 sub = dp * (D * T + after);
-            mc.template add<3>(at.material, score * (sub.x + sub.y + sub.z), s_g, s_c);
+            mc.add<3>(at.material, score * (sub.x + sub.y + sub.z), s_g, s_c);
         }
         if (cont_ok && pr.kind != 0) {
             const float cosl = dot(f.N, bs.dir);
             w = cdiv(bs.color * cosl, bs.pdf);
             if (pr.kind == 3) {
-                const float g = sample_dlnD(brdf, f, bs);   // dw/w = d ln f
+                const float g = sample_dlnD(brdf.rough, f.N, f.V, bs.dir);   // dw/w = d ln f
                 gcont = after * g;
             } else {
                 const float dw = kInvPiMacro * cosl / bs.pdf;  // d w_c / d diffuse_c
@@ -361,7 +261,7 @@ __device__ __forceinline__ void replay_path(const DevScene& sc, const PathParams
             }
         } else if (pr.kind == 3) {
             const float3 g = dp * (gdir * pr.dr + gcont * pr.dr);
-            mc.template add<3>(pr.index, g.x + g.y + g.z, s_g, s_c);
+            mc.add<3>(pr.index, g.x + g.y + g.z, s_g, s_c);
         }
         // the forward update, identical to pass 1
         if (!continue_path(brdf, bs, f.N, p.min_depth, rng, vtx, T, cont, kind, bounces)) break;
@@ -494,48 +394,94 @@ __global__ void __launch_bounds__(kAdjBlock) k_adjoint(DevScene sc, PathParams p
         for (int k = 0; k < 3; ++k) atomicAdd(&counters[k], v[k]);
 }
 
-// Replay form (pass 2 only): one thread per item of a record pass (sub-sample-major:
-// q * npix + pixel with q = sl * L + j, L = max(1, light_samples), camera sample
-// p.sample_offset + s0 + sl, random-number sample index (p.sample_offset + s0) * L + q).
-// The wavefront engine's record pass wrote the hit records rec[item][p.max_depth] and
-// lo_raw[item]; the sub-samples j > 0 of the render's sample 0 were not traced.
-// 8 resident blocks of 128 threads (64 registers). (A grid-stride loop over a resident
-// grid was 30% slower: the block scheduler already balances 128-thread blocks.)
-__global__ void __launch_bounds__(kAdjBlock, 8) k_adjoint_replay(DevScene sc, PathParams p, int s0, uint32_t items,
-                                                              const float4* __restrict__ rec,
+// Replay form (pass 2 over a record pass): one thread per path walks the vertex records that the
+// wavefront engine's record mode wrote (VertexRec; the derivative factors of a vertex were computed
+// where it was shaded), and needs nothing but the path's radiance to finish them. Items are
+// sub-sample-major: q * npix + pixel with q = sl * L + j, L = max(1, light_samples), camera sample
+// p.sample_offset + s0 + sl; the sub-samples j > 0 of the render's sample 0 were not traced.
+// Re-shading every vertex here instead took 28 of the 62 ms of a 256 x 256, 256 sample texture
+// adjoint, its warps waiting for instructions (28 per issue) of a large body that ran 8 of 32
+// lanes. What is left is bound by the records' 64 B per vertex and the texels' atomics.
+// Sums are in FP64: per thread column of shared memory and then one global add per block for the
+// materials (`cols` columns; threads share one where all of them do not fit), one reduction to the
+// L2 per texel channel.
+__global__ void __launch_bounds__(kAdjBlock) k_adjoint_replay(PathParams p, uint32_t npix, int s0, uint32_t items,
+                                                              const float4* __restrict__ rec, int stride,
                                                               const float4* __restrict__ lo_raw,
-                                                              const float4* __restrict__ dfilm, int nmat, float* g_mat,
-                                                              float* g_mat_c, float* g_tex, float* g_tex_c) {
-    __shared__ float s_g[kAdjMaxMat * 4], s_c[kAdjMaxMat * 4];
-    for (int i = threadIdx.x; i < nmat * 4; i += blockDim.x) { s_g[i] = 0.f; s_c[i] = 0.f; }
+                                                              const float4* __restrict__ dfilm, int nmat, int cols,
+                                                              double* g_mat, double* g_tex) {
+    extern __shared__ double s_acc[];   // [4 nmat][cols]
+    for (int i = threadIdx.x; i < 4 * nmat * cols; i += blockDim.x) s_acc[i] = 0.0;
     __syncthreads();
-    const uint32_t npix = (uint32_t)(sc.cam.w * sc.cam.h);
-    RayCounts rc;
-    DirectAcc mc;
-    const uint32_t item = blockIdx.x * blockDim.x + threadIdx.x;
-    if (item < items) {
-        const uint32_t lsub = p.light_samples > 1 ? (uint32_t)p.light_samples : 1u;
+    double* col = s_acc + threadIdx.x % cols;
+    auto add = [&](int param, float x) {
+        if (x == 0.f) return;
+        if (cols == kAdjBlock) col[(size_t)param * cols] += (double)x;   // the thread's own column
+        else atomicAdd(&col[(size_t)param * cols], (double)x);
+    };
+    const uint32_t lsub = p.light_samples > 1 ? (uint32_t)p.light_samples : 1u;
+    const float inv = 1.f / (float)p.spp;
+    for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item < items; item += gridDim.x * blockDim.x) {
         const uint32_t pixel = item % npix, q = item / npix;
         const uint32_t j = q % lsub, sample = (uint32_t)(p.sample_offset + s0) + q / lsub;
         const uint32_t n = sample == 0 ? 1u : lsub;
-        const float4 df = dfilm[pixel];
-        const float inv = 1.f / (float)p.spp;
+        if (j >= n) continue;
+        const float4 df = dfilm[pixel], lo = lo_raw[item];
+        const int nv = __float_as_int(lo.w);
         float3 delta = mk(df.x * inv, df.y * inv, df.z * inv);
         if (n > 1) delta = delta * (1.f / (float)n);
-        if (j < n && (delta.x != 0.f || delta.y != 0.f || delta.z != 0.f)) {
-            const uint32_t first = (uint32_t)(p.sample_offset + s0) * lsub;
-            PathRng rng, cam_rng;
-            rng.key = cam_rng.key = seed_key(p.seed);
-            rng.base = path_base(pixel, first + q);
-            cam_rng.base = path_base(pixel, first + q - j);
-            const float4 lo = lo_raw[item];
-            replay_path(sc, p, (int)(pixel % (uint32_t)sc.cam.w), (int)(pixel / (uint32_t)sc.cam.w), cam_rng, rng,
-                        rec + (size_t)item * p.max_depth, __float_as_int(lo.w), mk(lo.x, lo.y, lo.z), delta, mc, s_g,
-                        s_c, g_tex, g_tex_c, rc);
+        if (delta.x == 0.f && delta.y == 0.f && delta.z == 0.f) continue;
+        const float3 Lo = mk(lo.x, lo.y, lo.z);
+        if (!isfinite(Lo.x) || !isfinite(Lo.y) || !isfinite(Lo.z)) continue;
+        const float3 dp = delta * firefly_factor(Lo);
+        const float4* r = rec + (size_t)item * p.max_depth * stride;
+        for (int v = 0; v < nv; ++v, r += stride) {
+            const float4 r3 = __ldg(r + 3);
+            const uint32_t meta = __float_as_uint(r3.w);
+            const int kind = (int)(meta & 3u), index = (int)(meta >> 2);
+            if (kind == 0) continue;
+            const float4 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2);
+            const float3 after = Lo - mk(r0.x, r0.y, r0.z);
+            const float3 g = dp * (mk(r1.x, r1.y, r1.z) + after * mk(r3.x, r3.y, r3.z));
+            if (r2.w != 0.f) {   // the lobe choice depends on roughness: score-function term on the subtree radiance
+                const float3 sub = dp * (Lo - mk(r2.x, r2.y, r2.z));
+                add(4 * __float_as_int(r0.w) + 3, r2.w * (sub.x + sub.y + sub.z));
+            }
+            if (kind == 1) {
+                add(4 * index, g.x);
+                add(4 * index + 1, g.y);
+                add(4 * index + 2, g.z);
+            } else if (kind == 3) {
+                add(4 * index + 3, g.x + g.y + g.z);
+            } else {
+                auto tap = [&](int t, float w) {
+                    if (!(w > 0.f)) return;
+                    if (g.x != 0.f) atomicAdd(&g_tex[3 * (size_t)t], (double)(g.x * w));
+                    if (g.y != 0.f) atomicAdd(&g_tex[3 * (size_t)t + 1], (double)(g.y * w));
+                    if (g.z != 0.f) atomicAdd(&g_tex[3 * (size_t)t + 2], (double)(g.z * w));
+                };
+                if (stride == kVertexRec) {
+                    tap(index, 1.f);
+                } else {
+                    const float4 ti = __ldg(r + 4), tw = __ldg(r + 5);
+                    tap(__float_as_int(ti.x), tw.x);
+                    tap(__float_as_int(ti.y), tw.y);
+                    tap(__float_as_int(ti.z), tw.z);
+                }
+            }
         }
     }
-    mc.flush(s_g, s_c);
-    flush_block(s_g, s_c, nmat, g_mat, g_mat_c);
+    __syncthreads();
+    for (int i = threadIdx.x; i < 4 * nmat; i += blockDim.x) {
+        double sum = 0.0;
+        for (int c = 0; c < cols; ++c) sum += s_acc[(size_t)i * cols + (c + i) % cols];
+        if (sum != 0.0) atomicAdd(&g_mat[i], sum);
+    }
+}
+
+__global__ void k_to_float(const double* g, float* out, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = (float)g[i];
 }
 
 __global__ void k_add_comp(float* g, const float* c, int n) {
@@ -571,16 +517,22 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
     const int ntex = (int)sc->ntexel_floats;
     DevIn din;
     DevOut gm, gt;
-    float *cm = nullptr, *ct = nullptr;
+    // the sums beside the outputs: compensation terms (megakernel) or the FP64 sums themselves
+    const int nsum = 4 * nmat + ntex;
+    const size_t sum_bytes = (wavefront ? sizeof(double) : sizeof(float)) * nsum;
+    void* sums = nullptr;
     cudaError_t e = din.init(dfilm, sizeof(float4) * npix, 16, s);
     if (e == cudaSuccess) e = gm.init(grad_mat, sizeof(float) * 4 * nmat, 4, s);
     if (e == cudaSuccess && ntex) e = gt.init(grad_tex, sizeof(float) * ntex, 4, s);
-    if (e == cudaSuccess) e = cudaMallocAsync(&cm, sizeof(float) * (4 * nmat + ntex), s);
-    ct = cm ? cm + 4 * nmat : nullptr;
-    if (e == cudaSuccess) e = cudaMemsetAsync(gm.ptr, 0, sizeof(float) * 4 * nmat, s);
-    if (e == cudaSuccess && ntex) e = cudaMemsetAsync(gt.ptr, 0, sizeof(float) * ntex, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cm, 0, sizeof(float) * (4 * nmat + ntex), s);
+    if (e == cudaSuccess) e = cudaMallocAsync(&sums, sum_bytes, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(sums, 0, sum_bytes, s);
+    if (e == cudaSuccess && !wavefront) e = cudaMemsetAsync(gm.ptr, 0, sizeof(float) * 4 * nmat, s);
+    if (e == cudaSuccess && !wavefront && ntex) e = cudaMemsetAsync(gt.ptr, 0, sizeof(float) * ntex, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(sc->ctx->counters, 0, sizeof(unsigned long long) * 8, s);
+    float* cm = (float*)sums;
+    float* ct = cm ? cm + 4 * nmat : nullptr;
+    double* dm = (double*)sums;
+    double* dt = dm ? dm + 4 * nmat : nullptr;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -593,32 +545,48 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
     unsigned long long rays[2] = {0, 0};
     float4* rec = nullptr;
     if (wavefront) {
-        // record passes (wavefront engine) + replay kernels over chunks of the samples, sized
-        // so that the records stay within 2 GiB and item indices within 2^31
+        // record passes (wavefront engine) + replay kernels over chunks of the samples, sized so that
+        // the records stay within kRecBudget and their indices within 2^31; where the device has less
+        // memory left, the chunk is halved until its records fit
         const size_t lsub = (size_t)p.light_samples;   // items per pixel and camera sample
-        const size_t per_item = sizeof(float4) * ((size_t)p.max_depth + 1);
-        const size_t budget = (size_t)2 << 30;
-        int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)p.spp, budget / (per_item * npix * lsub)));
-        while (chunk > 1 && (size_t)chunk * npix * lsub * (p.max_depth + 1) >= (1ull << 31)) chunk /= 2;
-        if ((size_t)chunk * npix * lsub * (p.max_depth + 1) >= (1ull << 31)) e = cudaErrorInvalidValue;
-        if (e == cudaSuccess) e = ctx_scratch(sc->ctx, per_item * npix * lsub * chunk, (void**)&rec);
-        float4* lo_raw = rec ? rec + (size_t)npix * lsub * chunk * p.max_depth : nullptr;
+        const int stride = record_stride(sc);
+        const size_t per_item = sizeof(float4) * ((size_t)p.max_depth * stride + 1);
+        const size_t per_spp = npix * lsub;
+        int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)p.spp, kRecBudget / (per_item * per_spp)));
+        while (chunk > 1 && (size_t)chunk * per_spp * (p.max_depth + 1) >= (1ull << 31)) chunk /= 2;
+        if ((size_t)chunk * per_spp * (p.max_depth + 1) >= (1ull << 31)) e = cudaErrorInvalidValue;
+        // as many passes as the budget needs, of equal size
+        chunk = (p.spp + (p.spp + chunk - 1) / chunk - 1) / ((p.spp + chunk - 1) / chunk);
+        while (e == cudaSuccess) {
+            e = ctx_scratch(sc->ctx, per_item * per_spp * chunk, (void**)&rec);
+            if (e != cudaErrorMemoryAllocation || chunk == 1) break;
+            cudaGetLastError();
+            e = cudaSuccess;
+            chunk = (chunk + 1) / 2;
+        }
+        float4* lo_raw = rec ? rec + per_spp * chunk * p.max_depth * stride : nullptr;
+        // a column of shared sums per thread, or as many as fit 48 KB
+        const int cols = std::min<int>(kAdjBlock, (int)(48 * 1024 / (sizeof(double) * 4 * nmat)));
+        const size_t smem = sizeof(double) * 4 * nmat * cols;
+        int sms = 0, nb = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, sc->ctx->device);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_adjoint_replay, kAdjBlock, smem);
         for (int s0 = 0; s0 < p.spp && e == cudaSuccess; s0 += chunk) {
             const int n = std::min(chunk, p.spp - s0);
-            aur_status rs = wf_record_pass(sc, p, s0, n, rec, lo_raw, &launches, rays);
+            aur_status rs = wf_record_pass(sc, p, s0, n, rec, stride, lo_raw, &launches, rays);
             if (rs != AUR_OK) {
-                if (cm) cudaFreeAsync(cm, s);
+                if (sums) cudaFreeAsync(sums, s);
                 cudaEventDestroy(e0);
                 cudaEventDestroy(e1);
                 cudaEventDestroy(er0);
                 cudaEventDestroy(er1);
                 return rs;
             }
-            const uint32_t items = (uint32_t)(npix * lsub * (size_t)n);
+            const uint32_t items = (uint32_t)(per_spp * (size_t)n);
+            const unsigned grid = std::min<unsigned>((items + kAdjBlock - 1) / kAdjBlock, (unsigned)(std::max(1, nb) * sms));
             cudaEventRecord(er0, s);
-            k_adjoint_replay<<<(items + kAdjBlock - 1) / kAdjBlock, kAdjBlock, 0, s>>>(
-                sc->dev(), p, s0, items, rec, lo_raw, (const float4*)din.ptr, nmat, (float*)gm.ptr, cm,
-                ntex ? (float*)gt.ptr : nullptr, ct);
+            k_adjoint_replay<<<grid, kAdjBlock, smem, s>>>(p, (uint32_t)npix, s0, items, rec, stride, lo_raw,
+                                                           (const float4*)din.ptr, nmat, cols, dm, dt);
             ++launches;
             e = cudaGetLastError();
             cudaEventRecord(er1, s);
@@ -636,7 +604,12 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
         ++launches;
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) {
+    if (e == cudaSuccess && wavefront) {
+        k_to_float<<<(4 * nmat + 255) / 256, 256, 0, s>>>(dm, (float*)gm.ptr, 4 * nmat);
+        ++launches;
+        if (ntex) { k_to_float<<<(ntex + 255) / 256, 256, 0, s>>>(dt, (float*)gt.ptr, ntex); ++launches; }
+        e = cudaGetLastError();
+    } else if (e == cudaSuccess) {
         k_add_comp<<<(4 * nmat + 255) / 256, 256, 0, s>>>((float*)gm.ptr, cm, 4 * nmat);
         ++launches;
         if (ntex) { k_add_comp<<<(ntex + 255) / 256, 256, 0, s>>>((float*)gt.ptr, ct, ntex); ++launches; }
@@ -659,7 +632,7 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
     cudaEventDestroy(e1);
     cudaEventDestroy(er0);
     cudaEventDestroy(er1);
-    if (cm) cudaFreeAsync(cm, s);
+    if (sums) cudaFreeAsync(sums, s);
     if (e != cudaSuccess) return cuda_fail(e, "aur_render_adjoint");
     if (stats) {
         *stats = aur_render_stats{};

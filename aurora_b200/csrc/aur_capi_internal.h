@@ -77,8 +77,17 @@ aur_status bvh_options(const aur_bvh_opts* o, BvhBuildOptions* out);
 aur_status render_options(const aur_scene* sc, const aur_render_opts* o, PathParams* p);
 aur_status render_wavefront(aur_scene* sc, const aur_render_opts* o, float* film, aur_render_stats* stats);
 void wf_release_context(aur_ctx* ctx);   // frees the wavefront engines cached for a context
-aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsamples, float4* rec, float4* lo_raw,
-                          uint64_t* launches, unsigned long long* rays);
+// Record pass of the adjoint's wavefront form; a vertex record is `stride` float4s:
+//   0  radiance collected up to and including the vertex, material (int bits)
+//   1  T dD/dtheta of the next-event estimate, 0
+//   2  radiance before the vertex's next-event estimate, d ln P(lobe) / d roughness
+//   3  (dw/dtheta) / w of the continuation weight, parameter: kind | index << 2 (kind 0: none; the
+//      rest of the record is then not written; 1 diffuse colour of material `index`, 2 texel
+//      `index`, 3 roughness of material `index`)
+//   4, 5 (stride 6) the texels and weights of kind 2
+constexpr int kVertexRec = 4;
+aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsamples, float4* rec, int stride,
+                          float4* lo_raw, uint64_t* launches, unsigned long long* rays);
 
 struct DeviceGuard {
     explicit DeviceGuard(int dev);

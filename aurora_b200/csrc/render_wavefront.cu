@@ -21,6 +21,7 @@
 // sample order with the plain kernel's compensated sum, so both renderers
 // produce the same film for the same seed.
 #include "aur_capi_internal.h"
+#include "aur_adjoint.cuh"
 #include <algorithm>
 #include <climits>
 #include <cstddef>
@@ -37,6 +38,7 @@ namespace {
 // What regen has to do for a slot, alone or above the slot's number (below 2^26).
 constexpr uint32_t kPending = 1u << 31;   // next-event rays in flight: their radiance is to be added
 constexpr uint32_t kDone = 1u << 30;      // the path is finished: write its sample, take new work
+constexpr uint32_t kNoRec = 0xffffffffu;  // WfPool::rec_cur of a vertex without a parameter
 // lane refill: a warp takes new rays once this many lanes are idle, and runs kRounds
 // traversal rounds (interior phase + leaf phase) between refill checks
 // (swept on the quantised 4-wide tree, 1080p terrain frame, closest + any hit: rounds 3 / 4 / 5 at
@@ -69,7 +71,7 @@ struct WfScene {
     DevScene sc;
     PathParams p;          // spp = samples of this pass, sample_offset = first sample index of this pass
     uint64_t key;
-    uint32_t npix, item_base, items, rec_depth;
+    uint32_t npix, item_base, items, rec_depth, rec_stride;
     // Light samples: every camera sample of the pass has lsub sub-samples q = sl * lsub + j
     // (lsub = light_samples, 1 without them); sub-sample j of sample s traces the path j of
     // Integrator::integrateCameraSample(sample, numSamples) and draws from random-number sample
@@ -81,7 +83,7 @@ struct WfScene {
     float4 *film, *acc_s, *acc_c;
     int32_t total_spp, first_pass, last_pass;
     // record mode (path-replay adjoint): per item (sample-major, sl * npix + pixel)
-    float4* rec;           // [items][rec_depth] hit records (t, u, v, prim | visibility << 30)
+    float4* rec;           // [items][rec_depth][rec_stride] vertex records (kVertexRec)
     float4* lo_raw;        // [items] unclamped path radiance, w = number of recorded vertices
 };
 
@@ -99,7 +101,8 @@ struct WfPool {
     float4 *ray, *hitid, *tplo, *neeA, *neeB, *neeC;   // [P][2] each
     uint32_t* q_regen;          // what regen has to do: by slot (sweep), or a list of the slots (see k_regen)
     uint32_t* sh_vis;           // bit k: next-event ray k of the slot is unoccluded
-    uint32_t* rec_cur;          // record mode: record index of the vertex whose next-event rays are in flight
+    uint32_t* rec_cur;          // record mode: record index << 1 | specular lobe of the vertex whose next-event rays
+                                // are in flight, kNoRec if it has no parameter
     uint8_t* bucket;            // material bucket of the slot's last hit (written by the sorting extend)
     uint32_t *q_ext0, *q_ext1, *q_sort, *q_shadow;
     uint32_t* ctr;              // WfState::ctr
@@ -238,9 +241,23 @@ __global__ void k_regen(WfPool w, int in_q) {
                 const float3 add = (res * nvis) * mk(t.x, t.y, t.z);
                 lo.x += add.x; lo.y += add.y; lo.z += add.z;
                 if (!(e & kDone)) w.lo(i) = lo;
-                if (kRec) {   // the visibility of the vertex's next-event rays goes into its record
-                    float4* r = w.scenes[id.x].rec + w.rec_cur[i];
-                    r->w = __int_as_float(__float_as_int(r->w) | (int)(vis << 30));
+                if (kRec) {   // the next-event estimate's derivative and the radiance so far complete the record
+                    const uint32_t rc = w.rec_cur[i];
+                    if (rc != kNoRec) {
+                        const WfScene& S = w.scenes[id.x];
+                        float4* r = S.rec + (size_t)(rc >> 1) * S.rec_stride;
+                        const float4 c1 = w.sh_c1(i);
+                        float3 d = mk(0.f, 0.f, 0.f);
+                        if (rc & 1u) {   // roughness: each contribution times its d ln f (c0.w, c1.w)
+                            if (vis & 1u) d += mk(c0.x, c0.y, c0.z) * c0.w;
+                            if (vis & 2u) d += mk(c1.x, c1.y, c1.z) * c1.w;
+                        } else if (vis & 1u) {
+                            d = mk(c1.x, c1.y, c1.z);
+                        }
+                        const float3 g = mk(t.x, t.y, t.z) * (d * nvis);
+                        r->x = lo.x; r->y = lo.y; r->z = lo.z;
+                        r[1] = make_float4(g.x, g.y, g.z, 0.f);
+                    }
                 }
             }
             if (e & kDone) {
@@ -493,6 +510,12 @@ __device__ __noinline__ float4 shade_env_miss(const WfPool* w, const WfScene* S,
     return make_float4(lo.x + a.x, lo.y + a.y, lo.z + a.z, lo.w);
 }
 
+// The record mode's derivatives, out of line: one copy of their double-precision transcendentals.
+static __device__ __noinline__ float rec_eval_dlnD(float rough, float3 N, float3 V, float3 L) { return eval_dlnD(rough, N, V, L); }
+static __device__ __noinline__ float rec_sample_dlnD(float rough, float3 N, float3 V, float3 L) {
+    return sample_dlnD(rough, N, V, L);
+}
+
 // Three resident 256-thread blocks per SM (85 registers, some spilled) instead of the two that
 // its 106 registers allow: 50.7 vs 52.3 ms per 1080p frame.
 // kPart selects the entries: SHADE_ALL every queued one; with the queue sorted by bucket,
@@ -559,14 +582,17 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                 float3 Lo = mk(lo.x, lo.y, lo.z);
                 if (vtx == 0) lo.w = 1.f;   // camera ray hit: alpha
                 const uint32_t rec_at = (id.z * S.npix + id.y) * S.rec_depth + (uint32_t)vtx;
-                if (kRec) S.rec[rec_at] = make_float4(hh.x, hh.y, hh.z, __int_as_float(prim));
                 const Frame f = hit_frame(sc.sh, prim, hh.x, hh.y, hh.z, mk(ro.x, ro.y, ro.z), mk(rd.x, rd.y, rd.z), true);
                 const Attr at = sc.sh.attrs[f.attr];
                 if (kind == RAY_DIFFUSE) matte = true;
                 if (collects_emission(kind)) Lo += T * at.emission;
-                const Brdf brdf = kPart == SHADE_MATTE
-                                      ? matte_brdf(sc.sh, sc.sh.mats[at.material], f)
-                                      : get_brdf(sc.sh, at.material, f, matte, rng.u(vertex_dim(vtx, kDimLobe)));
+                const float lobe_u = kPart == SHADE_MATTE ? 0.f : rng.u(vertex_dim(vtx, kDimLobe));
+                const Brdf brdf = kPart == SHADE_MATTE ? matte_brdf(sc.sh, sc.sh.mats[at.material], f)
+                                                       : get_brdf(sc.sh, at.material, f, matte, lobe_u);
+                ParamRef pr;
+                if (kRec) pr = param_of(sc.sh, at.material, brdf, f, matte, lobe_u);
+                const float3 pre = Lo;       // record: the radiance before the next-event estimate
+                bool nee_rec = false;
                 // next-event estimation: rays and their unoccluded contributions
                 if (brdf.lobe == LOBE_MATTE || brdf.lobe == LOBE_SPEC) {
                     int nvis;
@@ -580,10 +606,12 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                         float3 d0 = ls.dir, d1 = ls.dir;
                         float m0 = ls.maxt, m1 = 0.f;
                         bool r0 = false, r1 = false;
+                        float g0 = 0.f, g1 = 0.f;   // record: d ln c / d roughness
                         if (brdf.lobe == LOBE_MATTE) {
                             if (cost >= 0.f && ls.pdf > 0.f) {
                                 r0 = true;
                                 c0 = cdiv((ls.color * brdf_eval(brdf, ls.dir, f.V, f.N)) * cost, ls.pdf);
+                                if (kRec && cost > 0.f) c1 = cdiv((ls.color * kInvPiMacro) * cost, ls.pdf);   // d c0 / d colour
                             }
                         } else {
                             if (cost > 0.f && ls.pdf > 0.f) {
@@ -592,6 +620,7 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                                     r0 = true;
                                     const float wgt = power_heuristic(ls.pdf, bp);
                                     c0 = cdiv(((ls.color * wgt) * brdf_eval(brdf, ls.dir, f.V, f.N)) * cost, ls.pdf);
+                                    if (kRec && pr.kind == 3) g0 = rec_eval_dlnD(brdf.rough, f.N, f.V, ls.dir) * pr.dr;
                                 }
                             }
                             const BrdfSample bs = brdf_sample(brdf, f.V, f.N, rng.u(vertex_dim(vtx, kDimMisBrdf)),
@@ -606,16 +635,20 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                                     m1 = maxt;
                                     const float wgt = power_heuristic(bs.pdf, lp);
                                     c1 = cdiv(((bs.color * wgt) * light_eval(sc.sh, L, bs.dir)) * cost, bs.pdf);
+                                    if (kRec && pr.kind == 3) g1 = rec_sample_dlnD(brdf.rough, f.N, f.V, bs.dir) * pr.dr;
                                 }
                             }
                         }
                         if (r0 || r1) {
-                            if (kRec) w.rec_cur[slot] = rec_at;
+                            if (kRec) {
+                                w.rec_cur[slot] = pr.kind == 0 ? kNoRec : (rec_at << 1) | (pr.kind == 3 ? 1u : 0u);
+                                nee_rec = true;
+                            }
                             w.sh_p(slot) = make_float4(f.P.x, f.P.y, f.P.z, 0.f);
                             w.sh_d0(slot) = make_float4(d0.x, d0.y, d0.z, m0);
                             w.sh_d1(slot) = make_float4(d1.x, d1.y, d1.z, m1);
-                            w.sh_c0(slot) = make_float4(c0.x, c0.y, c0.z, 0.f);
-                            w.sh_c1(slot) = make_float4(c1.x, c1.y, c1.z, 0.f);
+                            w.sh_c0(slot) = make_float4(c0.x, c0.y, c0.z, g0);
+                            w.sh_c1(slot) = make_float4(c1.x, c1.y, c1.z, g1);
                             w.sh_t(slot) = make_float4(T.x, T.y, T.z, (float)nvis);
                             w.sh_vis[slot] = 0u;
                             push_sh0 = r0;
@@ -627,6 +660,45 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                 bool alive = false;
                 const BrdfSample bs = brdf_sample(brdf, f.V, f.N, rng.u(vertex_dim(vtx, kDimBrdf)),
                                                   rng.u(vertex_dim(vtx, kDimBrdf + 1)));
+                if (kRec) {
+                    // the vertex's record; regen completes it where next-event rays are in flight
+                    float4* r = S.rec + (size_t)rec_at * S.rec_stride;
+                    float3 q = mk(0.f, 0.f, 0.f);
+                    if (pr.kind != 0) {
+                        if (bs.pdf > 0.f) {
+                            if (pr.kind == 3) {
+                                const float g = rec_sample_dlnD(brdf.rough, f.N, f.V, bs.dir) * pr.dr;   // dw/w = d ln f
+                                q = mk(g, g, g);
+                            } else {
+                                const float cosl = dot(f.N, bs.dir);
+                                const float3 wt = cdiv(bs.color * cosl, bs.pdf);
+                                const float dw = kInvPiMacro * cosl / bs.pdf;   // d w_c / d diffuse_c
+                                q = mk(wt.x != 0.f ? dw / wt.x : 0.f, wt.y != 0.f ? dw / wt.y : 0.f,
+                                       wt.z != 0.f ? dw / wt.z : 0.f);
+                            }
+                        }
+                        float score = 0.f;
+                        if (kPart != SHADE_MATTE) {
+                            const Material& m = sc.sh.mats[at.material];
+                            if (m.type == MAT_KELEMEN && m.refl < 1.f && m.rough_tex < 0)
+                                score = kelemen_score(sc.sh, m, f, brdf, matte);
+                        }
+                        if (nee_rec) {
+                            r->w = __int_as_float(at.material);
+                        } else {
+                            r[0] = make_float4(pre.x, pre.y, pre.z, __int_as_float(at.material));
+                            r[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+                        r[2] = make_float4(pre.x, pre.y, pre.z, score);
+                        if (S.rec_stride > kVertexRec && pr.kind == 2) {
+                            r[4] = make_float4(__int_as_float(pr.taps.idx[0]), __int_as_float(pr.taps.idx[1]),
+                                               __int_as_float(pr.taps.idx[2]), 0.f);
+                            r[5] = make_float4(pr.taps.w[0], pr.taps.w[1], pr.taps.w[2], 0.f);
+                        }
+                    }
+                    const uint32_t index = (uint32_t)(pr.kind == 2 ? pr.taps.idx[0] : pr.index);
+                    r[3] = make_float4(q.x, q.y, q.z, __uint_as_float((uint32_t)pr.kind | (index << 2)));
+                }
                 // after the last vertex the reference traces one more ray, which only an
                 // escaping mirror ray in a scene with an environment light turns into radiance
                 // (integrator.cpp:256-274): that ray is queued and its hit is not shaded
@@ -787,7 +859,7 @@ struct WfConfig {
     uint32_t pool = 1u << 21;
     int block = 128;
     int sort = 1;
-    int record = 0;   // record mode: hit records + unclamped radiance per item instead of samples
+    int record = 0;   // record mode: vertex records + unclamped radiance per item instead of samples
     // the trees traversed by closest-hit and any-hit rays (TREE_*; the 4-wide ones only when every
     // scene has them), chosen by tree_for
     int tree = TREE_BINARY, tree_any = TREE_BINARY;
@@ -1308,10 +1380,10 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
 
 // Record pass of the path-replay adjoint: traces samples [s0, s0 + nsamples) of every
 // pixel with the wavefront engine in record mode and writes, per item (sample-major:
-// sl * npix + pixel), the hit records of its vertices (p.max_depth slots) and its
+// sl * npix + pixel), the records of its vertices (p.max_depth of `stride` float4s) and its
 // unclamped radiance. Ordered after the caller's stream and before its later work.
-aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsamples, float4* rec, float4* lo_raw,
-                          uint64_t* launches, unsigned long long* rays) {
+aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsamples, float4* rec, int stride,
+                          float4* lo_raw, uint64_t* launches, unsigned long long* rays) {
     aur_ctx* ctx = sc->ctx;
     WfConfig cfg;
     if (sc->wf_tuned) { cfg.pool = (uint32_t)sc->wf_pool; cfg.block = sc->wf_block; cfg.sort = sc->wf_sort; }
@@ -1330,6 +1402,7 @@ aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsampl
     run.h_scenes[0].rec = rec;
     run.h_scenes[0].lo_raw = lo_raw;
     run.h_scenes[0].rec_depth = (uint32_t)p.max_depth;
+    run.h_scenes[0].rec_stride = (uint32_t)stride;
     e = run.begin_pass(total, 1, true);
     if (e == cudaSuccess) e = run.run_pass(total, max_rays(items), launches);
     if (e == cudaSuccess) e = run.read_state();
