@@ -75,15 +75,13 @@ struct BvhBuildOptions {
     int ploc_radius = 16;         // PLOC nearest-neighbour search radius
 };
 
-// Builds into freshly allocated device buffers (cudaMallocAsync on `stream`).
-// verts: device float3[nvert]; idx: device uint32[3*ntri]. Returns cudaSuccess
-// or the first CUDA error. ntri must be >= 1.
-cudaError_t bvh_build_device(const float* verts, const uint32_t* idx, int ntri, const BvhBuildOptions& opt,
-                             DeviceBvh* out, cudaStream_t stream);
+// Builds into freshly allocated device buffers (cudaMallocAsync on `stream`), the 4-wide forms
+// included (left null where the tree is too deep for any of their stacks). verts: device
+// float3[nvert]; idx: device uint32[3*ntri]. Returns cudaSuccess or the first CUDA error; what was
+// allocated until then is the caller's to free. *in_range = false, and nothing is built, when an
+// index is not below nvert. ntri must be >= 1. Synchronises the stream.
+cudaError_t bvh_build_device(const float* verts, const uint32_t* idx, int ntri, uint32_t nvert, const BvhBuildOptions& opt,
+                             DeviceBvh* out, bool* in_range, cudaStream_t stream);
 void bvh_free_device(DeviceBvh* bvh, cudaStream_t stream);
-// Collapses the binary tree of `bvh` into its 4-wide form (nodes4): each 4-wide node
-// takes a binary node's two children and opens its largest-area interior child until
-// it holds four, level by level from the root.
-cudaError_t bvh_collapse4(DeviceBvh* bvh, cudaStream_t stream);
 
 }  // namespace aur

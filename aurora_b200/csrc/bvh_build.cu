@@ -6,23 +6,35 @@
 // (Aurora/src/frontend/renderer.cpp:99-145, triangleMesh.cpp:57-81).
 //
 // Pipeline (all kernels in this file, no library calls):
-//   1. triangle boxes + centroid bounds            k_prim_setup
-//   2. 30-bit Morton codes, stable LSD radix sort   k_morton, k_radix_hist/k_radix_scatter
+//   1. scene and centroid bounds, index check         k_bounds
+//   2. 30-bit Morton codes, stable LSD radix sort     k_morton, k_sort_*
 //   3. PLOC agglomerative clustering (Meister & Bittner, "Parallel Locally-
 //      Ordered Clustering for BVH Construction", IEEE TVCG 2018): every cluster
 //      finds its nearest neighbour (smallest merged surface area) within a
 //      window of the Morton order; mutual pairs merge; the list is compacted
-//      with an order-preserving scan. Ties are broken on the index pair so that
-//      the globally best pair is always mutual (guaranteed progress).
-//   4. bottom-up SAH leaf collapse (atomic second-arrival walk)
-//   5. deterministic depth-first layout: every node derives its output slot by
+//      in order. Ties are broken on the index pair so that the globally best
+//      pair is always mutual (guaranteed progress).
+//      A merge also decides, from its two finished children, whether the new
+//      node collapses into a leaf by the SAH, and its row of the dynamic
+//      program that groups binary nodes into 4-wide ones (step 5); both need
+//      nothing but the children, and as passes of their own they climbed the
+//      finished tree with an atomic and a fence a level.
+//   4. deterministic depth-first layout: every node derives its output slot by
 //      walking to the root, so the result is independent of thread timing.
-//   6. the 4-wide tree: an SAH-optimal grouping of the binary nodes (a bottom-up
-//      dynamic program), built level by level.
+//   5. the 4-wide tree: an SAH-optimal grouping of the binary nodes, built
+//      level by level, and its quantised form.
+//
+// Small meshes are bound by launches and host reads, large ones by the traffic of each pass:
+// two launches a PLOC iteration (search and merge, compaction) where there were eight, one block
+// for all iterations from kFinish clusters on, no pass over the finished tree for the SAH and the
+// grouping, boxes recomputed from the vertices instead of kept, one allocation. Build and a
+// batch of rays: 3.4 M triangles from device arrays with 262,144 rays 6.2 -> 2.7 ms, 20,482
+// triangles from host arrays with 16,384 rays 2.1 -> 0.93 ms.
 #include "aur_bvh.cuh"
 #include "aur_shading.cuh"
+#include <algorithm>
 #include <cfloat>
-#include <vector>
+#include <cstring>
 
 namespace aur {
 namespace {
@@ -31,15 +43,8 @@ namespace {
 
 template <typename T>
 cudaError_t dalloc(T** p, size_t n, cudaStream_t s) { return cudaMallocAsync((void**)p, sizeof(T) * (n ? n : 1), s); }
-template <typename T>
-void dfree(T*& p, cudaStream_t s) { if (p) cudaFreeAsync(p, s); p = nullptr; }
 
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
-
-// ------------------------------------------------------------ exclusive scan
-constexpr int kScanThreads = 512;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
     const int lane = threadIdx.x & 31;
@@ -51,148 +56,192 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
     return v;
 }
 
-// In-place safe: each thread reads its own items before writing them.
-__global__ void k_scan_tiles(const uint32_t* in, uint32_t* out, uint32_t* sums, int n) {
-    __shared__ uint32_t s_warp[kScanThreads / 32];
-    const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t local = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) { int i = base + k; v[k] = i < n ? in[i] : 0u; local += v[k]; }
-    uint32_t incl = warp_incl_scan(local);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 31) s_warp[warp] = incl;
+// Exclusive prefix of v over the block (at most 1024 threads; all of them call it) and the
+// block's total. s: 33 words, free for reuse after the caller's next barrier.
+__device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* s, uint32_t* total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const uint32_t incl = warp_incl_scan(v);
+    if (lane == 31) s[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = lane < kScanThreads / 32 ? s_warp[lane] : 0u;
-        w = warp_incl_scan(w);
-        if (lane < kScanThreads / 32) s_warp[lane] = w;
+        const uint32_t x = lane < nw ? s[lane] : 0u;
+        const uint32_t y = warp_incl_scan(x);
+        s[lane] = y - x;
+        if (lane == 31) s[32] = y;
     }
     __syncthreads();
-    uint32_t excl = incl - local + (warp > 0 ? s_warp[warp - 1] : 0u);
-#pragma unroll
-    for (int k = 0; k < kScanItems; ++k) { int i = base + k; if (i < n) out[i] = excl; excl += v[k]; }
-    if (sums && threadIdx.x == 0) sums[blockIdx.x] = s_warp[kScanThreads / 32 - 1];
-}
-
-__global__ void k_scan_add(uint32_t* out, const uint32_t* add, int n) {
-    const int base = blockIdx.x * kScanTile;
-    const uint32_t a = add[blockIdx.x];
-    const int end = min(base + kScanTile, n);
-    for (int i = base + threadIdx.x; i < end; i += blockDim.x) out[i] += a;
-}
-
-cudaError_t exclusive_scan(const uint32_t* in, uint32_t* out, int n, cudaStream_t s) {
-    const int nb = div_up(n, kScanTile);
-    if (nb <= 1) { k_scan_tiles<<<1, kScanThreads, 0, s>>>(in, out, nullptr, n); return cudaGetLastError(); }
-    uint32_t* sums = nullptr;
-    CK(dalloc(&sums, nb, s));
-    k_scan_tiles<<<nb, kScanThreads, 0, s>>>(in, out, sums, n);
-    CK(exclusive_scan(sums, sums, nb, s));
-    k_scan_add<<<nb, 256, 0, s>>>(out, sums, n);
-    dfree(sums, s);
-    return cudaGetLastError();
+    *total = s[32];
+    return incl - v + s[warp];
 }
 
 // ------------------------------------------------------------ radix sort
-// Stable LSD sort of (key, value) pairs, 8 bits per pass. One warp per block
-// walks its 2048-key tile in order, so ranks within a digit follow input order.
-constexpr int kSortTile = 2048;
+// Stable LSD sort of (key, value) pairs, 10 bits per pass, three passes for the 30-bit codes. A
+// block of 8 warps takes a tile of up to 4096 pairs in order, each warp a contiguous eighth: per warp
+// and digit counts (phase 1), a prefix over the warps (phase 2), then every pair's place from its
+// warp's counter and its rank among the equal digits of its 32 (phase 3). One warp per block
+// over 2048 pairs, 8 bits a pass, spent 56 + 36 us a pass however small the array.
+constexpr int kDigits = 1024;
+constexpr int kSortThreads = 256;
+constexpr int kSortWarps = kSortThreads / 32;
+// pairs per thread: 16, or 4 (tiles of 1024) for arrays of up to kSmallSort pairs, which
+// otherwise occupy a few SMs for the length of a tile
+constexpr int kSmallSort = 1 << 18;
 
-__global__ void k_radix_hist(const uint32_t* keys, int n, int shift, uint32_t* hist, int nb) {
-    __shared__ uint32_t s_h[256];
-    const int lane = threadIdx.x;
-    for (int d = lane; d < 256; d += 32) s_h[d] = 0;
-    __syncwarp();
-    const int base = blockIdx.x * kSortTile;
-    for (int k = 0; k < kSortTile / 32; ++k) {
-        int i = base + k * 32 + lane;
-        if (i < n) atomicAdd(&s_h[(keys[i] >> shift) & 255u], 1u);
+template <int kItems>
+__global__ void __launch_bounds__(kSortThreads) k_sort_hist(const uint32_t* __restrict__ keys, int n, int shift,
+                                                            uint32_t* __restrict__ hist, int nb) {
+    __shared__ uint32_t s_h[kDigits];
+    for (int d = threadIdx.x; d < kDigits; d += kSortThreads) s_h[d] = 0;
+    __syncthreads();
+    const int base = blockIdx.x * (kSortThreads * kItems);
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int i = base + k * kSortThreads + threadIdx.x;
+        if (i < n) atomicAdd(&s_h[(keys[i] >> shift) & (kDigits - 1)], 1u);
     }
-    __syncwarp();
-    for (int d = lane; d < 256; d += 32) hist[d * nb + blockIdx.x] = s_h[d];
+    __syncthreads();
+    for (int d = threadIdx.x; d < kDigits; d += kSortThreads) hist[(size_t)d * nb + blockIdx.x] = s_h[d];
 }
 
-__global__ void k_radix_scatter(const uint32_t* keys, const uint32_t* vals, uint32_t* okeys, uint32_t* ovals,
-                                int n, int shift, const uint32_t* offs, int nb) {
-    __shared__ uint32_t s_off[256];
-    const int lane = threadIdx.x;
-    for (int d = lane; d < 256; d += 32) s_off[d] = offs[d * nb + blockIdx.x];
-    __syncwarp();
-    const int base = blockIdx.x * kSortTile;
-    for (int k = 0; k < kSortTile / 32; ++k) {
+inline int sort_tile(long long n) { return kSortThreads * (n <= kSmallSort ? 4 : 16); }
+
+// One warp per digit: exclusive prefix of the digit's counts over the tiles, in place, and its total.
+__global__ void k_sort_rows(uint32_t* hist, int nb, uint32_t* __restrict__ total) {
+    const int d = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (d >= kDigits) return;
+    uint32_t* row = hist + (size_t)d * nb;
+    uint32_t run = 0;
+    for (int b = 0; b < nb; b += 32) {
+        const uint32_t v = b + lane < nb ? row[b + lane] : 0u;
+        const uint32_t incl = warp_incl_scan(v);
+        if (b + lane < nb) row[b + lane] = run + incl - v;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) total[d] = run;
+}
+
+template <int kItems>
+__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const uint32_t* __restrict__ keys,
+                                                               const uint32_t* __restrict__ vals, uint32_t* okeys,
+                                                               uint32_t* ovals, int n, int shift,
+                                                               const uint32_t* __restrict__ rows,
+                                                               const uint32_t* __restrict__ total, int nb) {
+    __shared__ uint32_t s_cnt[kSortWarps][kDigits];
+    __shared__ uint32_t s_scan[33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int d = threadIdx.x; d < kSortWarps * kDigits; d += kSortThreads) (&s_cnt[0][0])[d] = 0;
+    __syncthreads();
+    const int base = blockIdx.x * (kSortThreads * kItems) + warp * (32 * kItems);
+    uint32_t key[kItems], val[kItems], rank[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
         const int i = base + k * 32 + lane;
-        const bool valid = i < n;
-        const uint32_t active = __ballot_sync(0xffffffffu, valid);
-        if (!active) break;
-        if (valid) {
-            const uint32_t key = keys[i], val = vals[i];
-            const uint32_t d = (key >> shift) & 255u;
-            const uint32_t peers = __match_any_sync(active, d);
-            const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-            const int leader = __ffs(peers) - 1;
-            const uint32_t b = s_off[d];
-            __syncwarp(active);
-            if (lane == leader) s_off[d] = b + __popc(peers);
-            okeys[b + rank] = key;
-            ovals[b + rank] = val;
-        }
+        key[k] = i < n ? keys[i] : 0xffffffffu;
+        val[k] = i < n ? vals[i] : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const bool valid = base + k * 32 + lane < n;
+        const uint32_t d = (key[k] >> shift) & (kDigits - 1);
+        const uint32_t peers = __match_any_sync(0xffffffffu, valid ? d : kDigits);
+        rank[k] = 0;
+        if (valid) rank[k] = s_cnt[warp][d] + __popc(peers & ((1u << lane) - 1u));
+        __syncwarp();
+        if (valid && lane == __ffs(peers) - 1) s_cnt[warp][d] += __popc(peers);
         __syncwarp();
     }
-}
-
-cudaError_t radix_sort_pairs(uint32_t* keys, uint32_t* vals, int n, int bits, cudaStream_t s) {
-    const int nb = div_up(n, kSortTile);
-    uint32_t *k2 = nullptr, *v2 = nullptr, *hist = nullptr;
-    CK(dalloc(&k2, n, s)); CK(dalloc(&v2, n, s)); CK(dalloc(&hist, (size_t)256 * nb, s));
-    uint32_t *ka = keys, *va = vals, *kb = k2, *vb = v2;
-    for (int shift = 0; shift < bits; shift += 8) {
-        k_radix_hist<<<nb, 32, 0, s>>>(ka, n, shift, hist, nb);
-        CK(exclusive_scan(hist, hist, 256 * nb, s));
-        k_radix_scatter<<<nb, 32, 0, s>>>(ka, va, kb, vb, n, shift, hist, nb);
-        std::swap(ka, kb); std::swap(va, vb);
+    __syncthreads();
+    // digits 4 t .. 4 t + 3 of thread t: the digit's first place in the output, then its warps in order
+    uint32_t sum = 0, tot[kDigits / kSortThreads], unused;
+#pragma unroll
+    for (int q = 0; q < kDigits / kSortThreads; ++q) { tot[q] = total[threadIdx.x * (kDigits / kSortThreads) + q]; sum += tot[q]; }
+    uint32_t first = block_excl_scan(sum, s_scan, &unused);
+#pragma unroll
+    for (int q = 0; q < kDigits / kSortThreads; ++q) {
+        const int d = threadIdx.x * (kDigits / kSortThreads) + q;
+        uint32_t at = first + rows[(size_t)d * nb + blockIdx.x];
+        for (int w = 0; w < kSortWarps; ++w) { const uint32_t c = s_cnt[w][d]; s_cnt[w][d] = at; at += c; }
+        first += tot[q];
     }
-    if (ka != keys) {
-        CK(cudaMemcpyAsync(keys, ka, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-        CK(cudaMemcpyAsync(vals, va, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        if (base + k * 32 + lane >= n) continue;
+        const uint32_t at = s_cnt[warp][(key[k] >> shift) & (kDigits - 1)] + rank[k];
+        okeys[at] = key[k];
+        ovals[at] = val[k];
     }
-    dfree(k2, s); dfree(v2, s); dfree(hist, s);
-    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ primitives
 __device__ __forceinline__ int f2ord(float f) { int i = __float_as_int(f); return i >= 0 ? i : i ^ 0x7fffffff; }
 __device__ __forceinline__ float ord2f(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+inline float host_ord2f(int i) { const int b = i >= 0 ? i : i ^ 0x7fffffff; float f; memcpy(&f, &b, 4); return f; }
 
-__device__ __forceinline__ float3 ld3(const float* v, uint32_t i) { return mk(v[3 * i], v[3 * i + 1], v[3 * i + 2]); }
+__device__ __forceinline__ float3 ld3(const float* v, uint32_t i) { return mk(v[3 * (size_t)i], v[3 * (size_t)i + 1], v[3 * (size_t)i + 2]); }
 
-__global__ void k_prim_setup(const float* verts, const uint32_t* idx, int n, float4* plo, float4* phi, float4* cent,
-                             int* gb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float c[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, C[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
-    if (i < n) {
-        float3 a = ld3(verts, idx[3 * i]), b = ld3(verts, idx[3 * i + 1]), d = ld3(verts, idx[3 * i + 2]);
-        float3 lo = mk(fminf(fminf(a.x, b.x), d.x), fminf(fminf(a.y, b.y), d.y), fminf(fminf(a.z, b.z), d.z));
-        float3 hi = mk(fmaxf(fmaxf(a.x, b.x), d.x), fmaxf(fmaxf(a.y, b.y), d.y), fmaxf(fmaxf(a.z, b.z), d.z));
-        plo[i] = make_float4(lo.x, lo.y, lo.z, 0.f);
-        phi[i] = make_float4(hi.x, hi.y, hi.z, 0.f);
-        float3 ce = (lo + hi) * 0.5f;
-        cent[i] = make_float4(ce.x, ce.y, ce.z, 0.f);
-        c[0] = C[0] = ce.x; c[1] = C[1] = ce.y; c[2] = C[2] = ce.z;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            c[k] = fminf(c[k], __shfl_xor_sync(0xffffffffu, c[k], o));
-            C[k] = fmaxf(C[k], __shfl_xor_sync(0xffffffffu, C[k], o));
-        }
-    if ((threadIdx.x & 31) == 0)
-        for (int k = 0; k < 3; ++k) { atomicMin(&gb[k], f2ord(c[k])); atomicMax(&gb[3 + k], f2ord(C[k])); }
+__device__ __forceinline__ void tri_box(const float* verts, const uint32_t* idx, size_t i, float3* lo, float3* hi) {
+    const float3 a = ld3(verts, idx[3 * i]), b = ld3(verts, idx[3 * i + 1]), d = ld3(verts, idx[3 * i + 2]);
+    *lo = mk(fminf(fminf(a.x, b.x), d.x), fminf(fminf(a.y, b.y), d.y), fminf(fminf(a.z, b.z), d.z));
+    *hi = mk(fmaxf(fmaxf(a.x, b.x), d.x), fmaxf(fmaxf(a.y, b.y), d.y), fmaxf(fmaxf(a.z, b.z), d.z));
 }
 
-__global__ void k_init_bounds(int* gb) {
-    if (threadIdx.x < 3) { gb[threadIdx.x] = f2ord(FLT_MAX); gb[3 + threadIdx.x] = f2ord(-FLT_MAX); }
+// What the build keeps beside its arrays; read back by the host between its phases.
+constexpr int kMaxLevels = 96;
+struct BuildState {
+    int gb[12];                   // ordered ints: centroid min, max, scene min, max
+    uint32_t bad;                 // an index out of range
+    int m[2];                     // cluster counts, ping-pong
+    int node;                     // next node id
+    int root, num_nodes;          // after the last merge
+    int depth;                    // binary levels
+    int front[kMaxLevels + 2];    // 4-wide nodes per level
+};
+
+__global__ void k_init_state(BuildState* st, int n) {
+    const int t = threadIdx.x;
+    if (t < 12) st->gb[t] = f2ord((t / 3) % 2 == 0 ? FLT_MAX : -FLT_MAX);
+    if (t < kMaxLevels + 2) st->front[t] = t == 0 ? 1 : 0;
+    if (t == 0) { st->bad = 0u; st->m[0] = n; st->m[1] = n; st->node = n; st->root = 0; st->num_nodes = 0; st->depth = 0; }
+}
+
+// Bounds of the boxes and of their centroids, and the check that every vertex index is below nvert
+// (a triangle with a bad one is not read). A resident grid reduces per block before its twelve
+// atomics: one set per warp of a thread-per-triangle grid took 456 us for 3.4 M triangles.
+__global__ void __launch_bounds__(256) k_bounds(const float* __restrict__ verts, const uint32_t* __restrict__ idx, int n,
+                                                uint32_t nvert, BuildState* st) {
+    float v[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) v[k] = (k / 3) % 2 == 0 ? FLT_MAX : -FLT_MAX;
+    uint32_t bad = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        if (idx[3 * (size_t)i] >= nvert || idx[3 * (size_t)i + 1] >= nvert || idx[3 * (size_t)i + 2] >= nvert) { bad = 1; continue; }
+        float3 lo, hi;
+        tri_box(verts, idx, i, &lo, &hi);
+        const float3 c = (lo + hi) * 0.5f;
+        const float a[12] = {c.x, c.y, c.z, c.x, c.y, c.z, lo.x, lo.y, lo.z, hi.x, hi.y, hi.z};
+#pragma unroll
+        for (int k = 0; k < 12; ++k) v[k] = (k / 3) % 2 == 0 ? fminf(v[k], a[k]) : fmaxf(v[k], a[k]);
+    }
+    __shared__ int s_v[12];
+    __shared__ uint32_t s_bad;
+    if (threadIdx.x < 12) s_v[threadIdx.x] = f2ord((threadIdx.x / 3) % 2 == 0 ? FLT_MAX : -FLT_MAX);
+    if (threadIdx.x == 0) s_bad = 0;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+        const bool mn = (k / 3) % 2 == 0;
+        const int o = f2ord(v[k]);
+        const int r = mn ? __reduce_min_sync(0xffffffffu, o) : __reduce_max_sync(0xffffffffu, o);
+        if ((threadIdx.x & 31) == 0) { if (mn) atomicMin(&s_v[k], r); else atomicMax(&s_v[k], r); }
+    }
+    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) s_bad = 1;
+    __syncthreads();
+    if (threadIdx.x < 12) {
+        if ((threadIdx.x / 3) % 2 == 0) atomicMin(&st->gb[threadIdx.x], s_v[threadIdx.x]);
+        else atomicMax(&st->gb[threadIdx.x], s_v[threadIdx.x]);
+    }
+    if (threadIdx.x == 0 && s_bad) atomicOr(&st->bad, 1u);
 }
 
 __device__ __forceinline__ uint32_t expand10(uint32_t v) {
@@ -203,16 +252,19 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
     return v;
 }
 
-__global__ void k_morton(const float4* cent, int n, const int* gb, uint32_t* keys, uint32_t* vals) {
+__global__ void k_morton(const float* __restrict__ verts, const uint32_t* __restrict__ idx, int n,
+                         const BuildState* __restrict__ st, uint32_t* keys, uint32_t* vals) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float lo[3], sc[3];
     for (int k = 0; k < 3; ++k) {
-        lo[k] = ord2f(gb[k]);
-        float ext = ord2f(gb[3 + k]) - lo[k];
+        lo[k] = ord2f(st->gb[k]);
+        float ext = ord2f(st->gb[3 + k]) - lo[k];
         sc[k] = ext > 0.f ? 1023.f / ext : 0.f;
     }
-    float4 c = cent[i];
+    float3 blo, bhi;
+    tri_box(verts, idx, i, &blo, &bhi);
+    const float3 c = (blo + bhi) * 0.5f;
     uint32_t q[3];
     float cc[3] = {c.x, c.y, c.z};
     for (int k = 0; k < 3; ++k) {
@@ -224,155 +276,11 @@ __global__ void k_morton(const float4* cent, int n, const int* gb, uint32_t* key
     vals[i] = (uint32_t)i;
 }
 
-// ------------------------------------------------------------ PLOC
-struct Tree {
-    float4 *lo, *hi;
-    int *left, *right, *parent;
-};
-
-__global__ void k_init_leaves(const uint32_t* sorted, int n, const float4* plo, const float4* phi, Tree t, int* clusters) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const uint32_t p = sorted[k];
-    t.lo[k] = plo[p];
-    t.hi[k] = phi[p];
-    t.left[k] = -1;
-    t.right[k] = -1;
-    t.parent[k] = -1;
-    clusters[k] = k;
-}
-
 __device__ __forceinline__ float half_area(float3 lo, float3 hi) {
     float3 d = hi - lo;
     return d.x * d.y + d.y * d.z + d.z * d.x;
 }
 
-constexpr int kNnBlock = 256;
-constexpr int kPlocBatch = 8;
-constexpr int kMaxRadius = 32;
-
-// The cluster count m lives on the device (dm) so that several iterations run between host
-// synchronisations; grids are sized for an upper bound of it.
-__global__ void __launch_bounds__(kNnBlock) k_ploc_nn(const int* clusters, const int* dm, Tree t, int* nn, int r) {
-    __shared__ float3 s_lo[kNnBlock + 2 * kMaxRadius], s_hi[kNnBlock + 2 * kMaxRadius];
-    const int m = *dm;
-    const int start = blockIdx.x * kNnBlock - r;
-    const int count = kNnBlock + 2 * r;
-    for (int k = threadIdx.x; k < count; k += kNnBlock) {
-        const int g = start + k;
-        if (g >= 0 && g < m) {
-            const int c = clusters[g];
-            float4 a = t.lo[c], b = t.hi[c];
-            s_lo[k] = mk(a.x, a.y, a.z);
-            s_hi[k] = mk(b.x, b.y, b.z);
-        }
-    }
-    __syncthreads();
-    const int i = blockIdx.x * kNnBlock + threadIdx.x;
-    if (i >= m) return;
-    const float3 mlo = s_lo[threadIdx.x + r], mhi = s_hi[threadIdx.x + r];
-    float best = FLT_MAX;
-    int bj = -1;
-    const int j0 = max(0, i - r), j1 = min(m - 1, i + r);
-    for (int j = j0; j <= j1; ++j) {
-        if (j == i) continue;
-        const int sj = j - start;
-        float3 lo = mk(fminf(mlo.x, s_lo[sj].x), fminf(mlo.y, s_lo[sj].y), fminf(mlo.z, s_lo[sj].z));
-        float3 hi = mk(fmaxf(mhi.x, s_hi[sj].x), fmaxf(mhi.y, s_hi[sj].y), fmaxf(mhi.z, s_hi[sj].z));
-        const float a = half_area(lo, hi);
-        // strict order on unordered pairs: (area, min index, max index); j increases,
-        // so for equal area the first j seen has the smaller pair key.
-        if (a < best) { best = a; bj = j; }
-    }
-    nn[i] = bj;
-}
-
-__global__ void k_ploc_merge(int* clusters, const int* dm, int bound, const int* nn, Tree t, int* node_counter,
-                             uint32_t* keep) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= bound) return;
-    if (i >= *dm) { keep[i] = 0u; return; }   // the scan runs over the bound
-    const int j = nn[i];
-    if (j >= 0 && nn[j] == i) {
-        if (i < j) {
-            const int a = clusters[i], b = clusters[j];
-            const int node = atomicAdd(node_counter, 1);
-            float4 la = t.lo[a], lb = t.lo[b], ha = t.hi[a], hb = t.hi[b];
-            t.lo[node] = make_float4(fminf(la.x, lb.x), fminf(la.y, lb.y), fminf(la.z, lb.z), 0.f);
-            t.hi[node] = make_float4(fmaxf(ha.x, hb.x), fmaxf(ha.y, hb.y), fmaxf(ha.z, hb.z), 0.f);
-            t.left[node] = a;
-            t.right[node] = b;
-            t.parent[node] = -1;
-            t.parent[a] = node;
-            t.parent[b] = node;
-            clusters[i] = node;
-            keep[i] = 1u;
-        } else {
-            keep[i] = 0u;
-        }
-    } else {
-        keep[i] = 1u;
-    }
-}
-
-__global__ void k_compact(const int* in, const uint32_t* keep, const uint32_t* pos, const int* dm, int* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < *dm && keep[i]) out[pos[i]] = in[i];
-}
-
-// The next cluster count: the kept clusters of the compaction.
-__global__ void k_ploc_count(const uint32_t* keep, const uint32_t* pos, int* dm) {
-    const int m = *dm;
-    *dm = (int)(pos[m - 1] + keep[m - 1]);
-}
-
-// ------------------------------------------------------------ SAH collapse
-struct Sah {
-    int *cnt, *icount, *visit;
-    float* cost;
-    unsigned char* collapsed;
-};
-
-__global__ void k_bottom_up(int n, Tree t, Sah s, int max_leaf, float ct, float ci) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    {
-        float4 a = t.lo[k], b = t.hi[k];
-        s.cnt[k] = 1;
-        s.cost[k] = ci * half_area(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z));
-        s.icount[k] = 0;
-        s.collapsed[k] = 1;
-    }
-    __threadfence();
-    int node = t.parent[k];
-    while (node >= 0) {
-        if (atomicAdd(&s.visit[node], 1) == 0) return;
-        __threadfence();
-        const int l = t.left[node], r = t.right[node];
-        const int cl = __ldcg(&s.cnt[l]), cr = __ldcg(&s.cnt[r]);
-        const float kl = __ldcg(&s.cost[l]), kr = __ldcg(&s.cost[r]);
-        const int il = __ldcg(&s.icount[l]), ir = __ldcg(&s.icount[r]);
-        float4 a = t.lo[node], b = t.hi[node];
-        const float A = half_area(mk(a.x, a.y, a.z), mk(b.x, b.y, b.z));
-        const int c = cl + cr;
-        const float split = ct * A + kl + kr;
-        const float leaf = c <= max_leaf ? ci * A * (float)c : FLT_MAX;
-        s.cnt[node] = c;
-        if (leaf <= split) { s.cost[node] = leaf; s.icount[node] = 0; s.collapsed[node] = 1; }
-        else { s.cost[node] = split; s.icount[node] = 1 + il + ir; s.collapsed[node] = 0; }
-        __threadfence();
-        node = t.parent[node];
-    }
-}
-
-__global__ void k_fix_root(int root, Tree t, Sah s) {
-    if (s.collapsed[root]) {
-        s.collapsed[root] = 0;
-        s.icount[root] = 1 + s.icount[t.left[root]] + s.icount[t.right[root]];
-    }
-}
-
-// ------------------------------------------------------------ layout
 // Outward padding: 2^-19 of the box's own magnitude, and at least 2^-20 of the
 // scene's magnitude (covers the rounding of slab distances for rays whose
 // origin lies anywhere inside the scene bounds).
@@ -383,17 +291,353 @@ __device__ __forceinline__ void pad_box(float& lo, float& hi, float floor_pad) {
     hi += p;
 }
 
-__global__ void k_layout_tris(int n, Tree t, Sah s, const uint32_t* sorted, const float* verts, const uint32_t* idx,
-                              BvhTri* out) {
+// ------------------------------------------------------------ nodes
+// The tree under construction, by node id (the n leaves in Morton order, then the merges).
+struct Tree {
+    float4* lo;       // box, SAH cost
+    float4* hi;       // box, triangles << 1 | collapsed (int bits)
+    int* icount;      // interior nodes of the subtree that are not inside collapsed ones
+    int2* child;
+    // To the parent: (parent, what the depth-first index and the first triangle grow by on the way
+    // down from it, whether it is collapsed). Parent -1 at the root.
+    int4* up;
+    // SAH-optimal grouping into 4-wide nodes: a dynamic program over the binary tree, bottom up
+    // (the 8-wide form is in Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs
+    // Through Compressed Wide BVHs", HPG 2017). The leaves are fixed, so groupings differ in SAH
+    // cost only by the summed surface area of the 4-wide nodes. S(x, j) is the least such sum for
+    // the subtree of binary node x when it may fill j of its parent's child slots (a leaf costs
+    // nothing): S(x, 1) = A(x) + D(x, 4), and for j > 1 S(x, j) = min(S(x, 1), D(x, j)), with
+    // D(x, j) = min over k in [1, j) of S(left, k) + S(right, j - k). dec(x, j) is the k that
+    // reaches S(x, j), or 0 where x fills one slot; dec(x, 4) is the split of x's slots when x
+    // roots a 4-wide node.
+    float4* S;        // S(x, 1..4)
+    uchar4* dec;      // dec(x, 1..4) (dec(x, 1) = 0)
+};
+struct Sah { int max_leaf; float ct, ci, floor_pad; };
+
+struct Kid { float3 lo, hi; float cost; int cnt, icount; bool collapsed; float4 S; };
+
+__device__ __forceinline__ Kid load_kid(const Tree& t, int x) {
+    const float4 a = __ldcg(&t.lo[x]), b = __ldcg(&t.hi[x]);
+    Kid k;
+    k.lo = mk(a.x, a.y, a.z);
+    k.hi = mk(b.x, b.y, b.z);
+    k.cost = a.w;
+    const int w = __float_as_int(b.w);
+    k.cnt = w >> 1;
+    k.collapsed = (w & 1) != 0;
+    k.icount = __ldcg(&t.icount[x]);
+    k.S = k.collapsed ? make_float4(0.f, 0.f, 0.f, 0.f) : __ldcg(&t.S[x]);
+    return k;
+}
+
+__global__ void k_init_leaves(const uint32_t* __restrict__ sorted, int n, const float* __restrict__ verts,
+                              const uint32_t* __restrict__ idx, Tree t, Sah sah, int* clusters) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    int pos = 0, x = k, p;
-    while ((p = t.parent[x]) >= 0) {
-        if (t.right[p] == x) pos += s.cnt[t.left[p]];
-        x = p;
+    float3 lo, hi;
+    tri_box(verts, idx, sorted[k], &lo, &hi);
+    t.lo[k] = make_float4(lo.x, lo.y, lo.z, sah.ci * half_area(lo, hi));
+    t.hi[k] = make_float4(hi.x, hi.y, hi.z, __int_as_float((1 << 1) | 1));
+    t.icount[k] = 0;
+    clusters[k] = k;
+}
+
+// Makes node `x` the parent of clusters a and b: its box, SAH cost and collapse, and its row of the
+// 4-wide grouping.
+__device__ __forceinline__ void merge_node(const Tree& t, const Sah& sah, int x, int a, int b) {
+    const Kid l = load_kid(t, a), r = load_kid(t, b);
+    const float3 lo = mk(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z));
+    const float3 hi = mk(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z));
+    const float A = half_area(lo, hi);
+    const int c = l.cnt + r.cnt;
+    const float split = sah.ct * A + l.cost + r.cost;
+    const float leaf = c <= sah.max_leaf ? sah.ci * A * (float)c : FLT_MAX;
+    const bool collapsed = leaf <= split;
+    t.lo[x] = make_float4(lo.x, lo.y, lo.z, collapsed ? leaf : split);
+    t.hi[x] = make_float4(hi.x, hi.y, hi.z, __int_as_float((c << 1) | (collapsed ? 1 : 0)));
+    t.icount[x] = collapsed ? 0 : 1 + l.icount + r.icount;
+    t.child[x] = make_int2(a, b);
+    t.up[a] = make_int4(x, 1, 0, collapsed ? 1 : 0);
+    t.up[b] = make_int4(x, 1 + l.icount, l.cnt, collapsed ? 1 : 0);
+    // the grouping's areas are of the padded child boxes' union, as the stored nodes have them
+    float al[3] = {l.lo.x, l.lo.y, l.lo.z}, ah[3] = {l.hi.x, l.hi.y, l.hi.z};
+    float bl[3] = {r.lo.x, r.lo.y, r.lo.z}, bh[3] = {r.hi.x, r.hi.y, r.hi.z};
+    float d[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        pad_box(al[k], ah[k], sah.floor_pad);
+        pad_box(bl[k], bh[k], sah.floor_pad);
+        d[k] = fmaxf(ah[k], bh[k]) - fminf(al[k], bl[k]);
+    }
+    const float sc[2][5] = {{0.f, l.S.x, l.S.y, l.S.z, l.S.w}, {0.f, r.S.x, r.S.y, r.S.z, r.S.w}};
+    float D[5] = {0.f, 0.f, FLT_MAX, FLT_MAX, FLT_MAX};
+    int kd[5] = {0, 0, 0, 0, 0};
+#pragma unroll
+    for (int j = 2; j <= 4; ++j)
+#pragma unroll
+        for (int k = 1; k < j; ++k) {
+            const float cost = sc[0][k] + sc[1][j - k];
+            if (cost < D[j]) { D[j] = cost; kd[j] = k; }
+        }
+    const float s1 = (d[0] * d[1] + d[1] * d[2] + d[2] * d[0]) + D[4];
+    const bool one2 = s1 <= D[2], one3 = s1 <= D[3];      // s1 = A + D(x, 4) > D(x, 4)
+    t.S[x] = make_float4(s1, one2 ? s1 : D[2], one3 ? s1 : D[3], D[4]);
+    t.dec[x] = make_uchar4(0, (unsigned char)(one2 ? 0 : kd[2]), (unsigned char)(one3 ? 0 : kd[3]), (unsigned char)kd[4]);
+}
+
+// ------------------------------------------------------------ PLOC
+constexpr int kPlocThreads = 256;
+constexpr int kPlocTile = 2 * kPlocThreads;
+constexpr int kPlocBatch = 8;      // iterations between host reads of the count
+constexpr int kMaxRadius = 32;
+constexpr int kSuper = 64;         // tiles per partial sum of the compaction
+constexpr int kFinish = 2048;      // from this many clusters on, one block does the rest
+
+// The nearest neighbour of cluster i of m: boxes lo/hi are those of clusters i - r.. (s + 0) on,
+// limited to [0, m). Strict order on unordered pairs: (area, min index, max index); j increases,
+// so for equal area the first j seen has the smaller pair key.
+__device__ __forceinline__ int nearest(const float3* lo, const float3* hi, int at, int i, int m, int r) {
+    const float3 mlo = lo[at], mhi = hi[at];
+    float best = FLT_MAX;
+    int bj = -1;
+    const int j0 = max(0, i - r), j1 = min(m - 1, i + r);
+    for (int j = j0; j <= j1; ++j) {
+        if (j == i) continue;
+        const int k = at + (j - i);
+        const float3 ulo = mk(fminf(mlo.x, lo[k].x), fminf(mlo.y, lo[k].y), fminf(mlo.z, lo[k].z));
+        const float3 uhi = mk(fmaxf(mhi.x, hi[k].x), fmaxf(mhi.y, hi[k].y), fmaxf(mhi.z, hi[k].z));
+        const float a = half_area(ulo, uhi);
+        if (a < best) { best = a; bj = j; }
+    }
+    return bj;
+}
+
+// The same for clusters i and i + 1 (either may lie outside [0, m)): every box of the joint window is
+// read once.
+__device__ __forceinline__ void nearest2(const float3* lo, const float3* hi, int at, int i, int m, int r, int (&nn)[2]) {
+    const bool in0 = i >= 0 && i < m, in1 = i + 1 >= 0 && i + 1 < m;
+    const float3 z = mk(0.f, 0.f, 0.f);
+    const float3 lo0 = in0 ? lo[at] : z, hi0 = in0 ? hi[at] : z;
+    const float3 lo1 = in1 ? lo[at + 1] : z, hi1 = in1 ? hi[at + 1] : z;
+    float b0 = FLT_MAX, b1 = FLT_MAX;
+    int n0 = -1, n1 = -1;
+    const int j0 = max(0, i - r), j1 = min(m - 1, i + 1 + r);
+    for (int j = j0; j <= j1; ++j) {
+        const int k = at + (j - i);
+        const float3 l = lo[k], h = hi[k];
+        const float a0 = half_area(mk(fminf(lo0.x, l.x), fminf(lo0.y, l.y), fminf(lo0.z, l.z)),
+                                   mk(fmaxf(hi0.x, h.x), fmaxf(hi0.y, h.y), fmaxf(hi0.z, h.z)));
+        const float a1 = half_area(mk(fminf(lo1.x, l.x), fminf(lo1.y, l.y), fminf(lo1.z, l.z)),
+                                   mk(fmaxf(hi1.x, h.x), fmaxf(hi1.y, h.y), fmaxf(hi1.z, h.z)));
+        if (a0 < b0 && j != i && j <= i + r) { b0 = a0; n0 = j; }
+        if (a1 < b1 && j != i + 1 && j >= i + 1 - r) { b1 = a1; n1 = j; }
+    }
+    nn[0] = in0 ? n0 : -1;
+    nn[1] = in1 ? n1 : -1;
+}
+
+// One iteration's search and merges. A block owns kPlocTile - 2 r clusters and finds the
+// neighbours of r more on either side, so that it can tell its own mutual pairs without another
+// launch. Each thread searches for two adjacent clusters, whose windows share all but two boxes:
+// the search is bound by the shared-memory reads of its 2 r boxes a cluster.
+// out[i]: cluster i after the iteration, -1 if it was merged into its partner. Counts of
+// kept clusters per tile and per kSuper tiles. From kFinish clusters on it only passes them on.
+__global__ void __launch_bounds__(kPlocThreads) k_ploc_merge(const int* __restrict__ clusters, BuildState* st, int parity,
+                                                             Tree t, Sah sah, int r, int* __restrict__ out,
+                                                             uint32_t* __restrict__ cnt, uint32_t* super) {
+    __shared__ float3 s_lo[kPlocTile + 2 * kMaxRadius], s_hi[kPlocTile + 2 * kMaxRadius];
+    __shared__ int s_nn[kPlocTile];
+    __shared__ uint32_t s_scan[33];
+    __shared__ int s_base;
+    const int m = st->m[parity];
+    const int tile = kPlocTile - 2 * r, start = blockIdx.x * tile;
+    if (start >= m) return;
+    const int tid = threadIdx.x, g0 = start - r + 2 * tid;
+    bool own[2], keep[2], merges[2] = {false, false};
+    int id[2], j[2] = {-1, -1};
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int k = 2 * tid + q, g = g0 + q;
+        own[q] = k >= r && k < r + tile && g < m;
+        keep[q] = own[q];
+        id[q] = own[q] ? clusters[g] : -1;
+    }
+    if (m > kFinish) {
+        for (int k = tid; k < kPlocTile + 2 * r; k += kPlocThreads) {
+            const int q = start - 2 * r + k;
+            if (q >= 0 && q < m) {
+                const int c = clusters[q];
+                const float4 a = t.lo[c], b = t.hi[c];
+                s_lo[k] = mk(a.x, a.y, a.z);
+                s_hi[k] = mk(b.x, b.y, b.z);
+            }
+        }
+        __syncthreads();
+        int nn[2] = {-1, -1};
+        if (g0 + 1 >= 0 && g0 < m) nearest2(s_lo, s_hi, 2 * tid + r, g0, m, r, nn);
+        s_nn[2 * tid] = nn[0];
+        s_nn[2 * tid + 1] = nn[1];
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (!own[q]) continue;
+            const int g = g0 + q;
+            j[q] = nn[q];
+            const bool mutual = j[q] >= 0 && s_nn[j[q] - (start - r)] == g;
+            merges[q] = mutual && g < j[q];
+            keep[q] = !mutual || merges[q];
+        }
+    }
+    // both counts in one scan: merges in the low half, kept clusters in the high one
+    uint32_t total;
+    const uint32_t pre = block_excl_scan((uint32_t)(merges[0] + merges[1]) | ((uint32_t)(keep[0] + keep[1]) << 16), s_scan, &total);
+    const int nmerge = (int)(total & 0xffffu);
+    if (tid == 0) {
+        s_base = nmerge ? atomicAdd(&st->node, nmerge) : 0;
+        cnt[blockIdx.x] = total >> 16;
+        atomicAdd(&super[blockIdx.x / kSuper], total >> 16);
+    }
+    __syncthreads();
+    int x = s_base + (int)(pre & 0xffffu);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        if (!own[q]) continue;
+        if (merges[q]) {
+            merge_node(t, sah, x, id[q], clusters[j[q]]);
+            id[q] = x++;
+        }
+        out[g0 + q] = keep[q] ? id[q] : -1;
+    }
+}
+
+// Compacts the iteration's clusters in order (same tiles) and hands on their count; clears the
+// partial sums of the next iteration.
+__global__ void __launch_bounds__(kPlocThreads) k_ploc_compact(const int* __restrict__ in, BuildState* st, int parity, int r,
+                                                               const uint32_t* __restrict__ cnt,
+                                                               const uint32_t* __restrict__ super, uint32_t* next_super,
+                                                               int* __restrict__ clusters) {
+    __shared__ uint32_t s_scan[33];
+    const int m = st->m[parity];
+    const int tile = kPlocTile - 2 * r, start = blockIdx.x * tile;
+    if (start >= m) return;
+    const int tid = threadIdx.x, sb = blockIdx.x / kSuper;
+    uint32_t before = 0, base, own;
+    for (int k = tid; k < sb; k += kPlocThreads) before += super[k];
+    for (int k = sb * kSuper + tid; k < (int)blockIdx.x; k += kPlocThreads) before += cnt[k];
+    block_excl_scan(before, s_scan, &base);
+    __syncthreads();
+    int id[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) id[q] = 2 * tid + q < tile && start + 2 * tid + q < m ? in[start + 2 * tid + q] : -1;
+    uint32_t at = base + block_excl_scan((uint32_t)(id[0] >= 0) + (uint32_t)(id[1] >= 0), s_scan, &own);
+    if (id[0] >= 0) clusters[at++] = id[0];
+    if (id[1] >= 0) clusters[at] = id[1];
+    if (blockIdx.x % kSuper == 0 && tid == 0) next_super[sb] = 0u;
+    if (tid == 0 && start + tile >= m) st->m[parity ^ 1] = (int)(base + own);
+}
+
+// All remaining iterations in one block, the clusters' boxes in shared memory. Then the root: never
+// a leaf (a tree has at least one interior node).
+__global__ void __launch_bounds__(1024) k_ploc_finish(const int* __restrict__ clusters, BuildState* st, int parity, Tree t,
+                                                      Sah sah, int r) {
+    extern __shared__ char s_mem[];
+    float3* s_lo = reinterpret_cast<float3*>(s_mem);
+    float3* s_hi = s_lo + kFinish;
+    int* s_id = reinterpret_cast<int*>(s_hi + kFinish);
+    int* s_nn = s_id + kFinish;
+    __shared__ uint32_t s_scan[33];
+    __shared__ int s_base;
+    int m = st->m[parity];
+    if (m > kFinish) return;
+    const int tid = threadIdx.x;
+    for (int k = tid; k < m; k += 1024) {
+        const int c = clusters[k];
+        const float4 a = t.lo[c], b = t.hi[c];
+        s_id[k] = c;
+        s_lo[k] = mk(a.x, a.y, a.z);
+        s_hi[k] = mk(b.x, b.y, b.z);
+    }
+    __syncthreads();
+    while (m > 1) {
+        for (int k = tid; k < m; k += 1024) s_nn[k] = nearest(s_lo, s_hi, k, k, m, r);
+        __syncthreads();
+        // thread t has clusters 2 t and 2 t + 1, so that ranks follow the order
+        int id[2];
+        float3 lo[2], hi[2];
+        bool keep[2], mer[2];
+        int partner[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int k = 2 * tid + q;
+            keep[q] = mer[q] = false;
+            partner[q] = -1;
+            id[q] = -1;
+            if (k >= m) continue;
+            const int j = s_nn[k];
+            const bool mutual = j >= 0 && s_nn[j] == k;
+            mer[q] = mutual && k < j;
+            keep[q] = !mutual || mer[q];
+            id[q] = s_id[k];
+            lo[q] = s_lo[k];
+            hi[q] = s_hi[k];
+            if (mer[q]) {
+                partner[q] = s_id[j];
+                lo[q] = mk(fminf(lo[q].x, s_lo[j].x), fminf(lo[q].y, s_lo[j].y), fminf(lo[q].z, s_lo[j].z));
+                hi[q] = mk(fmaxf(hi[q].x, s_hi[j].x), fmaxf(hi[q].y, s_hi[j].y), fmaxf(hi[q].z, s_hi[j].z));
+            }
+        }
+        // both counts in one scan: merges in the low half, kept clusters in the high one
+        uint32_t total;
+        const uint32_t pre = block_excl_scan((mer[0] + mer[1]) | ((uint32_t)(keep[0] + keep[1]) << 16), s_scan, &total);
+        const int nmerge = (int)(total & 0xffffu), nkeep = (int)(total >> 16);
+        if (nmerge == 0) break;                      // no progress: the host reports it
+        if (tid == 0) { s_base = st->node; st->node = s_base + nmerge; }
+        __syncthreads();
+        int mr = (int)(pre & 0xffffu), kr = (int)(pre >> 16);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (mer[q]) {
+                const int x = s_base + mr++;
+                merge_node(t, sah, x, id[q], partner[q]);
+                id[q] = x;
+            }
+            if (keep[q]) {
+                s_id[kr] = id[q];
+                s_lo[kr] = lo[q];
+                s_hi[kr] = hi[q];
+                ++kr;
+            }
+        }
+        m = nkeep;
+        __syncthreads();
+    }
+    if (tid != 0) return;
+    st->m[0] = st->m[1] = m;
+    if (m != 1) return;
+    const int root = s_id[0];
+    const int2 c = t.child[root];
+    const int n = 1 + t.icount[c.x] + t.icount[c.y];   // as if the root were not collapsed
+    t.up[root] = make_int4(-1, 0, 0, 0);
+    t.up[c.x].w = 0;
+    t.up[c.y].w = 0;
+    st->root = root;
+    st->num_nodes = n;
+}
+
+// ------------------------------------------------------------ layout
+__global__ void k_layout_tris(int n, Tree t, const uint32_t* __restrict__ sorted, const float* __restrict__ verts,
+                              const uint32_t* __restrict__ idx, BvhTri* __restrict__ out) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    int pos = 0;
+    for (int x = k; x >= 0;) {
+        const int4 u = __ldg(&t.up[x]);
+        pos += u.z;
+        x = u.x;
     }
     const uint32_t prim = sorted[k];
-    float3 a = ld3(verts, idx[3 * prim]), b = ld3(verts, idx[3 * prim + 1]), c = ld3(verts, idx[3 * prim + 2]);
+    float3 a = ld3(verts, idx[3 * (size_t)prim]), b = ld3(verts, idx[3 * (size_t)prim + 1]), c = ld3(verts, idx[3 * (size_t)prim + 2]);
     float3 e1 = xsub(b, a), e2 = xsub(c, a);
     BvhTri tr;
     tr.p1 = make_float4(a.x, a.y, a.z, __int_as_float((int)prim));
@@ -402,44 +646,54 @@ __global__ void k_layout_tris(int n, Tree t, Sah s, const uint32_t* sorted, cons
     out[pos] = tr;
 }
 
-__global__ void k_layout_nodes(int n, int total, Tree t, Sah s, float floor_pad, BvhNode* out, int* max_depth) {
+// dec: the 4-wide grouping's decisions, by depth-first index
+__global__ void k_layout_nodes(int n, int total, Tree t, float floor_pad, BuildState* st, BvhNode* __restrict__ out,
+                               uchar4* __restrict__ dec) {
     const int x = n + blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= total || s.collapsed[x]) return;
-    int idx = 0, start = 0, y = x, p, depth = 1;
-    while ((p = t.parent[y]) >= 0) {
-        if (s.collapsed[p]) return;      // inside a collapsed leaf subtree
-        const int l = t.left[p];
-        if (t.right[p] == y) { idx += 1 + s.icount[l]; start += s.cnt[l]; }
-        else idx += 1;
-        y = p;
-        ++depth;
+    int depth = 0;
+    bool live = x < total && (x == st->root || !(__float_as_int(t.hi[x].w) & 1));
+    if (live) {
+        int idx = 0, start = 0;
+        depth = 1;
+        for (int4 u = __ldg(&t.up[x]); u.x >= 0; u = __ldg(&t.up[u.x])) {
+            if (u.w) { live = false; depth = 0; break; }      // inside a collapsed leaf subtree
+            idx += u.y;
+            start += u.z;
+            ++depth;
+        }
+        if (live) {
+            const int2 ch = t.child[x];
+            const int c[2] = {ch.x, ch.y};
+            const int lw = __float_as_int(t.hi[ch.x].w);
+            const int cidx[2] = {idx + 1, idx + 1 + t.icount[ch.x]};
+            const int cstart[2] = {start, start + (lw >> 1)};
+            int ref[2], cnt[2];
+            float blo[2][3], bhi[2][3];
+            for (int k = 0; k < 2; ++k) {
+                const float4 a = t.lo[c[k]], b = t.hi[c[k]];
+                const int w = __float_as_int(b.w);
+                if (w & 1) { ref[k] = ~((cstart[k] << 5) | (w >> 1)); cnt[k] = w >> 1; }
+                else { ref[k] = cidx[k]; cnt[k] = 0; }
+                blo[k][0] = a.x; blo[k][1] = a.y; blo[k][2] = a.z;
+                bhi[k][0] = b.x; bhi[k][1] = b.y; bhi[k][2] = b.z;
+                for (int d = 0; d < 3; ++d) pad_box(blo[k][d], bhi[k][d], floor_pad);
+            }
+            BvhNode nd;
+            nd.a = make_float4(blo[0][0], bhi[0][0], blo[0][1], bhi[0][1]);
+            nd.b = make_float4(blo[1][0], bhi[1][0], blo[1][1], bhi[1][1]);
+            nd.c = make_float4(blo[0][2], bhi[0][2], blo[1][2], bhi[1][2]);
+            nd.d = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(cnt[0]), __int_as_float(cnt[1]));
+            out[idx] = nd;
+            dec[idx] = t.dec[x];
+        }
     }
-    atomicMax(max_depth, depth);
-    const int l = t.left[x], r = t.right[x];
-    int ref[2], cnt[2];
-    const int ch[2] = {l, r};
-    const int cidx[2] = {idx + 1, idx + 1 + s.icount[l]};
-    const int cstart[2] = {start, start + s.cnt[l]};
-    float blo[2][3], bhi[2][3];
-    for (int k = 0; k < 2; ++k) {
-        const int c = ch[k];
-        if (c < n || s.collapsed[c]) { ref[k] = ~((cstart[k] << 5) | s.cnt[c]); cnt[k] = s.cnt[c]; }
-        else { ref[k] = cidx[k]; cnt[k] = 0; }
-        float4 a = t.lo[c], b = t.hi[c];
-        blo[k][0] = a.x; blo[k][1] = a.y; blo[k][2] = a.z;
-        bhi[k][0] = b.x; bhi[k][1] = b.y; bhi[k][2] = b.z;
-        for (int d = 0; d < 3; ++d) pad_box(blo[k][d], bhi[k][d], floor_pad);
-    }
-    BvhNode nd;
-    nd.a = make_float4(blo[0][0], bhi[0][0], blo[0][1], bhi[0][1]);
-    nd.b = make_float4(blo[1][0], bhi[1][0], blo[1][1], bhi[1][1]);
-    nd.c = make_float4(blo[0][2], bhi[0][2], blo[1][2], bhi[1][2]);
-    nd.d = make_float4(__int_as_float(ref[0]), __int_as_float(ref[1]), __int_as_float(cnt[0]), __int_as_float(cnt[1]));
-    out[idx] = nd;
+    depth = __reduce_max_sync(0xffffffffu, depth);
+    if ((threadIdx.x & 31) == 0 && depth > *(volatile int*)&st->depth) atomicMax(&st->depth, depth);
 }
 
 // single triangle: one node with a leaf child and an empty child
-__global__ void k_single(const float* verts, const uint32_t* idx, BvhNode* nodes, BvhTri* tris) {
+__global__ void k_single(const float* verts, const uint32_t* idx, BvhNode* nodes, BvhTri* tris,
+                         uchar4* dec, BuildState* st) {
     float3 a = ld3(verts, idx[0]), b = ld3(verts, idx[1]), c = ld3(verts, idx[2]);
     float lo[3] = {fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y), fminf(fminf(a.z, b.z), c.z)};
     float hi[3] = {fmaxf(fmaxf(a.x, b.x), c.x), fmaxf(fmaxf(a.y, b.y), c.y), fmaxf(fmaxf(a.z, b.z), c.z)};
@@ -450,122 +704,16 @@ __global__ void k_single(const float* verts, const uint32_t* idx, BvhNode* nodes
     nd.c = make_float4(lo[2], hi[2], FLT_MAX, -FLT_MAX);
     nd.d = make_float4(__int_as_float(~1), __int_as_float(~0), __int_as_float(1), __int_as_float(0));
     nodes[0] = nd;
+    dec[0] = make_uchar4(0, 1, 1, 1);   // two leaves
+    st->depth = 1;
+    st->num_nodes = 1;
     float3 e1 = xsub(b, a), e2 = xsub(c, a);
     tris[0].p1 = make_float4(a.x, a.y, a.z, __int_as_float(0));
     tris[0].e1 = make_float4(e1.x, e1.y, e1.z, 0.f);
     tris[0].e2 = make_float4(e2.x, e2.y, e2.z, 0.f);
 }
 
-}  // namespace
-
-cudaError_t bvh_build_device(const float* verts, const uint32_t* idx, int n, const BvhBuildOptions& opt,
-                             DeviceBvh* out, cudaStream_t s) {
-    if (n < 1) return cudaErrorInvalidValue;
-    *out = DeviceBvh();
-    out->num_tris = n;
-    CK(dalloc(&out->tris, n, s));
-    if (n == 1) {
-        CK(dalloc(&out->nodes, 1, s));
-        out->num_nodes = 1;
-        out->depth = 1;
-        k_single<<<1, 1, 0, s>>>(verts, idx, out->nodes, out->tris);
-        return cudaGetLastError();
-    }
-    const int total = 2 * n - 1;
-    const int T = 256;
-    float4 *plo, *phi, *cent;
-    uint32_t *keys, *vals;
-    int* gb;
-    CK(dalloc(&plo, n, s)); CK(dalloc(&phi, n, s)); CK(dalloc(&cent, n, s));
-    CK(dalloc(&keys, n, s)); CK(dalloc(&vals, n, s)); CK(dalloc(&gb, 8, s));
-    k_init_bounds<<<1, 32, 0, s>>>(gb);
-    k_prim_setup<<<div_up(n, T), T, 0, s>>>(verts, idx, n, plo, phi, cent, gb);
-    k_morton<<<div_up(n, T), T, 0, s>>>(cent, n, gb, keys, vals);
-    CK(radix_sort_pairs(keys, vals, n, 32, s));
-
-    Tree t;
-    CK(dalloc(&t.lo, total, s)); CK(dalloc(&t.hi, total, s));
-    CK(dalloc(&t.left, total, s)); CK(dalloc(&t.right, total, s)); CK(dalloc(&t.parent, total, s));
-    int *ca, *cb, *nn, *counter;
-    uint32_t *keep, *pos;
-    CK(dalloc(&ca, n, s)); CK(dalloc(&cb, n, s)); CK(dalloc(&nn, n, s)); CK(dalloc(&counter, 1, s));
-    CK(dalloc(&keep, n, s)); CK(dalloc(&pos, n, s));
-    k_init_leaves<<<div_up(n, T), T, 0, s>>>(vals, n, plo, phi, t, ca);
-    CK(cudaMemcpyAsync(counter, &n, sizeof(int), cudaMemcpyHostToDevice, s));
-    const int r = opt.ploc_radius < 1 ? 1 : (opt.ploc_radius > kMaxRadius ? kMaxRadius : opt.ploc_radius);
-    // kPlocBatch iterations between host reads of the count; once one cluster is left the
-    // remaining iterations of a batch keep it as it is
-    int m = n;
-    int* dm = nullptr;
-    CK(dalloc(&dm, 1, s));
-    CK(cudaMemcpyAsync(dm, &n, sizeof(int), cudaMemcpyHostToDevice, s));
-    while (m > 1) {
-        for (int it = 0; it < kPlocBatch; ++it) {
-            k_ploc_nn<<<div_up(m, kNnBlock), kNnBlock, 0, s>>>(ca, dm, t, nn, r);
-            k_ploc_merge<<<div_up(m, T), T, 0, s>>>(ca, dm, m, nn, t, counter, keep);
-            CK(exclusive_scan(keep, pos, m, s));
-            k_compact<<<div_up(m, T), T, 0, s>>>(ca, keep, pos, dm, cb);
-            k_ploc_count<<<1, 1, 0, s>>>(keep, pos, dm);
-            std::swap(ca, cb);
-        }
-        int m2 = 0;
-        CK(cudaMemcpyAsync(&m2, dm, sizeof(int), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (m2 < 1 || (m2 > 1 && m2 >= m)) return cudaErrorUnknown;   // no progress: impossible with the strict pair order
-        m = m2;
-    }
-    dfree(dm, s);
-    int root = 0;
-    CK(cudaMemcpyAsync(&root, ca, sizeof(int), cudaMemcpyDeviceToHost, s));
-
-    Sah sah;
-    CK(dalloc(&sah.cnt, total, s)); CK(dalloc(&sah.icount, total, s)); CK(dalloc(&sah.visit, total, s));
-    CK(dalloc(&sah.cost, total, s)); CK(dalloc(&sah.collapsed, total, s));
-    CK(cudaMemsetAsync(sah.visit, 0, sizeof(int) * total, s));
-    k_bottom_up<<<div_up(n, T), T, 0, s>>>(n, t, sah, opt.max_leaf < 1 ? 1 : opt.max_leaf, opt.cost_traverse,
-                                           opt.cost_intersect);
-    CK(cudaStreamSynchronize(s));
-    k_fix_root<<<1, 1, 0, s>>>(root, t, sah);
-    int num_nodes = 0;
-    CK(cudaMemcpyAsync(&num_nodes, sah.icount + root, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    out->num_nodes = num_nodes;
-    CK(dalloc(&out->nodes, num_nodes, s));
-    // scene bounds for the caller and the scene-relative box padding
-    float4 rb[2];
-    CK(cudaMemcpyAsync(&rb[0], t.lo + root, sizeof(float4), cudaMemcpyDeviceToHost, s));
-    CK(cudaMemcpyAsync(&rb[1], t.hi + root, sizeof(float4), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    out->lo[0] = rb[0].x; out->lo[1] = rb[0].y; out->lo[2] = rb[0].z;
-    out->hi[0] = rb[1].x; out->hi[1] = rb[1].y; out->hi[2] = rb[1].z;
-    float scale = 0.f;
-    for (int k = 0; k < 3; ++k) scale = fmaxf(scale, fmaxf(fabsf(out->lo[k]), fabsf(out->hi[k])));
-    k_layout_tris<<<div_up(n, T), T, 0, s>>>(n, t, sah, vals, verts, idx, out->tris);
-    int* dmax;
-    CK(dalloc(&dmax, 1, s));
-    CK(cudaMemsetAsync(dmax, 0, sizeof(int), s));
-    k_layout_nodes<<<div_up(n - 1, T), T, 0, s>>>(n, total, t, sah, scale * 9.5367432e-7f, out->nodes, dmax);
-    CK(cudaMemcpyAsync(&out->depth, dmax, sizeof(int), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    dfree(dmax, s);
-
-    dfree(plo, s); dfree(phi, s); dfree(cent, s); dfree(keys, s); dfree(vals, s); dfree(gb, s);
-    dfree(t.lo, s); dfree(t.hi, s); dfree(t.left, s); dfree(t.right, s); dfree(t.parent, s);
-    dfree(ca, s); dfree(cb, s); dfree(nn, s); dfree(counter, s); dfree(keep, s); dfree(pos, s);
-    dfree(sah.cnt, s); dfree(sah.icount, s); dfree(sah.visit, s); dfree(sah.cost, s); dfree(sah.collapsed, s);
-    return cudaGetLastError();
-}
-
-void bvh_free_device(DeviceBvh* bvh, cudaStream_t s) {
-    if (bvh->nodes) cudaFreeAsync(bvh->nodes, s);
-    if (bvh->tris) cudaFreeAsync(bvh->tris, s);
-    if (bvh->nodes4) cudaFreeAsync(bvh->nodes4, s);
-    if (bvh->nodes4q) cudaFreeAsync(bvh->nodes4q, s);
-    *bvh = DeviceBvh();
-}
-
-namespace {
-
+// ------------------------------------------------------------ 4-wide tree
 __device__ __forceinline__ void child_of(const BvhNode& nd, int k, float lo[3], float hi[3], int* ref) {
     if (k == 0) {
         lo[0] = nd.a.x; hi[0] = nd.a.y; lo[1] = nd.a.z; hi[1] = nd.a.w; lo[2] = nd.c.x; hi[2] = nd.c.y;
@@ -576,178 +724,88 @@ __device__ __forceinline__ void child_of(const BvhNode& nd, int k, float lo[3], 
     }
 }
 
-__device__ __forceinline__ float half_area(const float lo[3], const float hi[3]) {
-    const float dx = hi[0] - lo[0], dy = hi[1] - lo[1], dz = hi[2] - lo[2];
-    return dx * dy + dy * dz + dz * dx;
-}
-
-// Writes the 4-wide node at index `at` with children (lo, hi, ref)[0..n): interior children
-// get the next 4-wide indices and join the next level's front.
-__device__ void write_node4(const float (&lo)[4][3], const float (&hi)[4][3], const int (&ref)[4], int n, int at,
-                            BvhNode4* __restrict__ out, int* counters, int2* __restrict__ next, int cap) {
-    float v[6][4];
-    int r[4];
-    for (int k = 0; k < 4; ++k) {
-        if (k >= n) {
-            for (int d = 0; d < 6; ++d) v[d][k] = __int_as_float(0x7f800000);   // +inf: never entered
-            r[k] = ~0;
-            continue;
-        }
-        v[0][k] = lo[k][0]; v[1][k] = hi[k][0]; v[2][k] = lo[k][1];
-        v[3][k] = hi[k][1]; v[4][k] = lo[k][2]; v[5][k] = hi[k][2];
-        if (ref[k] >= 0) {
-            const int j = atomicAdd(&counters[0], 1);
-            const int q = atomicAdd(&counters[1], 1);
-            if (j < cap && q < cap) next[q] = make_int2(ref[k], j);
-            r[k] = j;
-        } else {
-            r[k] = ref[k];
-        }
-    }
-    if (at >= cap) return;
-    BvhNode4 o;
-    o.lox = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
-    o.hix = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
-    o.loy = make_float4(v[2][0], v[2][1], v[2][2], v[2][3]);
-    o.hiy = make_float4(v[3][0], v[3][1], v[3][2], v[3][3]);
-    o.loz = make_float4(v[4][0], v[4][1], v[4][2], v[4][3]);
-    o.hiz = make_float4(v[5][0], v[5][1], v[5][2], v[5][3]);
-    o.ref = make_int4(r[0], r[1], r[2], r[3]);
-    o.pad = make_int4(0, 0, 0, 0);
-    out[at] = o;
-}
-
-// SAH-optimal grouping of the binary tree into 4-wide nodes: a dynamic program over the
-// binary tree, bottom up (the 8-wide form is in Ylitie, Karras and Laine, "Efficient
-// Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs", HPG 2017). The leaves are
-// fixed, so groupings differ in SAH cost only by the summed surface area of the 4-wide
-// nodes. S(x, j) is the least such sum for the subtree of binary node x when it may fill j
-// of its parent's child slots (a leaf costs nothing): S(x, 1) = A(x) + D(x, 4), and for
-// j > 1 S(x, j) = min(S(x, 1), D(x, j)), with D(x, j) = min over k in [1, j) of
-// S(left, k) + S(right, j - k). dec(x, j) is the k that reaches S(x, j), or 0 where x fills
-// one slot; dec(x, 4) is the split of x's slots when x roots a 4-wide node.
-struct Dp4 {
-    float4* S;          // S(x, 1..4)
-    uchar4* dec;        // dec(x, 1..4) (dec(x, 1) = 0)
-    int* parent;        // binary parent, -1 at the root
-    int* visit;         // arrivals so far, started at the number of leaf children
-};
-
-__global__ void k_dp4_init(const BvhNode* __restrict__ n2, int nn, Dp4 d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nn) return;
-    const BvhNode nd = n2[i];
-    const int r0 = __float_as_int(nd.d.x), r1 = __float_as_int(nd.d.y);
-    d.visit[i] = (r0 < 0) + (r1 < 0);
-    if (i == 0) d.parent[0] = -1;
-    if (r0 >= 0) d.parent[r0] = i;
-    if (r1 >= 0) d.parent[r1] = i;
-}
-
-__device__ void dp4_node(const BvhNode* __restrict__ n2, int x, Dp4 d) {
-    const BvhNode nd = n2[x];
-    float lo[2][3], hi[2][3];
-    int r[2];
-    child_of(nd, 0, lo[0], hi[0], &r[0]);
-    child_of(nd, 1, lo[1], hi[1], &r[1]);
-    float ulo[3], uhi[3];
-    for (int a = 0; a < 3; ++a) { ulo[a] = fminf(lo[0][a], lo[1][a]); uhi[a] = fmaxf(hi[0][a], hi[1][a]); }
-    float sc[2][5];
-    for (int c = 0; c < 2; ++c) {
-        sc[c][0] = 0.f;
-        if (r[c] >= 0) {
-            const float4 v = __ldcg(&d.S[r[c]]);
-            sc[c][1] = v.x; sc[c][2] = v.y; sc[c][3] = v.z; sc[c][4] = v.w;
-        } else {
-            sc[c][1] = sc[c][2] = sc[c][3] = sc[c][4] = 0.f;
-        }
-    }
-    float D[5] = {0.f, 0.f, FLT_MAX, FLT_MAX, FLT_MAX};
-    int kd[5] = {0, 0, 0, 0, 0};
-    for (int j = 2; j <= 4; ++j)
-        for (int k = 1; k < j; ++k) {
-            const float c = sc[0][k] + sc[1][j - k];
-            if (c < D[j]) { D[j] = c; kd[j] = k; }
-        }
-    const float s1 = half_area(ulo, uhi) + D[4];
-    float S[5];
-    int dec[5];
-    S[1] = s1; dec[1] = 0;
-    for (int j = 2; j <= 3; ++j) {
-        if (s1 <= D[j]) { S[j] = s1; dec[j] = 0; }
-        else { S[j] = D[j]; dec[j] = kd[j]; }
-    }
-    S[4] = D[4]; dec[4] = kd[4];   // s1 = A + D(x, 4) > D(x, 4)
-    d.S[x] = make_float4(S[1], S[2], S[3], S[4]);
-    d.dec[x] = make_uchar4(0, (unsigned char)dec[2], (unsigned char)dec[3], (unsigned char)dec[4]);
-}
-
-// Bottom-up sweep: a thread starts at each node whose children are both leaves; the last
-// child to finish carries on to the parent.
-__global__ void k_dp4(const BvhNode* __restrict__ n2, int nn, Dp4 d) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nn) return;
-    const BvhNode nd = n2[i];
-    if (__float_as_int(nd.d.x) >= 0 || __float_as_int(nd.d.y) >= 0) return;
-    int x = i;
-    while (true) {
-        dp4_node(n2, x, d);
-        __threadfence();
-        const int p = d.parent[x];
-        if (p < 0) return;
-        if (atomicAdd(&d.visit[p], 1) == 0) return;   // the sibling subtree is still running
-        __threadfence();
-        x = p;
-    }
-}
-
-// Between two levels: the next front becomes the current one (c[2]) and a non-empty level
-// is counted (c[3]).
-constexpr int kCollapseBatch = 8;
-__global__ void k_collapse_next(int* c) {
-    if (c[2] > 0) ++c[3];
-    c[2] = c[1];
-    c[1] = 0;
-}
-
 __device__ __forceinline__ int dec_for(uchar4 v, int j) { return j == 2 ? v.y : j == 3 ? v.z : j == 4 ? v.w : 0; }
 
 // One level of the collapse by the program's decisions: the node's four slots are split
 // between its binary children by dec(x, 4), and a child given j > 1 slots is opened while
 // dec(child, j) says so. Slots always add up to four, so a node gets at most four children.
-__global__ void k_collapse4_dp(const BvhNode* __restrict__ n2, const uchar4* __restrict__ dec,
-                               const int2* __restrict__ front, const int* nfront, BvhNode4* __restrict__ out,
-                               int* counters, int2* __restrict__ next, int cap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *nfront) return;
-    const int2 f = front[i];
-    float lo[4][3], hi[4][3];
-    int ref[4], bud[4];
-    int n = 2;
-    {
-        const BvhNode nd = n2[f.x];
-        child_of(nd, 0, lo[0], hi[0], &ref[0]);
-        child_of(nd, 1, lo[1], hi[1], &ref[1]);
-        const int k = dec[f.x].w;
-        bud[0] = k;
-        bud[1] = 4 - k;
-    }
-    while (n < 4) {
-        int e = -1, dd = 0;
-        for (int q = 0; q < n && e < 0; ++q) {
-            if (ref[q] < 0 || bud[q] < 2) continue;
-            const int v = dec_for(dec[ref[q]], bud[q]);
-            if (v > 0) { e = q; dd = v; }
+// front: the level's binary nodes, whose 4-wide nodes are first + 0, 1, ...; interior children
+// get the next indices in the order their warps arrive (one add a warp) and form the next level.
+__global__ void __launch_bounds__(256) k_collapse4_dp(const BvhNode* __restrict__ n2, const uchar4* __restrict__ dec,
+                                                      const int* __restrict__ front, BuildState* st, int level,
+                                                      BvhNode4* __restrict__ out, int* __restrict__ next, int cap) {
+    int first = 0;
+    for (int k = 0; k < level; ++k) first += st->front[k];
+    const int m = st->front[level], child0 = first + m;
+    const int lane = threadIdx.x & 31;
+    for (int b = blockIdx.x * blockDim.x; b < m; b += gridDim.x * blockDim.x) {
+        const int i = b + threadIdx.x;
+        const bool valid = i < m;
+        float lo[4][3], hi[4][3];
+        int ref[4] = {~0, ~0, ~0, ~0}, bud[4], n = 0, interior = 0;
+        if (valid) {
+            const int x = front[i];
+            n = 2;
+            {
+                const BvhNode nd = n2[x];
+                child_of(nd, 0, lo[0], hi[0], &ref[0]);
+                child_of(nd, 1, lo[1], hi[1], &ref[1]);
+                const int k = dec[x].w;
+                bud[0] = k;
+                bud[1] = 4 - k;
+            }
+            while (n < 4) {
+                int e = -1, dd = 0;
+                for (int q = 0; q < n && e < 0; ++q) {
+                    if (ref[q] < 0 || bud[q] < 2) continue;
+                    const int v = dec_for(dec[ref[q]], bud[q]);
+                    if (v > 0) { e = q; dd = v; }
+                }
+                if (e < 0) break;
+                const BvhNode c = n2[ref[e]];
+                child_of(c, 1, lo[n], hi[n], &ref[n]);
+                bud[n] = bud[e] - dd;
+                child_of(c, 0, lo[e], hi[e], &ref[e]);
+                bud[e] = dd;
+                ++n;
+            }
+            for (int k = 0; k < n; ++k) interior += ref[k] >= 0 ? 1 : 0;
         }
-        if (e < 0) break;
-        const BvhNode c = n2[ref[e]];
-        child_of(c, 1, lo[n], hi[n], &ref[n]);
-        bud[n] = bud[e] - dd;
-        child_of(c, 0, lo[e], hi[e], &ref[e]);
-        bud[e] = dd;
-        ++n;
+        const uint32_t incl = warp_incl_scan((uint32_t)interior);
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        int base = 0;
+        if (lane == 0 && all) base = atomicAdd(&st->front[level + 1], (int)all);
+        base = __shfl_sync(0xffffffffu, base, 0) + (int)incl - interior;
+        if (!valid) continue;
+        float v[6][4];
+        int r[4];
+        for (int k = 0; k < 4; ++k) {
+            if (k >= n) {
+                for (int d = 0; d < 6; ++d) v[d][k] = __int_as_float(0x7f800000);   // +inf: never entered
+                r[k] = ~0;
+                continue;
+            }
+            v[0][k] = lo[k][0]; v[1][k] = hi[k][0]; v[2][k] = lo[k][1];
+            v[3][k] = hi[k][1]; v[4][k] = lo[k][2]; v[5][k] = hi[k][2];
+            r[k] = ref[k];
+            if (ref[k] >= 0) {
+                if (base < cap) next[base] = ref[k];
+                r[k] = child0 + base;
+                ++base;
+            }
+        }
+        if (first + i >= cap) continue;
+        BvhNode4 o;
+        o.lox = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
+        o.hix = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
+        o.loy = make_float4(v[2][0], v[2][1], v[2][2], v[2][3]);
+        o.hiy = make_float4(v[3][0], v[3][1], v[3][2], v[3][3]);
+        o.loz = make_float4(v[4][0], v[4][1], v[4][2], v[4][3]);
+        o.hiz = make_float4(v[5][0], v[5][1], v[5][2], v[5][3]);
+        o.ref = make_int4(r[0], r[1], r[2], r[3]);
+        o.pad = make_int4(0, 0, 0, 0);
+        out[first + i] = o;
     }
-    write_node4(lo, hi, ref, n, f.y, out, counters, next, cap);
 }
 
 // One axis of a node's quantised boxes. The decoded plane of byte q is p + s (1 + q 2^-15) in
@@ -800,68 +858,187 @@ __global__ void k_quantise4(const BvhNode4* __restrict__ in, int n, BvhNode4Q* _
     out[i] = q;
 }
 
-}  // namespace
 
-cudaError_t bvh_collapse4(DeviceBvh* b, cudaStream_t s) {
-    if (!b->nodes || b->num_nodes < 1) return cudaErrorInvalidValue;
-    const int cap = b->num_nodes;             // a 4-wide tree has at most as many nodes as the binary one
-    int2 *fa = nullptr, *fb = nullptr;
-    int* counters = nullptr;
-    CK(dalloc(&b->nodes4, cap, s));
+// Scratch of one build: one allocation, cut into arrays.
+struct Arena {
+    char* base = nullptr;
+    size_t used = 0;
+    template <typename T> T* take(size_t n) {
+        T* p = reinterpret_cast<T*>(base + used);
+        used += (sizeof(T) * (n ? n : 1) + 255) & ~(size_t)255;
+        return p;
+    }
+};
+
+struct Scratch {
+    BuildState* st;
+    uint32_t *keys, *vals, *keys2, *vals2, *hist, *dsum;
+    Tree t;
+    int *ca, *cb, *out;
+    uint32_t *cnt, *super[2];
+    uchar4* dec;
+    int *fa, *fb;
+    void cut(Arena& a, size_t n, int tile) {
+        const size_t total = 2 * n, nb = (n + sort_tile(n) - 1) / sort_tile(n), tiles = (n + tile - 1) / tile;
+        st = a.take<BuildState>(1);
+        keys = a.take<uint32_t>(n); vals = a.take<uint32_t>(n);
+        keys2 = a.take<uint32_t>(n); vals2 = a.take<uint32_t>(n);
+        hist = a.take<uint32_t>(kDigits * nb); dsum = a.take<uint32_t>(kDigits);
+        t.lo = a.take<float4>(total); t.hi = a.take<float4>(total); t.icount = a.take<int>(total);
+        t.child = a.take<int2>(total); t.up = a.take<int4>(total);
+        t.S = a.take<float4>(total); t.dec = a.take<uchar4>(total);
+        ca = a.take<int>(n); cb = a.take<int>(n); out = a.take<int>(n);
+        cnt = a.take<uint32_t>(tiles);
+        for (uint32_t*& s : super) s = a.take<uint32_t>(tiles / kSuper + 1);
+        dec = a.take<uchar4>(n);
+        fa = a.take<int>(n); fb = a.take<int>(n);
+    }
+};
+
+cudaError_t read_state(BuildState* host, const BuildState* st, cudaStream_t s) {
+    cudaError_t e = cudaMemcpyAsync(host, st, sizeof(BuildState), cudaMemcpyDeviceToHost, s);
+    return e != cudaSuccess ? e : cudaStreamSynchronize(s);
+}
+
+cudaError_t build_with(Scratch& w, const float* verts, const uint32_t* idx, int n, uint32_t nvert,
+                       const BvhBuildOptions& opt, DeviceBvh* out, bool* in_range, cudaStream_t s) {
+    const int T = 256;
+    BuildState h;
+    int sms = 148;
+    {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    }
+    k_init_state<<<1, 128, 0, s>>>(w.st, n);
+    k_bounds<<<std::min(div_up(n, T), sms * 8), T, 0, s>>>(verts, idx, n, nvert, w.st);
+    CK(cudaGetLastError());
+    CK(read_state(&h, w.st, s));
+    *in_range = h.bad == 0;
+    if (h.bad) return cudaSuccess;
+    // scene bounds for the caller and the scene-relative box padding
+    float scale = 0.f;
+    for (int k = 0; k < 3; ++k) {
+        out->lo[k] = host_ord2f(h.gb[6 + k]);
+        out->hi[k] = host_ord2f(h.gb[9 + k]);
+        scale = fmaxf(scale, fmaxf(fabsf(out->lo[k]), fabsf(out->hi[k])));
+    }
+    const Sah sah{opt.max_leaf < 1 ? 1 : opt.max_leaf, opt.cost_traverse, opt.cost_intersect, scale * 9.5367432e-7f};
+    CK(dalloc(&out->tris, n, s));
+    if (n == 1) {
+        CK(dalloc(&out->nodes, 1, s));
+        k_single<<<1, 1, 0, s>>>(verts, idx, out->nodes, out->tris, w.dec, w.st);
+        out->num_nodes = 1;
+        out->lo[0] = out->lo[1] = out->lo[2] = out->hi[0] = out->hi[1] = out->hi[2] = 0.f;
+    } else {
+        k_morton<<<div_up(n, T), T, 0, s>>>(verts, idx, n, w.st, w.keys, w.vals);
+        const int nb = div_up(n, sort_tile(n));
+        for (int shift = 0; shift < 30; shift += 10) {
+            const bool small = n <= kSmallSort;
+            auto hist = small ? k_sort_hist<4> : k_sort_hist<16>;
+            auto scatter = small ? k_sort_scatter<4> : k_sort_scatter<16>;
+            hist<<<nb, kSortThreads, 0, s>>>(w.keys, n, shift, w.hist, nb);
+            k_sort_rows<<<kDigits / 8, 256, 0, s>>>(w.hist, nb, w.dsum);
+            scatter<<<nb, kSortThreads, 0, s>>>(w.keys, w.vals, w.keys2, w.vals2, n, shift, w.hist, w.dsum, nb);
+            std::swap(w.keys, w.keys2);
+            std::swap(w.vals, w.vals2);
+        }
+        k_init_leaves<<<div_up(n, T), T, 0, s>>>(w.vals, n, verts, idx, w.t, sah, w.ca);
+        CK(cudaGetLastError());
+        const int r = opt.ploc_radius < 1 ? 1 : (opt.ploc_radius > kMaxRadius ? kMaxRadius : opt.ploc_radius);
+        const int tile = kPlocTile - 2 * r;
+        const size_t smem = kFinish * (2 * sizeof(float3) + 2 * sizeof(int));
+        CK(cudaFuncSetAttribute(k_ploc_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        for (int m = n; ;) {
+            if (m > kFinish) {
+                const int tiles = div_up(m, tile);
+                CK(cudaMemsetAsync(w.super[0], 0, sizeof(uint32_t) * (tiles / kSuper + 1), s));
+                for (int it = 0; it < kPlocBatch; ++it) {
+                    k_ploc_merge<<<tiles, kPlocThreads, 0, s>>>(w.ca, w.st, it & 1, w.t, sah, r, w.out, w.cnt, w.super[it & 1]);
+                    k_ploc_compact<<<tiles, kPlocThreads, 0, s>>>(w.out, w.st, it & 1, r, w.cnt, w.super[it & 1],
+                                                                  w.super[(it & 1) ^ 1], w.cb);
+                    std::swap(w.ca, w.cb);
+                }
+            }
+            k_ploc_finish<<<1, 1024, smem, s>>>(w.ca, w.st, 0, w.t, sah, r);
+            CK(cudaGetLastError());
+            CK(read_state(&h, w.st, s));
+            if (h.m[0] == 1) break;
+            // no progress: impossible with the strict pair order, unless areas are not finite
+            if (h.m[0] < 1 || h.m[0] >= m || h.m[0] <= kFinish) return cudaErrorUnknown;
+            m = h.m[0];
+        }
+        out->num_nodes = h.num_nodes;
+        CK(dalloc(&out->nodes, h.num_nodes, s));
+        k_layout_tris<<<div_up(n, T), T, 0, s>>>(n, w.t, w.vals, verts, idx, out->tris);
+        k_layout_nodes<<<div_up(n - 1, T), T, 0, s>>>(n, 2 * n - 1, w.t, sah.floor_pad, w.st, out->nodes, w.dec);
+    }
+    CK(cudaGetLastError());
+    // the 4-wide form, level by level
+    const int cap = out->num_nodes;             // it has at most as many nodes as the binary tree
+    CK(dalloc(&out->nodes4, cap, s));
     // every 4-wide node must start on a 128-byte line (the traversals read it in 32-byte and
     // 16-byte vector loads): the allocator's alignment, checked rather than assumed
-    if ((uintptr_t)b->nodes4 % sizeof(BvhNode4) != 0) {
-        cudaFreeAsync(b->nodes4, s);
-        b->nodes4 = nullptr;
-        return cudaErrorMisalignedAddress;
-    }
-    CK(dalloc(&fa, cap, s));
-    CK(dalloc(&fb, cap, s));
-    CK(dalloc(&counters, 4, s));
-    Dp4 dp{};
-    CK(dalloc(&dp.S, cap, s));
-    CK(dalloc(&dp.dec, cap, s));
-    CK(dalloc(&dp.parent, cap, s));
-    CK(dalloc(&dp.visit, cap, s));
-    k_dp4_init<<<div_up(cap, 256), 256, 0, s>>>(b->nodes, cap, dp);
-    k_dp4<<<div_up(cap, 256), 256, 0, s>>>(b->nodes, cap, dp);
-    CK(cudaGetLastError());
-    const int2 root = make_int2(0, 0);
-    // counters: next 4-wide index, next front's size, this front's size, non-empty levels.
-    // kCollapseBatch levels run between host reads; the grid covers an upper bound of the
-    // front (at most four times the previous one, and at most cap)
-    const int init[4] = {1, 0, 1, 0};
-    CK(cudaMemcpyAsync(fa, &root, sizeof(int2), cudaMemcpyHostToDevice, s));
-    CK(cudaMemcpyAsync(counters, init, sizeof(init), cudaMemcpyHostToDevice, s));
-    int bound = 1, launched = 0, hc[4] = {1, 0, 1, 0};
-    while (true) {
-        for (int it = 0; it < kCollapseBatch; ++it) {
-            k_collapse4_dp<<<div_up(bound, 256), 256, 0, s>>>(b->nodes, dp.dec, fa, counters + 2, b->nodes4, counters,
-                                                              fb, cap);
-            k_collapse_next<<<1, 1, 0, s>>>(counters);
-            std::swap(fa, fb);
-            bound = (int)std::min<long long>(cap, 4ll * bound);
+    if ((uintptr_t)out->nodes4 % sizeof(BvhNode4) != 0) return cudaErrorMisalignedAddress;
+    CK(cudaMemsetAsync(w.fa, 0, sizeof(int), s));   // the root
+    // levels between host reads: as many as a balanced tree has, and a few more
+    int levels = 6;
+    for (long long c = 1; c < cap; c *= 3) ++levels;
+    bool done = false;
+    for (int level = 0; level < kMaxLevels && !done;) {
+        for (int k = 0; k < levels && level < kMaxLevels; ++k, ++level) {
+            const long long bound = level < 12 ? std::min<long long>(cap, 1ll << (2 * level)) : cap;
+            k_collapse4_dp<<<std::min(div_up(bound, T), sms * 8), T, 0, s>>>(out->nodes, w.dec, w.fa, w.st, level, out->nodes4,
+                                                                            w.fb, cap);
+            std::swap(w.fa, w.fb);
         }
-        launched += kCollapseBatch;
-        CK(cudaMemcpyAsync(hc, counters, sizeof(hc), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (hc[0] > cap || hc[2] > cap) return cudaErrorUnknown;
-        if (hc[2] == 0) break;
-        if (launched > 64) return cudaErrorUnknown;   // the binary tree's depth is at most 63
-        bound = hc[2];
+        CK(cudaGetLastError());
+        CK(read_state(&h, w.st, s));
+        done = h.front[level] == 0;
     }
-    b->num_nodes4 = hc[0];
-    CK(dalloc(&b->nodes4q, b->num_nodes4, s));
-    k_quantise4<<<div_up(b->num_nodes4, 128), 128, 0, s>>>(b->nodes4, b->num_nodes4, b->nodes4q);
-    b->depth4 = hc[3];
-    dfree(fa, s);
-    dfree(fb, s);
-    dfree(counters, s);
-    dfree(dp.S, s);
-    dfree(dp.dec, s);
-    dfree(dp.parent, s);
-    dfree(dp.visit, s);
+    out->depth = h.depth;
+    int nodes4 = 0, depth4 = 0;
+    for (int k = 0; k < kMaxLevels && h.front[k] > 0; ++k) { nodes4 += h.front[k]; ++depth4; }
+    if (!done) {                      // deeper than any stack holds: the binary tree only
+        cudaFreeAsync(out->nodes4, s);
+        out->nodes4 = nullptr;
+        return cudaSuccess;
+    }
+    if (nodes4 > cap) return cudaErrorUnknown;
+    out->num_nodes4 = nodes4;
+    out->depth4 = depth4;
+    CK(dalloc(&out->nodes4q, nodes4, s));
+    k_quantise4<<<div_up(nodes4, 128), 128, 0, s>>>(out->nodes4, nodes4, out->nodes4q);
     return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t bvh_build_device(const float* verts, const uint32_t* idx, int n, uint32_t nvert, const BvhBuildOptions& opt,
+                             DeviceBvh* out, bool* in_range, cudaStream_t s) {
+    *in_range = true;
+    if (n < 1) return cudaErrorInvalidValue;
+    *out = DeviceBvh();
+    out->num_tris = n;
+    const int tile = kPlocTile - 2 * kMaxRadius;      // the smallest tile
+    Arena a;
+    Scratch w;
+    w.cut(a, n, tile);                                // sizes
+    const size_t bytes = a.used;
+    CK(cudaMallocAsync((void**)&a.base, bytes, s));
+    a.used = 0;
+    w.cut(a, n, tile);
+    const cudaError_t e = build_with(w, verts, idx, n, nvert, opt, out, in_range, s);
+    cudaFreeAsync(a.base, s);
+    return e;
+}
+
+void bvh_free_device(DeviceBvh* bvh, cudaStream_t s) {
+    if (bvh->nodes) cudaFreeAsync(bvh->nodes, s);
+    if (bvh->tris) cudaFreeAsync(bvh->tris, s);
+    if (bvh->nodes4) cudaFreeAsync(bvh->nodes4, s);
+    if (bvh->nodes4q) cudaFreeAsync(bvh->nodes4q, s);
+    *bvh = DeviceBvh();
 }
 
 }  // namespace aur

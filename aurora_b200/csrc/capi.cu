@@ -256,21 +256,22 @@ aur_status aur_bvh_build(aur_ctx* ctx, const float* verts, uint32_t nvert, const
     DevIn dv, di, da;
     CUDA_TRY(dv.init(verts, sizeof(float) * 3 * nvert, 4, s), "aur_bvh_build(upload)");
     CUDA_TRY(di.init(tri_vidx, sizeof(uint32_t) * 3 * ntri, 4, s), "aur_bvh_build(upload)");
-    // vertex indices must be in range before any build kernel reads vertices through them:
-    // checked on the device copy (host and device inputs alike)
-    bool in_range = true;
-    CUDA_TRY(indices_below((const uint32_t*)di.ptr, 3 * (size_t)ntri, nvert, &in_range, s), "aur_bvh_build(check)");
-    if (!in_range) return fail(AUR_ERR_INVALID_ARG, "aur_bvh_build: vertex index out of range");
     aur_bvh* b = new aur_bvh();
     b->ctx = ctx;
-    cudaError_t e = bvh_build_device((const float*)dv.ptr, (const uint32_t*)di.ptr, (int)ntri, bo, &b->bvh, s);
+    // vertex indices are checked on the device copy (host and device inputs alike) before any
+    // build kernel reads vertices through them
+    bool in_range = true;
+    cudaError_t e = bvh_build_device((const float*)dv.ptr, (const uint32_t*)di.ptr, (int)ntri, nvert, bo, &b->bvh, &in_range, s);
+    if (e == cudaSuccess && !in_range) {
+        delete b;
+        return fail(AUR_ERR_INVALID_ARG, "aur_bvh_build: vertex index out of range");
+    }
     if (e == cudaSuccess && b->bvh.depth >= kTraversalStack) {
         bvh_free_device(&b->bvh, s);
         delete b;
         return fail(AUR_ERR_UNSUPPORTED, "aur_bvh_build: tree deeper than the traversal stack");
     }
-    if (e == cudaSuccess) e = bvh_collapse4(&b->bvh, s);
-    if (e == cudaSuccess && 3 * b->bvh.depth4 + 1 > kTraversalStack4) {
+    if (e == cudaSuccess && b->bvh.nodes4 && 3 * b->bvh.depth4 + 1 > kTraversalStack4) {
         // a 4-wide node pushes up to three entries: too deep for its stack, keep the binary tree only
         cudaFreeAsync(b->bvh.nodes4, s);
         cudaFreeAsync(b->bvh.nodes4q, s);
