@@ -1,9 +1,11 @@
-// render_plain.cu — the plain renderer: one thread per pixel runs that pixel's
+// render_plain.cu — the plain renderer's pixel loop: one thread per pixel runs that pixel's
 // spp camera paths back to back (Renderer::renderImage's spp passes of
 // IntegrateParallel, Aurora/src/frontend/renderer.cpp:147-186,201-271, folded
 // into one launch) and writes the running mean the reference keeps in
 // OpenexrDisplay::appendValue (openexrDisplay.cpp:61-72). Accumulation is
-// Neumaier-compensated FP32, or FP64 for oracle images.
+// Neumaier-compensated FP32, or FP64 for oracle images. aur_render runs one lane per path
+// (render_paths.cu); this form counts work, serves callers that have no memory for samples, and
+// scenes whose tree is too deep for the 4-wide stack.
 #include "aur_kernels.h"
 
 namespace aur {
@@ -26,10 +28,9 @@ __device__ __forceinline__ void add_counters(unsigned long long* counters, const
         for (int k = 0; k < kN; ++k) atomicAdd(&counters[k], v[k]);
 }
 
-// kWidth: the tree traversed (2 binary, 4 four-wide, 8 quantised four-wide). The timed kernels use the binary
-// tree, on which this one-thread-per-path kernel is fastest (its code holds five
-// traversals; the 4-wide ones made it 30% slower); the counting pass can use either, to
-// count the work of the wavefront renderer's traversal.
+// kWidth: the tree traversed (2 binary, 4 four-wide, 8 quantised four-wide). Rendering uses the binary
+// tree, on which this kernel is fastest (its code holds five traversals; the 4-wide ones made it
+// 30% slower); the counting pass walks the tree that the wavefront renderer's closest-hit rays do.
 // kMulti: light_samples > 1 (several paths per camera sample after the first pass); the
 // one-path form keeps the single-path loop, whose code is smaller and 6% faster.
 template <bool kFp64, bool kCount, int kWidth, bool kMulti>

@@ -401,6 +401,9 @@ aur_status render_options(const aur_scene* sc, const aur_render_opts* o, PathPar
 
 }  // namespace aur
 
+// Samples that the plain renderer keeps before it sums them (ctx_scratch).
+constexpr size_t kPlainSampleBudget = (size_t)1 << 30;
+
 static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, void* film, bool f64,
                                     aur_render_stats* stats) {
     if (!sc || !o || !film) return fail(AUR_ERR_INVALID_ARG, "aur_render: NULL argument");
@@ -413,15 +416,33 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
     DevOut fo, fo64;
     double* d64 = nullptr;
     float4* f32 = nullptr;
+    // one lane per path where the scene has its 4-wide trees and samples fit a buffer; the pixel
+    // loop counts work, and renders what is left
+    const DeviceBvh& tree = sc->bvh.bvh;
+    const bool quant = tree.num_nodes4 >= kQuantMinNodes4;
+    void* scratch = nullptr;
+    int chunk = 0;
+    if (!o->count_work && tree.nodes4) {
+        size_t budget = kPlainSampleBudget;
+        cudaError_t e = cudaErrorMemoryAllocation;
+        while (e == cudaErrorMemoryAllocation) {
+            e = ctx_scratch(sc->ctx, paths_scratch_bytes(sc->dev(), p, budget, &chunk), &scratch);
+            if (e != cudaErrorMemoryAllocation || chunk == 1) break;
+            cudaGetLastError();
+            budget = (size_t)(chunk / 2) * npix * sizeof(float4);
+        }
+        if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); scratch = nullptr; }
+        else if (e != cudaSuccess) return cuda_fail(e, "aur_render(samples)");
+    }
+    const bool fp64_acc = f64 || o->fp64_film != 0;
     if (f64) {
         CUDA_TRY(fo64.init(film, sizeof(double) * 4 * npix, 8, s), "aur_render(film)");
         d64 = (double*)fo64.ptr;
-        CUDA_TRY(cudaMallocAsync(&f32, sizeof(float4) * npix, s), "aur_render(film)");
+        if (!scratch) CUDA_TRY(cudaMallocAsync(&f32, sizeof(float4) * npix, s), "aur_render(film)");
     } else {
-        const bool fp64_acc = o->fp64_film != 0;
         CUDA_TRY(fo.init(film, sizeof(float4) * npix, 16, s), "aur_render(film)");
         f32 = (float4*)fo.ptr;
-        if (fp64_acc) CUDA_TRY(cudaMallocAsync(&d64, sizeof(double) * 4 * npix, s), "aur_render(film)");
+        if (fp64_acc && !scratch) CUDA_TRY(cudaMallocAsync(&d64, sizeof(double) * 4 * npix, s), "aur_render(film)");
     }
     CUDA_TRY(cudaMemsetAsync(sc->ctx->counters, 0, sizeof(unsigned long long) * 8, s), "aur_render");
     cudaEvent_t e0, e1;
@@ -429,9 +450,15 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
     // the counting pass walks the tree that the wavefront renderer's closest-hit rays do
-    const DeviceBvh& tree = sc->bvh.bvh;
-    const int count_width = !o->count_work ? 0 : !tree.nodes4 ? 2 : tree.num_nodes4 >= kQuantMinNodes4 ? 8 : 4;
-    cudaError_t e = launch_render_plain(sc->dev(), p, f32, d64, sc->ctx->counters, count_width, s);
+    const int count_width = !o->count_work ? 0 : !tree.nodes4 ? 2 : quant ? 8 : 4;
+    uint64_t launches = 0;
+    cudaError_t e;
+    if (scratch) {
+        e = launch_render_paths(sc->dev(), p, quant, fp64_acc, chunk, scratch, f32, d64, sc->ctx->counters, &launches, s);
+    } else {
+        e = launch_render_plain(sc->dev(), p, f32, d64, sc->ctx->counters, count_width, s);
+        launches = 1;
+    }
     cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = f64 ? fo64.finish() : fo.finish();
     unsigned long long cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -441,22 +468,27 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (f64) cudaFreeAsync(f32, s);
+    if (f64) { if (f32) cudaFreeAsync(f32, s); }
     else if (d64) cudaFreeAsync(d64, s);
     if (e != cudaSuccess) return cuda_fail(e, "aur_render");
+    if (scratch) {   // the sample 0 of a render has one path, every other one light_samples
+        cnt[0] = npix * (unsigned long long)p.spp;
+        cnt[3] = npix * ((unsigned long long)p.spp * p.light_samples - (p.sample_offset == 0 ? p.light_samples - 1 : 0));
+    }
     if (stats) {
         stats->camera_rays = cnt[0];
         stats->closest_rays = cnt[1];
         stats->shadow_rays = cnt[2];
         stats->paths = cnt[3];
-        stats->node_visits = cnt[4];
-        stats->tri_tests = cnt[5];
-        stats->shadow_node_visits = cnt[6];
-        stats->shadow_tri_tests = cnt[7];
-        stats->launches = 1;
+        stats->node_visits = scratch ? 0 : cnt[4];
+        stats->tri_tests = scratch ? 0 : cnt[5];
+        stats->shadow_node_visits = scratch ? 0 : cnt[6];
+        stats->shadow_tri_tests = scratch ? 0 : cnt[7];
+        stats->launches = launches;
         stats->kernel_ms = ms;
-        stats->node_bytes = (int32_t)(count_width == 4 ? sizeof(BvhNode4) : count_width == 8 ? sizeof(BvhNode4Q)
-                                                                                             : sizeof(BvhNode));
+        stats->node_bytes = (int32_t)(scratch ? (quant ? sizeof(BvhNode4Q) : sizeof(BvhNode4))
+                                              : count_width == 4 ? sizeof(BvhNode4)
+                                              : count_width == 8 ? sizeof(BvhNode4Q) : sizeof(BvhNode));
     }
     return AUR_OK;
 }
