@@ -14,7 +14,7 @@ __device__ __forceinline__ float dlnD_dr(float r, float tan2, bool floored) {
     return 2.f * tan2 / (r2 * r) - 2.f / r;
 }
 __device__ __forceinline__ float tan2_of(float ndoth) {
-    const float t = xtanf(xacosf(ndoth));
+    const float t = xtan_acosf(ndoth);
     return t * t;
 }
 
@@ -30,7 +30,7 @@ __device__ __forceinline__ float eval_dlnD(float rough, float3 N, float3 V, floa
 __device__ __forceinline__ float sample_dlnD(float rough, float3 N, float3 V, float3 L) {
     const float3 H = normalize(L + V);
     const float ndoth = dot(N, H);
-    const float tana = ndoth > 0.999f ? 0.f : xtanf(xacosf(ndoth));
+    const float tana = ndoth > 0.999f ? 0.f : xtan_acosf(ndoth);
     if (ct_d(rough, ndoth, tana) >= 1000.f) return 0.f;
     return dlnD_dr(rough, tana * tana, true);
 }

@@ -65,7 +65,12 @@ AUR_HD float rng_u01(uint64_t key, uint64_t counter) {
 }
 struct PathRng {
     uint64_t key, base;
-    AUR_HD float u(uint32_t dim) const { return rng_u01(key, base | (uint64_t)dim); }
+    // rng_u01(key, base | dim): the counter's bits do not overlap, so its product with the golden gamma
+    // splits, and the part that a path's draws share is computed once
+    AUR_HD float u(uint32_t dim) const {
+        const uint64_t golden = 0x9e3779b97f4a7c15ull;
+        return (float)(uint32_t)(mix64((key + base * golden) + (uint64_t)dim * golden) >> 40) * (1.0f / 16777216.0f);
+    }
 };
 
 // ---------------------------------------------------------------- transcendentals
@@ -84,14 +89,61 @@ struct PathRng {
 #define AUR_MATH AUR_HD
 #endif
 AUR_MATH float xexpf(float x) { return (float)exp((double)x); }
-AUR_MATH float xlogf(float x) { return (float)log((double)x); }
-AUR_MATH float xpowf(float x, float y) { return (float)pow((double)x, (double)y); }
-AUR_MATH float xacosf(float x) { return (float)acos((double)x); }
-AUR_MATH float xtanf(float x) { return (float)tan((double)x); }
-AUR_MATH float xatanf(float x) { return (float)atan((double)x); }
-AUR_MATH float xcosf(float x) { return (float)cos((double)x); }
-AUR_MATH float xsinf(float x) { return (float)sin((double)x); }
 AUR_MATH float xatan2f(float y, float x) { return (float)atan2((double)y, (double)x); }
+// Compositions of two roundings, each of which the reference does in float, without evaluating both
+// functions: a few double operations around one call give the same floats, at a fraction of
+// the instructions of a shading vertex (its code was waited for as much as its data).
+// x^3 and x^5: the float of the double product. (float)pow rounds 204 (8) of the 2^32 inputs the
+// other way, all of them exact ties of the float rounding that pow's own error breaks.
+AUR_HD float xpow3f(float x) { const double d = x; return (float)(d * d * d); }
+AUR_HD float xpow5f(float x) { const double d = x, q = d * d; return (float)(q * q * d); }
+// tan of the float a = (float)acos(x): with t = acos(x) and e = a - t, the addition theorem for
+// tan(t + e), tan t = sqrt(1 - x^2) / x and tan e = e. Equal to (float)tan((double)a) for every
+// float x (all 2^32 compared on the device).
+AUR_MATH float xtan_acosf(float x) {
+    const double n = x, t = acos(n);
+    const double e = (double)(float)t - t;
+    const double s = sqrt(1.0 - n * n);
+    return (float)((s + n * e) / (n - s * e));
+}
+// cos of the float a = (float)atan(y), y >= 0, the same way with cos t = 1 / sqrt(1 + y^2) and sin t =
+// y cos t. Equal to (float)cos((double)a) for every float y below 256, where it is used.
+AUR_MATH float xcos_atanf(float y) {
+    const double d = y, t = atan(d);
+    if (!(y < 256.f)) return (float)cos((double)(float)t);
+    const double e = (double)(float)t - t;
+#ifdef __CUDA_ARCH__
+    const double c = rsqrt(1.0 + d * d);
+#else
+    const double c = 1.0 / sqrt(1.0 + d * d);
+#endif
+    return (float)(c * (1.0 - 0.5 * e * e) - d * c * e);
+}
+// (sin x, cos x) of an angle in [0, 2 pi]: the nearest multiple of pi / 2 taken off (pi / 2 in two
+// doubles), then the Taylor series to y^15 and y^16 (|y| <= pi / 4: the next terms are below
+// 5e-17). Equal to the float of the double functions for every angle that two_pi_times makes
+// of a random number (all 2^24 compared).
+AUR_MATH float2 xsincosf(float x) {
+    const double d = x;
+    const int q = (int)(d * 0.6366197723675814 + 0.5);
+    const double y = (d - q * 1.5707963267948966) - q * 6.123233995736766e-17;
+    const double z = y * y;
+    double s = -1.0 / 1307674368000.0, c = 1.0 / 20922789888000.0;
+    s = fma(s, z, 1.0 / 6227020800.0);  c = fma(c, z, -1.0 / 87178291200.0);
+    s = fma(s, z, -1.0 / 39916800.0);   c = fma(c, z, 1.0 / 479001600.0);
+    s = fma(s, z, 1.0 / 362880.0);      c = fma(c, z, -1.0 / 3628800.0);
+    s = fma(s, z, -1.0 / 5040.0);       c = fma(c, z, 1.0 / 40320.0);
+    s = fma(s, z, 1.0 / 120.0);         c = fma(c, z, -1.0 / 720.0);
+    s = fma(s, z, -1.0 / 6.0);          c = fma(c, z, 1.0 / 24.0);
+    s = fma(s * z, y, y);               c = fma(c, z, -0.5);
+    c = fma(c, z, 1.0);
+    float2 r;
+    r.x = (float)(q & 1 ? c : s);
+    r.y = (float)(q & 1 ? s : c);
+    if (q & 2) r.x = -r.x;
+    if ((q + 1) & 2) r.y = -r.y;
+    return r;
+}
 
 // ---------------------------------------------------------------- float3 helpers
 AUR_HD float3 mk(float x, float y, float z) { float3 r; r.x = x; r.y = y; r.z = z; return r; }
@@ -119,7 +171,7 @@ AUR_HD float lum(float3 c) { return (float)(0.2126 * c.x + 0.7152 * c.y + 0.0722
 AUR_HD bool is_black(float3 c) {   // compared with the double ISBLACK as in color.h:149-151
     return (double)c.x < 0.0001 && (double)c.y < 0.0001 && (double)c.z < 0.0001;
 }
-AUR_HD float schlick(float vdoth, float refl) { return refl + xpowf(1.f - vdoth, 5.f) * (1.f - refl); }
+AUR_HD float schlick(float vdoth, float refl) { return refl + xpow5f(1.f - vdoth) * (1.f - refl); }
 
 AUR_HD void coordinate_system(float3 v1, float3* v2, float3* v3) {
     if (!(v1.x != 0.f) && v1.y != 0.f && !(v1.z != 0.f)) *v2 = cross(v1, mk(1.f, 0.f, 0.f));
@@ -138,8 +190,8 @@ AUR_HD float two_pi_times(float r) { return (float)(6.283185307179586 * (double)
 AUR_HD float3 sample_hemisphere_uniform(float r1, float r2) {
     float z = r1;
     float r = sqrtf(fmaxf(0.f, 1.f - z * z));
-    float phi = two_pi_times(r2);
-    return mk(r * xcosf(phi), r * xsinf(phi), z);
+    const float2 sc = xsincosf(two_pi_times(r2));
+    return mk(r * sc.y, r * sc.x, z);
 }
 
 // Neumaier-compensated FP32 accumulator (film and gradient sums).

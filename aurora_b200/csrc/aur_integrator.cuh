@@ -36,14 +36,24 @@ struct PathParams {
 
 struct RayCounts { uint32_t closest = 0, shadow = 0; TraceWork work, shadow_work; };
 
-// Picks the k-th light for which light_visible() holds; returns -1 if none.
+// Picks the k-th light for which light_visible() holds; returns -1 if none. Up to 32 lights are
+// tested once, their answers kept as bits.
 __device__ __forceinline__ int pick_visible_light(const ShadeScene& sh, float3 P, float3 N, float u, int* nvis) {
     int n = 0;
-    for (int i = 0; i < sh.nlights; ++i) n += light_visible(sh.lights[i], P, N) ? 1 : 0;
+    uint32_t seen = 0;
+    for (int i = 0; i < sh.nlights; ++i)
+        if (light_visible(sh.lights[i], P, N)) {
+            ++n;
+            seen |= i < 32 ? 1u << i : 0u;
+        }
     *nvis = n;
     if (n == 0) return -1;
     int k = (int)(u * (float)n);
     k = k < n ? k : n - 1;
+    if (sh.nlights <= 32) {
+        for (; k > 0; --k) seen &= seen - 1;
+        return __ffs(seen) - 1;
+    }
     for (int i = 0; i < sh.nlights; ++i) {
         if (light_visible(sh.lights[i], P, N)) {
             if (k == 0) return i;

@@ -286,7 +286,7 @@ constexpr float kInvPiMacro = 1.f / 3.14159265358979323846f;
 AUR_HD float ct_d(float rough, float cosa, float tana) {        // cookTorrance.cpp:40-45
     float rough2 = fmaxf(0.001f, rough * rough);
     float e = xexpf(-(tana * tana) / rough2);
-    float div = (float)((double)rough2 * 3.141592653589793 * (double)xpowf(cosa, 3.f));   // rough2 * M_PI in double
+    float div = (float)((double)rough2 * 3.141592653589793 * (double)xpow3f(cosa));   // rough2 * M_PI in double
     return e / div;
 }
 
@@ -301,10 +301,10 @@ AUR_HD BrdfSample brdf_sample(const Brdf& b, float3 V, float3 N, float r1, float
         return s;
     }
     if (b.lobe == LOBE_SPEC) {                                       // cookTorrance.cpp:47-99
-        float z = xcosf(xatanf(b.rough * sqrtf((float)(-log(1.0 - (double)r1)))));
+        float z = xcos_atanf(b.rough * sqrtf((float)(-log(1.0 - (double)r1))));
         float r = sqrtf(fmaxf(0.f, 1.f - z * z));
-        float phi = two_pi_times(r2);
-        float3 dir = normalize(mk(r * xcosf(phi), r * xsinf(phi), z));
+        const float2 sc = xsincosf(two_pi_times(r2));
+        float3 dir = normalize(mk(r * sc.y, r * sc.x, z));
         float3 H = normalize(tangent_to_world(dir, N));
         float vdoth = dot(V, H);
         float3 L = normalize((H * 2.f) * vdoth - V);
@@ -312,7 +312,7 @@ AUR_HD BrdfSample brdf_sample(const Brdf& b, float3 V, float3 N, float r1, float
         s.color = mk(0.f, 0.f, 0.f);
         s.pdf = 1.f;
         if (vdoth > 0.0001f) {
-            float tana = (ndoth > 0.999f) ? 0.f : xtanf(xacosf(ndoth));
+            float tana = (ndoth > 0.999f) ? 0.f : xtan_acosf(ndoth);
             float D = ct_d(b.rough, ndoth, tana);
             D = fminf(D, 1000.f);
             s.pdf = D / (4.f * vdoth);
@@ -364,8 +364,8 @@ AUR_HD float3 brdf_eval(const Brdf& b, float3 L, float3 V, float3 N) {
         float3 H = normalize(L + V);
         float vdoth = dot(V, H), vdotn = dot(V, N), ndoth = dot(H, N), ldotn = dot(L, N);
         float r2 = b.rough * b.rough;
-        float ta = xtanf(xacosf(ndoth));
-        float D = (float)((1.f / ((double)r2 * 3.141592653589793 * (double)xpowf(ndoth, 3.f))) *
+        float ta = xtan_acosf(ndoth);
+        float D = (float)((1.f / ((double)r2 * 3.141592653589793 * (double)xpow3f(ndoth))) *
                           (double)xexpf(-(ta * ta) / r2));
         if (vdoth <= 0.001f || ldotn <= 0.001f || vdotn <= 0.001f || isnan(D)) return mk(0.f, 0.f, 0.f);
         return cdiv(b.color * D, (float)(4.0 * vdoth * vdoth));
@@ -378,7 +378,7 @@ AUR_HD float brdf_pdf(const Brdf& b, float3 L, float3 V, float3 N) {
     if (b.lobe == LOBE_SPEC) {                                       // cookTorrance.cpp:101-117
         float3 H = normalize(L + V);
         float vdoth = dot(V, H), ndoth = dot(N, H);
-        float D = ct_d(b.rough, ndoth, xtanf(xacosf(ndoth)));
+        float D = ct_d(b.rough, ndoth, xtan_acosf(ndoth));
         if (isnan(D)) D = 0.f;
         return D / (4.f * vdoth);
     }
@@ -591,8 +591,8 @@ static __host__ __device__ __noinline__ LightSample env_light_sample(const Textu
         if (l.tex >= 0) {   // a uniform direction on the sphere, weighted by the map's pdf at (u1, u2)
             const float vy = 1.f - 2.f * u2;
             const float r = sqrtf(fmaxf(0.f, 1.f - vy * vy));
-            const float phi = two_pi_times(u1);
-            dirw = xform_vector(l.minv, mk(r * xcosf(phi), vy, r * xsinf(phi)));
+            const float2 sc = xsincosf(two_pi_times(u1));
+            dirw = xform_vector(l.minv, mk(r * sc.y, vy, r * sc.x));
             pdf = env_texel_pdf(sh, l, u1, u2);
         } else {
             pdf = 2.f;
@@ -631,8 +631,8 @@ AUR_HD LightSample light_sample(const ShadeScene& sh, const Light& l, float3 P, 
     float cosmax = sphere_cone_cos(l, P);
     float cost = (1.f - u1) + u1 * cosmax;
     float sint = sqrtf(fmaxf(0.f, 1.f - cost * cost));
-    float phi = two_pi_times(u2);
-    float3 dir = normalize(tangent_to_world(mk(sint * xcosf(phi), sint * xsinf(phi), cost), w));
+    const float2 sc = xsincosf(two_pi_times(u2));
+    float3 dir = normalize(tangent_to_world(mk(sint * sc.y, sint * sc.x, cost), w));
     float t;
     sphere_hit(l.center, l.radius, P, dir, 0.f, &t);
     s.dir = dir;
