@@ -29,10 +29,9 @@ struct aur_bvh {
     int* tri_attr = nullptr;                   // device, per original triangle id
     bool owns_attr = false;
     bool owned_by_scene = false;
-    // per-corner normals (9 floats) and uvs (6 floats) per triangle for aur_bvh_intersect:
-    // the scene's arrays for a scene's BVH, else uploaded by aur_bvh_set_shading (owned)
-    float* corner_n = nullptr;
-    float* corner_uv = nullptr;
+    // corner normals and uvs per triangle for aur_bvh_intersect: the scene's records for a scene's
+    // BVH, else made by aur_bvh_set_shading (owned)
+    aur::TriShade* tri = nullptr;
     bool owns_shading = false;
 };
 
@@ -40,8 +39,9 @@ struct aur_scene {
     aur_ctx* ctx = nullptr;
     aur_bvh bvh;                               // owned_by_scene = true
     // device buffers
-    float* corner_n = nullptr;
-    float* corner_uv = nullptr;
+    aur::TriShade* tri = nullptr;
+    uint8_t* tri_type = nullptr;
+    bool has_uv = false;
     aur::Attr* attrs = nullptr;
     aur::Material* mats = nullptr;
     aur::Light* lights = nullptr;
@@ -88,6 +88,14 @@ void wf_release_context(aur_ctx* ctx);   // frees the wavefront engines cached f
 constexpr int kVertexRec = 4;
 aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsamples, float4* rec, int stride,
                           float4* lo_raw, uint64_t* launches, unsigned long long* rays);
+
+// Packs the triangles' shading records from device arrays (corner uvs and attributes may be null: 0)
+// into a new buffer of the stream's pool.
+cudaError_t pack_tri_shade(const float* corner_n, const float* corner_uv, const int* tri_attr, size_t ntri, TriShade** out,
+                           cudaStream_t s);
+// The material type of every triangle, into a new buffer.
+cudaError_t make_tri_type(const int* tri_attr, const Attr* attrs, const Material* mats, size_t ntri, uint8_t** out,
+                          cudaStream_t s);
 
 struct DeviceGuard {
     explicit DeviceGuard(int dev);

@@ -69,6 +69,15 @@ struct Light {
 struct Texture { int w, h, offset; float tri_scale; };
 struct Camera { float fov; int w, h; int pad; };
 
+// What shading reads of a triangle, in two 32-byte sectors: the corners' normals and uvs and the
+// attribute index. As arrays of their own (36 + 24 + 4 bytes a triangle, unaligned) they took ten
+// to sixteen loads and three to five sectors a vertex.
+struct alignas(64) TriShade {
+    float n[9];              // corner normals (EmbreeMesh::normals[3 * triangle + k])
+    int attr;                // attribute index
+    float uv[6];             // corner uvs (EmbreeMesh::uvs), 0 without any
+};
+
 struct ShadeScene {          // device pointers for the shading stage
     const Material* mats;
     const Attr* attrs;
@@ -77,9 +86,9 @@ struct ShadeScene {          // device pointers for the shading stage
     const float* texels;
     const float* albedo;     // Kelemen tables, [table][cos 64][rough 32]
     int nenv;                // environment lights among the lights
-    const float* corner_n;   // per-corner normals, 9 floats per triangle
-    const float* corner_uv;  // per-corner uvs, 6 floats per triangle
-    const int* tri_attr;     // attribute index per triangle
+    const TriShade* tri;     // per triangle
+    const uint8_t* tri_type; // its material's type: the wavefront's sort key without the way over attribute and material
+    int uses_uv;             // a uv-mapped shader reads the interpolated uvs (else they are not computed)
     int nlights;
     int nnormal;             // materials with a normal map
     const float* attr_c2o;   // camera-to-object transform per attribute, 16 floats row major
@@ -705,12 +714,31 @@ static __host__ __device__ __noinline__ float3 normal_map(const Material* mats, 
     return normalize(ns);
 }
 
+// A triangle's shading record in two 256-bit read-only loads.
+AUR_HD TriShade load_tri(const TriShade* t) {
+    TriShade r;
+#ifdef __CUDA_ARCH__
+    float w;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.n[0]), "=f"(r.n[1]), "=f"(r.n[2]), "=f"(r.n[3]), "=f"(r.n[4]), "=f"(r.n[5]), "=f"(r.n[6]), "=f"(r.n[7])
+        : "l"(t));
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.n[8]), "=f"(w), "=f"(r.uv[0]), "=f"(r.uv[1]), "=f"(r.uv[2]), "=f"(r.uv[3]), "=f"(r.uv[4]), "=f"(r.uv[5])
+        : "l"(reinterpret_cast<const char*>(t) + 32));
+    r.attr = __float_as_int(w);
+#else
+    r = *t;
+#endif
+    return r;
+}
+
 // Shading frame at a hit (embreeAccelerator.cpp:54-90 + integrator.cpp:132-150):
 // interpolated, face-forwarded, normalised normal; the normal map; V = -normalize(dir);
 // back-facing fix.
 AUR_HD Frame hit_frame(const ShadeScene& s, int prim, float t, float u, float v, float3 o, float3 d, bool need_uv) {
     Frame f;
-    const float* n = s.corner_n + (size_t)prim * 9;
+    const TriShade r = load_tri(s.tri + prim);
+    const float* n = r.n;
     float w = (float)(1.0 - u - v);      // 1. - u - v in double (embreeAccelerator.cpp:54)
     float3 nn = mk(w * n[0] + u * n[3] + v * n[6],
                    w * n[1] + u * n[4] + v * n[7],
@@ -719,10 +747,10 @@ AUR_HD Frame hit_frame(const ShadeScene& s, int prim, float t, float u, float v,
     f.Ng = normalize(nn);
     f.N = f.Ng;
     f.P = o + d * t;
-    f.attr = s.tri_attr[prim];
+    f.attr = r.attr;
     f.su = f.sv = 0.f;
-    if (need_uv && s.corner_uv) {
-        const float* uv = s.corner_uv + (size_t)prim * 6;
+    if (need_uv && s.uses_uv) {
+        const float* uv = r.uv;
         f.su = w * uv[0] + u * uv[2] + v * uv[4];
         f.sv = w * uv[1] + u * uv[3] + v * uv[5];
     }

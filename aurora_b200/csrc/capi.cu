@@ -305,8 +305,7 @@ aur_status aur_bvh_destroy(aur_bvh* b) {
     DeviceGuard g(b->ctx->device);
     bvh_free_device(&b->bvh, b->ctx->stream);
     if (b->owns_attr && b->tri_attr) cudaFreeAsync(b->tri_attr, b->ctx->stream);
-    if (b->owns_shading && b->corner_n) cudaFreeAsync(b->corner_n, b->ctx->stream);
-    if (b->owns_shading && b->corner_uv) cudaFreeAsync(b->corner_uv, b->ctx->stream);
+    if (b->owns_shading && b->tri) cudaFreeAsync(b->tri, b->ctx->stream);
     cudaStreamSynchronize(b->ctx->stream);
     delete b;
     return AUR_OK;

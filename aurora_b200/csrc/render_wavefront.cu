@@ -119,8 +119,6 @@ struct WfPool {
     __device__ __forceinline__ float4& sh_d0(uint32_t i) const { return neeA[2 * (size_t)i + 1]; }
     __device__ __forceinline__ float4& sh_d1(uint32_t i) const { return neeB[2 * (size_t)i]; }
     __device__ __forceinline__ float4& sh_c1(uint32_t i) const { return neeB[2 * (size_t)i + 1]; }
-    __device__ __forceinline__ float4& sh_c0(uint32_t i) const { return neeC[2 * (size_t)i]; }
-    __device__ __forceinline__ float4& sh_t(uint32_t i) const { return neeC[2 * (size_t)i + 1]; }
 };
 
 // flags in id.w; kNoClamp: the sample is the environment seen by the camera ray, which
@@ -133,6 +131,18 @@ __device__ __forceinline__ int f_vtx(uint32_t f) { return f & 511; }
 __device__ __forceinline__ int f_bounces(uint32_t f) { return (f >> 9) & 511; }
 __device__ __forceinline__ int f_kind(uint32_t f) { return (f >> 18) & 3; }
 __device__ __forceinline__ bool f_matte(uint32_t f) { return (f >> 20) & 1; }
+
+// A slot's 32-byte pair in one 256-bit access (the pool's arrays are written and read by the stages
+// in turn: no read-only loads, and no reordering around the stage's own stores)
+__device__ __forceinline__ void ld_pair(const float4* p, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_pair(float4* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w) : "memory");
+}
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << lane_id()) - 1u; }
@@ -233,7 +243,8 @@ __global__ void k_regen(WfPool w, int in_q) {
                 // next-event estimate of the last vertex: Lo += ((vis0 c0 + vis1 c1) nvis) T, the
                 // plain kernel's order of operations (integrate_direct)
                 const uint32_t vis = w.sh_vis[i];
-                const float4 t = w.sh_t(i), c0 = w.sh_c0(i);
+                float4 c0, t;
+                ld_pair(w.neeC + 2 * (size_t)i, c0, t);
                 const float nvis = t.w;   // the number of visible lights rides in the throughput record
                 float3 res = mk(0.f, 0.f, 0.f);
                 if (vis & 1u) res += mk(c0.x, c0.y, c0.z);   // only unoccluded contributions are added
@@ -292,10 +303,8 @@ __global__ void k_regen(WfPool w, int in_q) {
             rng.base = path_base(pixel, cam_index(S, q));
             const RayF r = camera_ray(S.sc.cam, (int)(pixel % (uint32_t)S.sc.cam.w), (int)(pixel / (uint32_t)S.sc.cam.w),
                                       rng.u(kDimCamera), rng.u(kDimCamera + 1));
-            w.ray_o(i) = make_float4(r.o.x, r.o.y, r.o.z, r.mint);
-            w.ray_d(i) = make_float4(r.d.x, r.d.y, r.d.z, r.maxt);
-            w.tp(i) = make_float4(1.f, 1.f, 1.f, 1.f);
-            w.lo(i) = make_float4(0.f, 0.f, 0.f, 0.f);
+            st_pair(w.ray + 2 * (size_t)i, make_float4(r.o.x, r.o.y, r.o.z, r.mint), make_float4(r.d.x, r.d.y, r.d.z, r.maxt));
+            st_pair(w.tplo + 2 * (size_t)i, make_float4(1.f, 1.f, 1.f, 1.f), make_float4(0.f, 0.f, 0.f, 0.f));
             w.id(i) = make_uint4((uint32_t)s, pixel, q, pack_flags(0, 0, RAY_CAMERA, false));
         }
         {
@@ -310,9 +319,9 @@ __global__ void k_regen(WfPool w, int in_q) {
 // ------------------------------------------------------------------ extend
 __device__ __forceinline__ int bucket_of(const ShadeScene& sh, int prim) {
     if (prim < 0) return B_MISS;
-    const int mt = sh.mats[sh.attrs[sh.tri_attr[prim]].material].type;
-    return mt == MAT_MATTE ? B_MATTE : mt == MAT_KELEMEN ? B_KELEMEN : mt == MAT_COOKTORRANCE ? B_CT
-         : mt == MAT_METAL ? B_METAL : B_CONST;
+    static_assert(B_MATTE == MAT_MATTE + 1 && B_KELEMEN == MAT_KELEMEN + 1 && B_CT == MAT_COOKTORRANCE + 1 &&
+                  B_METAL == MAT_METAL + 1 && B_CONST == MAT_CONSTANT + 1 && MAT_GLASS > MAT_CONSTANT, "bucket order");
+    return min((int)__ldg(sh.tri_type + prim), (int)MAT_CONSTANT) + 1;
 }
 
 // The tree a traversal kernel walks.
@@ -391,7 +400,8 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
                     S = &w.scenes[w.id(slot).x];
                     nodes = Tree::nodes(S->sc);
                     tris = S->sc.tris;
-                    const float4 o = w.ray_o(slot), d = w.ray_d(slot);
+                    float4 o, d;
+                    ld_pair(w.ray + 2 * (size_t)slot, o, d);
                     ts.begin(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, d.w);
                     has = true;
                 } else {
@@ -550,21 +560,23 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
         uint32_t slot = 0;
         if (k < n) {
             slot = qin[kPart == SHADE_ALL ? k : kPart == SHADE_MATTE ? nmiss + k : (k < nmiss ? k : k + nm)];
-            const float4 hh = w.hit(slot);
+            float4 hh, idf, tpv, lo;
+            ld_pair(w.hitid + 2 * (size_t)slot, hh, idf);
+            ld_pair(w.tplo + 2 * (size_t)slot, tpv, lo);
+            const uint4 id = make_uint4(__float_as_uint(idf.x), __float_as_uint(idf.y), __float_as_uint(idf.z),
+                                        __float_as_uint(idf.w));
             const int prim = __float_as_int(hh.w);
-            float4 lo = w.lo(slot);
             if (prim < 0) {
-                const uint4 id = w.id(slot);
                 const WfScene& S = w.scenes[id.x];
                 const int kind = f_kind(id.w), vtx = f_vtx(id.w);
                 if (S.sc.sh.nenv && (vtx == 0 || kind == RAY_MIRROR))
                     lo = shade_env_miss(&w, &S, slot, id, vtx, lo);
                 done = true;
-            } else if (f_vtx(w.id(slot).w) >= w.scenes[w.id(slot).x].p.max_depth) {
+                w.lo(slot) = lo;
+            } else if (f_vtx(id.w) >= w.scenes[id.x].p.max_depth) {
                 // the reference's unshaded last ray hit something: the path ends
                 done = true;
             } else {
-                const uint4 id = w.id(slot);
                 const WfScene& S = w.scenes[id.x];
                 const DevScene& sc = S.sc;
                 const uint32_t flags = id.w;
@@ -575,8 +587,8 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                 PathRng rng;
                 rng.key = S.key;
                 rng.base = path_base(id.y, rng_index(S, id.z));
-                const float4 ro = w.ray_o(slot), rd = w.ray_d(slot);
-                float4 tpv = w.tp(slot);
+                float4 ro, rd;
+                ld_pair(w.ray + 2 * (size_t)slot, ro, rd);
                 float3 T = mk(tpv.x, tpv.y, tpv.z);
                 float cont = tpv.w;
                 float3 Lo = mk(lo.x, lo.y, lo.z);
@@ -644,12 +656,13 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                                 w.rec_cur[slot] = pr.kind == 0 ? kNoRec : (rec_at << 1) | (pr.kind == 3 ? 1u : 0u);
                                 nee_rec = true;
                             }
-                            w.sh_p(slot) = make_float4(f.P.x, f.P.y, f.P.z, 0.f);
-                            w.sh_d0(slot) = make_float4(d0.x, d0.y, d0.z, m0);
-                            w.sh_d1(slot) = make_float4(d1.x, d1.y, d1.z, m1);
-                            w.sh_c0(slot) = make_float4(c0.x, c0.y, c0.z, g0);
-                            w.sh_c1(slot) = make_float4(c1.x, c1.y, c1.z, g1);
-                            w.sh_t(slot) = make_float4(T.x, T.y, T.z, (float)nvis);
+                            st_pair(w.neeA + 2 * (size_t)slot, make_float4(f.P.x, f.P.y, f.P.z, 0.f),
+                                    make_float4(d0.x, d0.y, d0.z, m0));
+                            if (kRec || r1)   // nothing else reads the second ray's pair
+                                st_pair(w.neeB + 2 * (size_t)slot, make_float4(d1.x, d1.y, d1.z, m1),
+                                        make_float4(c1.x, c1.y, c1.z, g1));
+                            st_pair(w.neeC + 2 * (size_t)slot, make_float4(c0.x, c0.y, c0.z, g0),
+                                    make_float4(T.x, T.y, T.z, (float)nvis));
                             w.sh_vis[slot] = 0u;
                             push_sh0 = r0;
                             push_sh1 = r1;
@@ -705,18 +718,16 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
                 if (continue_path(brdf, bs, f.N, S.p.min_depth, rng, vtx, T, cont, kind, bounces) &&
                     (vtx + 1 < S.p.max_depth || (kind == RAY_MIRROR && sc.sh.nenv))) {
                     alive = true;
-                    w.ray_o(slot) = make_float4(f.P.x, f.P.y, f.P.z, kRayBias);
-                    w.ray_d(slot) = make_float4(bs.dir.x, bs.dir.y, bs.dir.z, bs.maxt);
-                    w.tp(slot) = make_float4(T.x, T.y, T.z, cont);
+                    st_pair(w.ray + 2 * (size_t)slot, make_float4(f.P.x, f.P.y, f.P.z, kRayBias),
+                            make_float4(bs.dir.x, bs.dir.y, bs.dir.z, bs.maxt));
                     w.id(slot).w = pack_flags(vtx + 1, bounces, kind, matte);
                 }
-                lo = make_float4(Lo.x, Lo.y, Lo.z, lo.w);
+                st_pair(w.tplo + 2 * (size_t)slot, make_float4(T.x, T.y, T.z, cont), make_float4(Lo.x, Lo.y, Lo.z, lo.w));
                 // a finished path's flags count its recorded vertices (a missed ray's vertex is not recorded)
                 if (kRec && !alive) w.id(slot).w = pack_flags(vtx + 1, bounces, kind, matte);
                 done = !alive;
                 push_ext = alive;
             }
-            w.lo(slot) = lo;
         }
         {
             const bool nee = push_sh0 || push_sh1;

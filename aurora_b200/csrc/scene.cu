@@ -109,7 +109,7 @@ static void scene_free(aur_scene* sc) {
     cudaStreamSynchronize(s);
     bvh_free_device(&sc->bvh.bvh, s);
     cudaStreamSynchronize(s);
-    void* bufs[] = {sc->bvh.tri_attr, sc->corner_n, sc->corner_uv, sc->attrs, sc->mats, sc->lights, sc->texs, sc->texels,
+    void* bufs[] = {sc->bvh.tri_attr, sc->tri, sc->tri_type, sc->attrs, sc->mats, sc->lights, sc->texs, sc->texels,
                     sc->attr_c2o};
     for (void* b : bufs) if (b) cudaFreeAsync(b, s);
     cudaStreamSynchronize(s);
@@ -130,15 +130,14 @@ DevScene aur_scene::dev() const {
     d.sh.texs = texs;
     d.sh.texels = texels;
     d.sh.albedo = ctx->kelemen;
-    d.sh.corner_n = corner_n;
-    // the per-corner uvs are read only where a uv-mapped shader (texture2DShader) needs them:
-    // a scene without one skips their 24 bytes per shaded vertex
+    d.sh.tri = tri;
+    d.sh.tri_type = tri_type;
+    // the uvs are interpolated only where a uv-mapped shader (texture2DShader) needs them
     bool uses_uv = false;
     auto uv_tex = [&](int t) { return t >= 0 && t < (int)h_texs.size() && h_texs[t].tri_scale == 0.f; };
     for (const Material& m : h_mats)
         uses_uv = uses_uv || uv_tex(m.diff_tex) || uv_tex(m.spec_tex) || uv_tex(m.rough_tex) || uv_tex(m.norm_tex);
-    d.sh.corner_uv = uses_uv ? corner_uv : nullptr;
-    d.sh.tri_attr = bvh.tri_attr;
+    d.sh.uses_uv = uses_uv && has_uv ? 1 : 0;
     d.sh.nlights = (int)h_lights.size();
     d.sh.nenv = 0;
     for (const Light& l : h_lights) d.sh.nenv += l.type == LIGHT_ENV ? 1 : 0;
@@ -290,23 +289,26 @@ aur_status aur_scene_create(aur_ctx* ctx, const aur_scene_desc* d, const aur_bvh
     for (const Material& m : mats)
         if (m.type == MAT_KELEMEN && e == cudaSuccess) e = ctx_kelemen_ensure(ctx, m.table);
     if (us) {
-        sc->corner_n = cn;
-        sc->corner_uv = cu;
         if (e == cudaSuccess) e = up_err;
     } else {
-        if (e == cudaSuccess) e = upload(&sc->corner_n, d->corner_normals, 9 * (size_t)d->ntri, s);
-        if (e == cudaSuccess) e = upload(&sc->corner_uv, d->corner_uvs, 6 * (size_t)d->ntri, s);
+        if (e == cudaSuccess) e = upload(&cn, d->corner_normals, 9 * (size_t)d->ntri, s);
+        if (e == cudaSuccess) e = upload(&cu, d->corner_uvs, 6 * (size_t)d->ntri, s);
     }
+    // packed into the triangles' shading records; the uploads go back to the pool
+    if (e == cudaSuccess) e = pack_tri_shade(cn, cu, sc->bvh.tri_attr, d->ntri, &sc->tri, s);
+    sc->has_uv = cu != nullptr;
+    if (cn) cudaFreeAsync(cn, s);
+    if (cu) cudaFreeAsync(cu, s);
     if (e == cudaSuccess) e = upload(&sc->attrs, attrs.data(), attrs.size(), s);
     if (e == cudaSuccess) e = upload(&sc->mats, mats.data(), mats.size(), s);
+    if (e == cudaSuccess) e = make_tri_type(sc->bvh.tri_attr, sc->attrs, sc->mats, d->ntri, &sc->tri_type, s);
     if (e == cudaSuccess) e = upload(&sc->lights, lights.data(), lights.size(), s);
     if (e == cudaSuccess) e = upload(&sc->texs, texs.data(), texs.size(), s);
     if (e == cudaSuccess) e = upload(&sc->texels, d->texels, texel_floats, s);
     if (e == cudaSuccess) e = upload(&sc->attr_c2o, c2o.data(), c2o.size(), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { scene_free(sc); return cuda_fail(e, "aur_scene_create"); }
-    sc->bvh.corner_n = sc->corner_n;       // aur_bvh_intersect on aur_scene_bvh reads the scene's arrays
-    sc->bvh.corner_uv = sc->corner_uv;
+    sc->bvh.tri = sc->tri;                 // aur_bvh_intersect on aur_scene_bvh reads the scene's records
     *out = sc;
     return AUR_OK;
 }
