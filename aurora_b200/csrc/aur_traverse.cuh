@@ -279,7 +279,7 @@ __device__ __forceinline__ bool bvh_trace4(const Node4* __restrict__ nodes, cons
                 if (tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
                                   &t, &u, &v)) {
                     if (kAnyHit) return true;
-                    if (tie) *tie = *tie || (t == tbest && best >= 0);
+                    if (tie) *tie = *tie || (!(t < tbest) && best >= 0);   // equal, or not a number
                     tbest = t; bu = u; bv = v;
                     best = __float_as_int(p.w);
                     box_tmax = tbest * 1.00000095f;
@@ -399,7 +399,7 @@ struct TraceLane {
             if (tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
                               &t, &u, &v)) {
                 if (kAnyHit) { hit_any = true; node = kNoNode; sp = 0; return; }
-                tie = tie || (t == tbest && best >= 0);
+                tie = tie || (!(t < tbest) && best >= 0);   // equal, or not a number
                 tbest = t; bu = u; bv = v;
                 best = __float_as_int(p.w);
                 box_tmax = tbest * 1.00000095f;

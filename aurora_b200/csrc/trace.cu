@@ -1,47 +1,295 @@
 // trace.cu — batched closest-hit / occlusion queries over the device BVH.
-// The C-ABI entry points aur_trace_closest / aur_trace_occluded run these;
+// The C-ABI entry points aur_trace_closest / aur_trace_occluded / aur_bvh_intersect run these;
 // they replace EmbreeAccelerator::intersect / intersectBinary
 // (Aurora/src/geometry/embreeAccelerator.cpp:41-100) for arrays of rays.
+//
+// Three forms by the number of rays. Large batches run a resident grid whose lanes take the next ray
+// as soon as theirs is finished, over the tree form the wavefront renderer uses (full-precision
+// or quantised 4-wide nodes): 2^20 incoherent rays on 20,482 triangles 181 -> 144 us, 1,500,001
+// next-event rays on a 0.85 M triangle landscape 661 -> 411 us. Small ones cannot fill the chip and
+// take as long as their longest ray's walk: a warp per ray walks it side by side, 1,000 rays
+// 41 -> 24 us, of which 15 are the call's. In between, a thread per ray, spread over more warps
+// with fewer rays each where there are few.
 #include "aur_kernels.h"
 #include "aur_traverse.cuh"
+#include <algorithm>
 
 namespace aur {
 namespace {
 
 constexpr int kTraceBlock = 128;
+constexpr int kTraceRefill = 12;     // idle lanes of a warp that fetch new rays together
+constexpr int kTraceRounds = 4;      // rounds between fetches (both as in the wavefront's kernels)
+
+struct HitRec { float t, u, v; int prim, attr; };   // aur_hit
+
+__device__ __forceinline__ void put_hit(HitRec* out, const Hit& h, bool hit, float maxt, const int* tri_attr) {
+    out->t = hit ? h.t : maxt;
+    out->u = hit ? h.u : 0.f;
+    out->v = hit ? h.v : 0.f;
+    out->prim = hit ? h.prim : -1;
+    out->attr = hit ? (tri_attr ? tri_attr[h.prim] : 0) : -1;
+}
+
+// The ray of this thread when every warp takes `per_warp` of them; n or more: none.
+__device__ __forceinline__ uint32_t spread_index(int per_warp) {
+    const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    return lane < (uint32_t)per_warp ? warp * per_warp + lane : 0xffffffffu;
+}
 
 __global__ void __launch_bounds__(kTraceBlock) k_trace_closest(const BvhNode* __restrict__ nodes,
                                                                const BvhNode4* __restrict__ nodes4,
                                                                const BvhTri* __restrict__ tris,
                                                                const int* __restrict__ tri_attr,
-                                                               const float4* __restrict__ rays, float* hits,
-                                                               uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                               const float4* __restrict__ rays, HitRec* hits,
+                                                               uint32_t n, int per_warp) {
+    const uint32_t i = spread_index(per_warp);
     if (i >= n) return;
-    const float4 a = __ldg(&rays[2 * i]);
-    const float4 b = __ldg(&rays[2 * i + 1]);
+    const float4 a = __ldg(&rays[2 * (size_t)i]);
+    const float4 b = __ldg(&rays[2 * (size_t)i + 1]);
     Hit h;
     TraceWork w;
     const bool hit = bvh_closest(nodes, nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, &h, w);
-    float* o = hits + 5 * (size_t)i;
-    o[0] = hit ? h.t : b.w;
-    o[1] = hit ? h.u : 0.f;
-    o[2] = hit ? h.v : 0.f;
-    o[3] = __int_as_float(hit ? h.prim : -1);
-    o[4] = __int_as_float(hit ? (tri_attr ? tri_attr[h.prim] : 0) : -1);
+    put_hit(hits + i, h, hit, b.w, tri_attr);
 }
 
 __global__ void __launch_bounds__(kTraceBlock) k_trace_occluded(const BvhNode* __restrict__ nodes,
                                                                 const BvhNode4* __restrict__ nodes4,
                                                                 const BvhTri* __restrict__ tris,
                                                                 const float4* __restrict__ rays, uint8_t* occ,
-                                                                uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                                uint32_t n, int per_warp) {
+    const uint32_t i = spread_index(per_warp);
     if (i >= n) return;
-    const float4 a = __ldg(&rays[2 * i]);
-    const float4 b = __ldg(&rays[2 * i + 1]);
+    const float4 a = __ldg(&rays[2 * (size_t)i]);
+    const float4 b = __ldg(&rays[2 * (size_t)i + 1]);
     TraceWork w;
     occ[i] = bvh_occluded(nodes, nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, w) ? 1 : 0;
+}
+
+// One warp per ray: the lanes take up to 32 references off the warp's stack at a time, test their
+// boxes or triangles together and push the children entered, so a ray's visits go on side by side
+// instead of one dependent fetch after the other (a thousand rays take as long as the one with
+// the longest walk). Without an order among the references more of them are visited. Where
+// two triangles lie at exactly the closest distance the visiting order decides, and the ray is
+// traced again in bvh_trace4's.
+// The stack cannot overflow: fewer references are taken as it fills, down to one at a time, which
+// needs three entries a level (at most kTraversalStack4, checked at build).
+constexpr int kWarpStack = 1024;
+template <bool kAnyHit>
+__global__ void __launch_bounds__(kTraceBlock) k_trace_warp(const BvhNode4* __restrict__ nodes4,
+                                                            const BvhTri* __restrict__ tris,
+                                                            const int* __restrict__ tri_attr,
+                                                            const float4* __restrict__ rays, HitRec* hits, uint8_t* occ,
+                                                            uint32_t n) {
+    __shared__ int s_stack[kTraceBlock / 32][kWarpStack];
+    const int lane = threadIdx.x & 31;
+    const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, before = (1u << lane) - 1u;
+    if (i >= n) return;
+    int* st = s_stack[threadIdx.x >> 5];
+    const float4 ra = __ldg(&rays[2 * (size_t)i]), rb = __ldg(&rays[2 * (size_t)i + 1]);
+    const float3 o = mk(ra.x, ra.y, ra.z), d = mk(rb.x, rb.y, rb.z);
+    const float mint = ra.w;
+    const float3 id = mk(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
+    const float3 ood = mk(o.x * id.x, o.y * id.y, o.z * id.z);
+    const float box_tmin = mint > 0.f ? mint * 0.99999905f : mint * 1.00000095f;
+    const float kMiss = __int_as_float(0x7f800000);
+    float tbest = rb.w, box_tmax = tbest * 1.00000095f;   // of the warp
+    Hit h;                                                // of the lane
+    h.t = kMiss; h.u = h.v = 0.f; h.prim = -1;
+    bool tie = false, any = false;
+    int sp = 1;
+    if (lane == 0) st[0] = 0;
+    __syncwarp();
+    while (sp > 0) {
+        const int room = (kWarpStack - kTraversalStack4 - sp) / 3;
+        const int k = min(sp, max(1, min(32, room)));
+        const int ref = lane < k ? st[sp - 1 - lane] : ~0;     // ~0: an empty leaf
+        sp -= k;
+        __syncwarp();
+        float t[4] = {kMiss, kMiss, kMiss, kMiss};
+        int r[4] = {~0, ~0, ~0, ~0};
+        bool found = false;
+        if (ref >= 0) {
+            boxes4<kAnyHit>(nodes4 + ref, id, ood, box_tmin, box_tmax, t, r);
+        } else {
+            const int packed = ~ref;
+            const int start = packed >> 5, end = start + (packed & 31);
+            for (int q = start; q < end; ++q) {
+                const float4 p = __ldg(&tris[q].p1);
+                const float4 e1 = __ldg(&tris[q].e1);
+                const float4 e2 = __ldg(&tris[q].e2);
+                float tt, u, v;
+                if (!tri_intersect(mk(p.x, p.y, p.z), mk(e1.x, e1.y, e1.z), mk(e2.x, e2.y, e2.z), o, d, mint, tbest,
+                                   &tt, &u, &v)) continue;
+                found = true;
+                if (kAnyHit) break;
+                if (h.prim >= 0 && !(tt < h.t)) {
+                    tie = tie || !(tt > h.t);              // equal, or not a number
+                } else {
+                    tie = !(tt == tt);
+                    h.t = tt; h.u = u; h.v = v; h.prim = __float_as_int(p.w);
+                }
+            }
+        }
+        __syncwarp();
+        if (__any_sync(0xffffffffu, found)) {
+            if (kAnyHit) { any = true; break; }
+            float best = h.t;
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1) best = fminf(best, __shfl_xor_sync(0xffffffffu, best, s));
+            tbest = fminf(tbest, best);
+            box_tmax = tbest * 1.00000095f;
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const bool in = t[c] != kMiss;
+            const uint32_t m = __ballot_sync(0xffffffffu, in);
+            if (in) st[sp + __popc(m & before)] = r[c];
+            sp += __popc(m);
+        }
+        __syncwarp();
+    }
+    if (kAnyHit) {
+        if (lane == 0) occ[i] = any ? 1 : 0;
+        return;
+    }
+    // the lanes' closest hits: one of them is the ray's, unless several share its distance
+    const uint32_t have = __ballot_sync(0xffffffffu, h.prim >= 0);
+    const uint32_t bad = __ballot_sync(0xffffffffu, h.prim >= 0 && !(h.t == h.t));
+    const uint32_t win = __ballot_sync(0xffffffffu, h.prim >= 0 && h.t <= tbest);
+    const uint32_t tied = __ballot_sync(0xffffffffu, tie) & win;
+    if (!have) {
+        if (lane == 0) put_hit(hits + i, h, false, rb.w, tri_attr);
+    } else if (bad || tied || __popc(win) != 1) {
+        if (lane == 0) {
+            TraceWork w;
+            const bool hit = bvh_trace4<false>(nodes4, tris, o, d, mint, rb.w, &h, w);
+            put_hit(hits + i, h, hit, rb.w, tri_attr);
+        }
+    } else if (lane == __ffs(win) - 1) {
+        put_hit(hits + i, h, true, rb.w, tri_attr);
+    }
+}
+
+// The resident form. Warps fetch ranges of rays from *cursor. Closest hits that meet two triangles at
+// exactly the same distance are left to k_trace_ties: their indices are appended to `ties`.
+template <bool kAnyHit, class Node4>
+__global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restrict__ nodes, const BvhTri* __restrict__ tris,
+                                                           const int* __restrict__ tri_attr,
+                                                           const float4* __restrict__ rays, HitRec* __restrict__ hits,
+                                                           uint8_t* __restrict__ occ, uint32_t n, uint32_t* cursor,
+                                                           uint32_t* ties) {
+    extern __shared__ int s_stack[];
+    LaneStack4 stack;
+    stack.col = s_stack + threadIdx.x;
+    stack.stride = blockDim.x;
+    TraceState4<kAnyHit, Node4> ts;
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t i = 0;
+    bool has = false, exhausted = false;
+    while (true) {
+        const bool need = !has && !exhausted;
+        const uint32_t m = __ballot_sync(0xffffffffu, need);
+        const uint32_t act = __ballot_sync(0xffffffffu, has);
+        if (m && (__popc(m) >= kTraceRefill || act == 0)) {
+            const int leader = __ffs(m) - 1;
+            uint32_t b = 0;
+            if ((int)lane == leader) b = atomicAdd(&cursor[0], (uint32_t)__popc(m));
+            b = __shfl_sync(0xffffffffu, b, leader);
+            if (need) {
+                i = b + __popc(m & ((1u << lane) - 1u));
+                if (i < n) {
+                    const float4 o = __ldg(&rays[2 * (size_t)i]), d = __ldg(&rays[2 * (size_t)i + 1]);
+                    ts.begin(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, d.w);
+                    has = true;
+                } else {
+                    exhausted = true;
+                }
+            }
+        }
+        if (__ballot_sync(0xffffffffu, has || !exhausted) == 0) break;
+        for (int k = 0; k < kTraceRounds; ++k) ts.round(nodes, tris, stack);
+        if (has && ts.finished()) {
+            has = false;
+            if constexpr (kAnyHit) {
+                occ[i] = ts.hit_any ? 1 : 0;
+            } else if (sizeof(Node4) != sizeof(BvhNode4) && ts.tie) {
+                ties[atomicAdd(&cursor[1], 1u)] = i;
+            } else {
+                Hit h;
+                h.t = ts.tbest; h.u = ts.bu; h.v = ts.bv; h.prim = ts.best;
+                put_hit(hits + i, h, ts.best >= 0, ts.tbest, tri_attr);
+            }
+        }
+    }
+}
+
+// The rays left by the quantised traversal, over the full-precision nodes.
+__global__ void __launch_bounds__(kTraceBlock) k_trace_ties(const BvhNode4* __restrict__ nodes4, const BvhTri* __restrict__ tris,
+                                                            const int* __restrict__ tri_attr,
+                                                            const float4* __restrict__ rays, HitRec* hits,
+                                                            const uint32_t* __restrict__ cursor,
+                                                            const uint32_t* __restrict__ ties) {
+    const uint32_t m = cursor[1];
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
+        const uint32_t i = ties[k];
+        const float4 a = __ldg(&rays[2 * (size_t)i]), b = __ldg(&rays[2 * (size_t)i + 1]);
+        Hit h;
+        TraceWork w;
+        const bool hit = bvh_trace4<false>(nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, &h, w);
+        put_hit(hits + i, h, hit, b.w, tri_attr);
+    }
+}
+
+int sm_count() {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// Rays per warp of a small batch: the fewest (a power of two) that need at most kSpreadWarps warps per
+// SM; 32 once the batch is large.
+constexpr int kSpreadWarps = 16;
+int rays_per_warp(uint32_t n, int sms) {
+    int r = 1;
+    while (r < 32 && (n + r - 1) / r > (uint32_t)(kSpreadWarps * sms)) r *= 2;
+    return r;
+}
+
+unsigned spread_grid(uint32_t n, int per_warp) {
+    const uint64_t warps = ((uint64_t)n + per_warp - 1) / per_warp;
+    return (unsigned)((warps * 32 + kTraceBlock - 1) / kTraceBlock);
+}
+
+// Up to this many rays per SM each has a warp of its own (14,208 on 148 SMs). A warp per ray against
+// spread threads, closest hits, 1,000 / 8,000 / 16,384 / 32,000 rays on 20,482 triangles: 24 vs 54,
+// 28 vs 48, 34 vs 43, 43 vs 61 us; on 0.85 M triangles 29 vs 48, 45 vs 58, 64 vs 71, 101 vs 74 us.
+constexpr uint32_t kWarpRays = 96;
+// From this many rays on the resident form pays for its launches: 2^18 on trees with quantised
+// nodes for closest hits (260,000 rays 209 -> 173 us), 2^19 on smaller ones (300,000 rays 85 vs
+// 89 us, 524,288 rays 120 -> 108).
+uint32_t resident_min(const DeviceBvh& bvh) { return bvh.num_nodes4 >= kQuantMinNodes4 ? 1u << 18 : 1u << 19; }
+
+template <bool kAnyHit, class Node4>
+cudaError_t run_resident(const DeviceBvh& bvh, const Node4* nodes, const int* tri_attr, const void* rays, void* hits,
+                         uint8_t* occ, uint32_t n, int sms, cudaStream_t s) {
+    const bool ties = !kAnyHit && sizeof(Node4) != sizeof(BvhNode4);
+    uint32_t* cursor = nullptr;      // cursor, tie count, tie list
+    cudaError_t e = cudaMallocAsync((void**)&cursor, sizeof(uint32_t) * (2 + (ties ? (size_t)n : 0)), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, 2 * sizeof(uint32_t), s);
+    if (e != cudaSuccess) { if (cursor) cudaFreeAsync(cursor, s); return e; }
+    const size_t smem = sizeof(int) * kSharedDepth * 256;
+    int nb = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_resident<kAnyHit, Node4>, 256, smem);
+    k_trace_resident<kAnyHit, Node4><<<std::max(1, nb) * sms, 256, smem, s>>>(nodes, bvh.tris, tri_attr, (const float4*)rays,
+                                                                               (HitRec*)hits, occ, n, cursor, cursor + 2);
+    if (ties)
+        k_trace_ties<<<sms, kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays, (HitRec*)hits, cursor,
+                                                 cursor + 2);
+    e = cudaGetLastError();
+    cudaFreeAsync(cursor, s);
+    return e;
 }
 
 }  // namespace
@@ -49,15 +297,38 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_occluded(const BvhNode* _
 cudaError_t launch_trace_closest(const DeviceBvh& bvh, const int* tri_attr, const void* rays, void* hits, uint32_t n,
                                  cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_trace_closest<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(
-        bvh.nodes, bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays, (float*)hits, n);
+    const int sms = sm_count();
+    if (bvh.nodes4 && n >= resident_min(bvh)) {
+        return bvh.num_nodes4 >= kQuantMinNodes4
+                   ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, tri_attr, rays, hits, nullptr, n, sms, s)
+                   : run_resident<false, BvhNode4>(bvh, bvh.nodes4, tri_attr, rays, hits, nullptr, n, sms, s);
+    }
+    if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
+        k_trace_warp<false><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays,
+                                                                      (HitRec*)hits, nullptr, n);
+        return cudaGetLastError();
+    }
+    const int r = rays_per_warp(n, sms);
+    k_trace_closest<<<spread_grid(n, r), kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays,
+                                                              (HitRec*)hits, n, r);
     return cudaGetLastError();
 }
 
 cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
-    k_trace_occluded<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris,
-                                                                                 (const float4*)rays, occ, n);
+    const int sms = sm_count();
+    if (bvh.nodes4 && n >= resident_min(bvh)) {
+        return bvh.num_nodes4 >= kQuantMinNodes4Any
+                   ? run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, nullptr, rays, nullptr, occ, n, sms, s)
+                   : run_resident<true, BvhNode4>(bvh, bvh.nodes4, nullptr, rays, nullptr, occ, n, sms, s);
+    }
+    if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
+        k_trace_warp<true><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, nullptr, (const float4*)rays, nullptr,
+                                                                     occ, n);
+        return cudaGetLastError();
+    }
+    const int r = rays_per_warp(n, sms);
+    k_trace_occluded<<<spread_grid(n, r), kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris, (const float4*)rays, occ, n, r);
     return cudaGetLastError();
 }
 
