@@ -10,6 +10,8 @@ namespace aur {
 // trace.cu — batched ray queries (aur_ray / aur_hit layouts of aurora_b200.h)
 cudaError_t launch_trace_closest(const DeviceBvh& bvh, const int* tri_attr, const void* rays, void* hits, uint32_t n,
                                  cudaStream_t s);
+// the whole record of EmbreeAccelerator::intersect (aur_isect); shrinks rays[i].maxt on a hit
+cudaError_t launch_intersect(const DeviceBvh& bvh, const TriShade* tri, void* rays, void* isects, uint32_t n, cudaStream_t s);
 cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, cudaStream_t s);
 
 // kelemen.cu — directional-albedo table for reflectance index 0..20 into out[2048]

@@ -10,6 +10,7 @@
 // take as long as their longest ray's walk: a warp per ray walks it side by side, 1,000 rays
 // 41 -> 24 us, of which 15 are the call's. In between, a thread per ray, spread over more warps
 // with fewer rays each where there are few.
+#include "aurora_b200.h"
 #include "aur_kernels.h"
 #include "aur_traverse.cuh"
 #include <algorithm>
@@ -21,15 +22,69 @@ constexpr int kTraceBlock = 128;
 constexpr int kTraceRefill = 12;     // idle lanes of a warp that fetch new rays together
 constexpr int kTraceRounds = 4;      // rounds between fetches (both as in the wavefront's kernels)
 
-struct HitRec { float t, u, v; int prim, attr; };   // aur_hit
+// Where a closest hit goes: the plain record, or the whole record of EmbreeAccelerator::intersect.
+struct HitOut {
+    aur_hit* hits;
+    const int* tri_attr;
+    __device__ __forceinline__ void put(uint32_t i, const Hit& h, bool hit, const float4* rays) const {
+        aur_hit* out = hits + i;
+        out->t = hit ? h.t : rays[2 * (size_t)i + 1].w;
+        out->u = hit ? h.u : 0.f;
+        out->v = hit ? h.v : 0.f;
+        out->prim = hit ? h.prim : -1;
+        out->attr = hit ? (tri_attr ? tri_attr[h.prim] : 0) : -1;
+    }
+};
 
-__device__ __forceinline__ void put_hit(HitRec* out, const Hit& h, bool hit, float maxt, const int* tri_attr) {
-    out->t = hit ? h.t : maxt;
-    out->u = hit ? h.u : 0.f;
-    out->v = hit ? h.v : 0.f;
-    out->prim = hit ? h.prim : -1;
-    out->attr = hit ? (tri_attr ? tri_attr[h.prim] : 0) : -1;
-}
+// The hit's post-process of EmbreeAccelerator::intersect (embreeAccelerator.cpp:49-91) with the
+// per-corner normals and uvs the mesh retains (EmbreeMesh::normals / uvs, geometry/embreeMesh.h:62-63):
+//   w = 1. - u - v (in double, rounded to float)
+//   hitP = org + dir * t
+//   hitN = normalize(w n0 + u n1 + v n2), negated first when it faces along dir
+//   st   = w st0 + u st1 + v st2
+//   barCoords = (u, v, w); ray.maxt = t on a hit (embreeAccelerator.cpp:56)
+// The arithmetic is the shading frame's (hit_frame), so a hit reported here and the
+// same hit shaded by the renderers agree bit for bit.
+struct IsectOut {
+    aur_isect* out;
+    const TriShade* tri;
+    __device__ __forceinline__ void put(uint32_t i, const Hit& h, bool hit, float4* rays) const {
+        const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
+        aur_isect r;
+        if (!hit) {
+            r.t = b.w; r.u = r.v = 0.f; r.prim = -1; r.attr = -1;
+            for (int k = 0; k < 3; ++k) { r.hitP[k] = 0.f; r.hitN[k] = 0.f; r.bar[k] = 0.f; }
+            r.st[0] = r.st[1] = 0.f;
+            out[i] = r;
+            return;
+        }
+        const float3 o = mk(a.x, a.y, a.z), d = mk(b.x, b.y, b.z);
+        const float w = (float)(1.0 - h.u - h.v);
+        const TriShade ts = load_tri(tri + h.prim);
+        const float* nn = ts.n;
+        float3 N = mk(w * nn[0] + h.u * nn[3] + h.v * nn[6],
+                      w * nn[1] + h.u * nn[4] + h.v * nn[7],
+                      w * nn[2] + h.u * nn[5] + h.v * nn[8]);
+        if (dot(N, d) > 0.f) N *= -1.f;
+        N = normalize(N);
+        const float3 P = o + d * h.t;
+        const float* uv = ts.uv;
+        r.t = h.t; r.u = h.u; r.v = h.v; r.prim = h.prim;
+        r.attr = ts.attr;
+        r.hitP[0] = P.x; r.hitP[1] = P.y; r.hitP[2] = P.z;
+        r.hitN[0] = N.x; r.hitN[1] = N.y; r.hitN[2] = N.z;
+        r.st[0] = w * uv[0] + h.u * uv[2] + h.v * uv[4];
+        r.st[1] = w * uv[1] + h.u * uv[3] + h.v * uv[5];
+        r.bar[0] = h.u; r.bar[1] = h.v; r.bar[2] = w;
+        out[i] = r;
+        rays[2 * (size_t)i + 1].w = h.t;          // ray->maxt = t
+    }
+};
+
+// Occlusion: no hit is put.
+struct NoOut {
+    __device__ __forceinline__ void put(uint32_t, const Hit&, bool, const float4*) const {}
+};
 
 // The ray of this thread when every warp takes `per_warp` of them; n or more: none.
 __device__ __forceinline__ uint32_t spread_index(int per_warp) {
@@ -37,20 +92,19 @@ __device__ __forceinline__ uint32_t spread_index(int per_warp) {
     return lane < (uint32_t)per_warp ? warp * per_warp + lane : 0xffffffffu;
 }
 
+template <class Out>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_closest(const BvhNode* __restrict__ nodes,
                                                                const BvhNode4* __restrict__ nodes4,
-                                                               const BvhTri* __restrict__ tris,
-                                                               const int* __restrict__ tri_attr,
-                                                               const float4* __restrict__ rays, HitRec* hits,
+                                                               const BvhTri* __restrict__ tris, float4* rays, Out out,
                                                                uint32_t n, int per_warp) {
     const uint32_t i = spread_index(per_warp);
     if (i >= n) return;
-    const float4 a = __ldg(&rays[2 * (size_t)i]);
-    const float4 b = __ldg(&rays[2 * (size_t)i + 1]);
+    const float4 a = rays[2 * (size_t)i];
+    const float4 b = rays[2 * (size_t)i + 1];
     Hit h;
     TraceWork w;
     const bool hit = bvh_closest(nodes, nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, &h, w);
-    put_hit(hits + i, h, hit, b.w, tri_attr);
+    out.put(i, h, hit, rays);
 }
 
 __global__ void __launch_bounds__(kTraceBlock) k_trace_occluded(const BvhNode* __restrict__ nodes,
@@ -60,8 +114,8 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_occluded(const BvhNode* _
                                                                 uint32_t n, int per_warp) {
     const uint32_t i = spread_index(per_warp);
     if (i >= n) return;
-    const float4 a = __ldg(&rays[2 * (size_t)i]);
-    const float4 b = __ldg(&rays[2 * (size_t)i + 1]);
+    const float4 a = rays[2 * (size_t)i];
+    const float4 b = rays[2 * (size_t)i + 1];
     TraceWork w;
     occ[i] = bvh_occluded(nodes, nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, w) ? 1 : 0;
 }
@@ -75,18 +129,16 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_occluded(const BvhNode* _
 // The stack cannot overflow: fewer references are taken as it fills, down to one at a time, which
 // needs three entries a level (at most kTraversalStack4, checked at build).
 constexpr int kWarpStack = 1024;
-template <bool kAnyHit>
+template <bool kAnyHit, class Out>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_warp(const BvhNode4* __restrict__ nodes4,
-                                                            const BvhTri* __restrict__ tris,
-                                                            const int* __restrict__ tri_attr,
-                                                            const float4* __restrict__ rays, HitRec* hits, uint8_t* occ,
-                                                            uint32_t n) {
+                                                            const BvhTri* __restrict__ tris, float4* rays, Out out,
+                                                            uint8_t* occ, uint32_t n) {
     __shared__ int s_stack[kTraceBlock / 32][kWarpStack];
     const int lane = threadIdx.x & 31;
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, before = (1u << lane) - 1u;
     if (i >= n) return;
     int* st = s_stack[threadIdx.x >> 5];
-    const float4 ra = __ldg(&rays[2 * (size_t)i]), rb = __ldg(&rays[2 * (size_t)i + 1]);
+    const float4 ra = rays[2 * (size_t)i], rb = rays[2 * (size_t)i + 1];
     const float3 o = mk(ra.x, ra.y, ra.z), d = mk(rb.x, rb.y, rb.z);
     const float mint = ra.w;
     const float3 id = mk(safe_rcp(d.x), safe_rcp(d.y), safe_rcp(d.z));
@@ -159,25 +211,23 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_warp(const BvhNode4* __re
     const uint32_t win = __ballot_sync(0xffffffffu, h.prim >= 0 && h.t <= tbest);
     const uint32_t tied = __ballot_sync(0xffffffffu, tie) & win;
     if (!have) {
-        if (lane == 0) put_hit(hits + i, h, false, rb.w, tri_attr);
+        if (lane == 0) out.put(i, h, false, rays);
     } else if (bad || tied || __popc(win) != 1) {
         if (lane == 0) {
             TraceWork w;
             const bool hit = bvh_trace4<false>(nodes4, tris, o, d, mint, rb.w, &h, w);
-            put_hit(hits + i, h, hit, rb.w, tri_attr);
+            out.put(i, h, hit, rays);
         }
     } else if (lane == __ffs(win) - 1) {
-        put_hit(hits + i, h, true, rb.w, tri_attr);
+        out.put(i, h, true, rays);
     }
 }
 
 // The resident form. Warps fetch ranges of rays from *cursor. Closest hits that meet two triangles at
 // exactly the same distance are left to k_trace_ties: their indices are appended to `ties`.
-template <bool kAnyHit, class Node4>
+template <bool kAnyHit, class Node4, class Out>
 __global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restrict__ nodes, const BvhTri* __restrict__ tris,
-                                                           const int* __restrict__ tri_attr,
-                                                           const float4* __restrict__ rays, HitRec* __restrict__ hits,
-                                                           uint8_t* __restrict__ occ, uint32_t n, uint32_t* cursor,
+                                                           float4* rays, Out out, uint8_t* __restrict__ occ, uint32_t n, uint32_t* cursor,
                                                            uint32_t* ties) {
     extern __shared__ int s_stack[];
     LaneStack4 stack;
@@ -199,7 +249,7 @@ __global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restri
             if (need) {
                 i = b + __popc(m & ((1u << lane) - 1u));
                 if (i < n) {
-                    const float4 o = __ldg(&rays[2 * (size_t)i]), d = __ldg(&rays[2 * (size_t)i + 1]);
+                    const float4 o = rays[2 * (size_t)i], d = rays[2 * (size_t)i + 1];
                     ts.begin(mk(o.x, o.y, o.z), mk(d.x, d.y, d.z), o.w, d.w);
                     has = true;
                 } else {
@@ -218,26 +268,25 @@ __global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restri
             } else {
                 Hit h;
                 h.t = ts.tbest; h.u = ts.bu; h.v = ts.bv; h.prim = ts.best;
-                put_hit(hits + i, h, ts.best >= 0, ts.tbest, tri_attr);
+                out.put(i, h, ts.best >= 0, rays);
             }
         }
     }
 }
 
 // The rays left by the quantised traversal, over the full-precision nodes.
+template <class Out>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_ties(const BvhNode4* __restrict__ nodes4, const BvhTri* __restrict__ tris,
-                                                            const int* __restrict__ tri_attr,
-                                                            const float4* __restrict__ rays, HitRec* hits,
-                                                            const uint32_t* __restrict__ cursor,
+                                                            float4* rays, Out out, const uint32_t* __restrict__ cursor,
                                                             const uint32_t* __restrict__ ties) {
     const uint32_t m = cursor[1];
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
         const uint32_t i = ties[k];
-        const float4 a = __ldg(&rays[2 * (size_t)i]), b = __ldg(&rays[2 * (size_t)i + 1]);
+        const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
         Hit h;
         TraceWork w;
         const bool hit = bvh_trace4<false>(nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, &h, w);
-        put_hit(hits + i, h, hit, b.w, tri_attr);
+        out.put(i, h, hit, rays);
     }
 }
 
@@ -271,64 +320,68 @@ constexpr uint32_t kWarpRays = 96;
 // 89 us, 524,288 rays 120 -> 108).
 uint32_t resident_min(const DeviceBvh& bvh) { return bvh.num_nodes4 >= kQuantMinNodes4 ? 1u << 18 : 1u << 19; }
 
-template <bool kAnyHit, class Node4>
-cudaError_t run_resident(const DeviceBvh& bvh, const Node4* nodes, const int* tri_attr, const void* rays, void* hits,
-                         uint8_t* occ, uint32_t n, int sms, cudaStream_t s) {
-    const bool ties = !kAnyHit && sizeof(Node4) != sizeof(BvhNode4);
+template <bool kAnyHit, class Node4, class Out>
+cudaError_t run_resident(const DeviceBvh& bvh, const Node4* nodes, float4* rays, const Out& out, uint8_t* occ, uint32_t n,
+                         int sms, cudaStream_t s) {
+    constexpr bool ties = !kAnyHit && sizeof(Node4) != sizeof(BvhNode4);
     uint32_t* cursor = nullptr;      // cursor, tie count, tie list
     cudaError_t e = cudaMallocAsync((void**)&cursor, sizeof(uint32_t) * (2 + (ties ? (size_t)n : 0)), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, 2 * sizeof(uint32_t), s);
     if (e != cudaSuccess) { if (cursor) cudaFreeAsync(cursor, s); return e; }
     const size_t smem = sizeof(int) * kSharedDepth * 256;
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_resident<kAnyHit, Node4>, 256, smem);
-    k_trace_resident<kAnyHit, Node4><<<std::max(1, nb) * sms, 256, smem, s>>>(nodes, bvh.tris, tri_attr, (const float4*)rays,
-                                                                               (HitRec*)hits, occ, n, cursor, cursor + 2);
-    if (ties)
-        k_trace_ties<<<sms, kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays, (HitRec*)hits, cursor,
-                                                 cursor + 2);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_resident<kAnyHit, Node4, Out>, 256, smem);
+    k_trace_resident<kAnyHit, Node4, Out><<<std::max(1, nb) * sms, 256, smem, s>>>(nodes, bvh.tris, rays, out, occ, n, cursor,
+                                                                                    cursor + 2);
+    if constexpr (ties) k_trace_ties<Out><<<sms, kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, rays, out, cursor, cursor + 2);
     e = cudaGetLastError();
     cudaFreeAsync(cursor, s);
     return e;
 }
 
-}  // namespace
-
-cudaError_t launch_trace_closest(const DeviceBvh& bvh, const int* tri_attr, const void* rays, void* hits, uint32_t n,
-                                 cudaStream_t s) {
+template <class Out>
+cudaError_t run_closest(const DeviceBvh& bvh, float4* rays, const Out& out, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const int sms = sm_count();
-    if (bvh.nodes4 && n >= resident_min(bvh)) {
+    if (bvh.nodes4 && n >= resident_min(bvh))
         return bvh.num_nodes4 >= kQuantMinNodes4
-                   ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, tri_attr, rays, hits, nullptr, n, sms, s)
-                   : run_resident<false, BvhNode4>(bvh, bvh.nodes4, tri_attr, rays, hits, nullptr, n, sms, s);
-    }
+                   ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, rays, out, nullptr, n, sms, s)
+                   : run_resident<false, BvhNode4>(bvh, bvh.nodes4, rays, out, nullptr, n, sms, s);
     if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
-        k_trace_warp<false><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays,
-                                                                      (HitRec*)hits, nullptr, n);
+        k_trace_warp<false, Out><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, rays, out, nullptr, n);
         return cudaGetLastError();
     }
     const int r = rays_per_warp(n, sms);
-    k_trace_closest<<<spread_grid(n, r), kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris, tri_attr, (const float4*)rays,
-                                                              (HitRec*)hits, n, r);
+    k_trace_closest<Out><<<spread_grid(n, r), kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris, rays, out, n, r);
     return cudaGetLastError();
+}
+
+}  // namespace
+
+// rays: aur_ray records; written (maxt) by launch_intersect only
+cudaError_t launch_trace_closest(const DeviceBvh& bvh, const int* tri_attr, const void* rays, void* hits, uint32_t n,
+                                 cudaStream_t s) {
+    return run_closest(bvh, (float4*)const_cast<void*>(rays), HitOut{(aur_hit*)hits, tri_attr}, n, s);
+}
+
+cudaError_t launch_intersect(const DeviceBvh& bvh, const TriShade* tri, void* rays, void* isects, uint32_t n, cudaStream_t s) {
+    return run_closest(bvh, (float4*)rays, IsectOut{(aur_isect*)isects, tri}, n, s);
 }
 
 cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const int sms = sm_count();
-    if (bvh.nodes4 && n >= resident_min(bvh)) {
+    float4* r4 = (float4*)const_cast<void*>(rays);
+    if (bvh.nodes4 && n >= resident_min(bvh))
         return bvh.num_nodes4 >= kQuantMinNodes4Any
-                   ? run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, nullptr, rays, nullptr, occ, n, sms, s)
-                   : run_resident<true, BvhNode4>(bvh, bvh.nodes4, nullptr, rays, nullptr, occ, n, sms, s);
-    }
+                   ? run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, r4, NoOut{}, occ, n, sms, s)
+                   : run_resident<true, BvhNode4>(bvh, bvh.nodes4, r4, NoOut{}, occ, n, sms, s);
     if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
-        k_trace_warp<true><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, nullptr, (const float4*)rays, nullptr,
-                                                                     occ, n);
+        k_trace_warp<true, NoOut><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, r4, NoOut{}, occ, n);
         return cudaGetLastError();
     }
     const int r = rays_per_warp(n, sms);
-    k_trace_occluded<<<spread_grid(n, r), kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris, (const float4*)rays, occ, n, r);
+    k_trace_occluded<<<spread_grid(n, r), kTraceBlock, 0, s>>>(bvh.nodes, bvh.nodes4, bvh.tris, r4, occ, n, r);
     return cudaGetLastError();
 }
 
