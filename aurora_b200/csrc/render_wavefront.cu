@@ -1177,11 +1177,14 @@ static uint32_t fill_table(std::vector<BatchItem>& items, int s0, int chunk, flo
     return base;
 }
 
-// Autotuner: times every candidate (pool size x block size x material sort) on the
-// same probe — the first `limit` work items of the real workload (at most 2^25) — and
-// keeps the fastest. Pools larger than twice the probe are not tried. (On the 1080p
-// depth-8 terrain, pools of 2^21 / 2^22 / 2^23 / 2^24 slots gave 475 / 491 / 504 / 509 M
-// samples/s: more paths in flight hide more of the traversal's fetch latency.)
+// Autotuner: times candidates (pool size, material sort, block size) on the same probe, the first
+// `limit` work items of the real workload (at most 2^25), and keeps the fastest: first the pool
+// sizes with the sort on and blocks of 256, then the best pool without the sort, then the better of
+// those with blocks of 128. (All twenty combinations take twice the time and chose one of these
+// on every workload here.) Pools larger than twice the probe are not tried. More paths in flight hide
+// more of the traversal's fetch latency, 1080p terrain frame at 2^21 / 2^22 / 2^23 / 2^24 / 2^25 slots:
+// 204.6 / 196.1 / 189.6 / 185.2 / 183.3 ms. The largest (7.5 GB) is tried only where all paths fit
+// it and not the next smaller: a batch of 25.6 M paths 25.6 -> 22.9 ms.
 // Returns the chosen configuration.
 static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig* best_out) {
     cudaStream_t s = ctx->work_stream;
@@ -1207,46 +1210,47 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
     std::vector<WfScene> tab(items.size());
     limit = std::min(limit, fill_table(items, 0, chunk, samples, tab.data()));
     const int depth = max_rays(items), n = (int)items.size();
-    constexpr int kPools = 5;
-    const uint32_t pools[kPools] = {1u << 20, 1u << 21, 1u << 22, 1u << 23, 1u << 24};
-    const int blocks[2] = {128, 256};
     double best = -1.0;
     WfConfig bestc;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
-    for (int pi = 0; pi < kPools && e == cudaSuccess; ++pi) {
-        if (pi > 0 && (uint64_t)pools[pi] > 2ull * limit) break;   // a pool that would stay mostly empty
-        for (int bi = 0; bi < 2 && e == cudaSuccess; ++bi)
-            for (int so = 0; so < 2 && e == cudaSuccess; ++so) {
-                WfConfig c;
-                c.pool = pools[pi];
-                c.block = blocks[bi];
-                c.sort = so;
-                tree_for(items, &c);
-                WfRun run;
-                e = run.init(c, (int)items.size(), s);
-                if (e == cudaSuccess) memcpy(run.h_scenes, tab.data(), sizeof(WfScene) * n);
-                // a short probe runs twice: the first pass also builds its graph
-                uint64_t l = 0;
-                auto pass = [&](uint32_t items_in_pass) {
-                    cudaError_t pe = run.begin_pass(items_in_pass, n, true);
-                    if (pe == cudaSuccess) pe = cudaEventRecord(e0, s);
-                    if (pe == cudaSuccess) pe = run.run_pass(items_in_pass, depth, &l);
-                    if (pe == cudaSuccess) pe = cudaEventRecord(e1, s);
-                    const cudaError_t se = cudaStreamSynchronize(s);
-                    return pe != cudaSuccess ? pe : se;
-                };
-                if (e == cudaSuccess && limit <= (1u << 22)) e = pass(limit);
-                if (e == cudaSuccess) e = pass(limit);
-                float ms = 0.f;
-                if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-                run.release();
-                if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); e = cudaSuccess; continue; }
-                const double rate = ms > 0.f ? limit / ms : 0.0;
-                if (e == cudaSuccess && rate > best) { best = rate; bestc = c; }
-            }
+    auto probe = [&](uint32_t pool, int sort, int block) {
+        if (e != cudaSuccess) return;
+        WfConfig c;
+        c.pool = pool;
+        c.block = block;
+        c.sort = sort;
+        tree_for(items, &c);
+        WfRun run;
+        e = run.init(c, n, s);
+        if (e == cudaSuccess) memcpy(run.h_scenes, tab.data(), sizeof(WfScene) * n);
+        uint64_t l = 0;
+        auto pass = [&](uint32_t items_in_pass) {
+            cudaError_t pe = run.begin_pass(items_in_pass, n, true);
+            if (pe == cudaSuccess) pe = cudaEventRecord(e0, s);
+            if (pe == cudaSuccess) pe = run.run_pass(items_in_pass, depth, &l);
+            if (pe == cudaSuccess) pe = cudaEventRecord(e1, s);
+            const cudaError_t se = cudaStreamSynchronize(s);
+            return pe != cudaSuccess ? pe : se;
+        };
+        // a short probe runs twice: the first pass also builds its graph
+        if (e == cudaSuccess && limit <= (1u << 22)) e = pass(limit);
+        if (e == cudaSuccess) e = pass(limit);
+        float ms = 0.f;
+        if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
+        run.release();
+        if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); e = cudaSuccess; return; }
+        const double rate = ms > 0.f ? limit / ms : 0.0;
+        if (e == cudaSuccess && rate > best) { best = rate; bestc = c; }
+    };
+    for (uint32_t pool = 1u << 20; pool <= (1u << 24); pool <<= 1) {
+        if (pool > (1u << 20) && (uint64_t)pool > 2ull * limit) break;   // a pool that would stay mostly empty
+        probe(pool, 1, 256);
     }
+    if (total > (1ull << 24) && total <= (1ull << 25)) probe(1u << 25, 1, 256);
+    if (best >= 0) probe(bestc.pool, 0, 256);
+    if (best >= 0) probe(bestc.pool, bestc.sort, 128);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     cudaFreeAsync(samples, s);
