@@ -34,6 +34,7 @@
 #include "aur_shading.cuh"
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstring>
 
 namespace aur {
@@ -343,10 +344,9 @@ __global__ void k_init_leaves(const uint32_t* __restrict__ sorted, int n, const 
     clusters[k] = k;
 }
 
-// Makes node `x` the parent of clusters a and b: its box, SAH cost and collapse, and its row of the
-// 4-wide grouping.
-__device__ __forceinline__ void merge_node(const Tree& t, const Sah& sah, int x, int a, int b) {
-    const Kid l = load_kid(t, a), r = load_kid(t, b);
+// Makes node `x` the parent of clusters a and b, whose data are l and r: its box, SAH cost and
+// collapse, and its row of the 4-wide grouping. Returns the new node's data.
+__device__ __forceinline__ Kid merge_kids(const Tree& t, const Sah& sah, int x, int a, int b, const Kid& l, const Kid& r) {
     const float3 lo = mk(fminf(l.lo.x, r.lo.x), fminf(l.lo.y, r.lo.y), fminf(l.lo.z, r.lo.z));
     const float3 hi = mk(fmaxf(l.hi.x, r.hi.x), fmaxf(l.hi.y, r.hi.y), fmaxf(l.hi.z, r.hi.z));
     const float A = half_area(lo, hi);
@@ -382,39 +382,40 @@ __device__ __forceinline__ void merge_node(const Tree& t, const Sah& sah, int x,
         }
     const float s1 = (d[0] * d[1] + d[1] * d[2] + d[2] * d[0]) + D[4];
     const bool one2 = s1 <= D[2], one3 = s1 <= D[3];      // s1 = A + D(x, 4) > D(x, 4)
-    t.S[x] = make_float4(s1, one2 ? s1 : D[2], one3 ? s1 : D[3], D[4]);
+    const float4 S = make_float4(s1, one2 ? s1 : D[2], one3 ? s1 : D[3], D[4]);
+    t.S[x] = S;
     t.dec[x] = make_uchar4(0, (unsigned char)(one2 ? 0 : kd[2]), (unsigned char)(one3 ? 0 : kd[3]), (unsigned char)kd[4]);
+    Kid k;
+    k.lo = lo; k.hi = hi;
+    k.cost = collapsed ? leaf : split;
+    k.cnt = c;
+    k.icount = collapsed ? 0 : 1 + l.icount + r.icount;
+    k.collapsed = collapsed;
+    k.S = collapsed ? make_float4(0.f, 0.f, 0.f, 0.f) : S;
+    return k;
+}
+__device__ __forceinline__ void merge_node(const Tree& t, const Sah& sah, int x, int a, int b) {
+    merge_kids(t, sah, x, a, b, load_kid(t, a), load_kid(t, b));
 }
 
 // ------------------------------------------------------------ PLOC
 constexpr int kPlocThreads = 256;
 constexpr int kPlocTile = 2 * kPlocThreads;
-constexpr int kPlocBatch = 8;      // iterations between host reads of the count
+// Iterations between host reads of the count: as many as it takes to get to kFinish if each keeps
+// kPlocKeep of the clusters, 16 at most (an even number, so that the count ends in m[0]).
+// Iterations past that point cost two empty launches each (8 us), a further read of the count
+// 20 us: of the 16 iterations that a fixed eight between reads took at 20,480 triangles, seven
+// were empty.
+constexpr double kPlocKeep = 0.78;
+constexpr int kPlocBatch = 16;
 constexpr int kMaxRadius = 32;
 constexpr int kSuper = 64;         // tiles per partial sum of the compaction
 constexpr int kFinish = 2048;      // from this many clusters on, one block does the rest
 
-// The nearest neighbour of cluster i of m: boxes lo/hi are those of clusters i - r.. (s + 0) on,
-// limited to [0, m). Strict order on unordered pairs: (area, min index, max index); j increases,
-// so for equal area the first j seen has the smaller pair key.
-__device__ __forceinline__ int nearest(const float3* lo, const float3* hi, int at, int i, int m, int r) {
-    const float3 mlo = lo[at], mhi = hi[at];
-    float best = FLT_MAX;
-    int bj = -1;
-    const int j0 = max(0, i - r), j1 = min(m - 1, i + r);
-    for (int j = j0; j <= j1; ++j) {
-        if (j == i) continue;
-        const int k = at + (j - i);
-        const float3 ulo = mk(fminf(mlo.x, lo[k].x), fminf(mlo.y, lo[k].y), fminf(mlo.z, lo[k].z));
-        const float3 uhi = mk(fmaxf(mhi.x, hi[k].x), fmaxf(mhi.y, hi[k].y), fmaxf(mhi.z, hi[k].z));
-        const float a = half_area(ulo, uhi);
-        if (a < best) { best = a; bj = j; }
-    }
-    return bj;
-}
-
-// The same for clusters i and i + 1 (either may lie outside [0, m)): every box of the joint window is
-// read once.
+// The nearest neighbours of clusters i and i + 1 of m (either may lie outside [0, m)), whose boxes are
+// at lo/hi[at] on: within r places, limited to [0, m). Strict order on unordered pairs: (area, min
+// index, max index); j increases, so for equal area the first j seen has the smaller pair key.
+// Every box of the joint window is read once.
 __device__ __forceinline__ void nearest2(const float3* lo, const float3* hi, int at, int i, int m, int r, int (&nn)[2]) {
     const bool in0 = i >= 0 && i < m, in1 = i + 1 >= 0 && i + 1 < m;
     const float3 z = mk(0.f, 0.f, 0.f);
@@ -537,90 +538,171 @@ __global__ void __launch_bounds__(kPlocThreads) k_ploc_compact(const int* __rest
     if (tid == 0 && start + tile >= m) st->m[parity ^ 1] = (int)(base + own);
 }
 
-// All remaining iterations in one block, the clusters' boxes in shared memory. Then the root: never
-// a leaf (a tree has at least one interior node).
+// The nearest neighbour of cluster i, its window dealt out to a group of `lanes` lanes (all of the
+// warp take part), which all get the result: the smallest area, of equal ones the smallest j.
+__device__ __forceinline__ int nearest_lanes(const float3* lo, const float3* hi, int i, int m, int r, int lanes, int q) {
+    float best = FLT_MAX;
+    int bj = -1;
+    if (i < m) {
+        const float3 mlo = lo[i], mhi = hi[i];
+        const int j1 = min(m - 1, i + r);
+        for (int j = max(0, i - r) + q; j <= j1; j += lanes) {
+            if (j == i) continue;
+            const float a = half_area(mk(fminf(mlo.x, lo[j].x), fminf(mlo.y, lo[j].y), fminf(mlo.z, lo[j].z)),
+                                      mk(fmaxf(mhi.x, hi[j].x), fmaxf(mhi.y, hi[j].y), fmaxf(mhi.z, hi[j].z)));
+            if (a < best) { best = a; bj = j; }
+        }
+    }
+    for (int o = lanes >> 1; o; o >>= 1) {
+        const float a = __shfl_xor_sync(0xffffffffu, best, o);
+        const int j = __shfl_xor_sync(0xffffffffu, bj, o);
+        if (a < best || (a == best && (uint32_t)j < (uint32_t)bj)) { best = a; bj = j; }
+    }
+    return bj;
+}
+
+// The clusters of the last iterations, in shared memory. Order, boxes and slots move every
+// iteration; what only a merge reads stays in a slot, and the parent takes the slot of its first child.
+struct FinishMem {
+    float3 lo[kFinish], hi[kFinish];
+    int slot[kFinish], nn[kFinish];
+    int2 merge[kFinish / 2];                        // slots of the iteration's pairs
+    float3 klo[kFinish], khi[kFinish];
+    float4 S[kFinish];
+    float cost[kFinish];
+    int id[kFinish], cnt[kFinish], icount[kFinish];   // cnt: as in Tree::hi, with the collapse bit
+    __device__ __forceinline__ Kid get(int k) const {
+        Kid r;
+        r.lo = klo[k]; r.hi = khi[k]; r.cost = cost[k];
+        r.cnt = cnt[k] >> 1; r.collapsed = (cnt[k] & 1) != 0;
+        r.icount = icount[k]; r.S = S[k];
+        return r;
+    }
+    __device__ __forceinline__ void put(int k, int id_, const Kid& r) {
+        id[k] = id_;
+        klo[k] = r.lo; khi[k] = r.hi; cost[k] = r.cost;
+        cnt[k] = (r.cnt << 1) | (r.collapsed ? 1 : 0);
+        icount[k] = r.icount; S[k] = r.S;
+    }
+};
+
+// All remaining iterations in one block, whatever a merge reads in shared memory. Then the root:
+// never a leaf (a tree has at least one interior node). Some thirty iterations, bound by the
+// search while there are many clusters and by their chain of barriers after that: few clusters
+// share the block's threads for their search; the pairs are put in a list, so that full warps
+// merge them, beside the next iteration's search, which needs the boxes alone; warps without a
+// cluster go from barrier to barrier. A thread per cluster that merges where it stands, its nodes in
+// global memory: 179 us from 2048 clusters; nodes in shared memory and shared searches 131; the
+// list 115; now 105 (at 59% of the SM's issue slots).
 __global__ void __launch_bounds__(1024) k_ploc_finish(const int* __restrict__ clusters, BuildState* st, int parity, Tree t,
                                                       Sah sah, int r) {
     extern __shared__ char s_mem[];
-    float3* s_lo = reinterpret_cast<float3*>(s_mem);
-    float3* s_hi = s_lo + kFinish;
-    int* s_id = reinterpret_cast<int*>(s_hi + kFinish);
-    int* s_nn = s_id + kFinish;
-    __shared__ uint32_t s_scan[33];
-    __shared__ int s_base;
+    FinishMem& c = *reinterpret_cast<FinishMem*>(s_mem);
+    __shared__ uint32_t s_scan[32];
     int m = st->m[parity];
     if (m > kFinish) return;
     const int tid = threadIdx.x;
+    int node = st->node, nmerge = 0;
     for (int k = tid; k < m; k += 1024) {
-        const int c = clusters[k];
-        const float4 a = t.lo[c], b = t.hi[c];
-        s_id[k] = c;
-        s_lo[k] = mk(a.x, a.y, a.z);
-        s_hi[k] = mk(b.x, b.y, b.z);
+        const int x = clusters[k];
+        const Kid kid = load_kid(t, x);
+        c.put(k, x, kid);
+        c.lo[k] = kid.lo; c.hi[k] = kid.hi;
+        c.slot[k] = k;
     }
     __syncthreads();
+    // the merges of the iteration before, from the last thread on (the first ones search)
+    auto merge_pairs = [&]() {
+        const int q = 1023 - tid;                    // at most kFinish / 2 = 1024 pairs
+        if (q >= nmerge) return;
+        const int2 e = c.merge[q];
+        const int x = node - nmerge + q;
+        const Kid kid = merge_kids(t, sah, x, c.id[e.x], c.id[e.y], c.get(e.x), c.get(e.y));
+        c.put(e.x, x, kid);
+    };
     while (m > 1) {
-        for (int k = tid; k < m; k += 1024) s_nn[k] = nearest(s_lo, s_hi, k, k, m, r);
+        merge_pairs();
+        if (m > 1024) {
+            int nn[2] = {-1, -1};
+            if (2 * tid < m) nearest2(c.lo, c.hi, 2 * tid, 2 * tid, m, r, nn);
+            if (2 * tid < m) c.nn[2 * tid] = nn[0];
+            if (2 * tid + 1 < m) c.nn[2 * tid + 1] = nn[1];
+        } else {
+            int shift = 0;
+            while (shift < 3 && (m << (shift + 1)) <= 1024) ++shift;
+            const int i = tid >> shift, q = tid & ((1 << shift) - 1);
+            if ((tid & ~31) >> shift < m) {          // the warp has a cluster
+                const int nn = nearest_lanes(c.lo, c.hi, i, m, r, 1 << shift, q);
+                if (i < m && q == 0) c.nn[i] = nn;
+            }
+        }
         __syncthreads();
         // thread t has clusters 2 t and 2 t + 1, so that ranks follow the order
-        int id[2];
+        int j[2];
+        bool keep[2] = {false, false}, mer[2] = {false, false};
+        const bool busy = 2 * (tid & ~31) < m;       // the warp has any
+        uint32_t own = 0, incl = 0;                  // merges in the low half, kept clusters in the high one
+        if (busy) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int k = 2 * tid + q;
+                j[q] = k < m ? c.nn[k] : -1;
+                const bool mutual = j[q] >= 0 && c.nn[j[q]] == k;
+                mer[q] = mutual && k < j[q];
+                keep[q] = k < m && (!mutual || mer[q]);
+            }
+            own = (mer[0] + mer[1]) | ((uint32_t)(keep[0] + keep[1]) << 16);
+            incl = warp_incl_scan(own);
+        }
+        if ((tid & 31) == 31) s_scan[tid >> 5] = incl;
+        __syncthreads();
+        // every warp adds up the warps before its own
+        const uint32_t w = s_scan[tid & 31];
+        const uint32_t total = __reduce_add_sync(0xffffffffu, w);
+        uint32_t pre = 0;
+        if (busy) pre = __reduce_add_sync(0xffffffffu, (tid & 31) < tid >> 5 ? w : 0u) + incl - own;
+        nmerge = (int)(total & 0xffffu);
+        if (nmerge == 0) break;                      // no progress: the host reports it
+        int mr = (int)(pre & 0xffffu), kr = (int)(pre >> 16);
+        int slot[2];
         float3 lo[2], hi[2];
-        bool keep[2], mer[2];
-        int partner[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int k = 2 * tid + q;
-            keep[q] = mer[q] = false;
-            partner[q] = -1;
-            id[q] = -1;
-            if (k >= m) continue;
-            const int j = s_nn[k];
-            const bool mutual = j >= 0 && s_nn[j] == k;
-            mer[q] = mutual && k < j;
-            keep[q] = !mutual || mer[q];
-            id[q] = s_id[k];
-            lo[q] = s_lo[k];
-            hi[q] = s_hi[k];
-            if (mer[q]) {
-                partner[q] = s_id[j];
-                lo[q] = mk(fminf(lo[q].x, s_lo[j].x), fminf(lo[q].y, s_lo[j].y), fminf(lo[q].z, s_lo[j].z));
-                hi[q] = mk(fmaxf(hi[q].x, s_hi[j].x), fmaxf(hi[q].y, s_hi[j].y), fmaxf(hi[q].z, s_hi[j].z));
-            }
+            if (!keep[q]) continue;
+            lo[q] = c.lo[k];
+            hi[q] = c.hi[k];
+            slot[q] = c.slot[k];
+            if (!mer[q]) continue;
+            const float3 l = c.lo[j[q]], h = c.hi[j[q]];
+            lo[q] = mk(fminf(lo[q].x, l.x), fminf(lo[q].y, l.y), fminf(lo[q].z, l.z));
+            hi[q] = mk(fmaxf(hi[q].x, h.x), fmaxf(hi[q].y, h.y), fmaxf(hi[q].z, h.z));
+            c.merge[mr++] = make_int2(slot[q], c.slot[j[q]]);
         }
-        // both counts in one scan: merges in the low half, kept clusters in the high one
-        uint32_t total;
-        const uint32_t pre = block_excl_scan((mer[0] + mer[1]) | ((uint32_t)(keep[0] + keep[1]) << 16), s_scan, &total);
-        const int nmerge = (int)(total & 0xffffu), nkeep = (int)(total >> 16);
-        if (nmerge == 0) break;                      // no progress: the host reports it
-        if (tid == 0) { s_base = st->node; st->node = s_base + nmerge; }
         __syncthreads();
-        int mr = (int)(pre & 0xffffu), kr = (int)(pre >> 16);
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-            if (mer[q]) {
-                const int x = s_base + mr++;
-                merge_node(t, sah, x, id[q], partner[q]);
-                id[q] = x;
-            }
-            if (keep[q]) {
-                s_id[kr] = id[q];
-                s_lo[kr] = lo[q];
-                s_hi[kr] = hi[q];
-                ++kr;
-            }
+            if (!keep[q]) continue;
+            c.lo[kr] = lo[q];
+            c.hi[kr] = hi[q];
+            c.slot[kr++] = slot[q];
         }
-        m = nkeep;
+        node += nmerge;
+        m = (int)(total >> 16);
         __syncthreads();
     }
+    merge_pairs();
+    __syncthreads();
     if (tid != 0) return;
+    st->node = node;
     st->m[0] = st->m[1] = m;
     if (m != 1) return;
-    const int root = s_id[0];
-    const int2 c = t.child[root];
-    const int n = 1 + t.icount[c.x] + t.icount[c.y];   // as if the root were not collapsed
+    const int root = c.id[c.slot[0]];
+    const int2 ch = t.child[root];
+    const int n = 1 + t.icount[ch.x] + t.icount[ch.y];   // as if the root were not collapsed
     t.up[root] = make_int4(-1, 0, 0, 0);
-    t.up[c.x].w = 0;
-    t.up[c.y].w = 0;
+    t.up[ch.x].w = 0;
+    t.up[ch.y].w = 0;
     st->root = root;
     st->num_nodes = n;
 }
@@ -947,13 +1029,14 @@ cudaError_t build_with(Scratch& w, const float* verts, const uint32_t* idx, int 
         CK(cudaGetLastError());
         const int r = opt.ploc_radius < 1 ? 1 : (opt.ploc_radius > kMaxRadius ? kMaxRadius : opt.ploc_radius);
         const int tile = kPlocTile - 2 * r;
-        const size_t smem = kFinish * (2 * sizeof(float3) + 2 * sizeof(int));
+        const size_t smem = sizeof(FinishMem);
         CK(cudaFuncSetAttribute(k_ploc_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         for (int m = n; ;) {
             if (m > kFinish) {
                 const int tiles = div_up(m, tile);
                 CK(cudaMemsetAsync(w.super[0], 0, sizeof(uint32_t) * (tiles / kSuper + 1), s));
-                for (int it = 0; it < kPlocBatch; ++it) {
+                const int its = std::min(kPlocBatch, ((int)std::ceil(std::log((double)m / kFinish) / -std::log(kPlocKeep)) + 1) & ~1);
+                for (int it = 0; it < its; ++it) {
                     k_ploc_merge<<<tiles, kPlocThreads, 0, s>>>(w.ca, w.st, it & 1, w.t, sah, r, w.out, w.cnt, w.super[it & 1]);
                     k_ploc_compact<<<tiles, kPlocThreads, 0, s>>>(w.out, w.st, it & 1, r, w.cnt, w.super[it & 1],
                                                                   w.super[(it & 1) ^ 1], w.cb);
