@@ -420,8 +420,8 @@ def main():
 
     # Roofline of the dominant kernel. Algorithmic bytes come from a counting pass of the
     # plain renderer (1 spp, untimed): both renderers trace the same rays through the same
-    # tree (the 4-wide one: 128-B node records; the binary one: 64 B), so node visits and
-    # triangle tests (48 B) per path are the same.
+    # tree (4-wide: 64-B quantised node records from 32,768 nodes on, else 128 B; binary:
+    # 64 B), so node visits and triangle tests (48 B) per path are the same.
     cw = frame(_abi.RENDER_PLAIN, count_work=1, spp_=1).stats
     node_b = cw["node_bytes"]
     if st.get("node_bytes", node_b) != node_b:

@@ -304,8 +304,9 @@ typedef struct aur_render_stats {
     uint64_t shadow_tri_tests;
     double stage_ms[5];     /* wavefront: device time of regen, extend, sort, shade, shadow */
     int32_t wf_pool, wf_block, wf_sort;   /* wavefront configuration used (tuned or given) */
-    int32_t node_bytes;     /* bytes of one interior-node record of the tree traversed: 128 for the
-                               4-wide tree, 64 for the binary one */
+    int32_t node_bytes;     /* bytes of one interior-node record of the tree traversed: 64 for the
+                               quantised 4-wide tree and the binary one, 128 for the full-
+                               precision 4-wide tree */
 } aur_render_stats;
 
 AUR_API aur_status aur_render(aur_scene* scene, const aur_render_opts* opts, float* film_rgba, aur_render_stats* stats);
