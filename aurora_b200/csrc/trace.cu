@@ -20,6 +20,7 @@ namespace {
 
 constexpr int kTraceBlock = 128;
 constexpr int kTraceRefill = 12;     // idle lanes of a warp that fetch new rays together
+constexpr uint32_t kResidentMax = 1u << 31;   // its 32-bit cursor runs past the last ray by what is fetched at once
 constexpr int kTraceRounds = 4;      // rounds between fetches (both as in the wavefront's kernels)
 
 // Where a closest hit goes: the plain record, or the whole record of EmbreeAccelerator::intersect.
@@ -343,10 +344,13 @@ template <class Out>
 cudaError_t run_closest(const DeviceBvh& bvh, float4* rays, const Out& out, uint32_t n, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const int sms = sm_count();
-    if (bvh.nodes4 && n >= resident_min(bvh))
-        return bvh.num_nodes4 >= kQuantMinNodes4
-                   ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, rays, out, nullptr, n, sms, s)
-                   : run_resident<false, BvhNode4>(bvh, bvh.nodes4, rays, out, nullptr, n, sms, s);
+    if (bvh.nodes4 && n >= resident_min(bvh) && n <= kResidentMax) {
+        const cudaError_t e = bvh.num_nodes4 >= kQuantMinNodes4
+                                  ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, rays, out, nullptr, n, sms, s)
+                                  : run_resident<false, BvhNode4>(bvh, bvh.nodes4, rays, out, nullptr, n, sms, s);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();                       // no room for its lists: the form below needs none
+    }
     if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
         k_trace_warp<false, Out><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, rays, out, nullptr, n);
         return cudaGetLastError();
@@ -372,10 +376,13 @@ cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_
     if (n == 0) return cudaSuccess;
     const int sms = sm_count();
     float4* r4 = (float4*)const_cast<void*>(rays);
-    if (bvh.nodes4 && n >= resident_min(bvh))
-        return bvh.num_nodes4 >= kQuantMinNodes4Any
-                   ? run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, r4, NoOut{}, occ, n, sms, s)
-                   : run_resident<true, BvhNode4>(bvh, bvh.nodes4, r4, NoOut{}, occ, n, sms, s);
+    if (bvh.nodes4 && n >= resident_min(bvh) && n <= kResidentMax) {
+        const cudaError_t e = bvh.num_nodes4 >= kQuantMinNodes4Any
+                                  ? run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, r4, NoOut{}, occ, n, sms, s)
+                                  : run_resident<true, BvhNode4>(bvh, bvh.nodes4, r4, NoOut{}, occ, n, sms, s);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();
+    }
     if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
         k_trace_warp<true, NoOut><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, r4, NoOut{}, occ, n);
         return cudaGetLastError();
