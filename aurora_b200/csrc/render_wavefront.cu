@@ -5,8 +5,8 @@
 // a pool of P path slots lives in HBM (structure of arrays) and every
 // iteration runs one bounce of every live path as separate stages:
 //
-//   regen   the slots that the shading stage listed: next-event radiance is added, finished
-//           slots write their sample and take the next work item (scene, pixel, sample)
+//   regen   the slots that the shading stage left work for: next-event radiance is added,
+//           finished slots write their sample and take the next work item (scene, pixel, sample)
 //           from a global counter -> camera ray
 //   extend  closest hit for the extension queue (persistent warps, traversal only)
 //   sort    optional: counting sort of the hits by material type
