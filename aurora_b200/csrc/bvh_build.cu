@@ -596,7 +596,7 @@ struct FinishMem {
 // list 115; now 105 (at 59% of the SM's issue slots).
 __global__ void __launch_bounds__(1024) k_ploc_finish(const int* __restrict__ clusters, BuildState* st, int parity, Tree t,
                                                       Sah sah, int r) {
-    extern __shared__ char s_mem[];
+    extern __shared__ __align__(16) char s_mem[];
     FinishMem& c = *reinterpret_cast<FinishMem*>(s_mem);
     __shared__ uint32_t s_scan[32];
     int m = st->m[parity];
