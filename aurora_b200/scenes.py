@@ -128,7 +128,7 @@ def value_noise_fbm(x, z, octaves, amplitude, seed, base_freq=0.5):
         fx, fz = (x * freq) % 256.0, (z * freq) % 256.0
         ix, iz = np.floor(fx).astype(np.int64), np.floor(fz).astype(np.int64)
         tx, tz = fx - ix, fz - iz
-        ix, iz = ix % 256, iz % 256          # just below 0 the remainder rounds to 256 itself
+        ix, iz = ix & 255, iz & 255          # just below 0 the remainder rounds to 256 itself
         sx, sz = tx * tx * (3 - 2 * tx), tz * tz * (3 - 2 * tz)
         a = lat[ix, iz] * (1 - sx) + lat[ix + 1, iz] * sx
         b = lat[ix, iz + 1] * (1 - sx) + lat[ix + 1, iz + 1] * sx

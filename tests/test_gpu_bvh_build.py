@@ -51,6 +51,16 @@ def test_sizes(ctx, oracle_lib, n, radius):
     _check(ctx, oracle_lib, *_soup(n, n), ab.bvh_opts(ploc_radius=radius))
 
 
+# binary trees just below and above 12,288 nodes: the 4-wide collapse in one block, and level by level
+@pytest.mark.parametrize("n,block", [(12300, True), (13000, False)])
+def test_collapse_forms(ctx, oracle_lib, n, block):
+    verts, idx = _soup(n, 11)
+    bvh = ab.Bvh(ctx, verts, idx, None, None)
+    assert (bvh.info()["num_nodes"] <= 12288) == block
+    bvh.close()
+    _check(ctx, oracle_lib, verts, idx)
+
+
 # the larger sort tile (4096 pairs) from 2^18 triangles on
 @pytest.mark.parametrize("n", [1 << 18, (1 << 18) + 1])
 def test_large_sort_tile(ctx, oracle_lib, n):
