@@ -517,6 +517,7 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
     const int ntex = (int)sc->ntexel_floats;
     DevIn din;
     DevOut gm, gt;
+    DevBuf counters, records;              // this call's own
     // the sums beside the outputs: compensation terms (megakernel) or the FP64 sums themselves
     const int nsum = 4 * nmat + ntex;
     const size_t sum_bytes = (wavefront ? sizeof(double) : sizeof(float)) * nsum;
@@ -528,7 +529,8 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
     if (e == cudaSuccess) e = cudaMemsetAsync(sums, 0, sum_bytes, s);
     if (e == cudaSuccess && !wavefront) e = cudaMemsetAsync(gm.ptr, 0, sizeof(float) * 4 * nmat, s);
     if (e == cudaSuccess && !wavefront && ntex) e = cudaMemsetAsync(gt.ptr, 0, sizeof(float) * ntex, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(sc->ctx->counters, 0, sizeof(unsigned long long) * 8, s);
+    if (e == cudaSuccess) e = counters.init(sizeof(unsigned long long) * 8, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(counters.ptr, 0, sizeof(unsigned long long) * 8, s);
     float* cm = (float*)sums;
     float* ct = cm ? cm + 4 * nmat : nullptr;
     double* dm = (double*)sums;
@@ -543,7 +545,6 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
     double replay_ms = 0.0;
     uint64_t launches = 0;
     unsigned long long rays[2] = {0, 0};
-    float4* rec = nullptr;
     if (wavefront) {
         // record passes (wavefront engine) + replay kernels over chunks of the samples, sized so that
         // the records stay within kRecBudget and their indices within 2^31; where the device has less
@@ -558,12 +559,13 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
         // as many passes as the budget needs, of equal size
         chunk = (p.spp + (p.spp + chunk - 1) / chunk - 1) / ((p.spp + chunk - 1) / chunk);
         while (e == cudaSuccess) {
-            e = ctx_scratch(sc->ctx, per_item * per_spp * chunk, (void**)&rec);
+            e = records.init(per_item * per_spp * chunk, s);
             if (e != cudaErrorMemoryAllocation || chunk == 1) break;
             cudaGetLastError();
             e = cudaSuccess;
             chunk = (chunk + 1) / 2;
         }
+        float4* rec = (float4*)records.ptr;
         float4* lo_raw = rec ? rec + per_spp * chunk * p.max_depth * stride : nullptr;
         // a column of shared sums per thread, or as many as fit 48 KB
         const int cols = std::min<int>(kAdjBlock, (int)(48 * 1024 / (sizeof(double) * 4 * nmat)));
@@ -600,7 +602,7 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
         auto kern = p.light_samples > 1 ? (dsc.sh.nenv ? k_adjoint<true, true> : k_adjoint<true, false>)
                                         : (dsc.sh.nenv ? k_adjoint<false, true> : k_adjoint<false, false>);
         kern<<<grid, kAdjBlock, 0, s>>>(dsc, p, (const float4*)din.ptr, nmat, (float*)gm.ptr, cm,
-                                        ntex ? (float*)gt.ptr : nullptr, ct, sc->ctx->counters);
+                                        ntex ? (float*)gt.ptr : nullptr, ct, (unsigned long long*)counters.ptr);
         ++launches;
         e = cudaGetLastError();
     }
@@ -624,7 +626,7 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
                                  (unsigned long long)npix * ((unsigned long long)p.spp * lpaths -
                                                              (p.sample_offset == 0 ? lpaths - 1 : 0))};
     if (e == cudaSuccess && !wavefront)
-        e = cudaMemcpyAsync(cnt, sc->ctx->counters, sizeof(cnt), cudaMemcpyDeviceToHost, s);
+        e = cudaMemcpyAsync(cnt, counters.ptr, sizeof(cnt), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     float ms = 0.f;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
@@ -645,6 +647,7 @@ extern "C" aur_status aur_render_adjoint(aur_scene* sc, const aur_render_opts* o
         if (wavefront) {   // stage_ms[0]: record passes (and the rest), stage_ms[1]: replay kernels
             stats->stage_ms[1] = replay_ms;
             stats->stage_ms[0] = ms - replay_ms;
+            std::lock_guard<std::mutex> lock(sc->ctx->wf_mutex);
             if (sc->wf_tuned) { stats->wf_pool = sc->wf_pool; stats->wf_block = sc->wf_block; stats->wf_sort = sc->wf_sort; }
         }
     }

@@ -3,7 +3,9 @@
 #include "aurora_b200.h"
 #include "aur_kernels.h"
 #include <array>
+#include <atomic>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -13,14 +15,13 @@ struct aur_ctx {
     bool own_stream = false;
     float* kelemen = nullptr;                  // 21 tables x 2048 floats
     bool kel_ready[aur::kAlbedoRefl] = {};
-    unsigned long long* counters = nullptr;    // 8 render counters
     cudaStream_t work_stream = nullptr;        // non-blocking stream for captured work (wavefront graphs)
     cudaEvent_t ev_order = nullptr;            // orders work_stream after `stream`
     std::map<uint64_t, std::array<int, 3>> wf_batch_tuned;   // autotuned batch configs (pool, block, sort)
     std::map<uint64_t, std::array<int, 3>> wf_scene_tuned;   // autotuned configs by scene signature
-    int live = 0;                              // BVHs and scenes created on this context and not destroyed
-    void* scratch = nullptr;                   // grow-only device scratch (adjoint hit records)
-    size_t scratch_bytes = 0;
+    std::atomic<int> live{0};                  // BVHs and scenes created on this context and not destroyed
+    std::mutex kelemen_mutex;                  // kelemen, kel_ready
+    std::mutex wf_mutex;                       // the wavefront engines, work_stream, ev_order and the tuned configurations
 };
 
 struct aur_bvh {
@@ -69,9 +70,6 @@ bool is_device_ptr(const void* p);
 // Checks on the device that v[0, n) < bound (device pointer v); synchronises the stream.
 cudaError_t indices_below(const uint32_t* v, size_t n, uint32_t bound, bool* ok, cudaStream_t s);
 cudaError_t ctx_kelemen_ensure(aur_ctx* ctx, int refl_index);
-// The context's scratch buffer of at least `bytes` (kept and reused by later calls;
-// freed with the context). Work on the context's stream must not still use it.
-cudaError_t ctx_scratch(aur_ctx* ctx, size_t bytes, void** out);
 int kelemen_index(float reflectance);
 aur_status bvh_options(const aur_bvh_opts* o, BvhBuildOptions* out);
 aur_status render_options(const aur_scene* sc, const aur_render_opts* o, PathParams* p);
@@ -101,6 +99,23 @@ struct DeviceGuard {
     explicit DeviceGuard(int dev);
     ~DeviceGuard();
     int prev_ = 0;
+};
+
+// Device memory of one call, from the stream's pool and given back to it in stream order: calls on one
+// context from several host threads interleave on its stream and must not share any.
+struct DevBuf {
+    void* ptr = nullptr;
+    cudaStream_t stream = nullptr;
+    cudaError_t init(size_t bytes, cudaStream_t s) {
+        stream = s;
+        const cudaError_t e = cudaMallocAsync(&ptr, bytes ? bytes : 1, s);
+        if (e != cudaSuccess) ptr = nullptr;
+        return e;
+    }
+    DevBuf() = default;
+    DevBuf(const DevBuf&) = delete;
+    DevBuf& operator=(const DevBuf&) = delete;
+    ~DevBuf() { if (ptr) cudaFreeAsync(ptr, stream); }
 };
 
 struct DevIn {

@@ -109,22 +109,8 @@ cudaError_t ctx_kelemen_tables(aur_ctx* ctx) {
     }
     return cudaSuccess;
 }
-cudaError_t ctx_scratch(aur_ctx* ctx, size_t bytes, void** out) {
-    if (bytes > ctx->scratch_bytes) {
-        cudaError_t e = cudaStreamSynchronize(ctx->stream);   // the old buffer may still be in use
-        if (e != cudaSuccess) return e;
-        if (ctx->scratch) cudaFree(ctx->scratch);
-        ctx->scratch = nullptr;
-        ctx->scratch_bytes = 0;
-        e = cudaMalloc(&ctx->scratch, bytes);
-        if (e != cudaSuccess) return e;
-        ctx->scratch_bytes = bytes;
-    }
-    *out = ctx->scratch;
-    return cudaSuccess;
-}
-
 cudaError_t ctx_kelemen_ensure(aur_ctx* ctx, int refl_index) {
+    std::lock_guard<std::mutex> lock(ctx->kelemen_mutex);
     cudaError_t e = ctx_kelemen_tables(ctx);
     if (e != cudaSuccess) return e;
     if (ctx->kel_ready[refl_index]) return cudaSuccess;
@@ -172,8 +158,7 @@ aur_status aur_ctx_create(int device, aur_ctx** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete c; return cuda_fail(e, "aur_ctx_create"); }
     c->own_stream = true;
-    e = cudaMalloc(&c->counters, sizeof(unsigned long long) * 8);
-    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->work_stream, cudaStreamNonBlocking);
+    e = cudaStreamCreateWithFlags(&c->work_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         // Scene and BVH buffers come from the device's stream-ordered pool; keeping freed
         // blocks reserved (instead of trimming at every synchronisation) makes a new scene's
@@ -187,7 +172,6 @@ aur_status aur_ctx_create(int device, aur_ctx** out) {
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_order, cudaEventDisableTiming);
     if (e != cudaSuccess) {
-        if (c->counters) cudaFree(c->counters);
         if (c->work_stream) cudaStreamDestroy(c->work_stream);
         cudaStreamDestroy(c->stream);
         delete c;
@@ -206,8 +190,6 @@ aur_status aur_ctx_destroy(aur_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     wf_release_context(ctx);
     if (ctx->kelemen) cudaFree(ctx->kelemen);
-    if (ctx->scratch) cudaFree(ctx->scratch);
-    if (ctx->counters) cudaFree(ctx->counters);
     if (ctx->work_stream) { cudaStreamSynchronize(ctx->work_stream); cudaStreamDestroy(ctx->work_stream); }
     if (ctx->ev_order) cudaEventDestroy(ctx->ev_order);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);

@@ -1415,6 +1415,7 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
 aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsamples, float4* rec, int stride,
                           float4* lo_raw, uint64_t* launches, unsigned long long* rays) {
     aur_ctx* ctx = sc->ctx;
+    std::lock_guard<std::mutex> lock(ctx->wf_mutex);
     WfConfig cfg;
     if (sc->wf_tuned) { cfg.pool = (uint32_t)sc->wf_pool; cfg.block = sc->wf_block; cfg.sort = sc->wf_sort; }
     cfg.record = 1;
@@ -1476,6 +1477,7 @@ aur_status render_wavefront(aur_scene* sc, const aur_render_opts* o, float* film
     WfConfig cfg = config_from(o, WfConfig());
     if ((st = check_config(cfg)) != AUR_OK) return st;
     DeviceGuard g(sc->ctx->device);
+    std::lock_guard<std::mutex> lock(sc->ctx->wf_mutex);
     cudaStream_t s = sc->ctx->stream;
     const uint32_t npix = (uint32_t)sc->cam.w * sc->cam.h;
     if ((uint64_t)npix * o->spp * (uint64_t)p.light_samples >= (1ull << 31))
@@ -1529,6 +1531,7 @@ extern "C" aur_status aur_render_batch(aur_scene* const* scenes, const aur_rende
     aur_status st = check_config(cfg);
     if (st != AUR_OK) return st;
     DeviceGuard g(ctx->device);
+    std::lock_guard<std::mutex> lock(ctx->wf_mutex);
     cudaStream_t s = ctx->stream;
     std::vector<BatchItem> items(n);
     std::vector<DevOut> outs(n);

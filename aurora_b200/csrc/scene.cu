@@ -403,7 +403,7 @@ aur_status render_options(const aur_scene* sc, const aur_render_opts* o, PathPar
 
 }  // namespace aur
 
-// Samples that the plain renderer keeps before it sums them (ctx_scratch).
+// Bytes of samples that the plain renderer keeps before it sums them.
 constexpr size_t kPlainSampleBudget = (size_t)1 << 30;
 
 static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, void* film, bool f64,
@@ -422,20 +422,25 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
     // loop counts work, and renders what is left
     const DeviceBvh& tree = sc->bvh.bvh;
     const bool quant = tree.num_nodes4 >= kQuantMinNodes4;
-    void* scratch = nullptr;
+    // counters (the paths' work cursor among them) and samples are this call's own
+    DevBuf counters, samples;
+    constexpr size_t kCounterBytes = sizeof(unsigned long long) * 8;
+    CUDA_TRY(counters.init(kCounterBytes, s), "aur_render");
+    unsigned long long* const ctr = (unsigned long long*)counters.ptr;
     int chunk = 0;
     if (!o->count_work && tree.nodes4) {
         size_t budget = kPlainSampleBudget;
         cudaError_t e = cudaErrorMemoryAllocation;
         while (e == cudaErrorMemoryAllocation) {
-            e = ctx_scratch(sc->ctx, paths_scratch_bytes(sc->dev(), p, budget, &chunk), &scratch);
+            e = samples.init(paths_scratch_bytes(sc->dev(), p, budget, &chunk), s);
             if (e != cudaErrorMemoryAllocation || chunk == 1) break;
             cudaGetLastError();
             budget = (size_t)(chunk / 2) * npix * sizeof(float4);
         }
-        if (e == cudaErrorMemoryAllocation) { cudaGetLastError(); scratch = nullptr; }
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
         else if (e != cudaSuccess) return cuda_fail(e, "aur_render(samples)");
     }
+    void* const scratch = samples.ptr;
     const bool fp64_acc = f64 || o->fp64_film != 0;
     if (f64) {
         CUDA_TRY(fo64.init(film, sizeof(double) * 4 * npix, 8, s), "aur_render(film)");
@@ -446,7 +451,7 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
         f32 = (float4*)fo.ptr;
         if (fp64_acc && !scratch) CUDA_TRY(cudaMallocAsync(&d64, sizeof(double) * 4 * npix, s), "aur_render(film)");
     }
-    CUDA_TRY(cudaMemsetAsync(sc->ctx->counters, 0, sizeof(unsigned long long) * 8, s), "aur_render");
+    CUDA_TRY(cudaMemsetAsync(ctr, 0, kCounterBytes, s), "aur_render");
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -456,15 +461,15 @@ static aur_status render_plain_impl(aur_scene* sc, const aur_render_opts* o, voi
     uint64_t launches = 0;
     cudaError_t e;
     if (scratch) {
-        e = launch_render_paths(sc->dev(), p, quant, fp64_acc, chunk, scratch, f32, d64, sc->ctx->counters, &launches, s);
+        e = launch_render_paths(sc->dev(), p, quant, fp64_acc, chunk, scratch, f32, d64, ctr, &launches, s);
     } else {
-        e = launch_render_plain(sc->dev(), p, f32, d64, sc->ctx->counters, count_width, s);
+        e = launch_render_plain(sc->dev(), p, f32, d64, ctr, count_width, s);
         launches = 1;
     }
     cudaEventRecord(e1, s);
     if (e == cudaSuccess) e = f64 ? fo64.finish() : fo.finish();
     unsigned long long cnt[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, sc->ctx->counters, sizeof(cnt), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, ctr, sizeof(cnt), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     float ms = 0.f;
     if (e == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);

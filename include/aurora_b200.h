@@ -7,6 +7,13 @@
  * Functions never abort: they return an aur_status and keep a thread-local
  * message readable with aur_last_error().
  *
+ * Several host threads may make calls on one context at the same time, on the
+ * same scenes and BVHs too while no call changes or destroys those
+ * (aur_scene_set_params, aur_bvh_set_shading, the destroy calls). Wavefront
+ * renders, batches and record passes of one context take turns.
+ * aur_ctx_set_stream and aur_ctx_destroy want the context for themselves, and
+ * aur_render_fp64acc_noalloc has a rule of its own.
+ *
  * Each entry point names the reference interface it replaces
  * (paths inside espennordahl/Aurora).
  */
