@@ -57,6 +57,7 @@ aur_status fail(aur_status s, const std::string& msg) {
 }
 aur_status cuda_fail(cudaError_t e, const char* where) {
     g_err = std::string(where) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
+    cudaGetLastError();   // reported here: not again by the next call's check of its launches
     return e == cudaErrorMemoryAllocation ? AUR_ERR_OOM : AUR_ERR_CUDA;
 }
 
