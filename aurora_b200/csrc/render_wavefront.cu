@@ -881,11 +881,14 @@ __global__ void k_resolve(const WfScene* scenes) {
 
 }  // namespace
 
+constexpr uint32_t kMinPool = 1u << 16;   // no pool smaller than this in the place of one that does not fit
+
 struct WfConfig {
     uint32_t pool = 1u << 21;
     int block = 128;
     int sort = 1;
     int record = 0;   // record mode: vertex records + unclamped radiance per item instead of samples
+    bool fixed_pool = false;   // the caller's size: no smaller pool in its place where it does not fit
     // the trees traversed by closest-hit and any-hit rays (TREE_*; the 4-wide ones only when every
     // scene has them), chosen by tree_for
     int tree = TREE_BINARY, tree_any = TREE_BINARY;
@@ -921,7 +924,8 @@ struct WfRun {
     float4* acc = nullptr;                     // per-pixel compensated sums, grown on demand
     size_t acc_bytes = 0;
     cudaStream_t stream = nullptr;
-    int grid_regen = 0, grid_ext = 0, grid_shade = 0, grid_shade_m = 0, grid_shade_r = 0, grid_shadow = 0, grid_sort = 0;
+    int grid_regen = 0, grid_shade = 0, grid_shade_m = 0, grid_shade_r = 0, grid_sort = 0;
+    int grid_ext[3] = {}, grid_shadow[3] = {};   // by tree
     size_t stack_smem = 0;                     // shared traversal stack of one block
     WfState* h_state = nullptr;                // pinned: [0] as read back, [1] as uploaded
     WfScene* h_scenes = nullptr;               // pinned scene table
@@ -931,7 +935,8 @@ struct WfRun {
     // by iterations and kind of pass: one that refills its slots, one that fits the pool, and one of
     // at most kSmallPass paths, whose launches need few blocks
     enum Kind : int { REFILL = 0, FITS = 1, SMALL = 2 };
-    cudaGraphExec_t exec[kItersPerGraph + 1][3] = {};
+    // and by the trees traversed: scenes on either side of their limits share an engine and its pool
+    cudaGraphExec_t exec[kItersPerGraph + 1][3][3][3] = {};
     static constexpr uint32_t kSmallPass = 1u << 18;
 
     int launches_per_iteration() const { return cfg.sort ? 6 : 4; }
@@ -977,11 +982,15 @@ struct WfRun {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, c.block, smem);
             return std::max(1, nb) * sms;
         };
-        grid_ext = persist((const void*)extend_kernel(c), stack_smem);
+        for (int t = TREE_BINARY; t <= TREE_QUANT; ++t) {
+            WfConfig ct = c;
+            ct.tree = ct.tree_any = t;
+            grid_ext[t] = persist((const void*)extend_kernel(ct), stack_smem);
+            grid_shadow[t] = persist((const void*)shadow_kernel(ct), stack_smem);
+        }
         grid_shade = persist(c.record ? (const void*)k_shade<true, SHADE_ALL> : (const void*)k_shade<false, SHADE_ALL>, 0);
         grid_shade_m = persist(c.record ? (const void*)k_shade<true, SHADE_MATTE> : (const void*)k_shade<false, SHADE_MATTE>, 0);
         grid_shade_r = persist(c.record ? (const void*)k_shade<true, SHADE_REST> : (const void*)k_shade<false, SHADE_REST>, 0);
-        grid_shadow = persist((const void*)shadow_kernel(c), stack_smem);
         grid_sort = persist((const void*)k_sort_scatter, 0);
         grid_regen = (int)std::min<size_t>((P + c.block - 1) / c.block, (size_t)sms * 64);
         return cudaSuccess;
@@ -1000,7 +1009,7 @@ struct WfRun {
         const int cap = kind == SMALL ? (int)(kSmallPass / cfg.block) : INT_MAX;
         const bool sweep = kind == REFILL;
         regen(in_q, kind);
-        extend_kernel(cfg)<<<std::min(grid_ext, cap), cfg.block, stack_smem, stream>>>(w, in_q);
+        extend_kernel(cfg)<<<std::min(grid_ext[cfg.tree], cap), cfg.block, stack_smem, stream>>>(w, in_q);
         if (cfg.sort) {   // the matte bucket, then the others
             k_sort_scatter<<<std::min(grid_sort, cap), cfg.block, 0, stream>>>(w, in_q);
             auto matte = cfg.record ? k_shade<true, SHADE_MATTE> : k_shade<false, SHADE_MATTE>;
@@ -1011,11 +1020,11 @@ struct WfRun {
             auto all = cfg.record ? k_shade<true, SHADE_ALL> : k_shade<false, SHADE_ALL>;
             all<<<std::min(grid_shade, cap), cfg.block, 0, stream>>>(w, in_q, 0, sweep);
         }
-        shadow_kernel(cfg)<<<std::min(grid_shadow, cap), cfg.block, stack_smem, stream>>>(w);
+        shadow_kernel(cfg)<<<std::min(grid_shadow[cfg.tree_any], cap), cfg.block, stack_smem, stream>>>(w);
     }
 
     cudaError_t launch_graph(int iters, Kind kind) {
-        cudaGraphExec_t& x = exec[iters][kind];
+        cudaGraphExec_t& x = exec[iters][kind][cfg.tree][cfg.tree_any];
         if (!x) {
             cudaGraph_t g;
             cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
@@ -1116,8 +1125,10 @@ struct WfRun {
         if (acc) cudaFree(acc);
         acc = nullptr;
         acc_bytes = 0;
-        for (auto& row : exec)
-            for (auto& x : row) { if (x) cudaGraphExecDestroy(x); x = nullptr; }
+        for (cudaGraphExec_t* x = &exec[0][0][0][0]; x != &exec[0][0][0][0] + sizeof(exec) / sizeof(*x); ++x) {
+            if (*x) cudaGraphExecDestroy(*x);
+            *x = nullptr;
+        }
         if (mem) cudaFree(mem);
         if (d_scenes) cudaFree(d_scenes);
         if (samples) cudaFree(samples);
@@ -1192,6 +1203,73 @@ static uint32_t fill_table(std::vector<BatchItem>& items, int s0, int chunk, flo
     return base;
 }
 
+// Engines (pool buffers, captured graphs, events, sample buffer) are cached per (context,
+// configuration) and reused by later calls; aur_ctx_destroy releases them, and so does a call
+// that finds no memory for its own. A context's engines are used by one call at a time (wf_mutex).
+static std::mutex g_engine_mutex;
+using EngineKey = std::tuple<aur_ctx*, uint32_t, int, int, int>;
+static std::map<EngineKey, std::unique_ptr<WfRun>> g_engines;
+static EngineKey engine_key(aur_ctx* ctx, const WfConfig& c) { return EngineKey(ctx, c.pool, c.block, c.sort, c.record); }
+
+// Gives back what the context holds for later calls: its engines but `keep`, and the free blocks of the
+// device's stream-ordered pool.
+static void wf_reclaim(aur_ctx* ctx, const WfRun* keep) {
+    {
+        std::lock_guard<std::mutex> lock(g_engine_mutex);
+        for (auto it = g_engines.begin(); it != g_engines.end();) {
+            if (std::get<0>(it->first) == ctx && it->second.get() != keep) { it->second->release(); it = g_engines.erase(it); }
+            else ++it;
+        }
+    }
+    cudaStreamSynchronize(ctx->stream);
+    cudaStreamSynchronize(ctx->work_stream);
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
+    cudaGetLastError();
+}
+
+static WfRun* engine_for(aur_ctx* ctx, const WfConfig& cfg, int nscenes, cudaError_t* err) {
+    const EngineKey key = engine_key(ctx, cfg);
+    {
+        std::lock_guard<std::mutex> lock(g_engine_mutex);
+        auto it = g_engines.find(key);
+        if (it != g_engines.end() && it->second->cap_scenes >= nscenes) {
+            it->second->cfg = cfg;                    // its trees are this call's
+            return it->second.get();
+        }
+        if (it != g_engines.end()) { it->second->release(); g_engines.erase(it); }
+    }
+    std::unique_ptr<WfRun> r(new WfRun());
+    *err = r->init(cfg, nscenes, ctx->work_stream);
+    if (*err == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        r->release();
+        wf_reclaim(ctx, nullptr);
+        *err = r->init(cfg, nscenes, ctx->work_stream);
+    }
+    if (*err != cudaSuccess) { r->release(); return nullptr; }
+    std::lock_guard<std::mutex> lock(g_engine_mutex);
+    return (g_engines[key] = std::move(r)).get();
+}
+
+// The engine of a configuration, or where its pool does not fit the device and the caller did not ask for
+// it, of the largest halving that does (cfg->pool; the films are the same).
+static WfRun* engine_that_fits(aur_ctx* ctx, WfConfig* cfg, int nscenes, cudaError_t* err) {
+    WfRun* r = engine_for(ctx, *cfg, nscenes, err);
+    while (!r && *err == cudaErrorMemoryAllocation && !cfg->fixed_pool && cfg->pool > kMinPool) {
+        cudaGetLastError();
+        cfg->pool /= 2;
+        r = engine_for(ctx, *cfg, nscenes, err);
+    }
+    return r;
+}
+
+static void wf_drop_engine(aur_ctx* ctx, const WfConfig& cfg) {
+    std::lock_guard<std::mutex> lock(g_engine_mutex);
+    auto it = g_engines.find(engine_key(ctx, cfg));
+    if (it != g_engines.end()) { it->second->release(); g_engines.erase(it); }
+}
+
 // Autotuner: times candidates (pool size, material sort, block size) on the same probe, the first
 // `limit` work items of the real workload (at most 2^25), and keeps the fastest: first the pool
 // sizes with the sort on and blocks of 256, then the best pool without the sort, then the better of
@@ -1221,6 +1299,11 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
     }
     float4* samples = nullptr;
     cudaError_t e = cudaMallocAsync(&samples, per_sample * chunk, s);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        wf_reclaim(ctx, nullptr);
+        e = cudaMallocAsync(&samples, per_sample * chunk, s);
+    }
     if (e != cudaSuccess) return cuda_fail(e, "wavefront autotune");
     std::vector<WfScene> tab(items.size());
     limit = std::min(limit, fill_table(items, 0, chunk, samples, tab.data()));
@@ -1276,31 +1359,6 @@ static aur_status autotune(aur_ctx* ctx, std::vector<BatchItem>& items, WfConfig
     return AUR_OK;
 }
 
-// Engines (pool buffers, captured graph, events, sample buffer) are cached per
-// (context, configuration) and reused by later calls; aur_ctx_destroy releases them.
-static std::mutex g_engine_mutex;
-static std::map<std::tuple<aur_ctx*, uint32_t, int, int, int, int, int>, std::unique_ptr<WfRun>> g_engines;
-
-static WfRun* engine_for(aur_ctx* ctx, const WfConfig& cfg, int nscenes, cudaError_t* err) {
-    std::lock_guard<std::mutex> lock(g_engine_mutex);
-    const auto key = std::make_tuple(ctx, cfg.pool, cfg.block, cfg.sort, cfg.record, cfg.tree, cfg.tree_any);
-    auto it = g_engines.find(key);
-    if (it != g_engines.end() && it->second->cap_scenes >= nscenes) return it->second.get();
-    if (it != g_engines.end()) { it->second->release(); g_engines.erase(it); }
-    std::unique_ptr<WfRun> r(new WfRun());
-    *err = r->init(cfg, nscenes, ctx->work_stream);
-    if (*err != cudaSuccess) { r->release(); return nullptr; }
-    WfRun* raw = r.get();
-    g_engines.emplace(key, std::move(r));
-    return raw;
-}
-
-static void wf_drop_engine(aur_ctx* ctx, const WfConfig& cfg) {
-    std::lock_guard<std::mutex> lock(g_engine_mutex);
-    auto it = g_engines.find(std::make_tuple(ctx, cfg.pool, cfg.block, cfg.sort, cfg.record, cfg.tree, cfg.tree_any));
-    if (it != g_engines.end()) { it->second->release(); g_engines.erase(it); }
-}
-
 void wf_release_context(aur_ctx* ctx) {
     std::lock_guard<std::mutex> lock(g_engine_mutex);
     for (auto it = g_engines.begin(); it != g_engines.end();) {
@@ -1332,7 +1390,7 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
     cudaEventRecord(ctx->ev_order, ctx->stream);
     cudaStreamWaitEvent(s, ctx->ev_order, 0);
     cudaError_t e = cudaSuccess;
-    WfRun* engine = engine_for(ctx, cfg, n, &e);
+    WfRun* engine = engine_that_fits(ctx, &cfg, n, &e);
     if (!engine) return cuda_fail(e, "wavefront: pool allocation");
     WfRun& run = *engine;
     // sample-buffer budget: passes over the spp range when all samples do not fit
@@ -1347,6 +1405,11 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
     }
     const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)max_spp, budget / std::max<size_t>(per_sample, 1)));
     e = run.ensure_samples(per_sample * chunk);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        wf_reclaim(ctx, &run);
+        e = run.ensure_samples(per_sample * chunk);
+    }
     if (chunk < max_spp) {   // several passes: two float4 sums per pixel between them
         size_t pixels = 0;
         for (auto& it : items) pixels += it.npix;
@@ -1426,7 +1489,7 @@ aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsampl
     cudaEventRecord(ctx->ev_order, ctx->stream);
     cudaStreamWaitEvent(s, ctx->ev_order, 0);
     cudaError_t e = cudaSuccess;
-    WfRun* engine = engine_for(ctx, cfg, 1, &e);
+    WfRun* engine = engine_that_fits(ctx, &cfg, 1, &e);
     if (!engine) return cuda_fail(e, "adjoint record pass: pool allocation");
     WfRun& run = *engine;
     const uint32_t total = fill_table(items, s0, nsamples, nullptr, run.h_scenes);
@@ -1454,7 +1517,7 @@ static bool wants_tuning(const aur_render_opts* o) { return o->wf_pool == 0 && o
 
 static WfConfig config_from(const aur_render_opts* o, const WfConfig& base) {
     WfConfig c = base;
-    if (o->wf_pool > 0) c.pool = (uint32_t)o->wf_pool;
+    if (o->wf_pool > 0) { c.pool = (uint32_t)o->wf_pool; c.fixed_pool = true; }
     if (o->wf_block > 0) c.block = o->wf_block;
     if (o->wf_sort >= 0) c.sort = o->wf_sort;
     return c;
