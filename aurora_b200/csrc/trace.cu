@@ -12,13 +12,13 @@
 // with fewer rays each where there are few.
 #include "aurora_b200.h"
 #include "aur_kernels.h"
+#include "aur_trace_split.h"
 #include "aur_traverse.cuh"
 #include <algorithm>
 
 namespace aur {
 namespace {
 
-constexpr int kTraceBlock = 128;
 constexpr int kTraceRefill = 12;     // idle lanes of a warp that fetch new rays together
 constexpr uint32_t kResidentMax = 1u << 31;   // its 32-bit cursor runs past the last ray by what is fetched at once
 constexpr int kTraceRounds = 4;      // rounds between fetches (both as in the wavefront's kernels)
@@ -87,18 +87,12 @@ struct NoOut {
     __device__ __forceinline__ void put(uint32_t, const Hit&, bool, const float4*) const {}
 };
 
-// The ray of this thread when every warp takes `per_warp` of them; n or more: none.
-__device__ __forceinline__ uint32_t spread_index(int per_warp) {
-    const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    return lane < (uint32_t)per_warp ? warp * per_warp + lane : 0xffffffffu;
-}
-
 template <class Out>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_closest(const BvhNode* __restrict__ nodes,
                                                                const BvhNode4* __restrict__ nodes4,
                                                                const BvhTri* __restrict__ tris, float4* rays, Out out,
                                                                uint32_t n, int per_warp) {
-    const uint32_t i = spread_index(per_warp);
+    const uint32_t i = spread_index(blockIdx.x, threadIdx.x, per_warp);
     if (i >= n) return;
     const float4 a = rays[2 * (size_t)i];
     const float4 b = rays[2 * (size_t)i + 1];
@@ -113,7 +107,7 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_occluded(const BvhNode* _
                                                                 const BvhTri* __restrict__ tris,
                                                                 const float4* __restrict__ rays, uint8_t* occ,
                                                                 uint32_t n, int per_warp) {
-    const uint32_t i = spread_index(per_warp);
+    const uint32_t i = spread_index(blockIdx.x, threadIdx.x, per_warp);
     if (i >= n) return;
     const float4 a = rays[2 * (size_t)i];
     const float4 b = rays[2 * (size_t)i + 1];
@@ -296,20 +290,6 @@ int sm_count() {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return sms;
-}
-
-// Rays per warp of a small batch: the fewest (a power of two) that need at most kSpreadWarps warps per
-// SM; 32 once the batch is large.
-constexpr int kSpreadWarps = 16;
-int rays_per_warp(uint32_t n, int sms) {
-    int r = 1;
-    while (r < 32 && (n + r - 1) / r > (uint32_t)(kSpreadWarps * sms)) r *= 2;
-    return r;
-}
-
-unsigned spread_grid(uint32_t n, int per_warp) {
-    const uint64_t warps = ((uint64_t)n + per_warp - 1) / per_warp;
-    return (unsigned)((warps * 32 + kTraceBlock - 1) / kTraceBlock);
 }
 
 // Up to this many rays per SM each has a warp of its own (14,208 on 148 SMs). A warp per ray against
