@@ -88,9 +88,11 @@ extern "C" aur_status aur_bvh_intersect(aur_bvh* b, aur_ray* rays, aur_isect* is
     if (dr.owned)
         CUDA_TRY(cudaMemcpyAsync(dr.ptr, rays, sizeof(aur_ray) * n, cudaMemcpyDefault, s), "aur_bvh_intersect(rays)");
     CUDA_TRY(dh.init(isects, sizeof(aur_isect) * n, 16, s), "aur_bvh_intersect(isects)");
-    CUDA_TRY(launch_intersect(b->bvh, b->tri, dr.ptr, dh.ptr, n, s), "aur_bvh_intersect");
+    TraceSlot slot(b->ctx);
+    CUDA_TRY(launch_intersect(b->bvh, b->tri, dr.ptr, dh.ptr, n, slot.ptr, s), "aur_bvh_intersect");
     CUDA_TRY(dr.finish(), "aur_bvh_intersect(download)");
     CUDA_TRY(dh.finish(), "aur_bvh_intersect(download)");
     CUDA_TRY(cudaStreamSynchronize(s), "aur_bvh_intersect");
+    slot.done();
     return AUR_OK;
 }

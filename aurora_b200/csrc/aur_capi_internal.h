@@ -19,6 +19,8 @@ struct aur_ctx {
     cudaEvent_t ev_order = nullptr;            // orders work_stream after `stream`
     std::map<uint64_t, std::array<int, 3>> wf_batch_tuned;   // autotuned batch configs (pool, block, sort)
     std::map<uint64_t, std::array<int, 3>> wf_scene_tuned;   // autotuned configs by scene signature
+    uint32_t* trace_cursors = nullptr;         // kTraceSlots of kCursorWords, for launch_trace_*
+    std::atomic<uint64_t> trace_slots{0};      // slots in use, by bit
     std::atomic<int> live{0};                  // BVHs and scenes created on this context and not destroyed
     std::mutex kelemen_mutex;                  // kelemen, kel_ready
     std::mutex wf_mutex;                       // the wavefront engines, work_stream, ev_order and the tuned configurations
@@ -116,6 +118,27 @@ struct DevBuf {
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { if (ptr) cudaFreeAsync(ptr, stream); }
+};
+
+// A ray query's place among the context's cursors (ptr null: all are taken). done() gives it back, once the
+// query's work is finished and has left it zero; a query that failed keeps it.
+constexpr int kTraceSlots = 64;
+struct TraceSlot {
+    aur_ctx* ctx;
+    int slot = -1;
+    uint32_t* ptr = nullptr;
+    explicit TraceSlot(aur_ctx* c) : ctx(c) {
+        uint64_t used = c->trace_slots.load();
+        while (~used) {
+            const int k = __builtin_ctzll(~used);
+            if (c->trace_slots.compare_exchange_weak(used, used | 1ull << k)) {
+                slot = k;
+                ptr = c->trace_cursors + aur::kCursorWords * k;
+                return;
+            }
+        }
+    }
+    void done() { if (slot >= 0) ctx->trace_slots.fetch_and(~(1ull << slot)); }
 };
 
 struct DevIn {

@@ -7,12 +7,16 @@
 
 namespace aur {
 
-// trace.cu — batched ray queries (aur_ray / aur_hit layouts of aurora_b200.h)
+// trace.cu — batched ray queries (aur_ray / aur_hit layouts of aurora_b200.h). cursor: kCursorWords words of device memory that
+// are zero, that the call has to itself until its work is done, and that are zero again then (TraceSlot); without
+// them the forms that need none are used.
+constexpr int kCursorWords = 2;
 cudaError_t launch_trace_closest(const DeviceBvh& bvh, const int* tri_attr, const void* rays, void* hits, uint32_t n,
-                                 cudaStream_t s);
+                                 uint32_t* cursor, cudaStream_t s);
 // the whole record of EmbreeAccelerator::intersect (aur_isect); shrinks rays[i].maxt on a hit
-cudaError_t launch_intersect(const DeviceBvh& bvh, const TriShade* tri, void* rays, void* isects, uint32_t n, cudaStream_t s);
-cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, cudaStream_t s);
+cudaError_t launch_intersect(const DeviceBvh& bvh, const TriShade* tri, void* rays, void* isects, uint32_t n, uint32_t* cursor,
+                             cudaStream_t s);
+cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, uint32_t* cursor, cudaStream_t s);
 
 // kelemen.cu — directional-albedo table for reflectance index 0..20 into out[2048]
 cudaError_t launch_kelemen_table(int refl_index, float* out, cudaStream_t s);

@@ -159,7 +159,10 @@ aur_status aur_ctx_create(int device, aur_ctx** out) {
     cudaError_t e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { delete c; return cuda_fail(e, "aur_ctx_create"); }
     c->own_stream = true;
-    e = cudaStreamCreateWithFlags(&c->work_stream, cudaStreamNonBlocking);
+    e = cudaMalloc(&c->trace_cursors, sizeof(uint32_t) * kCursorWords * kTraceSlots);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->trace_cursors, 0, sizeof(uint32_t) * kCursorWords * kTraceSlots, c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->work_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
         // Scene and BVH buffers come from the device's stream-ordered pool; keeping freed
         // blocks reserved (instead of trimming at every synchronisation) makes a new scene's
@@ -173,6 +176,7 @@ aur_status aur_ctx_create(int device, aur_ctx** out) {
     }
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_order, cudaEventDisableTiming);
     if (e != cudaSuccess) {
+        if (c->trace_cursors) cudaFree(c->trace_cursors);
         if (c->work_stream) cudaStreamDestroy(c->work_stream);
         cudaStreamDestroy(c->stream);
         delete c;
@@ -191,6 +195,7 @@ aur_status aur_ctx_destroy(aur_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     wf_release_context(ctx);
     if (ctx->kelemen) cudaFree(ctx->kelemen);
+    if (ctx->trace_cursors) cudaFree(ctx->trace_cursors);
     if (ctx->work_stream) { cudaStreamSynchronize(ctx->work_stream); cudaStreamDestroy(ctx->work_stream); }
     if (ctx->ev_order) cudaEventDestroy(ctx->ev_order);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
@@ -311,9 +316,11 @@ aur_status aur_trace_closest(aur_bvh* b, const aur_ray* rays, aur_hit* hits, uin
     DevOut dh;
     CUDA_TRY(dr.init(rays, sizeof(aur_ray) * n, 16, s), "aur_trace_closest(rays)");
     CUDA_TRY(dh.init(hits, sizeof(aur_hit) * n, 4, s), "aur_trace_closest(hits)");
-    CUDA_TRY(launch_trace_closest(b->bvh, b->tri_attr, dr.ptr, dh.ptr, n, s), "aur_trace_closest");
+    TraceSlot slot(b->ctx);
+    CUDA_TRY(launch_trace_closest(b->bvh, b->tri_attr, dr.ptr, dh.ptr, n, slot.ptr, s), "aur_trace_closest");
     CUDA_TRY(dh.finish(), "aur_trace_closest(download)");
     CUDA_TRY(cudaStreamSynchronize(s), "aur_trace_closest");
+    slot.done();
     return AUR_OK;
 }
 
@@ -326,9 +333,11 @@ aur_status aur_trace_occluded(aur_bvh* b, const aur_ray* rays, uint8_t* occluded
     DevOut dh;
     CUDA_TRY(dr.init(rays, sizeof(aur_ray) * n, 16, s), "aur_trace_occluded(rays)");
     CUDA_TRY(dh.init(occluded, n, 1, s), "aur_trace_occluded(out)");
-    CUDA_TRY(launch_trace_occluded(b->bvh, dr.ptr, (uint8_t*)dh.ptr, n, s), "aur_trace_occluded");
+    TraceSlot slot(b->ctx);
+    CUDA_TRY(launch_trace_occluded(b->bvh, dr.ptr, (uint8_t*)dh.ptr, n, slot.ptr, s), "aur_trace_occluded");
     CUDA_TRY(dh.finish(), "aur_trace_occluded(download)");
     CUDA_TRY(cudaStreamSynchronize(s), "aur_trace_occluded");
+    slot.done();
     return AUR_OK;
 }
 

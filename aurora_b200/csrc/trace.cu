@@ -3,12 +3,12 @@
 // they replace EmbreeAccelerator::intersect / intersectBinary
 // (Aurora/src/geometry/embreeAccelerator.cpp:41-100) for arrays of rays.
 //
-// Three forms by the number of rays. Large batches run a resident grid whose lanes take the next ray
-// as soon as theirs is finished, over the tree form the wavefront renderer uses (full-precision
-// or quantised 4-wide nodes): 2^20 incoherent rays on 20,482 triangles 181 -> 144 us, 1,500,001
-// next-event rays on a 0.85 M triangle landscape 661 -> 411 us. Small ones cannot fill the chip and
+// Three forms by the number of rays and the tree. Large batches run a resident grid whose lanes take the next
+// ray as soon as theirs is finished, over the tree form the wavefront renderer uses (full-precision
+// or quantised 4-wide nodes): 2^20 incoherent rays on 20,482 triangles 309 -> 254 us, 2^20 surface points
+// towards a light on a 0.85 M triangle landscape 555 -> 336. Small ones cannot fill the chip and
 // take as long as their longest ray's walk: a warp per ray walks it side by side, 1,000 rays
-// 41 -> 24 us, of which 15 are the call's. In between, a thread per ray, spread over more warps
+// 41 -> 22 us, of which 15 are the call's. In between, a thread per ray, spread over more warps
 // with fewer rays each where there are few.
 #include "aurora_b200.h"
 #include "aur_kernels.h"
@@ -27,6 +27,7 @@ constexpr int kTraceRounds = 4;      // rounds between fetches (both as in the w
 struct HitOut {
     aur_hit* hits;
     const int* tri_attr;
+    __device__ __forceinline__ int& link(uint32_t i) const { return hits[i].prim; }   // a word of a record not yet written
     __device__ __forceinline__ void put(uint32_t i, const Hit& h, bool hit, const float4* rays) const {
         aur_hit* out = hits + i;
         out->t = hit ? h.t : rays[2 * (size_t)i + 1].w;
@@ -49,6 +50,7 @@ struct HitOut {
 struct IsectOut {
     aur_isect* out;
     const TriShade* tri;
+    __device__ __forceinline__ int& link(uint32_t i) const { return out[i].prim; }
     __device__ __forceinline__ void put(uint32_t i, const Hit& h, bool hit, float4* rays) const {
         const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
         aur_isect r;
@@ -218,13 +220,18 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_warp(const BvhNode4* __re
     }
 }
 
-// The resident form. Warps fetch ranges of rays from *cursor. Closest hits that meet two triangles at
-// exactly the same distance are left to k_trace_ties: their indices are appended to `ties`.
+// The resident form. Warps fetch ranges of rays from cursor[0]; the last block to leave clears the
+// cursor (cursor[1] counts them), so that it is zero for its next user.
+// Closest hits of the quantised tree that meet two triangles at exactly the same distance are traced again over the
+// full-precision nodes: the thread keeps them in a list through their records (Out::link) until its warp is done.
 template <bool kAnyHit, class Node4, class Out>
-__global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restrict__ nodes, const BvhTri* __restrict__ tris,
-                                                           float4* rays, Out out, uint8_t* __restrict__ occ, uint32_t n, uint32_t* cursor,
-                                                           uint32_t* ties) {
+__global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restrict__ nodes, const BvhNode4* __restrict__ full,
+                                                           const BvhTri* __restrict__ tris, float4* rays, Out out,
+                                                           uint8_t* __restrict__ occ, uint32_t n, uint32_t* cursor) {
+    constexpr bool kTies = !kAnyHit && sizeof(Node4) != sizeof(BvhNode4);
     extern __shared__ int s_stack[];
+    __shared__ int s_tie[256];                    // first ray of the thread's list
+    s_tie[threadIdx.x] = -1;
     LaneStack4 stack;
     stack.col = s_stack + threadIdx.x;
     stack.stride = blockDim.x;
@@ -258,8 +265,9 @@ __global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restri
             has = false;
             if constexpr (kAnyHit) {
                 occ[i] = ts.hit_any ? 1 : 0;
-            } else if (sizeof(Node4) != sizeof(BvhNode4) && ts.tie) {
-                ties[atomicAdd(&cursor[1], 1u)] = i;
+            } else if (kTies && ts.tie) {
+                out.link(i) = s_tie[threadIdx.x];
+                s_tie[threadIdx.x] = (int)i;
             } else {
                 Hit h;
                 h.t = ts.tbest; h.u = ts.bu; h.v = ts.bv; h.prim = ts.best;
@@ -267,21 +275,21 @@ __global__ void __launch_bounds__(256, 4) k_trace_resident(const Node4* __restri
             }
         }
     }
-}
-
-// The rays left by the quantised traversal, over the full-precision nodes.
-template <class Out>
-__global__ void __launch_bounds__(kTraceBlock) k_trace_ties(const BvhNode4* __restrict__ nodes4, const BvhTri* __restrict__ tris,
-                                                            float4* rays, Out out, const uint32_t* __restrict__ cursor,
-                                                            const uint32_t* __restrict__ ties) {
-    const uint32_t m = cursor[1];
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) {
-        const uint32_t i = ties[k];
-        const float4 a = rays[2 * (size_t)i], b = rays[2 * (size_t)i + 1];
-        Hit h;
-        TraceWork w;
-        const bool hit = bvh_trace4<false>(nodes4, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, &h, w);
-        out.put(i, h, hit, rays);
+    if constexpr (kTies) {
+        for (int k = s_tie[threadIdx.x]; k >= 0;) {
+            const int next = out.link(k);
+            const float4 a = rays[2 * (size_t)k], b = rays[2 * (size_t)k + 1];
+            Hit h;
+            TraceWork w;
+            const bool hit = bvh_trace4<false>(full, tris, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, b.w, &h, w);
+            out.put(k, h, hit, rays);
+            k = next;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&cursor[1], 1u) == gridDim.x - 1) {
+        cursor[0] = 0u;
+        cursor[1] = 0u;
     }
 }
 
@@ -292,46 +300,48 @@ int sm_count() {
     return sms;
 }
 
-// Up to this many rays per SM each has a warp of its own (14,208 on 148 SMs). A warp per ray against
-// spread threads, closest hits, 1,000 / 8,000 / 16,384 / 32,000 rays on 20,482 triangles: 24 vs 54,
-// 28 vs 48, 34 vs 43, 43 vs 61 us; on 0.85 M triangles 29 vs 48, 45 vs 58, 64 vs 71, 101 vs 74 us.
-constexpr uint32_t kWarpRays = 96;
-// From this many rays on the resident form pays for its launches: 2^18 on trees with quantised
-// nodes for closest hits (260,000 rays 209 -> 173 us), 2^19 on smaller ones (300,000 rays 85 vs
-// 89 us, 524,288 rays 120 -> 108).
-uint32_t resident_min(const DeviceBvh& bvh) { return bvh.num_nodes4 >= kQuantMinNodes4 ? 1u << 18 : 1u << 19; }
+// Up to this many rays per SM each has a warp of its own (14,208 on 148 SMs; none without a 4-wide tree). A
+// warp per ray against spread threads, closest hits, 1,000 / 8,000 / 14,208 rays, incoherent: 20,482
+// triangles 22 vs 38, 29 vs 44, 38 vs 51 us; 3.4 M triangles 24 vs 41, 32 vs 53, 40 vs 61. Past that
+// camera rows and large trees turn: 20,000 rays of a camera on 0.85 M triangles 60 vs 58 us. A few
+// dozen triangles leave most of a warp's lanes without work: 34 triangles, closest hits 1,000 / 4,000 /
+// 8,000 rays 19.0 vs 19.1, 20.7 vs 19.8, 26.1 vs 21.0 us, any hit 15.3 vs 18.1, 16.4 vs 18.5, 19.6 vs 20.3.
+uint32_t warp_rays(const DeviceBvh& bvh, bool any) {
+    return !bvh.nodes4 ? 0u : bvh.num_nodes4 >= kQuantMinNodes4Any ? 96u : any ? 48u : 8u;
+}
+
+// The resident form from this many rays on. Against the thread form, closest hits, incoherent rays / surface points
+// towards a light / rows of a camera: 20,482 triangles, 2^19 rays 153 vs 179, 303 vs 327, 143 vs 135 us, 2^20 rays 254 vs
+// 309, 555 vs 599, 220 vs 205; any hit, 2^19 rays 123 vs 155, 205 vs 292, 114 vs 108. A camera's rows stay together by
+// themselves, and on trees that sit in the caches the thread form's dense blocks are 4 to 8% ahead on them
+// (walking them in step inside the resident grid, looking at a sample of the rays first, and ranges of
+// each warp's own were no better). On quantised trees it is ahead on all three from 2^18 rays on: 0.85 M triangles
+// 124 vs 121, 127 vs 177, 107 vs 105; 2^19 rays 164 vs 172, 195 vs 307, 152 vs 152; 3.4 M triangles, 2^20 rays 308
+// vs 402, 449 vs 744, 312 vs 374. On a few dozen triangles it gains nothing (34 triangles, 2^22 rays 269 vs
+// 273, 292 vs 290, 172 vs 143).
+uint32_t resident_min(const DeviceBvh& bvh) {
+    return !bvh.nodes4 || bvh.num_nodes4 < kQuantMinNodes4Any ? 0xffffffffu : bvh.num_nodes4 >= kQuantMinNodes4 ? 1u << 18 : 1u << 19;
+}
 
 template <bool kAnyHit, class Node4, class Out>
 cudaError_t run_resident(const DeviceBvh& bvh, const Node4* nodes, float4* rays, const Out& out, uint8_t* occ, uint32_t n,
-                         int sms, cudaStream_t s) {
-    constexpr bool ties = !kAnyHit && sizeof(Node4) != sizeof(BvhNode4);
-    uint32_t* cursor = nullptr;      // cursor, tie count, tie list
-    cudaError_t e = cudaMallocAsync((void**)&cursor, sizeof(uint32_t) * (2 + (ties ? (size_t)n : 0)), s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, 2 * sizeof(uint32_t), s);
-    if (e != cudaSuccess) { if (cursor) cudaFreeAsync(cursor, s); return e; }
+                         int sms, uint32_t* cursor, cudaStream_t s) {
     const size_t smem = sizeof(int) * kSharedDepth * 256;
     int nb = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_resident<kAnyHit, Node4, Out>, 256, smem);
-    k_trace_resident<kAnyHit, Node4, Out><<<std::max(1, nb) * sms, 256, smem, s>>>(nodes, bvh.tris, rays, out, occ, n, cursor,
-                                                                                    cursor + 2);
-    if constexpr (ties) k_trace_ties<Out><<<sms, kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, rays, out, cursor, cursor + 2);
-    e = cudaGetLastError();
-    cudaFreeAsync(cursor, s);
-    return e;
+    k_trace_resident<kAnyHit, Node4, Out><<<std::max(1, nb) * sms, 256, smem, s>>>(nodes, bvh.nodes4, bvh.tris, rays, out, occ, n,
+                                                                                    cursor);
+    return cudaGetLastError();
 }
 
 template <class Out>
-cudaError_t run_closest(const DeviceBvh& bvh, float4* rays, const Out& out, uint32_t n, cudaStream_t s) {
+cudaError_t run_closest(const DeviceBvh& bvh, float4* rays, const Out& out, uint32_t n, uint32_t* cursor, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const int sms = sm_count();
-    if (bvh.nodes4 && n >= resident_min(bvh) && n <= kResidentMax) {
-        const cudaError_t e = bvh.num_nodes4 >= kQuantMinNodes4
-                                  ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, rays, out, nullptr, n, sms, s)
-                                  : run_resident<false, BvhNode4>(bvh, bvh.nodes4, rays, out, nullptr, n, sms, s);
-        if (e != cudaErrorMemoryAllocation) return e;
-        cudaGetLastError();                       // no room for its lists: the form below needs none
-    }
-    if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
+    if (cursor && n >= resident_min(bvh) && n <= kResidentMax)
+        return bvh.num_nodes4 >= kQuantMinNodes4 ? run_resident<false, BvhNode4Q>(bvh, bvh.nodes4q, rays, out, nullptr, n, sms, cursor, s)
+                                                 : run_resident<false, BvhNode4>(bvh, bvh.nodes4, rays, out, nullptr, n, sms, cursor, s);
+    if (n <= warp_rays(bvh, false) * (uint32_t)sms) {
         k_trace_warp<false, Out><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, rays, out, nullptr, n);
         return cudaGetLastError();
     }
@@ -344,26 +354,22 @@ cudaError_t run_closest(const DeviceBvh& bvh, float4* rays, const Out& out, uint
 
 // rays: aur_ray records; written (maxt) by launch_intersect only
 cudaError_t launch_trace_closest(const DeviceBvh& bvh, const int* tri_attr, const void* rays, void* hits, uint32_t n,
-                                 cudaStream_t s) {
-    return run_closest(bvh, (float4*)const_cast<void*>(rays), HitOut{(aur_hit*)hits, tri_attr}, n, s);
+                                 uint32_t* cursor, cudaStream_t s) {
+    return run_closest(bvh, (float4*)const_cast<void*>(rays), HitOut{(aur_hit*)hits, tri_attr}, n, cursor, s);
 }
 
-cudaError_t launch_intersect(const DeviceBvh& bvh, const TriShade* tri, void* rays, void* isects, uint32_t n, cudaStream_t s) {
-    return run_closest(bvh, (float4*)rays, IsectOut{(aur_isect*)isects, tri}, n, s);
+cudaError_t launch_intersect(const DeviceBvh& bvh, const TriShade* tri, void* rays, void* isects, uint32_t n, uint32_t* cursor,
+                             cudaStream_t s) {
+    return run_closest(bvh, (float4*)rays, IsectOut{(aur_isect*)isects, tri}, n, cursor, s);
 }
 
-cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, cudaStream_t s) {
+cudaError_t launch_trace_occluded(const DeviceBvh& bvh, const void* rays, uint8_t* occ, uint32_t n, uint32_t* cursor, cudaStream_t s) {
     if (n == 0) return cudaSuccess;
     const int sms = sm_count();
     float4* r4 = (float4*)const_cast<void*>(rays);
-    if (bvh.nodes4 && n >= resident_min(bvh) && n <= kResidentMax) {
-        const cudaError_t e = bvh.num_nodes4 >= kQuantMinNodes4Any
-                                  ? run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, r4, NoOut{}, occ, n, sms, s)
-                                  : run_resident<true, BvhNode4>(bvh, bvh.nodes4, r4, NoOut{}, occ, n, sms, s);
-        if (e != cudaErrorMemoryAllocation) return e;
-        cudaGetLastError();
-    }
-    if (bvh.nodes4 && n <= kWarpRays * (uint32_t)sms) {
+    if (cursor && n >= resident_min(bvh) && n <= kResidentMax)   // such trees are past kQuantMinNodes4Any
+        return run_resident<true, BvhNode4Q>(bvh, bvh.nodes4q, r4, NoOut{}, occ, n, sms, cursor, s);
+    if (n <= warp_rays(bvh, true) * (uint32_t)sms) {
         k_trace_warp<true, NoOut><<<spread_grid(n, 1), kTraceBlock, 0, s>>>(bvh.nodes4, bvh.tris, r4, NoOut{}, occ, n);
         return cudaGetLastError();
     }

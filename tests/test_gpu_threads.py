@@ -77,3 +77,22 @@ def test_wavefront_renders(ctx):
     _together([_render_job(ctx, scenes.box_scene(96, 64), opts(4, 1 << 14)),
                _render_job(ctx, scenes.sphere_scene(128, 80), opts(6, 1 << 14)),
                _render_job(ctx, scenes.box_scene(50, 40), opts(2, 1 << 12))])
+
+
+def test_ray_queries(ctx):
+    """Batches of the resident form (2^19 rays), whose cursors are the context's, and small ones."""
+    def query_job(level, n, seed):
+        verts, idx = scenes.icosphere(level)
+        bvh = ab.Bvh(ctx, verts.astype(np.float32), idx.astype(np.uint32))
+        r = np.random.default_rng(seed)
+        rays = np.zeros((n, 8), np.float32)
+        rays[:, :3], rays[:, 4:7], rays[:, 7] = r.uniform(-2, 2, (n, 3)), r.normal(size=(n, 3)), 1e30
+        hits, occ = bvh.trace_closest(rays), bvh.trace_occluded(rays)
+
+        def job():
+            h = bvh.trace_closest(rays)
+            for k in h.dtype.names:
+                np.testing.assert_array_equal(h[k], hits[k])
+            np.testing.assert_array_equal(bvh.trace_occluded(rays), occ)
+        return job
+    _together([query_job(4, 1 << 19, 1), query_job(5, (1 << 19) + 99, 2), query_job(4, 5000, 3)])
