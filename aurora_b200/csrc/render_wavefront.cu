@@ -149,15 +149,18 @@ __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << lane_id()) - 1
 
 // Block 0's first thread charges the time since the previous stage began to that stage: two
 // timer reads and a few stores a launch, where event records between the launches cost every
-// graph as many nodes again.
-__device__ __forceinline__ void stage_begins(const WfPool& w, int stage) {
+// graph as many nodes again. Stage -1: nothing runs that is to be charged.
+__device__ __forceinline__ void stage_begins(WfState* st, int stage) {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
     unsigned long long now;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
-    if (w.st->stage >= 0) w.st->stage_ns[w.st->stage] += now - w.st->stamp;
-    w.st->stamp = now;
-    w.st->stage = stage;
+    if (st->stage >= 0) st->stage_ns[st->stage] += now - st->stamp;
+    st->stamp = now;
+    st->stage = stage;
 }
+
+// After the graphs that the host reads the counters between: its time is no stage's.
+__global__ void k_stage_end(WfPool w) { stage_begins(w.st, -1); }
 
 // Block-aggregated append to kQ queues: every thread of the block calls it (uniform control
 // flow) with its flags; it returns each flagged thread's slot in the queue. One atomic per
@@ -245,7 +248,7 @@ __device__ __forceinline__ int scene_of(const WfPool& w, uint32_t item) {
 template <bool kRec, bool kSweep>
 __global__ void k_regen(WfPool w, int in_q) {
     __shared__ BlockScan s_scan;
-    stage_begins(w, 0);
+    stage_begins(w.st, 0);
     uint32_t* qin = in_q ? w.q_ext1 : w.q_ext0;
     uint32_t* cin = &w.ctr[in_q ? C_EXT1 : C_EXT0];
     const uint32_t total = w.ctr[C_TOTAL];
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
     // Outputs of the later stages start empty. Only counters that no block of
     // this kernel touches are reset here; the bucket counters this kernel
     // increments were reset by the previous next-event stage (or the pass start).
-    stage_begins(w, 1);
+    stage_begins(w.st, 1);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.ctr[C_LIST] = 0;
         w.ctr[C_FRESH] = 0;
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_extend(WfPool w, int in_
 
 // counting-sort scatter of the extension queue into q_sort, grouped by bucket
 __global__ void k_sort_scatter(WfPool w, int in_q) {
-    stage_begins(w, 2);
+    stage_begins(w.st, 2);
     const uint32_t* qin = in_q ? w.q_ext1 : w.q_ext0;
     const uint32_t n = w.ctr[in_q ? C_EXT1 : C_EXT0];
     __shared__ uint32_t s_ofs[kBuckets], s_cnt[kBuckets], s_base[kBuckets];
@@ -564,7 +567,7 @@ __global__ void __launch_bounds__(256, kPart == SHADE_MATTE ? AUR_SHADE_MATTE_MI
     uint32_t* cout = &w.ctr[in_q ? C_EXT0 : C_EXT1];
     __shared__ BlockScan s_scan;
     __shared__ uint32_t s_fetch;
-    if (kPart != SHADE_REST) stage_begins(w, 3);
+    if (kPart != SHADE_REST) stage_begins(w.st, 3);
     while (true) {
         if (threadIdx.x == 0) s_fetch = atomicAdd(&w.ctr[kPart == SHADE_MATTE ? C_CUR_SHADE2 : C_CUR_SHADE], blockDim.x);
         __syncthreads();
@@ -766,7 +769,7 @@ template <int kTree>
 __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
     using Tree = TreeTypes<kTree, true>;
     const uint32_t n = w.ctr[C_SHADOW];
-    stage_begins(w, 4);
+    stage_begins(w.st, 4);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.st->rays[1] += n;
         // extend, scatter and shade are finished: reset their fetch and bucket counters
@@ -820,8 +823,9 @@ __global__ void __launch_bounds__(256, AUR_TRAV_MINB) k_shadow(WfPool w) {
 // ------------------------------------------------------------------ resolve
 // Adds this pass's samples of every pixel of every scene (blockIdx.y), in sample order, to the
 // pixel's compensated sum (the plain kernel's accumulation order), and after a scene's last pass
-// writes its film. A render of one pass keeps no sums in memory.
-__global__ void k_resolve(const WfScene* scenes) {
+// writes its film. A render of one pass keeps no sums in memory. It ends the pass's last stage.
+__global__ void k_resolve(const WfScene* scenes, WfState* st) {
+    if (blockIdx.y == 0) stage_begins(st, -1);
     const WfScene& S = scenes[blockIdx.y];
     if (S.p.spp == 0) return;
     for (uint32_t pixel = blockIdx.x * blockDim.x + threadIdx.x; pixel < S.npix; pixel += gridDim.x * blockDim.x) {
@@ -1030,6 +1034,7 @@ struct WfRun {
             cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
             if (e != cudaSuccess) return e;
             for (int it = 0; it < iters; ++it) enqueue_iteration(it & 1, kind);
+            if (iters == kItersPerGraph) k_stage_end<<<1, 1, 0, stream>>>(w);
             e = cudaStreamEndCapture(stream, &g);
             if (e != cudaSuccess) return e;
             e = cudaGraphInstantiate(&x, g, 0);
@@ -1071,7 +1076,7 @@ struct WfRun {
         if (kind != REFILL && depth <= kItersPerGraph) {   // as graph_iters
             e = launch_graph(depth, kind);
             if (e != cudaSuccess) return e;
-            *launches += depth * launches_per_iteration();
+            *launches += depth * launches_per_iteration() + (depth == kItersPerGraph ? 1 : 0);
         } else {
             // Bound on graph launches: each launch advances every live path by 8 bounces
             // and refills the pool, so a pass needs about total / P * depth / 8 launches.
@@ -1082,7 +1087,7 @@ struct WfRun {
                 if (e == cudaSuccess) e = read_state();
                 if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
                 if (e != cudaSuccess) return e;
-                *launches += kItersPerGraph * launches_per_iteration();
+                *launches += kItersPerGraph * launches_per_iteration() + 1;
                 done = drained(total, kItersPerGraph);
             }
             if (!done) return cudaErrorLaunchTimeout;
@@ -1432,7 +1437,7 @@ static aur_status wavefront_batch(aur_ctx* ctx, std::vector<BatchItem>& items, c
         if (e != cudaSuccess) break;
         for (int i = 0; i < n; i += 65535) {
             const dim3 grid((unsigned)std::min<uint32_t>((max_pix + 255) / 256, 1u << 20), (unsigned)std::min(n - i, 65535));
-            k_resolve<<<grid, 256, 0, s>>>(run.d_scenes + i);
+            k_resolve<<<grid, 256, 0, s>>>(run.d_scenes + i, run.w.st);
             ++launches;
         }
         e = cudaGetLastError();
