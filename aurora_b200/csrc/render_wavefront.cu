@@ -1557,13 +1557,15 @@ aur_status render_wavefront(aur_scene* sc, const aur_render_opts* o, float* film
     std::vector<BatchItem> items(1);
     items[0] = {sc, p, npix, (float4*)fo.ptr, nullptr, nullptr};
     if (wants_tuning(o)) {
-        // Tuned once per render shape (triangles, materials, lights, resolution, spp, depths)
-        // on this context: a scene rendered at another spp or depth is tuned for that too,
-        // and a new scene of the same shape reuses the configuration.
+        // Tuned once per render shape (triangles, materials, lights, resolution, spp, light samples,
+        // depths) on this context: a scene rendered at another spp or depth is tuned for that too,
+        // and a new scene of the same shape reuses the configuration. The first sample of a render
+        // has one path whatever the light samples, so a render that has it is another shape.
         uint64_t sig = 1469598103934665603ull;
-        const uint64_t parts[8] = {sc->ntri, sc->h_mats.size(), sc->h_lights.size(), (uint64_t)sc->cam.w,
-                                   (uint64_t)sc->cam.h, (uint64_t)o->spp, (uint64_t)o->max_depth,
-                                   (uint64_t)(int64_t)o->min_depth};
+        const uint64_t parts[10] = {sc->ntri, sc->h_mats.size(), sc->h_lights.size(), (uint64_t)sc->cam.w,
+                                    (uint64_t)sc->cam.h, (uint64_t)o->spp, (uint64_t)o->max_depth,
+                                    (uint64_t)(int64_t)o->min_depth, (uint64_t)p.light_samples,
+                                    (uint64_t)(p.light_samples > 1 && p.sample_offset == 0)};
         for (uint64_t v : parts) sig = (sig ^ v) * 1099511628211ull;
         auto it = sc->ctx->wf_scene_tuned.find(sig);
         if (it == sc->ctx->wf_scene_tuned.end()) {
