@@ -1042,7 +1042,6 @@ cudaError_t build_with(Scratch& w, const float* verts, const uint32_t* idx, int 
         CK(dalloc(&out->nodes, 1, s));
         k_single<<<1, 1, 0, s>>>(verts, idx, out->nodes, out->tris, w.dec, w.st);
         out->num_nodes = 1;
-        out->lo[0] = out->lo[1] = out->lo[2] = out->hi[0] = out->hi[1] = out->hi[2] = 0.f;
     } else {
         k_morton<<<div_up(n, T), T, 0, s>>>(verts, idx, n, w.st, w.keys, w.vals);
         const int nb = div_up(n, sort_tile(n));
