@@ -21,19 +21,23 @@ __global__ void k_pack_tri_shade(const float* __restrict__ cn, const float* __re
     o[3] = make_float4(r.uv[2], r.uv[3], r.uv[4], r.uv[5]);
 }
 
+// A material index out of range can come from a device-resident attribute table, which is not checked; it
+// matters only if such a triangle is shaded, so no material is read for it here.
 __global__ void k_tri_type(const int* __restrict__ attr, const Attr* __restrict__ attrs, const Material* __restrict__ mats,
-                           size_t ntri, uint8_t* __restrict__ out) {
+                           uint32_t nmat, size_t ntri, uint8_t* __restrict__ out) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < ntri) out[i] = (uint8_t)mats[attrs[attr[i]].material].type;
+    if (i >= ntri) return;
+    const uint32_t m = (uint32_t)attrs[attr[i]].material;
+    out[i] = (uint8_t)(m < nmat ? mats[m].type : MAT_CONSTANT);
 }
 
 }  // namespace
 
-cudaError_t make_tri_type(const int* tri_attr, const Attr* attrs, const Material* mats, size_t ntri, uint8_t** out,
-                          cudaStream_t s) {
+cudaError_t make_tri_type(const int* tri_attr, const Attr* attrs, const Material* mats, uint32_t nmat, size_t ntri,
+                          uint8_t** out, cudaStream_t s) {
     const cudaError_t e = cudaMallocAsync((void**)out, ntri, s);
     if (e != cudaSuccess) { *out = nullptr; return e; }
-    k_tri_type<<<(unsigned)((ntri + 255) / 256), 256, 0, s>>>(tri_attr, attrs, mats, ntri, *out);
+    k_tri_type<<<(unsigned)((ntri + 255) / 256), 256, 0, s>>>(tri_attr, attrs, mats, nmat, ntri, *out);
     return cudaGetLastError();
 }
 

@@ -94,8 +94,8 @@ aur_status wf_record_pass(aur_scene* sc, const PathParams& p, int s0, int nsampl
 cudaError_t pack_tri_shade(const float* corner_n, const float* corner_uv, const int* tri_attr, size_t ntri, TriShade** out,
                            cudaStream_t s);
 // The material type of every triangle, into a new buffer.
-cudaError_t make_tri_type(const int* tri_attr, const Attr* attrs, const Material* mats, size_t ntri, uint8_t** out,
-                          cudaStream_t s);
+cudaError_t make_tri_type(const int* tri_attr, const Attr* attrs, const Material* mats, uint32_t nmat, size_t ntri,
+                          uint8_t** out, cudaStream_t s);
 
 struct DeviceGuard {
     explicit DeviceGuard(int dev);

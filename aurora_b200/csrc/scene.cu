@@ -301,7 +301,7 @@ aur_status aur_scene_create(aur_ctx* ctx, const aur_scene_desc* d, const aur_bvh
     if (cu) cudaFreeAsync(cu, s);
     if (e == cudaSuccess) e = upload(&sc->attrs, attrs.data(), attrs.size(), s);
     if (e == cudaSuccess) e = upload(&sc->mats, mats.data(), mats.size(), s);
-    if (e == cudaSuccess) e = make_tri_type(sc->bvh.tri_attr, sc->attrs, sc->mats, d->ntri, &sc->tri_type, s);
+    if (e == cudaSuccess) e = make_tri_type(sc->bvh.tri_attr, sc->attrs, sc->mats, (uint32_t)mats.size(), d->ntri, &sc->tri_type, s);
     if (e == cudaSuccess) e = upload(&sc->lights, lights.data(), lights.size(), s);
     if (e == cudaSuccess) e = upload(&sc->texs, texs.data(), texs.size(), s);
     if (e == cudaSuccess) e = upload(&sc->texels, d->texels, texel_floats, s);
