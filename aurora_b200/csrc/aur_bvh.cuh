@@ -38,7 +38,14 @@ struct BvhNode4 { float4 lox, hix, loy, hiy, loz, hiz; int4 ref; int4 pad; };
 // node, at the same index; unused slots have an inverted box (255, 0) and ref ~0.
 // Its boxes contain the full-precision ones, so the traversals find the same hits; only the
 // visiting order differs, which decides a hit's identity where two triangles lie at exactly the
-// same distance. Such ties are detected and traced again over the full-precision nodes.
+// same distance. Such ties are detected and traced again over the full-precision nodes. (Any form's order
+// also decides for a ray that grazes an edge so flatly that a triangle's computed distance is off by more
+// than the boxes' slack: found first, the other triangle hides it. Of 524,288 rays towards a bumpy sheet, a
+// quarter of them at its vertices and half grazing, 3 to 30 differ between the forms of the ray queries.)
+// The padding covers origins within some sixteen scene magnitudes in both forms' terms but one: the
+// distance to the grid's origin is rounded once more here, which leaves about eleven. Of 13 million
+// such rays from half to 128 magnitudes away none lost a hit to the quantised boxes (any hit gains some that the
+// tighter boxes lose); from 1,024 on both forms lose hits, and not the same.
 struct __align__(64) BvhNode4Q {
     float p[3], s[3];
     uint32_t lox, hix, loy, hiy, loz, hiz;

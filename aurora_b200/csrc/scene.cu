@@ -403,7 +403,9 @@ aur_status render_options(const aur_scene* sc, const aur_render_opts* o, PathPar
 
 }  // namespace aur
 
-// Bytes of samples that the plain renderer keeps before it sums them.
+// Bytes of samples that the plain renderer takes from the stream's pool at a time (one sample a pixel at
+// least; with the sums of a render of several chunks beside them, 32 bytes a pixel). 1080p, 64 samples at
+// 1 GiB / 256 / 128 MiB: 189.4 / 190.3 / 191.5 ms.
 constexpr size_t kPlainSampleBudget = (size_t)1 << 30;
 
 // Films of up to this many pixels take the pixel loop where they have one path a pixel: there is nothing to
