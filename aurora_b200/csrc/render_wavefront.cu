@@ -937,7 +937,9 @@ struct WfRun {
     static constexpr int kStages = 5;          // regen, extend, sort, shade, shadow
     cudaEvent_t e0 = nullptr, e1 = nullptr;    // around a whole render
     // by iterations and kind of pass: one that refills its slots, one that fits the pool, and one of
-    // at most kSmallPass paths, whose launches need few blocks
+    // at most kSmallPass paths, whose launches need few blocks (box scene at depth 5, 128 x 128 with 1 / 4 samples
+    // 334 / 359 us against 346 / 371 without it, 256 x 256 with 2 / 4 samples 384 / 468 against 395 / 460;
+    // 20,480 triangles, the same four 700 / 761 / 817 / 901 against 716 / 778 / 828 / 900)
     enum Kind : int { REFILL = 0, FITS = 1, SMALL = 2 };
     // and by the trees traversed: scenes on either side of their limits share an engine and its pool
     cudaGraphExec_t exec[kItersPerGraph + 1][3][3][3] = {};

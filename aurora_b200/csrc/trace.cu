@@ -302,7 +302,8 @@ int sm_count() {
 
 // Up to this many rays per SM each has a warp of its own (14,208 on 148 SMs; none without a 4-wide tree). A
 // warp per ray against spread threads, closest hits, 1,000 / 8,000 / 14,208 rays, incoherent: 20,482
-// triangles 22 vs 38, 29 vs 44, 38 vs 51 us; 3.4 M triangles 24 vs 41, 32 vs 53, 40 vs 61. Past that
+// triangles 22 vs 38, 29 vs 44, 38 vs 51 us (occlusion 19 vs 36, 28 vs 42, 34 vs 45); 3.4 M triangles 24 vs 41,
+// 32 vs 53, 40 vs 61 (21 vs 37, 28 vs 43, 34 vs 46). Past that
 // camera rows and large trees turn: 20,000 rays of a camera on 0.85 M triangles 60 vs 58 us. A few
 // dozen triangles leave most of a warp's lanes without work: 34 triangles, closest hits 1,000 / 4,000 /
 // 8,000 rays 19.0 vs 19.1, 20.7 vs 19.8, 26.1 vs 21.0 us, any hit 15.3 vs 18.1, 16.4 vs 18.5, 19.6 vs 20.3.
@@ -316,9 +317,9 @@ uint32_t warp_rays(const DeviceBvh& bvh, bool any) {
 // themselves, and on trees that sit in the caches the thread form's dense blocks are 4 to 8% ahead on them
 // (walking them in step inside the resident grid, looking at a sample of the rays first, and ranges of
 // each warp's own were no better). On quantised trees it is ahead on all three from 2^18 rays on: 0.85 M triangles
-// 124 vs 121, 127 vs 177, 107 vs 105; 2^19 rays 164 vs 172, 195 vs 307, 152 vs 152; 3.4 M triangles, 2^20 rays 308
-// vs 402, 449 vs 744, 312 vs 374. On a few dozen triangles it gains nothing (34 triangles, 2^22 rays 269 vs
-// 273, 292 vs 290, 172 vs 143).
+// 124 vs 121, 127 vs 177, 107 vs 105 (any hit 111 vs 108, 108 vs 154, 87 vs 89); 2^19 rays 164 vs 172, 195 vs 307,
+// 152 vs 152; 3.4 M triangles, 2^20 rays 308 vs 402, 449 vs 744, 312 vs 374. On a few dozen triangles it gains
+// nothing (34 triangles, 2^22 rays 269 vs 273, 292 vs 290, 172 vs 143).
 uint32_t resident_min(const DeviceBvh& bvh) {
     return !bvh.nodes4 || bvh.num_nodes4 < kQuantMinNodes4Any ? 0xffffffffu : bvh.num_nodes4 >= kQuantMinNodes4 ? 1u << 18 : 1u << 19;
 }
